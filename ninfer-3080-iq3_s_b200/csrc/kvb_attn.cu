@@ -1,15 +1,16 @@
 // kvb_attn.cu -- paged split-K attention over the quantised cache for 1..8 query tokens (decode, MTP
-// verify), de-quantisation fused into the QK and PV loops.  head_dim 128.
+// verify), de-quantisation fused into the QK and PV loops.  head_dim 128 (one 128-dim slice per key) and 256 (two: the
+// template parameter S).
 //
 // Grid (splits, kv heads, row blocks).  A CTA owns one KV head, one contiguous range of sealed pages and a block
 // of up to 16 GQA-merged query rows (row = token * G + q head within the KV head); the last split of a head also
-// reads the open tile, whose rows are still un-quantised fp16 in the stage.  Inside a CTA each of the 12 warps
-// streams its own sub-range of pages through a private ring of three 4 KB slots in shared memory filled by bulk
-// async copies (one mbarrier per slot) and never synchronises with another warp until the final merge.  A page
+// reads the open tile, whose rows are still un-quantised fp16 in the stage.  Inside a CTA each of the 8, 12 or 16 warps
+// streams its own sub-range of pages through a private ring of two 4 KB slots (8 KB at 256 dims) in shared memory filled
+// by bulk async copies (one mbarrier per slot) and never synchronises with another warp until the final merge.  A page
 // arrives as two chunks: its K codes together with a small header (the page's V scale rows; its K scale rows when
-// it is the first page of a tile the warp sees), then its V codes as four 1 KB sub-blocks, each shifted 16 bytes
+// it is the first page of a tile the warp sees), then its V codes as 1 KB sub-blocks, each shifted 16 bytes
 // further, which makes the transposing ldmatrix reads of the V codes free of bank conflicts.  A slot is refilled
-// as soon as its chunk has been consumed, so two thirds of a warp's ring are in flight at any time.
+// as soon as its chunk has been consumed.
 //
 // Math per page (quantised-domain identities, no per-element de-quantisation), all on the int8 tensor path:
 //   logit[r][j] = sum_d (q'[r][d] * scale_K[d]) * code_K[j][d]  +  sum_d q'[r][d] * zp_K[d]
@@ -24,6 +25,11 @@
 //     byte permute and one AND per register; the integer sums of the page are converted once per page and
 //     enter the running fp32 accumulators with the weight exp2(page max - running max).
 // The page-local reference keeps 16 significant bits below each page's own maximum, whatever the global one is.
+// At head_dim 256 each slice has its own query integers (one scale_K, zp_K table per slice) and weights (scale_V per slice),
+// with a third byte each; the slices meet in the fp32 logits.  Bound by instruction issue like the 128-dim form (a 16 KB
+// page costs about as much as two 8 KB ones).  Measured on B200, 24 / 4 heads, balanced bf16 cache: decode at 30,011
+// tokens 21.4 us against 148.6 us for one warp per key on fp32 FMAs, a 5-row verify step at 20,000 tokens 35.7 against
+// 454 us (the whole difference: no per-element de-quantisation, rows of a KV head share every code read).
 #include <algorithm>
 #include <climits>
 #include <cstddef>
@@ -37,25 +43,36 @@ namespace {
 
 constexpr int D = 128;
 constexpr int kWarpsDecode = 16;    // warps per CTA for up to 8 merged query rows (one N block per warp): 128 registers per thread
-constexpr int kWarpsWide = 8;       // ... for 9..16 merged rows (two N blocks per warp: twice the accumulators): 255 registers
+constexpr int kWarpsWide = 8;       // ... for 9..16 merged rows (two N blocks per warp), and at head_dim 256: twice the accumulators, 255 registers
 constexpr int kRows = 16;           // query rows per CTA: one or two 8-row N blocks
-constexpr int kChunkBytes = kPage * (D / 2);  // 4096: the K or the V codes of one page
-#ifndef KVB_V_SHIFT
-#define KVB_V_SHIFT 16
-#endif
-constexpr int kVShift = KVB_V_SHIFT;  // 16: V codes lie as four sub-blocks of 16 keys, each shifted 16 bytes further (conflict-free ldmatrix, four copies); 0: one copy
-constexpr int kVSub = 1024 + kVShift;  // sub-block a at a * kVSub: key k at k * 64 + kVShift * (k / 16)
-constexpr int kSlotBytes = 4224;    // 4096 + 48 bytes of sub-block shifts, rounded up to 128
-#ifndef KVB_SLOTS
-#define KVB_SLOTS 2
-#endif
-constexpr int kSlots = KVB_SLOTS;   // ring slots per warp: the chunk in work and the next one(s) in flight
-constexpr int kHdrs = KVB_SLOTS;            // header buffers per warp (a header lives from the issue of its page's K chunk to the end of the page)
-constexpr int kHdrV = 512, kHdrK = 640, kHdrBytes = kHdrV + kHdrK;  // V scale rows of the page, then (first page of a tile) the K scale rows
+constexpr int kSlots = 2;           // ring slots per warp: the chunk in work and the next one in flight
+constexpr int kHdrs = 2;            // header buffers per warp (a header lives from the issue of its page's K chunk to the end of the page)
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kMagic = 12582912.0f;   // 1.5 * 2^23: x + kMagic has round(x) in its low mantissa bits (|x| < 2^22)
-constexpr float kPMax = 65000.0f;       // largest 16-bit weight (a margin below 65535 absorbs the rounding of the factor)
-constexpr int kTabPad = 4;          // the per-dim tables are padded by 4 floats per 32 dims: the four 32-dim chunks a warp reads at once fall in different banks
+constexpr int kTabPad = 4;          // the per-dim tables are padded by 4 floats per 32 dims: the 32-dim chunks a warp reads at once fall in different banks
+
+// What depends on the number of 128-dim slices of a head (head_dim 128 or 256).
+template <int S> struct Shape {
+    static constexpr int kDim = 128 * S;
+    static constexpr int kChunk = kPage * 64 * S;  // the K or the V codes of one page
+    // The V codes lie as 1 KB sub-blocks (16 keys at 128 dims, 8 at 256), each shifted 16 bytes further: the eight rows of
+    // every transposing ldmatrix fall in eight different bank groups.
+    static constexpr int kSubs = 4 * S, kSubBytes = 1024 + 16;
+    static constexpr int kSlot = (kChunk + (kSubs - 1) * 16 + 127) / 128 * 128;
+    static constexpr int kHdrV = 512 * S, kHdrK = 640 * S, kHdr = kHdrV + kHdrK;  // V scale rows of the page, then the K scale rows
+    static constexpr int kBlocks = 4 * S;          // 32-dim blocks
+    static constexpr int kTab = kDim + kBlocks * kTabPad;
+    // Bytes of a fixed-point query element or key weight: 16 bits at 128 dims; at 256 dims 22 and 23 bits, as much as the
+    // fp32 sums they enter keep.
+    static constexpr int kDigits = S == 1 ? 2 : 3;
+    static constexpr float kQMax = S == 1 ? 32639.0f : 4194000.0f;  // largest query integer
+    static constexpr float kPMagic = S == 1 ? kMagic : 8388608.0f;  // weights are >= 0: 2^23 leaves 23 bits
+    static constexpr float kPMax = S == 1 ? 65000.0f : 8380000.0f;  // largest weight (a margin below the full range absorbs the rounding of the factor)
+    // Key of m-row g (+ 8: kKeyH further) of 16-key group grp: key_lo(g) + key_grp(grp); see attn_cta.
+    static constexpr int kKeyH = 2 / S;
+    static __device__ __forceinline__ int key_lo(int g) { return S == 1 ? 16 * (g >> 1) + (g & 1) : 8 * g; }
+    static __device__ __forceinline__ constexpr int key_grp(int grp) { return (8 / S) * (grp >> 1) + (4 / S) * (grp & 1); }
+};
 
 struct AttnParams {
     LayerView L;
@@ -72,32 +89,32 @@ struct AttnParams {
     float* ws_o;         // [H][Z][nsplit][16][D]
 };
 
-struct __align__(128) WarpRing {
-    uint8_t slots[kSlots][kSlotBytes];
-    uint8_t hdr[kHdrs][kHdrBytes];
-    float scale_k[D + 4 * kTabPad], zp_k[D + 4 * kTabPad];  // per-dim scale / zero point of K for the tile in work: dim d at d + kTabPad * (d / 32)
+template <int S> struct __align__(128) WarpRing {
+    uint8_t slots[kSlots][Shape<S>::kSlot];
+    uint8_t hdr[kHdrs][Shape<S>::kHdr];
+    float scale_k[Shape<S>::kTab], zp_k[Shape<S>::kTab];  // per-dim scale / zero point of K for the tile in work: dim d at d + kTabPad * (d / 32)
     uint64_t bars[kSlots];      // completes when the copies of the chunk in the slot have landed
 };
 
-template <int W> struct __align__(128) AttnSmem {
-    WarpRing ring[W];
-    float4 qfrag[2][8][32];  // q' in per-lane fragment order: [row half][j][lane] = dims 32t+4j..+3 of row g(+8)
+template <int S, int W> struct __align__(128) AttnSmem {
+    WarpRing<S> ring[W];
+    float4 qfrag[2 / S][8 * S][32];  // q' in per-lane fragment order: [row half][8 slice + j][lane] = dims 128 slice + 32t+4j..+3 of row g(+8)
     int row_pos[kRows];
 };
 
 // Per-thread state of the running softmax.  Lane (g, t) owns query rows 8 nb + 2t, 2t+1 of n-block nb and dims
-// 32 db + 4g + i (db, i < 4):  o[nb][db][xy][c] is dim 32 db + 4g + xy + 2 (c >> 1), row 8 nb + 2t + (c & 1) -- the
-// accumulator layout of the two MMAs per 32-dim block (xy = 0: even dims, 1: odd dims).  l and z are partial over the
-// lane's keys; everything is relative to the running maximum m (log2 units).
-template <int NB> struct Acc {
-    float o[NB][4][2][4];
-    float m[NB][2], l[NB][2], z[NB][2];
+// 32 db + 4g + i (db < 4 S, i < 4):  o[nb][db][xy][c] is dim 32 db + 4g + xy + 2 (c >> 1), row 8 nb + 2t + (c & 1) -- the
+// accumulator layout of the two MMAs per 32-dim block (xy = 0: even dims, 1: odd dims).  l and z (per slice) are partial
+// over the lane's keys; everything is relative to the running maximum m (log2 units).
+template <int S, int NB> struct Acc {
+    float o[NB][4 * S][2][4];
+    float m[NB][2], l[NB][2], z[S][NB][2];
 };
 
 // B fragments of (q')^T per n-block and k-block (b0, b1), high and low fp16 parts: the open tile's rows are fp16.
-template <int NB> struct QFrag {
-    uint32_t hi[NB][8][2];
-    uint32_t lo[NB][8][2];
+template <int S, int NB> struct QFrag {
+    uint32_t hi[NB][8 * S][2];
+    uint32_t lo[NB][8 * S][2];
 };
 
 __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {
@@ -139,13 +156,14 @@ __device__ __forceinline__ void imma_uu0(int (&d)[4], uint32_t a0, uint32_t a1, 
 }
 
 // Q-side fragments for the open tile from q' (shared memory, fragment order).  Lane (g, t) prepares row 8 nb + g, dims
-// 32t .. 32t+31 in natural pairs (2e, 2e+1), split into an fp16 high and low part so the product keeps fp32 accuracy.
-template <int NB, typename Smem>
-__device__ __forceinline__ void build_qfrag(const Smem& sm, int lane, QFrag<NB>& f) {
+// 128 slice + 32t .. 32t+31 in natural pairs (2e, 2e+1), split into an fp16 high and low part so the product keeps fp32
+// accuracy.
+template <int S, int NB, typename Smem>
+__device__ __forceinline__ void build_qfrag(const Smem& sm, int lane, QFrag<S, NB>& f) {
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < 8 * S; ++j) {
             const float4 qv = sm.qfrag[nb][j][lane];
             const float x[4] = {qv.x, qv.y, qv.z, qv.w};
 #pragma unroll
@@ -159,96 +177,125 @@ __device__ __forceinline__ void build_qfrag(const Smem& sm, int lane, QFrag<NB>&
     }
 }
 
-// Integer form of (q' * scale_K)^T for the quantised pages: each row is scaled to 16-bit integers
-// (row scale f = max|.| / 32639), Qi = 256 hi + lo with hi = Qi >> 8 signed and lo = Qi & 255 unsigned, so that the
-// key side can feed its packed code bytes to the int8 tensor path without unpacking nibbles: with L = byte & 0x0F
-// (even dim) and H = byte & 0xF0 (16 x odd dim),   sum_d Qi[d] code[d] = sum_b Qi[2b] L_b + (1/16) sum_b Qi[2b+1] H_b.
-// b[nb][kb][part][digit] holds the B fragments (b0, b1) of 32-byte k-block kb: part 0 = even dims, 1 = odd dims;
-// digit 0 = high (s8), 1 = low (u8).  The two bytes are read straight out of the float kMagic + Qi.
-template <int NB> struct QInt {
-    uint32_t b[NB][2][2][2][2];
-    float f[NB][2];   // row scale / 16 of the lane's rows 2t, 2t+1
-    float qz[NB][2];  // sum_d q'[row][d] * zp_K[d]
+// Integer form of (q' * scale_K)^T for the quantised pages: each row (of a slice) is scaled to integers of kDigits bytes
+// (row scale f = max|.| / kQMax), Qi = 256 hi + lo with hi = Qi >> 8 signed and lo = Qi & 255 unsigned (three bytes at
+// 256 dims), so that the key side can feed its packed code bytes to the int8 tensor path without unpacking nibbles: with
+// L = byte & 0x0F (even dim) and H = byte & 0xF0 (16 x odd dim),
+//   sum_d Qi[d] code[d] = sum_b Qi[2b] L_b + (1/16) sum_b Qi[2b+1] H_b.
+// b[slice][nb][kb][part][digit] holds the B fragments (b0, b1) of 32-byte k-block kb: part 0 = even dims, 1 = odd dims;
+// digit 0 = highest (s8), then u8.  The bytes are read straight out of the float kMagic + Qi.
+template <int S, int NB> struct QInt {
+    uint32_t b[S][NB][2][2][Shape<S>::kDigits][2];
+    float f[S][NB][2];   // row scale / 16 of the lane's rows 2t, 2t+1
+    float qz[S][NB][2];  // sum_d q'[row][d] * zp_K[d]
 };
 
-template <int NB, typename Smem>
-__device__ __forceinline__ void build_qint(const Smem& sm, const WarpRing& R, int lane, QInt<NB>& f) {
+template <int S, int NB, typename Smem>
+__device__ __forceinline__ void build_qint(const Smem& sm, const WarpRing<S>& R, int lane, QInt<S, NB>& f) {
+    constexpr float kQMax = Shape<S>::kQMax;
     const int t = lane & 3;
 #pragma unroll
-    for (int nb = 0; nb < NB; ++nb) {
-        float qs[32];
-        float qz = 0.0f, amax = 0.0f;
+    for (int s = 0; s < S; ++s) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const float4 qv = sm.qfrag[nb][j][lane];
-            const float4 ks = *reinterpret_cast<const float4*>(&R.scale_k[(32 + kTabPad) * t + 4 * j]);
-            const float4 kz = *reinterpret_cast<const float4*>(&R.zp_k[(32 + kTabPad) * t + 4 * j]);
-            qs[4 * j + 0] = qv.x * ks.x; qs[4 * j + 1] = qv.y * ks.y;
-            qs[4 * j + 2] = qv.z * ks.z; qs[4 * j + 3] = qv.w * ks.w;
-            qz = fmaf(qv.x, kz.x, qz); qz = fmaf(qv.y, kz.y, qz);
-            qz = fmaf(qv.z, kz.z, qz); qz = fmaf(qv.w, kz.w, qz);
-            amax = fmaxf(fmaxf(amax, fmaxf(fabsf(qs[4 * j]), fabsf(qs[4 * j + 1]))), fmaxf(fabsf(qs[4 * j + 2]), fabsf(qs[4 * j + 3])));
+        for (int nb = 0; nb < NB; ++nb) {
+            float qs[32];
+            float qz = 0.0f, amax = 0.0f;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float4 qv = sm.qfrag[nb][8 * s + j][lane];
+                const float4 ks = *reinterpret_cast<const float4*>(&R.scale_k[(32 + kTabPad) * (4 * s + t) + 4 * j]);
+                const float4 kz = *reinterpret_cast<const float4*>(&R.zp_k[(32 + kTabPad) * (4 * s + t) + 4 * j]);
+                qs[4 * j + 0] = qv.x * ks.x; qs[4 * j + 1] = qv.y * ks.y;
+                qs[4 * j + 2] = qv.z * ks.z; qs[4 * j + 3] = qv.w * ks.w;
+                qz = fmaf(qv.x, kz.x, qz); qz = fmaf(qv.y, kz.y, qz);
+                qz = fmaf(qv.z, kz.z, qz); qz = fmaf(qv.w, kz.w, qz);
+                amax = fmaxf(fmaxf(amax, fmaxf(fabsf(qs[4 * j]), fabsf(qs[4 * j + 1]))), fmaxf(fabsf(qs[4 * j + 2]), fabsf(qs[4 * j + 3])));
+            }
+            qz += __shfl_xor_sync(0xffffffffu, qz, 1);
+            qz += __shfl_xor_sync(0xffffffffu, qz, 2);  // every lane of group g now holds qz of row 8 nb + g
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+            const float fr = amax > 0.0f ? amax * (1.0f / kQMax) : 1.0f, inv = amax > 0.0f ? kQMax / amax : 0.0f;
+            f.qz[s][nb][0] = __shfl_sync(0xffffffffu, qz, 8 * t);      // row 2t   lives in lanes 4 * (2t) ..
+            f.qz[s][nb][1] = __shfl_sync(0xffffffffu, qz, 8 * t + 4);  // row 2t+1 lives in lanes 4 * (2t+1) ..
+            f.f[s][nb][0] = __shfl_sync(0xffffffffu, fr, 8 * t) * 0.0625f;
+            f.f[s][nb][1] = __shfl_sync(0xffffffffu, fr, 8 * t + 4) * 0.0625f;
+            uint32_t x[32];
+#pragma unroll
+            for (int i = 0; i < 32; ++i) x[i] = __float_as_uint(fmaf(qs[i], inv, kMagic));  // low 16 bits (22 at 256 dims): Qi (two's complement)
+#pragma unroll
+            for (int kb = 0; kb < 2; ++kb)
+#pragma unroll
+                for (int part = 0; part < 2; ++part)
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {  // b0: local dims 16 kb + 2j + part, b1: +8
+                        const int i0 = 16 * kb + 8 * r + part;
+                        const uint32_t t01 = prmt(x[i0], x[i0 + 2], 0x5140), t23 = prmt(x[i0 + 4], x[i0 + 6], 0x5140);  // [lo lo hi hi]
+                        constexpr int kLast = Shape<S>::kDigits - 1;
+                        f.b[s][nb][kb][part][kLast][r] = prmt(t01, t23, 0x5410);
+                        f.b[s][nb][kb][part][kLast - 1][r] = prmt(t01, t23, 0x7632);
+                        if constexpr (S == 2) {  // third byte: 0x40 + (Qi >> 16), made a signed byte (flip bit 6, copy it to bit 7)
+                            const uint32_t h01 = prmt(x[i0], x[i0 + 2], 0x0062), h23 = prmt(x[i0 + 4], x[i0 + 6], 0x0062);
+                            const uint32_t h = prmt(h01, h23, 0x5410) ^ 0x40404040u;
+                            f.b[s][nb][kb][part][0][r] = h | ((h & 0x40404040u) << 1);
+                        }
+                    }
         }
-        qz += __shfl_xor_sync(0xffffffffu, qz, 1);
-        qz += __shfl_xor_sync(0xffffffffu, qz, 2);  // every lane of group g now holds qz of row 8 nb + g
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-        const float fr = amax > 0.0f ? amax * (1.0f / 32639.0f) : 1.0f, inv = amax > 0.0f ? 32639.0f / amax : 0.0f;
-        f.qz[nb][0] = __shfl_sync(0xffffffffu, qz, 8 * t);      // row 2t   lives in lanes 4 * (2t) ..
-        f.qz[nb][1] = __shfl_sync(0xffffffffu, qz, 8 * t + 4);  // row 2t+1 lives in lanes 4 * (2t+1) ..
-        f.f[nb][0] = __shfl_sync(0xffffffffu, fr, 8 * t) * 0.0625f;
-        f.f[nb][1] = __shfl_sync(0xffffffffu, fr, 8 * t + 4) * 0.0625f;
-        uint32_t x[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) x[i] = __float_as_uint(fmaf(qs[i], inv, kMagic));  // low 16 bits: Qi (two's complement)
-#pragma unroll
-        for (int kb = 0; kb < 2; ++kb)
-#pragma unroll
-            for (int part = 0; part < 2; ++part)
-#pragma unroll
-                for (int r = 0; r < 2; ++r) {  // b0: local dims 16 kb + 2j + part, b1: +8
-                    const int i0 = 16 * kb + 8 * r + part;
-                    const uint32_t t01 = prmt(x[i0], x[i0 + 2], 0x5140), t23 = prmt(x[i0 + 4], x[i0 + 6], 0x5140);  // [lo lo hi hi]
-                    f.b[nb][kb][part][1][r] = prmt(t01, t23, 0x5410);
-                    f.b[nb][kb][part][0][r] = prmt(t01, t23, 0x7632);
-                }
     }
 }
 
-// Scale rows of K -> per-dim tables in natural dim order, fp32.  A page row is 5 halves
-// [scale(2r) scale(2r+1) zp(2r) zp(2r+1) other(r)]; lane l converts rows 2l and 2l+1 (20 bytes): dims 4l .. 4l+3.
-__device__ __forceinline__ void transpose_k_scale(const uint8_t* kscale_rows, WarpRing& R, int lane) {
-    const uint32_t* w = reinterpret_cast<const uint32_t*>(kscale_rows + 20 * lane);
-    const uint32_t w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3], w4 = w[4];
-    // halves: w0 = s(4l) s(4l+1) | w1 = z(4l) z(4l+1) | w2 = o(2l) s(4l+2) | w3 = s(4l+3) z(4l+2) | w4 = z(4l+3) o(2l+1)
-    const float2 s01 = unpack_half2(w0), s23 = unpack_half2(prmt(w2, w3, 0x5432));
-    const float2 z01 = unpack_half2(w1), z23 = unpack_half2(prmt(w3, w4, 0x5432));
-    *reinterpret_cast<float4*>(&R.scale_k[4 * lane + kTabPad * (lane >> 3)]) = make_float4(s01.x, s01.y, s23.x, s23.y);
-    *reinterpret_cast<float4*>(&R.zp_k[4 * lane + kTabPad * (lane >> 3)]) = make_float4(z01.x, z01.y, z23.x, z23.y);
+// Scale rows of K -> per-dim tables in natural dim order, fp32; lane l converts rows 2l and 2l+1.
+// 128 dims: a page row is 5 halves [scale(2r) scale(2r+1) zp(2r) zp(2r+1) other(r)]: dims 4l .. 4l+3.
+// 256 dims: 10 halves [scale(4r) .. scale(4r+3) zp(4r) .. zp(4r+3) other(r), other(r) of the second slice]: dims 8l .. 8l+7.
+template <int S>
+__device__ __forceinline__ void transpose_k_scale(const uint8_t* kscale_rows, WarpRing<S>& R, int lane) {
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(kscale_rows + 20 * S * lane);
+    if constexpr (S == 1) {
+        const uint32_t w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3], w4 = w[4];
+        // halves: w0 = s(4l) s(4l+1) | w1 = z(4l) z(4l+1) | w2 = o(2l) s(4l+2) | w3 = s(4l+3) z(4l+2) | w4 = z(4l+3) o(2l+1)
+        const float2 s01 = unpack_half2(w0), s23 = unpack_half2(prmt(w2, w3, 0x5432));
+        const float2 z01 = unpack_half2(w1), z23 = unpack_half2(prmt(w3, w4, 0x5432));
+        *reinterpret_cast<float4*>(&R.scale_k[4 * lane + kTabPad * (lane >> 3)]) = make_float4(s01.x, s01.y, s23.x, s23.y);
+        *reinterpret_cast<float4*>(&R.zp_k[4 * lane + kTabPad * (lane >> 3)]) = make_float4(z01.x, z01.y, z23.x, z23.y);
+    } else {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const float2 s01 = unpack_half2(w[5 * r]), s23 = unpack_half2(w[5 * r + 1]), z01 = unpack_half2(w[5 * r + 2]), z23 = unpack_half2(w[5 * r + 3]);
+            const int at = 8 * lane + 4 * r + kTabPad * (lane >> 2);
+            *reinterpret_cast<float4*>(&R.scale_k[at]) = make_float4(s01.x, s01.y, s23.x, s23.y);
+            *reinterpret_cast<float4*>(&R.zp_k[at]) = make_float4(z01.x, z01.y, z23.x, z23.y);
+        }
+    }
 }
 
 // Running maximum moves to mnew: rescale the accumulators of one row pair.  alpha = exp2(m_old - m_new).
-template <int NB>
-__device__ __forceinline__ void rescale(Acc<NB>& acc, const float (&alpha)[NB][2]) {
+template <int S, int NB>
+__device__ __forceinline__ void rescale(Acc<S, NB>& acc, const float (&alpha)[NB][2]) {
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) {
 #pragma unroll
-        for (int db = 0; db < 4; ++db)
+        for (int db = 0; db < 4 * S; ++db)
 #pragma unroll
             for (int xy = 0; xy < 2; ++xy)
 #pragma unroll
                 for (int c = 0; c < 4; ++c) acc.o[nb][db][xy][c] *= alpha[nb][c & 1];
-        acc.l[nb][0] *= alpha[nb][0]; acc.z[nb][0] *= alpha[nb][0];
-        acc.l[nb][1] *= alpha[nb][1]; acc.z[nb][1] *= alpha[nb][1];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            acc.l[nb][j] *= alpha[nb][j];
+#pragma unroll
+            for (int s = 0; s < S; ++s) acc.z[s][nb][j] *= alpha[nb][j];
+        }
     }
 }
 
 // 16 keys of the open tile, read un-quantised (fp16, rotated) straight from the stage.
 // krow/vrow point at the first of the 16 stage rows of this head (row stride D halves).
-template <int NB>
-__device__ __forceinline__ void process_stage_group(const __half* krow, const __half* vrow, const QFrag<NB>& qf,
-                                                    Acc<NB>& acc, int lane, int first_pos, int kv_total,
+// At 256 dims the weights enter as an fp16 high and low part, like the query.
+template <int S, int NB>
+__device__ __forceinline__ void process_stage_group(const __half* krow, const __half* vrow, const QFrag<S, NB>& qf,
+                                                    Acc<S, NB>& acc, int lane, int first_pos, int kv_total,
                                                     const int (&row_lim)[NB][2], int key_begin, int key_end) {
+    constexpr int D = Shape<S>::kDim;
     const int g = lane >> 2, t = lane & 3;
     float s[NB][4];
     {
@@ -257,8 +304,9 @@ __device__ __forceinline__ void process_stage_group(const __half* krow, const __
 #pragma unroll
         for (int nb = 0; nb < NB; ++nb) s[nb][0] = s[nb][1] = s[nb][2] = s[nb][3] = 0.0f;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint4 a = *reinterpret_cast<const uint4*>(ka + 8 * i), b = *reinterpret_cast<const uint4*>(kb + 8 * i);
+        for (int i = 0; i < 4 * S; ++i) {
+            const int at = 128 * (i >> 2) + 8 * (i & 3);
+            const uint4 a = *reinterpret_cast<const uint4*>(ka + at), b = *reinterpret_cast<const uint4*>(kb + at);
 #pragma unroll
             for (int nb = 0; nb < NB; ++nb) {
                 mma16816(s[nb], a.x, b.x, a.y, b.y, qf.hi[nb][2 * i][0], qf.hi[nb][2 * i][1]);
@@ -294,8 +342,8 @@ __device__ __forceinline__ void process_stage_group(const __half* krow, const __
             acc.m[nb][j] = mnew;
         }
     }
-    if (__any_sync(0xffffffffu, moved)) rescale<NB>(acc, alpha);
-    uint32_t b0[NB], b1[NB];
+    if (__any_sync(0xffffffffu, moved)) rescale<S, NB>(acc, alpha);
+    uint32_t b0[NB], b1[NB], c0[NB], c1[NB];
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) {
 #pragma unroll
@@ -305,11 +353,16 @@ __device__ __forceinline__ void process_stage_group(const __half* krow, const __
         }
         b0[nb] = movmatrix_trans(pack_half2(s[nb][0], s[nb][1]));  // -> (row g; keys 2t, 2t+1)
         b1[nb] = movmatrix_trans(pack_half2(s[nb][2], s[nb][3]));  // -> (row g; keys 2t+8, 2t+9)
+        if constexpr (S == 2) {
+            const float2 h0 = unpack_half2(pack_half2(s[nb][0], s[nb][1])), h1 = unpack_half2(pack_half2(s[nb][2], s[nb][3]));
+            c0[nb] = movmatrix_trans(pack_half2(s[nb][0] - h0.x, s[nb][1] - h0.y));
+            c1[nb] = movmatrix_trans(pack_half2(s[nb][2] - h1.x, s[nb][3] - h1.y));
+        }
     }
     // A = V^T: the lane supplies dims 32 db + 4g .. +3 of keys 2t, 2t+1, 2t+8, 2t+9.  Keys at or beyond kv_total hold
     // stale rows: their p is exactly 0; zero V there so 0 * inf cannot appear.
 #pragma unroll
-    for (int db = 0; db < 4; ++db) {
+    for (int db = 0; db < 4 * S; ++db) {
         uint2 v[4];
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
@@ -325,6 +378,10 @@ __device__ __forceinline__ void process_stage_group(const __half* krow, const __
         for (int nb = 0; nb < NB; ++nb) {
             mma16816(acc.o[nb][db][0], x0, x1, x2, x3, b0[nb], b1[nb]);
             mma16816(acc.o[nb][db][1], y0, y1, y2, y3, b0[nb], b1[nb]);
+            if constexpr (S == 2) {
+                mma16816(acc.o[nb][db][0], x0, x1, x2, x3, c0[nb], c1[nb]);
+                mma16816(acc.o[nb][db][1], y0, y1, y2, y3, c0[nb], c1[nb]);
+            }
         }
     }
 }
@@ -336,28 +393,30 @@ __device__ __forceinline__ void process_stage_group(const __half* krow, const __
 // kOther: the cache was written with variance balancing (Sinkhorn iterations > 0): every key carries a factor other_K on
 // its logits and every dim of a tile a factor other_V on its output (reference kvarn128_codec.cuh:331-347); both are 1
 // otherwise and the arithmetic for them is compiled out.
-template <int NB, int W, bool kOther = false>
+template <int S, int NB, int W, bool kOther = false>
 __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int head, int zb, int64_t pidx) {
+    using Sh = Shape<S>;
+    constexpr int D = Sh::kDim, kChunkBytes = Sh::kChunk, kHdrV = Sh::kHdrV, kHdrK = Sh::kHdrK, kDigits = Sh::kDigits;
     constexpr int kWarps = W, kThreads = W * 32;
     constexpr int kGroups = kPage / 16;            // 16-key groups of a page
-    constexpr int kDimSweeps = 4;                  // the V chunk of a page is swept one 32-dim block at a time: a quarter of the integer accumulators live (measured 1.6 % faster than two halves)
-    constexpr int kORow = D + 4, kWarpFloats = 3 * kRows + kRows * kORow;  // merge buffer of a warp: m, l, z per row, then o
-    static_assert(kWarps * kWarpFloats * 4 <= static_cast<int>(sizeof(WarpRing)) * kWarps, "merge buffer exceeds the rings");
+    constexpr int kORow = D + 4, kWarpFloats = (2 + S) * kRows + kRows * kORow;  // merge buffer of a warp: m, l, z (per slice) per row, then o
+    static_assert(kWarps * kWarpFloats * 4 <= static_cast<int>(sizeof(WarpRing<S>)) * kWarps, "merge buffer exceeds the rings");
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    AttnSmem<W>& sm = *reinterpret_cast<AttnSmem<W>*>(smem_raw);
+    AttnSmem<S, W>& sm = *reinterpret_cast<AttnSmem<S, W>*>(smem_raw);
     const LayerView& L = P.L;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int G = L.q_heads / L.kv_heads;
-    WarpRing& R = sm.ring[warp];
+    WarpRing<S>& R = sm.ring[warp];
     // ---- order of the first memory requests: the few bytes everything waits for (positions, q rows, page table
     //      entries) go out first, then the first chunk of every warp, then -- after the rotation of q -- the rest of
     //      the ring.
     constexpr int kQIter = (8 * NB + W - 1) / W;  // warp w prepares rows w, w + W, ... of the block
-    uint16_t qraw[kQIter][4];
+    uint16_t qraw[kQIter][4 * S];
     int qpos[kQIter];
 #pragma unroll
     for (int i = 0; i < kQIter; ++i) {
-        qraw[i][0] = qraw[i][1] = qraw[i][2] = qraw[i][3] = 0;
+#pragma unroll
+        for (int j = 0; j < 4 * S; ++j) qraw[i][j] = 0;
         qpos[i] = -1;
         const int r = warp + W * i;
         if (r < 8 * NB) {
@@ -365,7 +424,7 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
             if (tq < P.T) {
                 const uint16_t* qrow = P.q + (static_cast<int64_t>(tq) * L.q_heads + head * G + gq) * D;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) qraw[i][j] = qrow[lane + 32 * j];
+                for (int j = 0; j < 4 * S; ++j) qraw[i][j] = qrow[lane + 32 * j];
                 qpos[i] = P.pos[tq];
             }
         }
@@ -427,12 +486,8 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
             if (n & 1) {
                 const uint8_t* src = vc + static_cast<size_t>(pid) * code_stride;
                 mbar_expect_tx(&R.bars[slot], kChunkBytes);
-                if constexpr (kVShift == 0) {
-                    bulk_g2s(dst, src, kChunkBytes, &R.bars[slot]);
-                } else {
 #pragma unroll
-                    for (int a = 0; a < 4; ++a) bulk_g2s(dst + a * kVSub, src + a * 1024, 1024, &R.bars[slot]);
-                }
+                for (int a = 0; a < Sh::kSubs; ++a) bulk_g2s(dst + a * Sh::kSubBytes, src + a * 1024, 1024, &R.bars[slot]);
             } else {
                 const int lp = w0 + (n >> 1);
                 const bool with_k = kOther || (lp & 1) == 0 || lp == w0;  // K scale rows: with the first page of a tile this warp reads (their fifth column is other_K of the page's own keys: always, when it is not 1)
@@ -451,17 +506,15 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
     for (int i = 0; i < kQIter; ++i) {
         const int r = warp + W * i;
         if (r < 8 * NB) {
-            float v[4];
+            float v[4 * S];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = L.dtype == KVB_DTYPE_BF16 ? in_to_f32<true>(qraw[i][j]) : in_to_f32<false>(qraw[i][j]);
+            for (int j = 0; j < 4 * S; ++j) v[j] = L.dtype == KVB_DTYPE_BF16 ? in_to_f32<true>(qraw[i][j]) : in_to_f32<false>(qraw[i][j]);
             hadamard_warp<D>(v, lane);  // rows beyond T are zeros and stay zeros
             if (lane == 0) sm.row_pos[r] = qpos[i];
             float* dst = reinterpret_cast<float*>(sm.qfrag);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int d = lane + 32 * j;  // -> lane' = (r%8)*4 + d/32, slot j' = (d%32)/4, component d%4
-                dst[(((r >> 3) * 8 + ((d & 31) >> 2)) * 32 + (r & 7) * 4 + (d >> 5)) * 4 + (d & 3)] = v[j] * P.scale_log2;
-            }
+            for (int j = 0; j < 4 * S; ++j)  // dim lane + 32 j -> lane' = (r%8)*4 + (d%128)/32, slot j' = 8 slice + (d%32)/4, component d%4
+                dst[(((r >> 3) * 8 * S + 8 * (j >> 2) + (lane >> 2)) * 32 + (r & 7) * 4 + (j & 3)) * 4 + (lane & 3)] = v[j] * P.scale_log2;
         }
     }
     while (n_issued < kSlots && n_issued < nchunks) issue_next(n_issued);
@@ -479,17 +532,19 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
     for (int r = 0; r < 8 * NB; ++r)
         if (sm.row_pos[r] >= 0) min_lim = min(min_lim, sm.row_pos[r]);
 
-    Acc<NB> acc;
+    Acc<S, NB> acc;
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) {
 #pragma unroll
-        for (int db = 0; db < 4; ++db)
+        for (int db = 0; db < Sh::kBlocks; ++db)
 #pragma unroll
             for (int xy = 0; xy < 2; ++xy)
 #pragma unroll
                 for (int c = 0; c < 4; ++c) acc.o[nb][db][xy][c] = 0.0f;
         acc.m[nb][0] = acc.m[nb][1] = -INFINITY;
-        acc.l[nb][0] = acc.l[nb][1] = acc.z[nb][0] = acc.z[nb][1] = 0.0f;
+        acc.l[nb][0] = acc.l[nb][1] = 0.0f;
+#pragma unroll
+        for (int s = 0; s < S; ++s) acc.z[s][nb][0] = acc.z[s][nb][1] = 0.0f;
     }
 
     // ---- open tile (last split of the head): its eight 16-key groups are dealt to the consumer warps, un-quantised,
@@ -499,9 +554,9 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
         for (int grp = warp; grp < 8; grp += W) {
             const int first = base + 16 * grp;
             if (first < key_end && first + 16 > key_begin && first < kv_total) {
-                QFrag<NB> qf;
-                build_qfrag<NB>(sm, lane, qf);
-                process_stage_group<NB>(L.stage_row(0, tile & 1, head, 16 * grp), L.stage_row(1, tile & 1, head, 16 * grp), qf,
+                QFrag<S, NB> qf;
+                build_qfrag<S, NB>(sm, lane, qf);
+                process_stage_group<S, NB>(L.stage_row(0, tile & 1, head, 16 * grp), L.stage_row(1, tile & 1, head, 16 * grp), qf,
                                         acc, lane, first, kv_total, row_lim, key_begin, key_end);
             }
         }
@@ -528,13 +583,15 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
         slot = slot + 1 == kSlots ? 0 : slot + 1;
     };
     // Key order inside a page: m-row i of 16-key group grp (lane g holds rows g and g + 8) is key
-    //   16 ((i & 7) >> 1) + 8 (grp >> 1) + 4 (grp & 1) + 2 (i >> 3) + (i & 1)
+    //   16 ((i & 7) >> 1) + 8 (grp >> 1) + 4 (grp & 1) + 2 (i >> 3) + (i & 1)     at 128 dims,
+    //   8 (i & 7) + 4 (grp >> 1) + 2 (grp & 1) + (i >> 3)                         at 256 dims,
     // so that, after the accumulator -> operand transposition, the weights of a group line up with the keys ldmatrix
-    // gathers from the four shifted sub-blocks of the V chunk.
-    const int key_lo = 16 * (g >> 1) + (g & 1);  // + 8 (grp >> 1) + 4 (grp & 1): key of m-row g; m-row g + 8 is 2 keys further
+    // gathers from the shifted sub-blocks of the V chunk.
+    const int key_lo = Sh::key_lo(g);
+    constexpr int kKeyH = Sh::kKeyH;
 
-    QInt<NB> qi;
-    float ov[4][2][2];  // kOther: other_V of dims 32 db + 4g + xy + 2h of the current tile
+    QInt<S, NB> qi;
+    float ov[Sh::kBlocks][2][2];  // kOther: other_V of dims 32 db + 4g + xy + 2h of the current tile
     int cur_tile = -1;
     for (int pi = 0; pi < npages; ++pi) {
         const int lp = w0 + pi;
@@ -551,15 +608,16 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
         if ((lp >> 1) != cur_tile) {  // per-dim scale / zero point of K belong to the tile
             cur_tile = lp >> 1;
             __syncwarp();
-            transpose_k_scale(hdr + kHdrV, R, lane);
+            transpose_k_scale<S>(hdr + kHdrV, R, lane);
             __syncwarp();
-            build_qint<NB>(sm, R, lane, qi);
-            if constexpr (kOther) {  // other_V of the lane's 16 dims: V scale row d / 2 starts with (other(d even), other(d odd))
+            build_qint<S, NB>(sm, R, lane, qi);
+            if constexpr (kOther) {  // other_V of the lane's dims: V scale row d / (2 S) starts with the other_V of its 2 S dims
 #pragma unroll
-                for (int db = 0; db < 4; ++db)
+                for (int db = 0; db < Sh::kBlocks; ++db)
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        const float2 o2 = unpack_half2(*reinterpret_cast<const uint32_t*>(hdr + (16 * db + 2 * g + h) * 8));
+                        const int at = S == 1 ? (16 * db + 2 * g + h) * 8 : (8 * db + g) * 16 + 4 * h;
+                        const float2 o2 = unpack_half2(*reinterpret_cast<const uint32_t*>(hdr + at));
                         ov[db][0][h] = o2.x;
                         ov[db][1][h] = o2.y;
                     }
@@ -567,43 +625,75 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
         }
         const int first = lp * kPage;
         const bool need_mask = first + kPage - 1 > min_lim || first < key_begin || first + kPage > key_end;
-        // ---- QK: integer logits of the page
+        // ---- QK: integer sums of the page.  One slice keeps them as integers (the row maximum is an integer maximum); with
+        //      two slices, each with its own row scale, they become fp32 logits right away.
         int tot[NB][kGroups][4];
+        float sl[NB][kGroups][4];  // logits, then logits relative to the page maximum (log2 units)
         {
-            const uint8_t* ch = R.slots[slot] + key_lo * 64 + 16 * t;
+            const uint8_t* ch = R.slots[slot] + key_lo * 64 * S + 16 * t;
 #pragma unroll
             for (int grp = 0; grp < kGroups; ++grp) {
-                const int koff = (8 * (grp >> 1) + 4 * (grp & 1)) * 64;
-                const uint4 ka = *reinterpret_cast<const uint4*>(ch + koff);
-                const uint4 kb8 = *reinterpret_cast<const uint4*>(ch + koff + 2 * 64);
-                const uint32_t wa[4] = {ka.x, ka.y, ka.z, ka.w}, wb[4] = {kb8.x, kb8.y, kb8.z, kb8.w};
-                int ceh[NB][4], cel[NB][4], coh[NB][4], col[NB][4];
+                const int koff = Sh::key_grp(grp) * 64 * S;
 #pragma unroll
-                for (int kb = 0; kb < 2; ++kb) {
-                    const uint32_t l0 = wa[2 * kb] & 0x0F0F0F0Fu, l1 = wb[2 * kb] & 0x0F0F0F0Fu, l2 = wa[2 * kb + 1] & 0x0F0F0F0Fu,
-                                   l3 = wb[2 * kb + 1] & 0x0F0F0F0Fu;
-                    const uint32_t h0 = wa[2 * kb] & 0xF0F0F0F0u, h1 = wb[2 * kb] & 0xF0F0F0F0u, h2 = wa[2 * kb + 1] & 0xF0F0F0F0u,
-                                   h3 = wb[2 * kb + 1] & 0xF0F0F0F0u;
+                for (int s = 0; s < S; ++s) {
+                    const uint4 ka = *reinterpret_cast<const uint4*>(ch + koff + 64 * s);
+                    const uint4 kb8 = *reinterpret_cast<const uint4*>(ch + koff + kKeyH * 64 * S + 64 * s);
+                    const uint32_t wa[4] = {ka.x, ka.y, ka.z, ka.w}, wb[4] = {kb8.x, kb8.y, kb8.z, kb8.w};
+                    int ce[NB][kDigits][4], co[NB][kDigits][4];  // even dims, odd dims (x 16)
 #pragma unroll
-                    for (int nb = 0; nb < NB; ++nb) {
-                        if (kb == 0) {
-                            imma_us0(ceh[nb], l0, l1, l2, l3, qi.b[nb][kb][0][0][0], qi.b[nb][kb][0][0][1]);
-                            imma_uu0(cel[nb], l0, l1, l2, l3, qi.b[nb][kb][0][1][0], qi.b[nb][kb][0][1][1]);
-                            imma_us0(coh[nb], h0, h1, h2, h3, qi.b[nb][kb][1][0][0], qi.b[nb][kb][1][0][1]);
-                            imma_uu0(col[nb], h0, h1, h2, h3, qi.b[nb][kb][1][1][0], qi.b[nb][kb][1][1][1]);
-                        } else {
-                            imma_us(ceh[nb], l0, l1, l2, l3, qi.b[nb][kb][0][0][0], qi.b[nb][kb][0][0][1]);
-                            imma_uu(cel[nb], l0, l1, l2, l3, qi.b[nb][kb][0][1][0], qi.b[nb][kb][0][1][1]);
-                            imma_us(coh[nb], h0, h1, h2, h3, qi.b[nb][kb][1][0][0], qi.b[nb][kb][1][0][1]);
-                            imma_uu(col[nb], h0, h1, h2, h3, qi.b[nb][kb][1][1][0], qi.b[nb][kb][1][1][1]);
+                    for (int kb = 0; kb < 2; ++kb) {
+                        const uint32_t l0 = wa[2 * kb] & 0x0F0F0F0Fu, l1 = wb[2 * kb] & 0x0F0F0F0Fu, l2 = wa[2 * kb + 1] & 0x0F0F0F0Fu,
+                                       l3 = wb[2 * kb + 1] & 0x0F0F0F0Fu;
+                        const uint32_t h0 = wa[2 * kb] & 0xF0F0F0F0u, h1 = wb[2 * kb] & 0xF0F0F0F0u, h2 = wa[2 * kb + 1] & 0xF0F0F0F0u,
+                                       h3 = wb[2 * kb + 1] & 0xF0F0F0F0u;
+#pragma unroll
+                        for (int nb = 0; nb < NB; ++nb) {
+#pragma unroll
+                            for (int d = 0; d < kDigits; ++d) {
+                                const uint32_t(&be)[2] = qi.b[s][nb][kb][0][d], (&bo)[2] = qi.b[s][nb][kb][1][d];
+                                if (d == 0) {
+                                    if (kb == 0) {
+                                        imma_us0(ce[nb][d], l0, l1, l2, l3, be[0], be[1]);
+                                        imma_us0(co[nb][d], h0, h1, h2, h3, bo[0], bo[1]);
+                                    } else {
+                                        imma_us(ce[nb][d], l0, l1, l2, l3, be[0], be[1]);
+                                        imma_us(co[nb][d], h0, h1, h2, h3, bo[0], bo[1]);
+                                    }
+                                } else {
+                                    if (kb == 0) {
+                                        imma_uu0(ce[nb][d], l0, l1, l2, l3, be[0], be[1]);
+                                        imma_uu0(co[nb][d], h0, h1, h2, h3, bo[0], bo[1]);
+                                    } else {
+                                        imma_uu(ce[nb][d], l0, l1, l2, l3, be[0], be[1]);
+                                        imma_uu(co[nb][d], h0, h1, h2, h3, bo[0], bo[1]);
+                                    }
+                                }
+                            }
                         }
                     }
+                    float ok[2] = {1.0f, 1.0f};
+                    if constexpr (S == 2 && kOther) {
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+                            ok[h] = __half2float(*reinterpret_cast<const __half*>(hdr + kHdrV + (key_lo + Sh::key_grp(grp) + kKeyH * h) * 20 + 16 + 2 * s));
+                    }
+#pragma unroll
+                    for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            if constexpr (S == 1) {
+                                // 16 * sum = 256 (16 even_hi + odd_hi) + (16 even_lo + odd_lo); |.| < 2^31
+                                tot[nb][grp][e] = ((ce[nb][0][e] * 16 + co[nb][0][e]) << 8) + (ce[nb][1][e] * 16 + co[nb][1][e]);
+                            } else {
+                                // the two low bytes' sums stay below 2^31 together; the high byte's joins in fp32
+                                const int low = ((ce[nb][1][e] * 16 + co[nb][1][e]) << 8) + (ce[nb][2][e] * 16 + co[nb][2][e]);
+                                const float sum = fmaf(static_cast<float>(ce[nb][0][e] * 16 + co[nb][0][e]), 65536.0f, static_cast<float>(low));
+                                const float x = fmaf(sum, qi.f[s][nb][e & 1], qi.qz[s][nb][e & 1]);
+                                if constexpr (kOther) sl[nb][grp][e] = s == 0 ? x * ok[e >> 1] : fmaf(x, ok[e >> 1], sl[nb][grp][e]);
+                                else sl[nb][grp][e] = s == 0 ? x : sl[nb][grp][e] + x;
+                            }
+                        }
                 }
-#pragma unroll
-                for (int nb = 0; nb < NB; ++nb)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)  // 16 * sum = 256 (16 even_hi + odd_hi) + (16 even_lo + odd_lo); |.| < 2^31
-                        tot[nb][grp][e] = ((ceh[nb][e] * 16 + coh[nb][e]) << 8) + (cel[nb][e] * 16 + col[nb][e]);
             }
         }
         release_chunk(true);
@@ -612,43 +702,63 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
             for (int grp = 0; grp < kGroups; ++grp)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    const int p = first + key_lo + 8 * (grp >> 1) + 4 * (grp & 1) + 2 * (e >> 1);
+                    const int p = first + key_lo + Sh::key_grp(grp) + kKeyH * (e >> 1);
                     const bool out = p < key_begin || p >= key_end;
 #pragma unroll
                     for (int nb = 0; nb < NB; ++nb)
-                        if (out || p > row_lim[nb][e & 1]) tot[nb][grp][e] = INT_MIN;
+                        if (out || p > row_lim[nb][e & 1]) {
+                            if constexpr (S == 1) tot[nb][grp][e] = INT_MIN;
+                            else sl[nb][grp][e] = -INFINITY;
+                        }
                 }
         }
         // ---- softmax of the page relative to its own row maxima; weights of the page against the running state
-        float wq[NB][2];     // weight of the integer sums of this page in the running accumulators
-        float zfull[NB][2];  // kOther: sum over the page's keys of p * zp_V, weighted like the integer sums
-        uint32_t bh[NB][kGroups], bl[NB][kGroups];  // 16-bit weights as B fragments: high and low bytes
+        float wq[S][NB][2];     // weight of the integer sums of this page in the running accumulators
+        float zfull[S][NB][2];  // kOther: sum over the page's keys of p * zp_V, weighted like the integer sums
+        uint32_t bw[S][NB][kDigits][kGroups];  // weights as B fragments, one byte each: highest digit first
         {
             // per-key scale of V: the largest of the page bounds p * scale_V; one factor for all rows
-            float svmax = fmaxf(fabsf(__half2float(*reinterpret_cast<const __half*>(hdr + lane * 8 + 4))),
-                                fabsf(__half2float(*reinterpret_cast<const __half*>(hdr + (lane + 32) * 8 + 4))));
+            float F[S], invF[S];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) svmax = fmaxf(svmax, __shfl_xor_sync(0xffffffffu, svmax, o));
-            const float F = svmax > 0.0f ? kPMax / svmax : 0.0f, invF = svmax * (1.0f / kPMax);
+            for (int s = 0; s < S; ++s) {
+                float svmax = fmaxf(fabsf(__half2float(*reinterpret_cast<const __half*>(hdr + lane * 8 * S + 4 * S + 2 * s))),
+                                    fabsf(__half2float(*reinterpret_cast<const __half*>(hdr + (lane + 32) * 8 * S + 4 * S + 2 * s))));
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) svmax = fmaxf(svmax, __shfl_xor_sync(0xffffffffu, svmax, o));
+                F[s] = svmax > 0.0f ? Sh::kPMax / svmax : 0.0f;
+                invF[s] = svmax * (1.0f / Sh::kPMax);
+            }
             float alpha[NB][2], wpass[NB][2], cst[NB][2];
             bool moved = false;
-            float sl[NB][kGroups][4];  // logits relative to the page maximum (log2 units)
-            if constexpr (kOther) {
-                // logits = other_K(key) * (f * integer sum + qz): the page maximum is taken on the floats
-                float ok[kGroups][2];
+            auto page_weights = [&](int nb, int j, float mpass) {  // the page's row maximum against the running one
+                const float mnew = fmaxf(acc.m[nb][j], mpass);
+                moved |= mnew > acc.m[nb][j];
+                const float muse = mnew == -INFINITY ? 0.0f : mnew;
+                alpha[nb][j] = fast_exp2(acc.m[nb][j] - muse);
+                wpass[nb][j] = fast_exp2(mpass - muse);
+                acc.m[nb][j] = mnew;
 #pragma unroll
-                for (int grp = 0; grp < kGroups; ++grp)
-#pragma unroll
-                    for (int h = 0; h < 2; ++h)
-                        ok[grp][h] = __half2float(*reinterpret_cast<const __half*>(hdr + kHdrV + (key_lo + 8 * (grp >> 1) + 4 * (grp & 1) + 2 * h) * 10 + 8));
-#pragma unroll
-                for (int nb = 0; nb < NB; ++nb)
+                for (int s = 0; s < S; ++s) wq[s][nb][j] = wpass[nb][j] * invF[s];
+            };
+            if constexpr (kOther || S == 2) {
+                if constexpr (S == 1) {
+                    // logits = other_K(key) * (f * integer sum + qz): the page maximum is taken on the floats
+                    float ok[kGroups][2];
 #pragma unroll
                     for (int grp = 0; grp < kGroups; ++grp)
 #pragma unroll
-                        for (int e = 0; e < 4; ++e)
-                            sl[nb][grp][e] = tot[nb][grp][e] == INT_MIN ? -INFINITY
-                                                                         : fmaf(static_cast<float>(tot[nb][grp][e]), qi.f[nb][e & 1], qi.qz[nb][e & 1]) * ok[grp][e >> 1];
+                        for (int h = 0; h < 2; ++h)
+                            ok[grp][h] = __half2float(*reinterpret_cast<const __half*>(hdr + kHdrV + (key_lo + Sh::key_grp(grp) + kKeyH * h) * 10 + 8));
+#pragma unroll
+                    for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+                        for (int grp = 0; grp < kGroups; ++grp)
+#pragma unroll
+                            for (int e = 0; e < 4; ++e)
+                                sl[nb][grp][e] = tot[nb][grp][e] == INT_MIN
+                                                     ? -INFINITY
+                                                     : fmaf(static_cast<float>(tot[nb][grp][e]), qi.f[0][nb][e & 1], qi.qz[0][nb][e & 1]) * ok[grp][e >> 1];
+                }
 #pragma unroll
                 for (int nb = 0; nb < NB; ++nb) {
 #pragma unroll
@@ -659,17 +769,11 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
                         mpass = fmaxf(mpass, __shfl_xor_sync(0xffffffffu, mpass, 4));
                         mpass = fmaxf(mpass, __shfl_xor_sync(0xffffffffu, mpass, 8));
                         mpass = fmaxf(mpass, __shfl_xor_sync(0xffffffffu, mpass, 16));
-                        const float mnew = fmaxf(acc.m[nb][j], mpass);
-                        moved |= mnew > acc.m[nb][j];
-                        const float muse = mnew == -INFINITY ? 0.0f : mnew;
-                        alpha[nb][j] = fast_exp2(acc.m[nb][j] - muse);
-                        wpass[nb][j] = fast_exp2(mpass - muse);
+                        page_weights(nb, j, mpass);
                         cst[nb][j] = mpass == -INFINITY ? 0.0f : mpass;
-                        acc.m[nb][j] = mnew;
-                        wq[nb][j] = wpass[nb][j] * invF;
                     }
                 }
-                if (__any_sync(0xffffffffu, moved)) rescale<NB>(acc, alpha);
+                if (__any_sync(0xffffffffu, moved)) rescale<S, NB>(acc, alpha);
 #pragma unroll
                 for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
@@ -678,56 +782,61 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
                         for (int e = 0; e < 4; ++e) sl[nb][grp][e] -= cst[nb][e & 1];  // masked keys stay at -inf
             } else {
 #pragma unroll
-            for (int nb = 0; nb < NB; ++nb) {
+                for (int nb = 0; nb < NB; ++nb) {
 #pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    int mx = INT_MIN;
+                    for (int j = 0; j < 2; ++j) {
+                        int mx = INT_MIN;
 #pragma unroll
-                    for (int grp = 0; grp < kGroups; ++grp) mx = max(mx, max(tot[nb][grp][j], tot[nb][grp][2 + j]));
-                    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
-                    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
-                    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-                    const float mpass = mx == INT_MIN ? -INFINITY : fmaf(static_cast<float>(mx), qi.f[nb][j], qi.qz[nb][j]);
-                    const float mnew = fmaxf(acc.m[nb][j], mpass);
-                    moved |= mnew > acc.m[nb][j];
-                    const float muse = mnew == -INFINITY ? 0.0f : mnew;
-                    alpha[nb][j] = fast_exp2(acc.m[nb][j] - muse);
-                    wpass[nb][j] = fast_exp2(mpass - muse);
-                    cst[nb][j] = qi.qz[nb][j] - (mpass == -INFINITY ? 0.0f : mpass);
-                    acc.m[nb][j] = mnew;
-                    wq[nb][j] = wpass[nb][j] * invF;
+                        for (int grp = 0; grp < kGroups; ++grp) mx = max(mx, max(tot[nb][grp][j], tot[nb][grp][2 + j]));
+                        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+                        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+                        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+                        const float mpass = mx == INT_MIN ? -INFINITY : fmaf(static_cast<float>(mx), qi.f[0][nb][j], qi.qz[0][nb][j]);
+                        page_weights(nb, j, mpass);
+                        cst[nb][j] = qi.qz[0][nb][j] - (mpass == -INFINITY ? 0.0f : mpass);
+                    }
+                }
+                if (__any_sync(0xffffffffu, moved)) rescale<S, NB>(acc, alpha);
+#pragma unroll
+                for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+                    for (int grp = 0; grp < kGroups; ++grp)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) sl[nb][grp][e] = fmaf(static_cast<float>(tot[nb][grp][e]), qi.f[0][nb][e & 1], cst[nb][e & 1]);
+                if (need_mask) {  // ... and get weight exactly zero
+#pragma unroll
+                    for (int grp = 0; grp < kGroups; ++grp)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const int p = first + key_lo + Sh::key_grp(grp) + kKeyH * (e >> 1);
+                            const bool out = p < key_begin || p >= key_end;
+#pragma unroll
+                            for (int nb = 0; nb < NB; ++nb)
+                                if (out || p > row_lim[nb][e & 1]) sl[nb][grp][e] = -INFINITY;
+                        }
                 }
             }
-            if (__any_sync(0xffffffffu, moved)) rescale<NB>(acc, alpha);
+            float lp_[NB][2], zp_[S][NB][2];
 #pragma unroll
-            for (int nb = 0; nb < NB; ++nb)
+            for (int nb = 0; nb < NB; ++nb) {
+                lp_[nb][0] = lp_[nb][1] = 0.0f;
 #pragma unroll
-                for (int grp = 0; grp < kGroups; ++grp)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) sl[nb][grp][e] = fmaf(static_cast<float>(tot[nb][grp][e]), qi.f[nb][e & 1], cst[nb][e & 1]);
-            if (need_mask) {  // ... and get weight exactly zero
-#pragma unroll
-                for (int grp = 0; grp < kGroups; ++grp)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int p = first + key_lo + 8 * (grp >> 1) + 4 * (grp & 1) + 2 * (e >> 1);
-                        const bool out = p < key_begin || p >= key_end;
-#pragma unroll
-                        for (int nb = 0; nb < NB; ++nb)
-                            if (out || p > row_lim[nb][e & 1]) sl[nb][grp][e] = -INFINITY;
-                    }
+                for (int s = 0; s < S; ++s) zp_[s][nb][0] = zp_[s][nb][1] = 0.0f;
             }
-            }
-            float lp_[NB][2], zp_[NB][2];
-#pragma unroll
-            for (int nb = 0; nb < NB; ++nb) lp_[nb][0] = lp_[nb][1] = zp_[nb][0] = zp_[nb][1] = 0.0f;
-            const uint8_t* vs = hdr + key_lo * 8 + 4;  // V scale rows are [other other scale zp] per key
+            const uint8_t* vs = hdr + key_lo * 8 * S + 4 * S;  // V scale rows per key: 2 S other_V, S scales, S zero points
 #pragma unroll
             for (int grp = 0; grp < kGroups; ++grp) {
-                const int koff = (8 * (grp >> 1) + 4 * (grp & 1)) * 8;
-                const float2 sz0 = unpack_half2(*reinterpret_cast<const uint32_t*>(vs + koff));           // (scale, zp) of the key of m-row g
-                const float2 sz1 = unpack_half2(*reinterpret_cast<const uint32_t*>(vs + koff + 2 * 8));   // ... of m-row g + 8
-                const float sf0 = sz0.x * F, sf1 = sz1.x * F;
+                const int koff = Sh::key_grp(grp) * 8 * S;
+                float sc0[S], zz0[S], sc1[S], zz1[S];  // scale and zero point of the keys of m-rows g and g + 8
+                if constexpr (S == 1) {
+                    const float2 sz0 = unpack_half2(*reinterpret_cast<const uint32_t*>(vs + koff)), sz1 = unpack_half2(*reinterpret_cast<const uint32_t*>(vs + koff + kKeyH * 8));
+                    sc0[0] = sz0.x; zz0[0] = sz0.y; sc1[0] = sz1.x; zz1[0] = sz1.y;
+                } else {
+                    const uint2 a = *reinterpret_cast<const uint2*>(vs + koff), b = *reinterpret_cast<const uint2*>(vs + koff + kKeyH * 16);
+                    const float2 sa = unpack_half2(a.x), za = unpack_half2(a.y), sb = unpack_half2(b.x), zb2 = unpack_half2(b.y);
+                    sc0[0] = sa.x; sc0[S - 1] = sa.y; zz0[0] = za.x; zz0[S - 1] = za.y;
+                    sc1[0] = sb.x; sc1[S - 1] = sb.y; zz1[0] = zb2.x; zz1[S - 1] = zb2.y;
+                }
 #pragma unroll
                 for (int nb = 0; nb < NB; ++nb) {
                     float p[4];
@@ -736,13 +845,23 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
                         p[e] = fast_exp2(sl[nb][grp][e]);
                         lp_[nb][e & 1] += p[e];
                     }
-                    zp_[nb][0] += p[0] * sz0.y + p[2] * sz1.y;
-                    zp_[nb][1] += p[1] * sz0.y + p[3] * sz1.y;
-                    // accumulator layout (m-row g; rows 2t, 2t+1) -> operand layout (row g; m-rows 2t, 2t+1 | 2t+8, 2t+9)
-                    const uint32_t y0 = movmatrix_trans(prmt(__float_as_uint(fmaf(p[0], sf0, kMagic)), __float_as_uint(fmaf(p[1], sf0, kMagic)), 0x5410));
-                    const uint32_t y1 = movmatrix_trans(prmt(__float_as_uint(fmaf(p[2], sf1, kMagic)), __float_as_uint(fmaf(p[3], sf1, kMagic)), 0x5410));
-                    bl[nb][grp] = prmt(y0, y1, 0x6420);
-                    bh[nb][grp] = prmt(y0, y1, 0x7531);
+#pragma unroll
+                    for (int s = 0; s < S; ++s) {
+                        zp_[s][nb][0] += p[0] * zz0[s] + p[2] * zz1[s];
+                        zp_[s][nb][1] += p[1] * zz0[s] + p[3] * zz1[s];
+                        // accumulator layout (m-row g; rows 2t, 2t+1) -> operand layout (row g; m-rows 2t, 2t+1 | 2t+8, 2t+9)
+                        const float sf0 = sc0[s] * F[s], sf1 = sc1[s] * F[s];
+                        uint32_t w[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) w[e] = __float_as_uint(fmaf(p[e], e < 2 ? sf0 : sf1, Sh::kPMagic));
+                        const uint32_t y0 = movmatrix_trans(prmt(w[0], w[1], 0x5410)), y1 = movmatrix_trans(prmt(w[2], w[3], 0x5410));
+                        bw[s][nb][kDigits - 1][grp] = prmt(y0, y1, 0x6420);
+                        bw[s][nb][kDigits - 2][grp] = prmt(y0, y1, 0x7531);
+                        if constexpr (S == 2) {  // the third bytes of both m-rows travel in one 16-bit element
+                            const uint32_t y2 = movmatrix_trans(prmt(prmt(w[0], w[2], 0x0062), prmt(w[1], w[3], 0x0062), 0x5410));
+                            bw[s][nb][0][grp] = prmt(y2, y2, 0x3120);
+                        }
+                    }
                 }
             }
 #pragma unroll
@@ -750,74 +869,75 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
                     acc.l[nb][j] = fmaf(lp_[nb][j], wpass[nb][j], acc.l[nb][j]);
-                    if constexpr (kOther) {  // the zero-point term takes other_V of the tile per dim: it enters the accumulators with the page
-                        float zs = zp_[nb][j];
-                        zs += __shfl_xor_sync(0xffffffffu, zs, 4);
-                        zs += __shfl_xor_sync(0xffffffffu, zs, 8);
-                        zs += __shfl_xor_sync(0xffffffffu, zs, 16);
-                        zfull[nb][j] = zs * wpass[nb][j];
-                    } else {
-                        acc.z[nb][j] = fmaf(zp_[nb][j], wpass[nb][j], acc.z[nb][j]);
+#pragma unroll
+                    for (int s = 0; s < S; ++s) {
+                        if constexpr (kOther) {  // the zero-point term takes other_V of the tile per dim: it enters the accumulators with the page
+                            float zs = zp_[s][nb][j];
+                            zs += __shfl_xor_sync(0xffffffffu, zs, 4);
+                            zs += __shfl_xor_sync(0xffffffffu, zs, 8);
+                            zs += __shfl_xor_sync(0xffffffffu, zs, 16);
+                            zfull[s][nb][j] = zs * wpass[nb][j];
+                        } else {
+                            acc.z[s][nb][j] = fmaf(zp_[s][nb][j], wpass[nb][j], acc.z[s][nb][j]);
+                        }
                     }
                 }
         }
-        // ---- PV on the int8 path.  Matrix i' of the page (8 rows) gathers keys 2i', 2i'+1 of each of the four sub-blocks:
-        //      eight distinct 16-byte bank groups.  ldmatrix.trans hands lane (g, t) the code bytes of dims 32 db + 4g .. +3
-        //      of keys 16t + 2i', +1; one byte permute gathers keys 16t + 8c + {0..3} (then + {4..7}) of a dim pair, one AND
-        //      isolates the even dim (x) or 16 x the odd dim (y): the k slots of MMA c, matching groups 2c and 2c + 1.
+        // ---- PV on the int8 path.  Matrix i' of half c of the page (8 rows) gathers keys 2i', 2i'+1 (+ 8c) of each of the four
+        //      sub-blocks at 128 dims, key i' + 4c of each of the eight at 256: eight distinct 16-byte bank groups.
+        //      ldmatrix.trans hands lane (g, t) the code bytes of dims 32 db + 4g .. +3 of matrix rows 2t, 2t+1; one byte permute
+        //      gathers the rows of two matrices of a dim pair, one AND isolates the even dim (x) or 16 x the odd dim (y): the k
+        //      slots of MMA c, matching groups 2c and 2c + 1.
         wait_slot(slot);
         {
-            // lane L addresses row L & 7 of matrix L >> 3: key 16 ((L & 7) >> 1) + 2 (L >> 3) + (L & 1) (+ 8c), shifted with its sub-block
-            const int vkey = 16 * ((lane & 7) >> 1) + 2 * (lane >> 3) + (lane & 1);
-            const uint8_t* ch = R.slots[slot] + vkey * 64 + kVShift * (vkey >> 4);
+            // lane L addresses row L & 7 of matrix L >> 3, shifted with its sub-block
+            const int vrow = lane & 7, vmat = lane >> 3;
+            const uint8_t* ch = S == 1 ? R.slots[slot] + (16 * (vrow >> 1) + 2 * vmat + (vrow & 1)) * 64 + 16 * (vrow >> 1)
+                                       : R.slots[slot] + (8 * vrow + vmat) * 128 + 16 * vrow;
+            // swept one 32-dim block at a time: a quarter of the integer accumulators live (measured 1.6 % faster than two halves)
 #pragma unroll
-            for (int sweep = 0; sweep < kDimSweeps; ++sweep) {
-                constexpr int kDb = 4 / kDimSweeps;
-                int ix[NB][kDb][2][2][4];  // [nb][db][xy][digit][c]
+            for (int db = 0; db < Sh::kBlocks; ++db) {
+                constexpr int kHi = 0;
+                const int s = db >> 2;
+                int ix[NB][2][kDigits][4];  // [nb][xy][digit][c]
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {  // 32-key halves of the page: keys 16t + 8c + {0..7}
+                for (int c = 0; c < 2; ++c) {  // 32-key halves of the page
+                    uint32_t r[4];
+                    ldsm_x4_trans(r, ch + c * 512 + 16 * db);
+                    const uint32_t u0 = prmt(r[0], r[1], 0x6420), v0 = prmt(r[0], r[1], 0x7531);
+                    const uint32_t u1 = prmt(r[2], r[3], 0x6420), v1 = prmt(r[2], r[3], 0x7531);
+                    const uint32_t ax0 = u0 & 0x0F0F0F0Fu, ax1 = v0 & 0x0F0F0F0Fu, ax2 = u1 & 0x0F0F0F0Fu, ax3 = v1 & 0x0F0F0F0Fu;
+                    const uint32_t ay0 = u0 & 0xF0F0F0F0u, ay1 = v0 & 0xF0F0F0F0u, ay2 = u1 & 0xF0F0F0F0u, ay3 = v1 & 0xF0F0F0F0u;
 #pragma unroll
-                    for (int d = 0; d < kDb; ++d) {
-                        const int db = sweep * kDb + d;
-                        uint32_t r[4];
-                        ldsm_x4_trans(r, ch + c * 8 * 64 + 16 * db);
-                        const uint32_t u0 = prmt(r[0], r[1], 0x6420), v0 = prmt(r[0], r[1], 0x7531);
-                        const uint32_t u1 = prmt(r[2], r[3], 0x6420), v1 = prmt(r[2], r[3], 0x7531);
-                        const uint32_t ax0 = u0 & 0x0F0F0F0Fu, ax1 = v0 & 0x0F0F0F0Fu, ax2 = u1 & 0x0F0F0F0Fu, ax3 = v1 & 0x0F0F0F0Fu;
-                        const uint32_t ay0 = u0 & 0xF0F0F0F0u, ay1 = v0 & 0xF0F0F0F0u, ay2 = u1 & 0xF0F0F0F0u, ay3 = v1 & 0xF0F0F0F0u;
+                    for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
-                        for (int nb = 0; nb < NB; ++nb) {
+                        for (int d = 0; d < kDigits; ++d) {
                             if (c == 0) {
-                                imma_uu0(ix[nb][d][0][0], ax0, ax1, ax2, ax3, bh[nb][0], bh[nb][1]);
-                                imma_uu0(ix[nb][d][0][1], ax0, ax1, ax2, ax3, bl[nb][0], bl[nb][1]);
-                                imma_uu0(ix[nb][d][1][0], ay0, ay1, ay2, ay3, bh[nb][0], bh[nb][1]);
-                                imma_uu0(ix[nb][d][1][1], ay0, ay1, ay2, ay3, bl[nb][0], bl[nb][1]);
+                                imma_uu0(ix[nb][0][d], ax0, ax1, ax2, ax3, bw[s][nb][d][0], bw[s][nb][d][1]);
+                                imma_uu0(ix[nb][1][d], ay0, ay1, ay2, ay3, bw[s][nb][d][0], bw[s][nb][d][1]);
                             } else {
-                                imma_uu(ix[nb][d][0][0], ax0, ax1, ax2, ax3, bh[nb][2], bh[nb][3]);
-                                imma_uu(ix[nb][d][0][1], ax0, ax1, ax2, ax3, bl[nb][2], bl[nb][3]);
-                                imma_uu(ix[nb][d][1][0], ay0, ay1, ay2, ay3, bh[nb][2], bh[nb][3]);
-                                imma_uu(ix[nb][d][1][1], ay0, ay1, ay2, ay3, bl[nb][2], bl[nb][3]);
+                                imma_uu(ix[nb][0][d], ax0, ax1, ax2, ax3, bw[s][nb][d][2], bw[s][nb][d][3]);
+                                imma_uu(ix[nb][1][d], ay0, ay1, ay2, ay3, bw[s][nb][d][2], bw[s][nb][d][3]);
                             }
                         }
-                    }
                 }
                 // ---- integer sums of the page -> running fp32 accumulators
 #pragma unroll
                 for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
-                    for (int d = 0; d < kDb; ++d)
+                    for (int xy = 0; xy < 2; ++xy)
 #pragma unroll
-                        for (int xy = 0; xy < 2; ++xy)
-#pragma unroll
-                            for (int c = 0; c < 4; ++c) {
-                                const float v = static_cast<float>((ix[nb][d][xy][0][c] << 8) + ix[nb][d][xy][1][c]);
-                                if constexpr (kOther) {  // (sum p code scale_V + sum p zp_V) * other_V(dim)
-                                    const float tv = fmaf(v, xy ? wq[nb][c & 1] * 0.0625f : wq[nb][c & 1], zfull[nb][c & 1]);
-                                    acc.o[nb][sweep * kDb + d][xy][c] = fmaf(tv, ov[sweep * kDb + d][xy][c >> 1], acc.o[nb][sweep * kDb + d][xy][c]);
-                                } else {
-                                    acc.o[nb][sweep * kDb + d][xy][c] = fmaf(v, xy ? wq[nb][c & 1] * 0.0625f : wq[nb][c & 1], acc.o[nb][sweep * kDb + d][xy][c]);
-                                }
+                        for (int c = 0; c < 4; ++c) {
+                            float v = static_cast<float>((ix[nb][xy][kDigits - 2][c] << 8) + ix[nb][xy][kDigits - 1][c]);
+                            if constexpr (S == 2) v = fmaf(static_cast<float>(ix[nb][xy][kHi][c]), 65536.0f, v);
+                            const float w = xy ? wq[s][nb][c & 1] * 0.0625f : wq[s][nb][c & 1];
+                            if constexpr (kOther) {  // (sum p code scale_V + sum p zp_V) * other_V(dim)
+                                const float tv = fmaf(v, w, zfull[s][nb][c & 1]);
+                                acc.o[nb][db][xy][c] = fmaf(tv, ov[db][xy][c >> 1], acc.o[nb][db][xy][c]);
+                            } else {
+                                acc.o[nb][db][xy][c] = fmaf(v, w, acc.o[nb][db][xy][c]);
                             }
+                        }
             }
         }
         release_chunk(true);
@@ -840,20 +960,22 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
 #pragma unroll
             for (int o = 4; o <= 16; o <<= 1) {
                 acc.l[nb][j] += __shfl_xor_sync(0xffffffffu, acc.l[nb][j], o);
-                acc.z[nb][j] += __shfl_xor_sync(0xffffffffu, acc.z[nb][j], o);
+#pragma unroll
+                for (int s = 0; s < S; ++s) acc.z[s][nb][j] += __shfl_xor_sync(0xffffffffu, acc.z[s][nb][j], o);
             }
             if (g == 0) {
                 const int row = 8 * nb + 2 * t + j;
                 mbuf[row] = acc.m[nb][j];
                 mbuf[kRows + row] = acc.l[nb][j];
-                mbuf[2 * kRows + row] = acc.z[nb][j];
+#pragma unroll
+                for (int s = 0; s < S; ++s) mbuf[(2 + s) * kRows + row] = acc.z[s][nb][j];
             }
         }
 #pragma unroll
-        for (int db = 0; db < 4; ++db)
+        for (int db = 0; db < Sh::kBlocks; ++db)
 #pragma unroll
             for (int j = 0; j < 2; ++j) {  // row 8 nb + 2t + j, dims 32 db + 4g .. +3
-                float* dst = mbuf + 3 * kRows + (8 * nb + 2 * t + j) * kORow + 32 * db + 4 * g;
+                float* dst = mbuf + (2 + S) * kRows + (8 * nb + 2 * t + j) * kORow + 32 * db + 4 * g;
                 *reinterpret_cast<float4*>(dst) = make_float4(acc.o[nb][db][0][j], acc.o[nb][db][1][j], acc.o[nb][db][0][2 + j], acc.o[nb][db][1][2 + j]);
             }
     }
@@ -871,8 +993,8 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
             for (int w = 0; w < kWarps; ++w) {
                 const float* wb = all + w * kWarpFloats;
                 const float wt = fast_exp2(wb[row] - m);  // exp2(-inf) = 0 for a warp that saw no key
-                const float4 v = *reinterpret_cast<const float4*>(wb + 3 * kRows + row * kORow + d);
-                const float z = wb[2 * kRows + row];
+                const float4 v = *reinterpret_cast<const float4*>(wb + (2 + S) * kRows + row * kORow + d);
+                const float z = wb[(2 + d / 128) * kRows + row];
                 l += wt * wb[kRows + row];
                 o.x += wt * (v.x + z); o.y += wt * (v.y + z); o.z += wt * (v.z + z); o.w += wt * (v.w + z);
             }
@@ -882,11 +1004,11 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
     }
 }
 
-template <int NB, int W, bool kOther = false>
+template <int S, int NB, int W, bool kOther = false>
 __global__ void __launch_bounds__(W * 32, 1) attn_kernel(const AttnParams P) {
     grid_dependency_wait();  // q, the positions and the cache come from the kernels before this one
     const int head = blockIdx.y, zb = blockIdx.z, split = blockIdx.x;
-    attn_cta<NB, W, kOther>(P, split, head, zb, ((static_cast<int64_t>(head) * gridDim.z + zb) * P.nsplit + split) * kRows);
+    attn_cta<S, NB, W, kOther>(P, split, head, zb, ((static_cast<int64_t>(head) * gridDim.z + zb) * P.nsplit + split) * kRows);
 }
 
 // Batched decode: `n` independent sequences (their caches described by device-resident kvb_layer structs, same
@@ -949,14 +1071,14 @@ __global__ void __launch_bounds__(W * 32, 1) attn_batch_kernel(const BatchParams
     P.ws_m = B.ws_m;
     P.ws_l = B.ws_l;
     P.ws_o = B.ws_o;
-    attn_cta<NB, W>(P, part - B.plan.prefix[b], head, 0, pidx);
+    attn_cta<1, NB, W>(P, part - B.plan.prefix[b], head, 0, pidx);
 }
 
 // Merge the partials of all splits of one query row, normalise, rotate back (H is its own inverse) and
 // store in the output dtype -- or, for a sharded decode, export the merged partial (m in natural-log
 // units, l, o in the rotated domain).  One CTA of 8 warps per (token, q head): warp w takes parts
 // w, w+8, ... and issues all its loads before using any (the kernel is pure load latency), lane l owns
-// dims 4l..4l+3; the eight warp sums meet in shared memory and warp 0 finishes the row.
+// dims 4l..4l+3 (of each 128-dim slice); the eight warp sums meet in shared memory and warp 0 finishes the row.
 constexpr int kReduceWarps = 8, kMaxPartsPerWarp = 8;  // up to 64 parts
 // Where a sharded decode sends its partial: the ring buffers of all ranks (peer memory over NVLink; this rank's
 // own buffer included), see kvb_peer_ring in the header.  A ring buffer holds [slot = call & 1][sender] blocks of
@@ -988,13 +1110,17 @@ __device__ __forceinline__ uint4 ring_load2(const unsigned long long* p) {
 }
 __device__ __forceinline__ bool ring_arrived(const uint4& w, uint32_t call) { return w.y == call && w.w == call; }
 
+// kPush: the ring exchange of a sharded decode (head_dim 128), compiled out of the other calls' kernel (it needs 242
+// registers per thread, the plain merge 72).
+template <int S, bool kPush>
 __global__ void __launch_bounds__(kReduceWarps * 32) reduce_kernel(const float* __restrict__ ws_m, const float* __restrict__ ws_l,
                                                                   const float* __restrict__ ws_o, int parts, int T, int q_heads,
                                                                   int kv_heads, int zblocks, int block_rows, int dtype, uint16_t* __restrict__ out,
                                                                   float* __restrict__ part_m, float* __restrict__ part_l,
                                                                   float* __restrict__ part_o, const PushTarget push,
                                                                   const BatchPlan plan) {
-    __shared__ float4 so[kReduceWarps][32];
+    constexpr int D = Shape<S>::kDim;
+    __shared__ float4 so[kReduceWarps][S][32];
     __shared__ float sl[kReduceWarps];
     const int row = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int G = q_heads / kv_heads, tq = row / q_heads, qh = row % q_heads, head = qh / G, gq = qh % G;
@@ -1009,11 +1135,11 @@ __global__ void __launch_bounds__(kReduceWarps * 32) reduce_kernel(const float* 
     grid_dependency_wait();  // launched while the attention kernel still runs: its partials are complete from here on
     launch_dependents();
     // the number of this call on the ring (read early: its latency hides behind the partial loads)
-    const uint32_t call = push.world > 0 && warp == 0 ? *reinterpret_cast<volatile uint32_t*>(push.state) + 1u : 0u;
+    const uint32_t call = kPush && warp == 0 ? *reinterpret_cast<volatile uint32_t*>(push.state) + 1u : 0u;
     // every warp finds the global maximum (parts <= 64: two loads per lane)
     float m = lane < parts ? ws_m[base + static_cast<int64_t>(lane) * kRows] : -INFINITY;
     if (lane + 32 < parts) m = fmaxf(m, ws_m[base + static_cast<int64_t>(lane + 32) * kRows]);
-    float4 v[kMaxPartsPerWarp];
+    float4 v[kMaxPartsPerWarp][S];
     float pm[kMaxPartsPerWarp], pl[kMaxPartsPerWarp];
 #pragma unroll
     for (int i = 0; i < kMaxPartsPerWarp; ++i) {
@@ -1022,33 +1148,44 @@ __global__ void __launch_bounds__(kReduceWarps * 32) reduce_kernel(const float* 
         const int64_t idx = base + static_cast<int64_t>(on ? p : 0) * kRows;
         pm[i] = on ? ws_m[idx] : -INFINITY;
         pl[i] = on ? ws_l[idx] : 0.0f;
-        v[i] = on ? *reinterpret_cast<const float4*>(ws_o + idx * D + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int s = 0; s < S; ++s)
+            v[i][s] = on ? *reinterpret_cast<const float4*>(ws_o + idx * D + 128 * s + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));  // after the loads are in flight
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 acc[S];
+#pragma unroll
+    for (int s = 0; s < S; ++s) acc[s] = make_float4(0.f, 0.f, 0.f, 0.f);
     float l = 0.0f;
     if (m != -INFINITY) {
 #pragma unroll
         for (int i = 0; i < kMaxPartsPerWarp; ++i) {
             const float w = fast_exp2(pm[i] - m);
             l += w * pl[i];
-            acc.x += w * v[i].x; acc.y += w * v[i].y; acc.z += w * v[i].z; acc.w += w * v[i].w;
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+                acc[s].x += w * v[i][s].x; acc[s].y += w * v[i][s].y; acc[s].z += w * v[i][s].z; acc[s].w += w * v[i][s].w;
+            }
         }
     }
-    so[warp][lane] = acc;
+#pragma unroll
+    for (int s = 0; s < S; ++s) so[warp][s][lane] = acc[s];
     if (lane == 0) sl[warp] = l;
     __syncthreads();
     if (warp != 0) return;
-    acc = so[0][lane];
     l = sl[0];
 #pragma unroll
     for (int w = 1; w < kReduceWarps; ++w) {
-        const float4 x = so[w][lane];
-        acc.x += x.x; acc.y += x.y; acc.z += x.z; acc.w += x.w;
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            const float4 x = so[w][s][lane];
+            acc[s].x += x.x; acc[s].y += x.y; acc[s].z += x.z; acc[s].w += x.w;
+        }
         l += sl[w];
     }
-    if (push.world > 0) {
+    if constexpr (kPush) {
+        static_assert(S == 1, "the ring holds rows of 128 dims");
         // Sharded decode: this CTA owns one query row on every rank.  It stores its partial of the row straight into
         // every peer's ring buffer, waits (bounded) for the peers' partials of the same row in its own ring buffer,
         // merges all of them in rank order (every rank computes the same bits), normalises, rotates back and
@@ -1064,8 +1201,8 @@ __global__ void __launch_bounds__(kReduceWarps * 32) reduce_kernel(const float* 
         for (int p = 0; p < kRingMaxWorld; ++p) {
             if (p >= push.world || p == push.rank) continue;
             unsigned long long* dst = push.peers[p] + my_block;
-            ring_store2(dst + o_off, acc.x, acc.y, call);
-            ring_store2(dst + o_off + 2, acc.z, acc.w, call);
+            ring_store2(dst + o_off, acc[0].x, acc[0].y, call);
+            ring_store2(dst + o_off + 2, acc[0].z, acc[0].w, call);
             if (lane == 0) ring_store2(dst + ml_off, mine, l, call);
         }
         const unsigned long long* in = push.local_buf + static_cast<int64_t>(slot) * push.world * block;
@@ -1137,7 +1274,7 @@ __global__ void __launch_bounds__(kReduceWarps * 32) reduce_kernel(const float* 
                 if (p == push.rank) {
                     const float w = gm == -INFINITY ? 0.0f : __expf(mine - gm);
                     gl += w * l;
-                    go.x += w * acc.x; go.y += w * acc.y; go.z += w * acc.z; go.w += w * acc.w;
+                    go.x += w * acc[0].x; go.y += w * acc[0].y; go.z += w * acc[0].z; go.w += w * acc[0].w;
                 } else {
                     const float w = gm == -INFINITY ? 0.0f : __expf(rm[p] - gm);
                     gl += w * rl[p];
@@ -1149,9 +1286,9 @@ __global__ void __launch_bounds__(kReduceWarps * 32) reduce_kernel(const float* 
         ok = __all_sync(0xffffffffu, ok);
         if (!ok && lane == 0 && push.error_word != nullptr) atomicOr(push.error_word, KVB_ERR_WAIT_TIMEOUT);
         const float ginv = ok && gl > 0.0f ? 1.0f / gl : 0.0f;  // a wait that ran out: zeros, not a half-merged row
-        so[0][lane] = make_float4(go.x * ginv, go.y * ginv, go.z * ginv, go.w * ginv);
+        so[0][0][lane] = make_float4(go.x * ginv, go.y * ginv, go.z * ginv, go.w * ginv);
         __syncwarp();
-        const float* gflat = reinterpret_cast<const float*>(so[0]);
+        const float* gflat = reinterpret_cast<const float*>(so[0][0]);
         float o[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) o[j] = gflat[lane + 32 * j];
@@ -1168,20 +1305,22 @@ __global__ void __launch_bounds__(kReduceWarps * 32) reduce_kernel(const float* 
     }
     if (part_m != nullptr) {
         if (lane == 0) { part_m[row] = m * kLn2; part_l[row] = l; }
-        *reinterpret_cast<float4*>(part_o + static_cast<int64_t>(row) * D + 4 * lane) = acc;
+#pragma unroll
+        for (int s = 0; s < S; ++s) *reinterpret_cast<float4*>(part_o + static_cast<int64_t>(row) * D + 128 * s + 4 * lane) = acc[s];
         return;
     }
     const float inv = l > 0.0f ? 1.0f / l : 0.0f;
     // the rotation wants lane l to hold dims l + 32 j: re-distribute through shared memory
-    so[0][lane] = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
+#pragma unroll
+    for (int s = 0; s < S; ++s) so[0][s][lane] = make_float4(acc[s].x * inv, acc[s].y * inv, acc[s].z * inv, acc[s].w * inv);
     __syncwarp();
     const float* flat = reinterpret_cast<const float*>(so[0]);
-    float o[4];
+    float o[4 * S];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) o[j] = flat[lane + 32 * j];
+    for (int j = 0; j < 4 * S; ++j) o[j] = flat[lane + 32 * j];
     hadamard_warp<D>(o, lane);
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < 4 * S; ++j)
         out[static_cast<int64_t>(row) * D + lane + 32 * j] = dtype == KVB_DTYPE_BF16 ? f32_to_out<true>(o[j]) : f32_to_out<false>(o[j]);
 }
 
@@ -1246,15 +1385,15 @@ int launch_general_attention(const kvb_layer* layer, const void* q, const int32_
 namespace {
 
 // One attention launch with W warps per CTA (the opt-in to large dynamic shared memory is made once per device and W).
-template <int NB, int W, bool kOther = false>
+template <int S, int NB, int W, bool kOther = false>
 cudaError_t launch_attn(dim3 grid, cudaStream_t stream, const AttnParams& P) {
-    constexpr int smem = static_cast<int>(sizeof(AttnSmem<W>));
+    constexpr int smem = static_cast<int>(sizeof(AttnSmem<S, W>));
     static unsigned long long opted = 0;
     if (first_call_on_device(opted)) {
-        const cudaError_t e = cudaFuncSetAttribute(attn_kernel<NB, W, kOther>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        const cudaError_t e = cudaFuncSetAttribute(attn_kernel<S, NB, W, kOther>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
     }
-    return launch_early(attn_kernel<NB, W, kOther>, grid, dim3(W * 32), smem, stream, P);
+    return launch_early(attn_kernel<S, NB, W, kOther>, grid, dim3(W * 32), smem, stream, P);
 }
 
 // Warps per CTA for a decode call: 8, 12 or 16 (whole warp quartets: an SM hands registers and issue slots out per
@@ -1285,14 +1424,14 @@ int decode_warps(int kv_len_max, int nsplit, float* cost_us = nullptr) {
 struct RowPlan {
     int nb, warps, block_rows, zblocks, nsplit;
 };
-RowPlan plan_rows(int kv_len_max, int kv_heads, int q_heads, int T, bool balanced) {
+RowPlan plan_rows(int kv_len_max, int kv_heads, int q_heads, int head_dim, int T, bool balanced) {
     const int merged = T * (q_heads / kv_heads);
     RowPlan one{1, 16, 8, zblocks_of(q_heads, kv_heads, T, 8), 0};
     one.nsplit = split_count(kv_len_max, kv_heads, one.zblocks);
     float cost_one = 0.0f;
     one.warps = decode_warps(kv_len_max, one.nsplit, &cost_one);
-    if (balanced) one.warps = 8;
-    if (merged <= 8) return one;
+    if (balanced || head_dim != 128) one.warps = kWarpsWide;
+    if (merged <= 8 || head_dim != 128) return one;
     RowPlan two{2, kWarpsWide, 16, zblocks_of(q_heads, kv_heads, T, 16), 0};
     two.nsplit = split_count(kv_len_max, kv_heads, two.zblocks);
     const int pages = 2 * (kv_len_max / kTile), per_cta = (pages + two.nsplit - 1) / two.nsplit;
@@ -1311,10 +1450,7 @@ int launch_attention(const kvb_layer* layer, const void* q, const int32_t* pos_d
     if (kv_len_max < 1) return fail(KVB_EINVAL, "%s: kv_len_max %d", who, kv_len_max);
     if (layer->stage == nullptr) return fail(KVB_EINVAL, "%s: layer has no stage buffer", who);
     if (layer->head_dim != 128 && push != nullptr) return fail(KVB_ERANGE, "%s: the sharded decode covers head_dim 128", who);
-    if (layer->head_dim != 128)  // two slices per key: general kernel, same semantics
-        return launch_general_attention(layer, q, pos_dev, total_pos_dev, T, scale, kv_len_max, key_begin, key_end, workspace, out,
-                                        part_m, part_l, part_o, stream);
-    const RowPlan plan = plan_rows(kv_len_max, layer->kv_heads, layer->q_heads, T, layer->sinkhorn_iters != 0);
+    const RowPlan plan = plan_rows(kv_len_max, layer->kv_heads, layer->q_heads, layer->head_dim, T, layer->sinkhorn_iters != 0);
     const int Z = plan.zblocks, nsplit = plan.nsplit;
     const int parts = nsplit;
     AttnParams P;
@@ -1334,23 +1470,30 @@ int launch_attention(const kvb_layer* layer, const void* q, const int32_t* pos_d
     P.ws_o = P.ws_l + rows;
     const bool upper = plan.nb == 2;
     const dim3 grid(parts, layer->kv_heads, Z);
-    if (layer->sinkhorn_iters != 0) {  // balanced caches: other_K per key, other_V per dim (more registers: 8 warps)
-        if (upper) {
-            KVB_CUDA_OK((launch_attn<2, kWarpsWide, true>(grid, stream, P)));
+    if (layer->head_dim != 128) {  // two slices per head: twice the accumulators and the wider integers leave room for 8 warps
+        if (layer->sinkhorn_iters != 0) {
+            KVB_CUDA_OK((launch_attn<2, 1, kWarpsWide, true>(grid, stream, P)));
         } else {
-            KVB_CUDA_OK((launch_attn<1, 8, true>(grid, stream, P)));
+            KVB_CUDA_OK((launch_attn<2, 1, kWarpsWide>(grid, stream, P)));
+        }
+    } else if (layer->sinkhorn_iters != 0) {  // balanced caches: other_K per key, other_V per dim (more registers: 8 warps)
+        if (upper) {
+            KVB_CUDA_OK((launch_attn<1, 2, kWarpsWide, true>(grid, stream, P)));
+        } else {
+            KVB_CUDA_OK((launch_attn<1, 1, 8, true>(grid, stream, P)));
         }
     } else if (upper) {
-        KVB_CUDA_OK((launch_attn<2, kWarpsWide>(grid, stream, P)));
+        KVB_CUDA_OK((launch_attn<1, 2, kWarpsWide>(grid, stream, P)));
     } else {
         switch (plan.warps) {
-            case 8: KVB_CUDA_OK((launch_attn<1, 8>(grid, stream, P))); break;
-            case 12: KVB_CUDA_OK((launch_attn<1, 12>(grid, stream, P))); break;
-            default: KVB_CUDA_OK((launch_attn<1, 16>(grid, stream, P))); break;
+            case 8: KVB_CUDA_OK((launch_attn<1, 1, 8>(grid, stream, P))); break;
+            case 12: KVB_CUDA_OK((launch_attn<1, 1, 12>(grid, stream, P))); break;
+            default: KVB_CUDA_OK((launch_attn<1, 1, 16>(grid, stream, P))); break;
         }
     }
     const int total_rows = T * layer->q_heads;
-    KVB_CUDA_OK(launch_early(reduce_kernel, dim3(total_rows), dim3(kReduceWarps * 32), 0, stream, P.ws_m, P.ws_l, P.ws_o, parts, T,
+    const auto reduce = layer->head_dim != 128 ? reduce_kernel<2, false> : push != nullptr ? reduce_kernel<1, true> : reduce_kernel<1, false>;
+    KVB_CUDA_OK(launch_early(reduce, dim3(total_rows), dim3(kReduceWarps * 32), 0, stream, P.ws_m, P.ws_l, P.ws_o, parts, T,
                              layer->q_heads, layer->kv_heads, Z, plan.block_rows, layer->dtype, static_cast<uint16_t*>(out), part_m, part_l, part_o,
                              push != nullptr ? *push : PushTarget{}, BatchPlan{}));
     return KVB_OK;
@@ -1365,7 +1508,7 @@ static constexpr int kDenseRows = 32;
 extern "C" int kvb_split_capacity(int kv_len_max, int kv_heads, int q_heads, int rows, int batch) {
     (void)batch;
     if (kv_heads < 1 || q_heads < kv_heads || rows < 1) return 0;
-    return kvb::plan_rows(kv_len_max, kv_heads, q_heads, rows > 8 ? 8 : rows, false).nsplit;
+    return kvb::plan_rows(kv_len_max, kv_heads, q_heads, 128, rows > 8 ? 8 : rows, false).nsplit;
 }
 
 // Bytes one call with `r` query tokens needs (the split count, hence the size, is not monotonic in r).
@@ -1599,7 +1742,7 @@ extern "C" int kvb_attn_decode_batch(const kvb_layer* layers_dev, int batch, int
     B.ws_m = static_cast<float*>(workspace);
     B.ws_l = B.ws_m + rows;
     B.ws_o = B.ws_l + rows;
-    constexpr int smem1 = static_cast<int>(sizeof(AttnSmem<kWarpsDecode>)), smem2 = static_cast<int>(sizeof(AttnSmem<kWarpsWide>));
+    constexpr int smem1 = static_cast<int>(sizeof(AttnSmem<1, kWarpsDecode>)), smem2 = static_cast<int>(sizeof(AttnSmem<1, kWarpsWide>));
     static unsigned long long opted = 0;
     if (first_call_on_device(opted)) {
         KVB_CUDA_OK(cudaFuncSetAttribute(attn_batch_kernel<1, kWarpsDecode>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem1));
@@ -1608,7 +1751,7 @@ extern "C" int kvb_attn_decode_batch(const kvb_layer* layers_dev, int batch, int
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (q_heads / kv_heads > 8) KVB_CUDA_OK(launch_early(attn_batch_kernel<2, kWarpsWide>, dim3(total, kv_heads, 1), dim3(kWarpsWide * 32), smem2, st, B));
     else KVB_CUDA_OK(launch_early(attn_batch_kernel<1, kWarpsDecode>, dim3(total, kv_heads, 1), dim3(kWarpsDecode * 32), smem1, st, B));
-    KVB_CUDA_OK(launch_early(reduce_kernel, dim3(batch * q_heads), dim3(kReduceWarps * 32), 0, st, B.ws_m, B.ws_l, B.ws_o, 0, batch, q_heads,
+    KVB_CUDA_OK(launch_early(reduce_kernel<1, false>, dim3(batch * q_heads), dim3(kReduceWarps * 32), 0, st, B.ws_m, B.ws_l, B.ws_o, 0, batch, q_heads,
                              kv_heads, 1, kRows, dtype, static_cast<uint16_t*>(out), static_cast<float*>(nullptr), static_cast<float*>(nullptr),
                              static_cast<float*>(nullptr), PushTarget{}, B.plan));
     return KVB_OK;
@@ -1648,12 +1791,12 @@ extern "C" int kvb_attn_chunk_partial(const kvb_layer* layer, const void* q, con
         return fail(KVB_EINVAL, "kvb_attn_chunk_partial: null argument");
     if (layer->stage == nullptr) return fail(KVB_EINVAL, "kvb_attn_chunk_partial: layer has no stage buffer");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (tokens <= 8 && (layer->head_dim != 128 || tokens * (layer->q_heads / layer->kv_heads) < kDenseRows))
+        return launch_attention(layer, q, positions_dev, positions_dev + (tokens - 1), tokens, scale, kv_len_max, 0, INT_MAX, workspace, nullptr,
+                                part_m, part_l, part_o, st, "kvb_attn_chunk_partial");
     if (layer->head_dim != 128)
         return launch_general_attention(layer, q, positions_dev, positions_dev + (tokens - 1), tokens, scale, kv_len_max, 0, INT_MAX, workspace,
                                         nullptr, part_m, part_l, part_o, st);
-    if (tokens <= 8 && tokens * (layer->q_heads / layer->kv_heads) < kDenseRows)
-        return launch_attention(layer, q, positions_dev, positions_dev + (tokens - 1), tokens, scale, kv_len_max, 0, INT_MAX, workspace, nullptr,
-                                part_m, part_l, part_o, st, "kvb_attn_chunk_partial");
     return launch_chunk_attention(layer, q, positions_dev, tokens, scale, kv_len_max, workspace, nullptr, st, part_m, part_l, part_o, nullptr);
 }
 
