@@ -1377,11 +1377,9 @@ namespace kvb {
 namespace {
 
 }  // namespace
-// kvb_attn_general.cu: head_dim 256 and caches written with Sinkhorn iterations > 0
-size_t general_workspace_bytes(int kv_len_max, int q_heads, int head_dim, int rows);
-int launch_general_attention(const kvb_layer* layer, const void* q, const int32_t* pos_dev, const int32_t* total_pos_dev, int T,
-                             float scale, int kv_len_max, int key_begin, int key_end, void* workspace, void* out, float* part_m,
-                             float* part_l, float* part_o, cudaStream_t stream);
+// kvb_chunk256.cu
+int launch_chunk_attention_256(const kvb_layer* layer, const void* q, const int32_t* positions_dev, int tokens, float scale,
+                               int kv_len_max, void* workspace, void* out, cudaStream_t s, float* part_m, float* part_l, float* part_o);
 namespace {
 
 // One attention launch with W warps per CTA (the opt-in to large dynamic shared memory is made once per device and W).
@@ -1519,9 +1517,7 @@ static size_t workspace_bytes_for_rows(int kv_len_max, int kv_heads, int q_heads
         const size_t parts = kvb::split_count(kv_len_max, kv_heads, Z);
         bytes = std::max(bytes, static_cast<size_t>(kv_heads) * Z * parts * kvb::kRows * (head_dim + 2) * sizeof(float));
     }
-    const size_t general = kvb::general_workspace_bytes(kv_len_max, q_heads, head_dim, r);
-    if (general > bytes) bytes = general;
-    if (r * (q_heads / kv_heads) >= kDenseRows) {  // verify steps this wide run on the chunk-attention kernel
+    if (r > 8 || r * (q_heads / kv_heads) >= kDenseRows) {  // steps this wide run on the chunk-attention kernels
         const size_t dense = kvb_prefill_workspace_bytes(kv_len_max, kv_heads, q_heads, head_dim, r);
         if (dense > bytes) bytes = dense;
     }
@@ -1795,8 +1791,7 @@ extern "C" int kvb_attn_chunk_partial(const kvb_layer* layer, const void* q, con
         return launch_attention(layer, q, positions_dev, positions_dev + (tokens - 1), tokens, scale, kv_len_max, 0, INT_MAX, workspace, nullptr,
                                 part_m, part_l, part_o, st, "kvb_attn_chunk_partial");
     if (layer->head_dim != 128)
-        return launch_general_attention(layer, q, positions_dev, positions_dev + (tokens - 1), tokens, scale, kv_len_max, 0, INT_MAX, workspace,
-                                        nullptr, part_m, part_l, part_o, st);
+        return launch_chunk_attention_256(layer, q, positions_dev, tokens, scale, kv_len_max, workspace, nullptr, st, part_m, part_l, part_o);
     return launch_chunk_attention(layer, q, positions_dev, tokens, scale, kv_len_max, workspace, nullptr, st, part_m, part_l, part_o, nullptr);
 }
 

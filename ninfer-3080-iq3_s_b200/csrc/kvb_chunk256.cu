@@ -1,0 +1,696 @@
+// kvb_chunk256.cu -- chunk attention over head_dim-256 caches (the reference engine's own geometry) on the
+// 5th-generation tensor cores, at fp32 accuracy.
+//
+// A CTA owns 128 GQA-packed (token, q head) rows of one KV head and one range of 64-key pages.  Every operand of the two
+// contractions is an fp32 value split into an fp16 high and low part (22 significant bits); a product takes three MMAs
+// (low x high, high x low, high x high; the low x low term is below fp32's own rounding).  So that neither part runs
+// into fp16's range, every query row, every page of K and the whole of V carry a power of two: rows and pages are scaled
+// to a largest magnitude of 2^14 .. 2^15 and their exponents return in the logits (a thread owns a row), V follows the
+// largest page seen so far and O is rescaled, exactly, when that grows.
+//
+// Roles (13 warps, one CTA per SM):
+//   warps 4-11   de-quantise K(i), then V(i-1): code -> fp32 (code * scale + zp) * other -> high | low, 64 KB a page each, in
+//                128-byte-swizzled tiles; thread = one key and 64 dims; codes and scales are fetched a page ahead;
+//   warp 12      issues S(i) = Q K(i)^T, then O += P(i-1) V(i-1);
+//   warps 0-3    softmax of S(i), thread = row: P (high | low) over S in tensor memory, O rescaled lazily.
+// K(i+1) is written while P V(i-1) runs, V(i) while Q K(i+1)^T runs.  Tensor memory (512 columns): two S buffers of
+// 64, the high part of Q (128, the A operand of two of the three Q K products), O (256).  The low part of Q stays in
+// shared memory (64 KB), beside one K and one V buffer.
+//
+// Bound by the chain of a page's hand-offs (de-quantise, MMA, softmax and back), with the tensor pipe (48 MMAs of 128x64x16
+// and 12 of 128x256x16 a page, about 3,300 cycles) and shared-memory traffic (MMA operands, 128 KB of tiles written a page)
+// close behind.  Measured on B200, 24 / 4 heads, 1,024 tokens over a prefix of 16,384, balanced bf16 cache: 1.5 ms (280
+// TFLOP/s of attention, 840 of MMA) against 69.8 ms for one warp per key on fp32 FMAs.
+// Accuracy: against float64 the un-normalised sums are off by 4e-7 .. 6e-6 (fp32 FMAs: 2e-7 .. 1.1e-5, sizes of 32 .. 65,576
+// keys), the fp16 / bf16 outputs by their rounding alone (2.09e-4 and 1.70e-3, as before).
+#include <climits>
+
+#include "kvb_chunk_merge.cuh"
+#include "kvb_common.cuh"
+#include "kvb_tcgen05.cuh"
+
+namespace kvb {
+namespace {
+
+constexpr int D = 256;
+constexpr int kM = 128;   // query rows per CTA
+constexpr int kN = 64;    // keys per step: one page
+constexpr int kSoftWarps = 4, kDqWarps = 8, kMmaWarp = kSoftWarps + kDqWarps, kThreads = 32 * (kMmaWarp + 1);
+constexpr int kDqThreads = 32 * kDqWarps;
+constexpr int kKvBlock = kN * 128;       // one 64-dim block of a K or V tile: 64 rows of 128 bytes
+constexpr int kKvTile = 4 * kKvBlock;
+constexpr int kQBlock = kM * 128;        // one 64-dim block of the Q tile
+constexpr int kSlotsMeta = 4;            // per-page words handed to the softmax warps: a writer is at most 2 pages ahead of a reader
+constexpr uint32_t kTmemCols = 512, kColQ = 128, kColO = 256;  // S buffers at columns 0 and 64
+constexpr int kTop = 14;                 // scaled operands reach 2^14 .. 2^15
+constexpr float kPBoost = 4.0f;          // P is taken 2^4 above the row's reference point (and stays below 2^12): more bits of small weights survive
+
+struct Chunk256Params {
+    LayerView L;
+    const uint16_t* q;         // [T][q_heads][D]
+    const int32_t* pos;        // [T]
+    const int32_t* total_pos;  // newest position in the cache
+    int T, mtiles, ksplit;
+    float scale_log2;
+    float* ws_m;               // [H][mtiles][ksplit][128]
+    float* ws_l;
+    float* ws_o;               // [H][mtiles][ksplit][128][D]
+};
+
+struct __align__(1024) Chunk256Smem {
+    uint8_t q_lo[4 * kQBlock];
+    uint8_t k[2][kKvTile];     // high, low part; holds the high part of Q before the walk
+    uint8_t v[2][kKvTile];
+    float ks[2][D], kz[2][D];            // per-dim factors of K by page parity; ks is divided by 16^(nibble position)
+    float vo[kSlotsMeta][D];             // per-dim factors of V (used a step later than those of K)
+    uint32_t red[2][kDqWarps][4];        // partial maxima: |K before other_K|, |other_K|, |other_V|, |V before other_V| (float bits)
+    uint32_t poison[kSlotsMeta][kDqWarps];  // keys with a non-finite V (ballots of the warps)
+    float k_unit[kSlotsMeta];            // page i: K = k_unit * (high + low)
+    int v_exp[kSlotsMeta];               // exponent of V and O as of page i
+    int bad_page[kSlotsMeta];
+    int row_pos[kM];
+    float row_unit[kM];                  // q' = row_unit * (high + low)
+    uint64_t s_full[2], p_full[2], k_full, v_full, o_done, drain;
+    uint32_t tmem_base;
+    int abort_flag;
+};
+
+__device__ __forceinline__ bool chunk_wait(uint64_t* bar, uint32_t parity, int* abort_flag) {
+    bool ok = false;
+    for (uint32_t i = 0; i < kSpinLimit && !ok; ++i) {
+        ok = mbar_try_wait(bar, parity);
+        if (!ok && *reinterpret_cast<volatile int*>(abort_flag) != 0) break;
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) *reinterpret_cast<volatile int*>(abort_flag) = 1;
+    return ok;
+}
+
+// Largest power of two that keeps values of magnitude `bits` (a non-negative float) below 2^(kTop + 1): exponent of the
+// scale that was taken out.  Zero and non-finite magnitudes: 0.
+__device__ __forceinline__ int scale_exponent(uint32_t bits) {
+    if (bits == 0u || bits >= 0x7F800000u) return 0;
+    return max(static_cast<int>(bits >> 23) - 127, -100) - kTop;
+}
+__device__ __forceinline__ float pow2i(int e) { return __uint_as_float(static_cast<uint32_t>(e + 127) << 23); }  // |e| <= 126
+__device__ __forceinline__ uint32_t abs_bits(float x) { return __float_as_uint(x) & 0x7FFFFFFFu; }
+
+// Two fp32 values in one register pair: half the issue slots of the scalar forms.
+struct F2 {
+    uint64_t v;
+    __device__ __forceinline__ F2() {}
+    __device__ __forceinline__ explicit F2(uint64_t x) : v(x) {}
+    __device__ __forceinline__ F2(float a, float b) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b)); }
+    __device__ __forceinline__ float2 get() const {
+        float2 r;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+        return r;
+    }
+};
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+// x = high + low in fp16 (22 significant bits)
+__device__ __forceinline__ void split2(F2 x, uint32_t& hi, uint32_t& lo) {
+    const float2 f = x.get();
+    hi = pack_half2(f.x, f.y);
+    const float2 h = unpack_half2(hi);
+    const float2 d = add2(x, F2(-h.x, -h.y)).get();
+    lo = pack_half2(d.x, d.y);
+}
+
+// Eight fp32 values -> one 16-byte chunk of the high and of the low tile.
+__device__ __forceinline__ void split_store(const F2 (&x)[4], uint8_t* hi_tile, uint8_t* lo_tile, uint32_t off) {
+    uint32_t h[4], l[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) split2(x[e], h[e], l[e]);
+    *reinterpret_cast<uint4*>(hi_tile + off) = make_uint4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<uint4*>(lo_tile + off) = make_uint4(l[0], l[1], l[2], l[3]);
+}
+// Eight fp16 values of an un-quantised row, times `f`.
+__device__ __forceinline__ void widen(const uint4& r, F2 f, F2 (&x)[4]) {
+    const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float2 h = unpack_half2(w[e]);
+        x[e] = mul2(F2(h.x, h.y), f);
+    }
+}
+
+// Eight codes of one word -> n * 16^p, p = 0 1 2 3 4 0 1 2: a nibble OR-ed under the exponent of 2^23 where it lies.
+__device__ __forceinline__ void unpack_f32(uint32_t w, F2 (&n)[4]) {
+    const uint32_t w5 = w >> 20;
+    float f[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(lop3_and_or(e < 5 ? w : w5, 0xFu << (4 * (e < 5 ? e : e - 5)), 0x4B000000u));
+#pragma unroll
+    for (int e = 0; e < 4; ++e) n[e] = add2(F2(f[2 * e], f[2 * e + 1]), F2(-8388608.0f, -8388608.0f));
+}
+__device__ __forceinline__ constexpr int nibble_shift(int d) { return 4 * ((d & 7) < 5 ? (d & 7) : (d & 7) - 5); }
+
+template <bool kOther>
+__global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Params P) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    Chunk256Smem& sm = *reinterpret_cast<Chunk256Smem*>(smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u));
+    const LayerView& L = P.L;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int mt = blockIdx.x, head = blockIdx.y, zs = blockIdx.z;
+    const int G = L.q_heads / L.kv_heads;
+    const int kv_total = *P.total_pos + 1;
+
+    if (warp == kMmaWarp) tc::tmem_alloc(&sm.tmem_base, kTmemCols);
+    if (tid == 0) {
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&sm.s_full[b], 1);
+            mbar_init(&sm.p_full[b], kSoftWarps);
+        }
+        mbar_init(&sm.k_full, kDqWarps);
+        mbar_init(&sm.v_full, kDqWarps);
+        mbar_init(&sm.o_done, 1);
+        mbar_init(&sm.drain, 1);
+        mbar_fence_init();
+        sm.abort_flag = 0;
+    }
+    // ---- Q: rows rotated, scaled, split; one warp per row, lane l holds dims l + 32 j, the loads of four rows in flight
+    constexpr int kQBatch = 4;
+    for (int r0 = warp; r0 < kM; r0 += kQBatch * (kMmaWarp + 1)) {
+        uint16_t raw[kQBatch][8];
+        int rp[kQBatch];
+#pragma unroll
+        for (int u = 0; u < kQBatch; ++u) {
+            const int r = r0 + u * (kMmaWarp + 1), R = mt * kM + r, tq = R / G, gq = R % G;
+            rp[u] = -1;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) raw[u][j] = 0;
+            if (r < kM && tq < P.T) {
+                const uint16_t* qrow = P.q + (static_cast<int64_t>(tq) * L.q_heads + head * G + gq) * D;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) raw[u][j] = qrow[lane + 32 * j];
+                rp[u] = P.pos[tq];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kQBatch; ++u) {
+            const int r = r0 + u * (kMmaWarp + 1);
+            if (r >= kM) break;
+            float v[8];
+            uint32_t top = 0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = L.dtype == KVB_DTYPE_BF16 ? in_to_f32<true>(raw[u][j]) : in_to_f32<false>(raw[u][j]);
+            hadamard_warp<D>(v, lane);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                v[j] *= P.scale_log2;
+                top = max(top, abs_bits(v[j]));
+            }
+            const int e = scale_exponent(__reduce_max_sync(0xffffffffu, top));
+            const float down = pow2i(-e);
+            if (lane == 0) {
+                sm.row_pos[r] = rp[u];
+                sm.row_unit[r] = pow2i(e);
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int d = lane + 32 * j;
+                const uint32_t off = (d >> 6) * kQBlock + r * 128 + ((((d & 63) >> 3) ^ (r & 7)) << 4) + (d & 7) * 2;
+                const float x = v[j] * down;
+                const __half h = __float2half_rn(x);
+                *reinterpret_cast<__half*>(sm.k[0] + off) = h;
+                *reinterpret_cast<__half*>(sm.q_lo + off) = __float2half_rn(x - __half2float(h));
+            }
+        }
+    }
+    fence_proxy_async();
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t tmem = sm.tmem_base;
+    if (warp < kSoftWarps) {  // the high part of Q moves to tensor memory: thread = row, two dims per column
+        const uint32_t lane_base = static_cast<uint32_t>(32 * warp) << 16;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            uint32_t w[32];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const uint4 x = *reinterpret_cast<const uint4*>(sm.k[0] + b * kQBlock + tid * 128 + ((c ^ (tid & 7)) << 4));
+                w[4 * c] = x.x; w[4 * c + 1] = x.y; w[4 * c + 2] = x.z; w[4 * c + 3] = x.w;
+            }
+            tc::tmem_st32(tmem + kColQ + lane_base + 32 * b, w);
+        }
+        tc::tmem_st_wait();
+    }
+    int max_pos = -1, min_pos = INT_MAX;
+#pragma unroll
+    for (int i = 0; i < kM / 32; ++i) {
+        const int p = sm.row_pos[lane + 32 * i];
+        max_pos = max(max_pos, p);
+        if (p >= 0) min_pos = min(min_pos, p);
+    }
+    max_pos = __reduce_max_sync(0xffffffffu, max_pos);
+    min_pos = __reduce_min_sync(0xffffffffu, min_pos);
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    // pages this CTA walks: those a row of the tile can see, cut into ksplit ranges
+    const int npages = max_pos < 0 ? 0 : min((kv_total + kN - 1) / kN, max_pos / kN + 1);
+    const int p0 = static_cast<int>(static_cast<int64_t>(npages) * zs / P.ksplit);
+    const int p1 = static_cast<int>(static_cast<int64_t>(npages) * (zs + 1) / P.ksplit);
+    const int n = p1 - p0;
+    const int sealed_pages = 2 * (kv_total / kTile);
+    bool failed = false;
+
+    if (warp >= kSoftWarps && warp < kMmaWarp) {
+        // =========================== de-quantise ===========================
+        const int dt = tid - 32 * kSoftWarps, dw = dt >> 5;        // dt: also the dim whose factors this thread fetches
+        const int quarter = dw & 3, key = 32 * (dw >> 2) + lane;   // 64 dims of one key of the page
+        const int s = quarter >> 1;
+        const uint32_t row_off = quarter * kKvBlock + key * 128;
+        const int32_t* tbl = L.table();
+        struct Meta {
+            __half ks, kz, vo, ko, sv, zp;
+            int32_t page;  // -1: unusable; the page is masked
+            bool sealed;
+        };
+        uint4 kcode[2], vcode[2];
+        int32_t pid_next = -1;  // page id of the page the next fetch asks for, looked up a page earlier
+        auto lookup = [&](int p) { pid_next = p < p1 && p < sealed_pages ? L.page_of(tbl, p) : -1; };
+        auto fetch_meta = [&](int p, Meta& m) {
+            m.sealed = p < sealed_pages;
+            m.page = pid_next;
+            m.ks = m.kz = m.vo = m.ko = m.sv = m.zp = __ushort_as_half(0);
+            if (p < p1 && m.page >= 0) {
+                const __half* ksp = L.k_scale + page_head_offset(10, L.kv_heads, m.page, head);
+                const __half* vsp = L.v_scale + page_head_offset(8, L.kv_heads, m.page, head);
+                m.ks = ksp[10 * (dt >> 2) + (dt & 3)];
+                m.kz = ksp[10 * (dt >> 2) + 4 + (dt & 3)];
+                m.ko = ksp[10 * key + 8 + s];
+                m.vo = vsp[8 * (dt >> 2) + (dt & 3)];
+                m.sv = vsp[8 * key + 4 + s];
+                m.zp = vsp[8 * key + 6 + s];
+            }
+        };
+        auto fetch_codes = [&](const uint8_t* plane, int32_t page, uint4 (&c)[2]) {
+            if (page >= 0) {
+                const uint4* src = reinterpret_cast<const uint4*>(plane + page_head_offset(128, L.kv_heads, page, head) + key * 128 + quarter * 32);
+                c[0] = src[0];
+                c[1] = src[1];
+            } else {
+                c[0] = c[1] = make_uint4(0u, 0u, 0u, 0u);
+            }
+        };
+        Meta cur, nxt;
+        if (n > 0) {
+            lookup(p0);
+            fetch_meta(p0, nxt);
+            fetch_codes(L.k_code, nxt.page, kcode);
+            fetch_codes(L.v_code, nxt.page, vcode);
+            lookup(p0 + 1);
+        }
+        int v_run = INT_MIN;  // exponent of V so far
+        // what V(i-1) needs: its page is de-quantised a step after K of the same page
+        struct {
+            float sv, zp, unit;
+            const __half* row;  // open tile: the un-quantised row of this thread's key (null: de-quantise)
+            bool live;
+        } vprev{};
+        for (int i = 0; i <= n; ++i) {
+            const int p = p0 + i, par = i & 1, slot = i & (kSlotsMeta - 1);
+            auto vnow = vprev;
+            if (i < n) {
+                cur = nxt;
+                const __half* krow = nullptr;  // open tile: this key's un-quantised row
+                float ko = __half2float(cur.ko);
+                vnow.sv = __half2float(cur.sv);
+                vnow.zp = __half2float(cur.zp);
+                vnow.row = nullptr;
+                vnow.live = true;
+                // ---- per-dim tables of the page, and the largest magnitudes that decide its scales
+                {
+                    const float ks = __half2float(cur.ks), kz = __half2float(cur.kz), vo = __half2float(cur.vo);
+                    uint32_t kb = max(abs_bits(kz), abs_bits(fmaf(15.0f, ks, kz))), vb = max(abs_bits(vnow.zp), abs_bits(fmaf(15.0f, vnow.sv, vnow.zp)));
+                    uint32_t ob = abs_bits(vo);
+                    if (!cur.sealed) {
+                        const int tile = kv_total / kTile, first = (p & 1) * kPage + key;
+                        krow = L.stage_row(0, tile & 1, head, first) + 64 * quarter;
+                        vnow.row = L.stage_row(1, tile & 1, head, first) + 64 * quarter;
+                        vnow.live = p * kN + key < kv_total;
+                        ob = __float_as_uint(1.0f);
+                        if (vnow.live) {
+#pragma unroll
+                            for (int c = 0; c < 8; ++c) {
+                                const uint4 a = reinterpret_cast<const uint4*>(vnow.row)[c], b = reinterpret_cast<const uint4*>(krow)[c];
+                                const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, wb[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) {
+                                    const float2 fa = unpack_half2(wa[e]), fb = unpack_half2(wb[e]);
+                                    vb = max(vb, max(abs_bits(fa.x), abs_bits(fa.y)));
+                                    kb = max(kb, max(abs_bits(fb.x), abs_bits(fb.y)));
+                                }
+                            }
+                        }
+                        ko = 1.0f;
+                    }
+                    const bool bad_key = vb >= 0x7F800000u;
+                    if (bad_key) { vnow.sv = vnow.zp = 0.0f; vb = 0u; vnow.live = false; }
+                    const uint32_t bad = __ballot_sync(0xffffffffu, bad_key);
+                    sm.ks[par][dt] = ks * pow2i(-nibble_shift(dt));
+                    sm.kz[par][dt] = kz;
+                    if constexpr (kOther) sm.vo[slot][dt] = ob >= 0x7F800000u ? 0.0f : vo;
+                    const uint32_t mk = __reduce_max_sync(0xffffffffu, kb), mo = __reduce_max_sync(0xffffffffu, abs_bits(ko));
+                    const uint32_t mov = __reduce_max_sync(0xffffffffu, ob), mv = __reduce_max_sync(0xffffffffu, vb);
+                    if (lane == 0) {
+                        *reinterpret_cast<uint4*>(sm.red[par][dw]) = make_uint4(mk, mo, mov, mv);
+                        sm.poison[slot][dw] = bad;
+                    }
+                }
+                if (named_barrier_or(1, kDqThreads, failed)) { failed = true; break; }
+                uint32_t mk = 0, mo = 0, mov = 0, mv = 0;
+#pragma unroll
+                for (int w = 0; w < kDqWarps; ++w) {
+                    const uint4 r = *reinterpret_cast<const uint4*>(sm.red[par][w]);
+                    mk = max(mk, r.x); mo = max(mo, r.y); mov = max(mov, r.z); mv = max(mv, r.w);
+                }
+                const int k_exp = scale_exponent(__float_as_uint(__uint_as_float(mk) * __uint_as_float(mo)));
+                const float vtop = __uint_as_float(mv) * (mov >= 0x7F800000u ? 1.0f : __uint_as_float(mov));
+                if (vtop > 0.0f) v_run = max(v_run, scale_exponent(__float_as_uint(vtop)));
+                const int v_exp = v_run == INT_MIN ? 0 : v_run;
+                vnow.unit = pow2i(-v_exp);
+                if (dt == 0) {
+                    sm.k_unit[slot] = pow2i(k_exp);
+                    sm.v_exp[slot] = v_exp;
+                    sm.bad_page[slot] = cur.sealed && cur.page < 0;
+                }
+                if (mov >= 0x7F800000u && lane == 0) sm.poison[slot][dw] = 0xffffffffu;  // a dim of every key
+                // ---- K(i): the buffer is free once S(i-1) has completed
+                if (i > 0 && !chunk_wait(&sm.s_full[(i - 1) & 1], ((i - 1) >> 1) & 1, &sm.abort_flag)) { failed = true; continue; }
+                const float kf = ko * pow2i(-k_exp);
+                const F2 kf2(kf, kf);
+                if (cur.sealed) {
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        const uint4 cc = kcode[c >> 2];
+                        const ulonglong2* st = reinterpret_cast<const ulonglong2*>(&sm.ks[par][64 * quarter + 8 * c]);
+                        const ulonglong2* zt = reinterpret_cast<const ulonglong2*>(&sm.kz[par][64 * quarter + 8 * c]);
+                        const ulonglong2 s0 = st[0], s1 = st[1], z0 = zt[0], z1 = zt[1];
+                        F2 x[4];
+                        unpack_f32((c & 3) == 0 ? cc.x : (c & 3) == 1 ? cc.y : (c & 3) == 2 ? cc.z : cc.w, x);
+                        x[0] = mul2(fma2(x[0], F2(s0.x), F2(z0.x)), kf2);
+                        x[1] = mul2(fma2(x[1], F2(s0.y), F2(z0.y)), kf2);
+                        x[2] = mul2(fma2(x[2], F2(s1.x), F2(z1.x)), kf2);
+                        x[3] = mul2(fma2(x[3], F2(s1.y), F2(z1.y)), kf2);
+                        split_store(x, sm.k[0], sm.k[1], row_off + ((c ^ (key & 7)) << 4));
+                    }
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        F2 x[4];
+                        widen(p * kN + key < kv_total ? reinterpret_cast<const uint4*>(krow)[c] : make_uint4(0u, 0u, 0u, 0u), kf2, x);
+                        split_store(x, sm.k[0], sm.k[1], row_off + ((c ^ (key & 7)) << 4));
+                    }
+                }
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sm.k_full);
+                fetch_meta(p + 1, nxt);
+                fetch_codes(L.k_code, nxt.page, kcode);
+                lookup(p + 2);
+            }
+            if (i > 0) {
+                // ---- V(i-1): the buffer is free once P V(i-2) has completed
+                const int vslot = (i - 1) & (kSlotsMeta - 1);
+                if (i > 1 && !chunk_wait(&sm.o_done, i & 1, &sm.abort_flag)) { failed = true; continue; }
+                if (vprev.row == nullptr) {
+                    const float z = vprev.zp * vprev.unit, s0 = vprev.sv * vprev.unit, s1 = s0 * 0.0625f, s2 = s1 * 0.0625f, s3 = s2 * 0.0625f, s4 = s3 * 0.0625f;
+                    const F2 z2(z, z), sc[4] = {F2(s0, s1), F2(s2, s3), F2(s4, s0), F2(s1, s2)};
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        const uint4 cc = vcode[c >> 2];
+                        F2 x[4];
+                        unpack_f32((c & 3) == 0 ? cc.x : (c & 3) == 1 ? cc.y : (c & 3) == 2 ? cc.z : cc.w, x);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) x[e] = fma2(x[e], sc[e], z2);
+                        if constexpr (kOther) {
+                            const ulonglong2* ot = reinterpret_cast<const ulonglong2*>(&sm.vo[vslot][64 * quarter + 8 * c]);
+                            const ulonglong2 o0 = ot[0], o1 = ot[1];
+                            x[0] = mul2(x[0], F2(o0.x));
+                            x[1] = mul2(x[1], F2(o0.y));
+                            x[2] = mul2(x[2], F2(o1.x));
+                            x[3] = mul2(x[3], F2(o1.y));
+                        }
+                        split_store(x, sm.v[0], sm.v[1], row_off + ((c ^ (key & 7)) << 4));
+                    }
+                } else {
+                    const F2 unit2(vprev.unit, vprev.unit);
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        F2 x[4];
+                        widen(vprev.live ? reinterpret_cast<const uint4*>(vprev.row)[c] : make_uint4(0u, 0u, 0u, 0u), unit2, x);
+                        split_store(x, sm.v[0], sm.v[1], row_off + ((c ^ (key & 7)) << 4));
+                    }
+                }
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sm.v_full);
+                if (i < n) fetch_codes(L.v_code, cur.page, vcode);
+            }
+            vprev = vnow;
+        }
+    } else if (warp == kMmaWarp) {
+        // =========================== MMA issue ===========================
+        constexpr uint32_t idesc_qk = tc::idesc_f16(kM, kN, false, false), idesc_pv = tc::idesc_f16(kM, D, false, true);
+        const uint32_t q_addr = smem_u32(sm.q_lo), k_hi = smem_u32(sm.k[0]), k_lo = smem_u32(sm.k[1]), v_hi = smem_u32(sm.v[0]), v_lo = smem_u32(sm.v[1]);
+        for (int i = 0; i <= n && !failed; ++i) {
+            if (i < n) {
+                // S(i) goes where P(i-2) was: P V(i-2) has to be over
+                if (!chunk_wait(&sm.k_full, i & 1, &sm.abort_flag) || (i > 1 && !chunk_wait(&sm.o_done, i & 1, &sm.abort_flag))) { failed = true; break; }
+                tc::fence_after_sync();
+                const uint32_t s = tmem + 64 * (i & 1);
+#pragma unroll
+                for (int kk = 0; kk < 16; ++kk) {
+                    const uint32_t ko = (kk >> 2) * kKvBlock + (kk & 3) * 32;
+                    tc::mma_f16_ss(s, tc::smem_desc(q_addr + (kk >> 2) * kQBlock + (kk & 3) * 32, 16, 1024), tc::smem_desc(k_hi + ko, 16, 1024), idesc_qk, kk > 0);
+                }
+#pragma unroll
+                for (int kk = 0; kk < 16; ++kk)
+                    tc::mma_f16_ts(s, tmem + kColQ + 8 * kk, tc::smem_desc(k_lo + (kk >> 2) * kKvBlock + (kk & 3) * 32, 16, 1024), idesc_qk, true);
+#pragma unroll
+                for (int kk = 0; kk < 16; ++kk)
+                    tc::mma_f16_ts(s, tmem + kColQ + 8 * kk, tc::smem_desc(k_hi + (kk >> 2) * kKvBlock + (kk & 3) * 32, 16, 1024), idesc_qk, true);
+                tc::commit(&sm.s_full[i & 1]);
+            }
+            if (i > 0) {
+                const int j = i - 1;
+                if (!chunk_wait(&sm.p_full[j & 1], (j >> 1) & 1, &sm.abort_flag) || !chunk_wait(&sm.v_full, j & 1, &sm.abort_flag)) { failed = true; break; }
+                tc::fence_after_sync();
+                const uint32_t p = tmem + 64 * (j & 1);
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk)
+                    tc::mma_f16_ts(tmem + kColO, p + 32 + 8 * kk, tc::smem_desc(v_hi + kk * 2048, kKvBlock, 1024), idesc_pv, j > 0 || kk > 0);
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk)
+                    tc::mma_f16_ts(tmem + kColO, p + 8 * kk, tc::smem_desc(v_lo + kk * 2048, kKvBlock, 1024), idesc_pv, true);
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk)
+                    tc::mma_f16_ts(tmem + kColO, p + 8 * kk, tc::smem_desc(v_hi + kk * 2048, kKvBlock, 1024), idesc_pv, true);
+                tc::commit(&sm.o_done);
+            }
+        }
+        if (failed) {  // nothing of this CTA may still run when its tensor memory is given back
+            tc::commit(&sm.drain);
+            mbar_wait_bounded(&sm.drain, 0);
+        }
+    } else {
+        // =========================== softmax ===========================
+        const uint32_t lane_base = static_cast<uint32_t>(32 * warp) << 16;
+        const int my_pos = sm.row_pos[tid];
+        const float row_unit = sm.row_unit[tid];
+        const bool warp_has_rows = __any_sync(0xffffffffu, my_pos >= 0);
+        float m_run = -INFINITY, l_run = 0.0f;
+        int v_exp = 0;
+        bool poisoned = false;
+        for (int i = 0; i < n; ++i) {
+            const int base = (p0 + i) * kN, slot = i & (kSlotsMeta - 1);
+            if (!chunk_wait(&sm.s_full[i & 1], (i >> 1) & 1, &sm.abort_flag)) { failed = true; break; }
+            tc::fence_after_sync();
+            if (warp_has_rows) {
+                const uint32_t ts = tmem + 64 * (i & 1) + lane_base;
+                float s[kN];
+                {
+                    uint32_t r0[32], r1[32];
+                    tc::tmem_ld32(ts, r0);
+                    tc::tmem_ld32(ts + 32, r1);
+                    tc::tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        s[j] = __uint_as_float(r0[j]);
+                        s[32 + j] = __uint_as_float(r1[j]);
+                    }
+                }
+                const float unit = fmaxf(row_unit * sm.k_unit[slot], 1.175494351e-38f);  // > 0: a masked key stays at -inf
+                const int v_new = sm.v_exp[slot];
+                const bool bad_page = sm.bad_page[slot] != 0;
+                if (base + kN - 1 > min_pos || base + kN > kv_total || bad_page) {
+#pragma unroll
+                    for (int j = 0; j < kN; ++j)
+                        if (base + j > my_pos || base + j >= kv_total || bad_page) s[j] = -INFINITY;
+                }
+                {  // a key whose V is not finite was left out of the product: rows that see it end as NaN
+                    const uint4 b0 = *reinterpret_cast<const uint4*>(&sm.poison[slot][0]), b1 = *reinterpret_cast<const uint4*>(&sm.poison[slot][4]);
+                    const uint32_t lo = b0.x | b0.y | b0.z | b0.w, hi = b1.x | b1.y | b1.z | b1.w;
+                    if ((lo | hi) != 0u && !bad_page) {
+                        for (int j = 0; j < kN; ++j)
+                            if (((j < 32 ? lo : hi) >> (j & 31) & 1u) && base + j <= my_pos && base + j < kv_total) poisoned = true;
+                    }
+                }
+                float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+                for (int j = 0; j < kN; ++j) mx4[j & 3] = fmaxf(mx4[j & 3], s[j]);
+                const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * unit;
+                constexpr float kLazy = 8.0f;  // the reference point moves only when the maximum has grown by more than 2^kLazy
+                const bool grown = mx > m_run + kLazy || (m_run == -INFINITY && mx > -INFINITY);
+                const float m_new = grown ? mx : m_run;
+                const float m_use = m_new == -INFINITY ? 0.0f : m_new;
+                float alpha = grown ? fast_exp2(m_run - m_use) : 1.0f;
+                m_run = m_new;
+                l_run *= alpha;
+                bool moved = grown;
+                if (v_new != v_exp) {  // the unit of V and O has grown: the sum so far is rescaled (powers of two: exact)
+                    alpha *= pow2i(max(v_exp - v_new, -126));
+                    v_exp = v_new;
+                    moved = true;
+                }
+                const float off = kPBoost - m_use;
+                const F2 unit2(unit, unit), off2(off, off);
+                F2 sum[2] = {F2(0.0f, 0.0f), F2(0.0f, 0.0f)};
+                uint32_t ph[32], pl[32];
+#pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                    const float2 e = fma2(F2(s[2 * j], s[2 * j + 1]), unit2, off2).get();
+                    const F2 x(fast_exp2(e.x), fast_exp2(e.y));
+                    sum[j & 1] = add2(sum[j & 1], x);
+                    split2(x, ph[j], pl[j]);
+                }
+                tc::tmem_st32(ts, ph);
+                tc::tmem_st32(ts + 32, pl);
+                const float2 sum2 = add2(sum[0], sum[1]).get();
+                l_run += sum2.x + sum2.y;
+                if (i > 0 && __any_sync(0xffffffffu, moved)) {
+                    if (!chunk_wait(&sm.o_done, (i - 1) & 1, &sm.abort_flag)) { failed = true; break; }
+                    tc::fence_after_sync();
+#pragma unroll 1
+                    for (int c = 0; c < D / 32; ++c) {
+                        uint32_t r[32];
+                        tc::tmem_ld32(tmem + kColO + lane_base + 32 * c, r);
+                        tc::tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * alpha);
+                        tc::tmem_st32(tmem + kColO + lane_base + 32 * c, r);
+                    }
+                }
+                tc::tmem_st_wait();
+            }
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.p_full[i & 1]);
+        }
+        // ---- partial of this (row tile, page range): m (log2 units), l, o
+        // (P V(n-2) first: a parity wait must not be more than one phase ahead of its barrier)
+        if (n > 1 && !failed && !chunk_wait(&sm.o_done, n & 1, &sm.abort_flag)) failed = true;
+        if (n > 0 && !failed && !chunk_wait(&sm.o_done, (n - 1) & 1, &sm.abort_flag)) failed = true;
+        tc::fence_after_sync();
+        const bool have = n > 0 && !failed;
+        const int64_t idx = ((static_cast<int64_t>(head) * P.mtiles + mt) * P.ksplit + zs) * kM + tid;
+        if (my_pos >= 0) {
+            P.ws_m[idx] = have && m_run != -INFINITY ? m_run - kPBoost : -INFINITY;
+            P.ws_l[idx] = have ? l_run : 0.0f;
+        }
+        const float unit = poisoned ? __uint_as_float(0x7FC00000u) : pow2i(v_exp);
+        float* orow = P.ws_o + idx * D;
+#pragma unroll 1
+        for (int c = 0; c < D / 32; ++c) {
+            if (!warp_has_rows) break;
+            uint32_t r[32];
+            if (have) {
+                tc::tmem_ld32(tmem + kColO + lane_base + 32 * c, r);
+                tc::tmem_ld_wait();
+            }
+            if (my_pos < 0) continue;
+#pragma unroll
+            for (int j = 0; j < 32; j += 4)
+                *reinterpret_cast<float4*>(orow + 32 * c + j) =
+                    have ? make_float4(__uint_as_float(r[j]) * unit, __uint_as_float(r[j + 1]) * unit, __uint_as_float(r[j + 2]) * unit, __uint_as_float(r[j + 3]) * unit)
+                         : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+    if (failed && lane == 0) L.flag(KVB_ERR_WAIT_TIMEOUT);
+    tc::fence_before_sync();
+    __syncthreads();
+    if (warp == kMmaWarp) tc::tmem_dealloc(tmem, kTmemCols);
+}
+
+// Row tiles and key ranges of a call.  One CTA per SM; a CTA costs its pages plus about six pages' worth of set-up and
+// epilogue, and every further range a partial per row: the number of ranges (at most four waves' worth, at least four
+// pages each) with the lowest (waves x CTA) is taken.
+void chunk256_shape(int kv_len_max, int kv_heads, int q_heads, int tokens, int* mtiles, int* ksplit) {
+    const int rows = tokens * (q_heads / kv_heads), sms = device_sm_count(), pages = (kv_len_max + kN - 1) / kN;
+    *mtiles = (rows + kM - 1) / kM;
+    const int ctas = *mtiles * kv_heads;
+    int best = 1;
+    int64_t best_cost = INT64_MAX;
+    for (int ks = 1; ks <= kMaxKeyRanges && (ks == 1 || (4 * ks <= pages && ctas * ks <= 4 * sms)); ++ks) {
+        const int64_t cost = static_cast<int64_t>((ctas * ks + sms - 1) / sms) * (6 + (pages + ks - 1) / ks);
+        if (cost < best_cost) { best_cost = cost; best = ks; }
+    }
+    *ksplit = best;
+}
+
+}  // namespace
+
+size_t chunk256_workspace_bytes(int kv_len_max, int kv_heads, int q_heads, int tokens) {
+    int mtiles, ksplit;
+    chunk256_shape(kv_len_max, kv_heads, q_heads, tokens, &mtiles, &ksplit);
+    return static_cast<size_t>(kv_heads) * mtiles * ksplit * kM * (D + 2) * sizeof(float);
+}
+
+// Chunk attention of `tokens` rows that are already appended, over a head_dim-256 cache.
+int launch_chunk_attention_256(const kvb_layer* layer, const void* q, const int32_t* positions_dev, int tokens, float scale,
+                               int kv_len_max, void* workspace, void* out, cudaStream_t s, float* part_m, float* part_l, float* part_o) {
+    Chunk256Params P;
+    P.L = make_view(*layer);
+    P.q = static_cast<const uint16_t*>(q);
+    P.pos = positions_dev;
+    P.total_pos = positions_dev + (tokens - 1);
+    P.T = tokens;
+    chunk256_shape(kv_len_max, layer->kv_heads, layer->q_heads, tokens, &P.mtiles, &P.ksplit);
+    P.scale_log2 = scale * 1.4426950408889634f;
+    const size_t rows = static_cast<size_t>(layer->kv_heads) * P.mtiles * P.ksplit * kM;
+    P.ws_m = static_cast<float*>(workspace);
+    P.ws_l = P.ws_m + rows;
+    P.ws_o = P.ws_l + rows;
+    const int smem = static_cast<int>(sizeof(Chunk256Smem)) + 1024;  // room to align the tiles to 1024 bytes
+    static unsigned long long opted = 0;
+    if (first_call_on_device(opted)) {
+        KVB_CUDA_OK(cudaFuncSetAttribute(chunk256_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        KVB_CUDA_OK(cudaFuncSetAttribute(chunk256_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    }
+    const dim3 grid(P.mtiles, layer->kv_heads, P.ksplit);
+    if (layer->sinkhorn_iters > 0) chunk256_kernel<true><<<grid, kThreads, smem, s>>>(P);
+    else chunk256_kernel<false><<<grid, kThreads, smem, s>>>(P);
+    KVB_CUDA_OK(cudaGetLastError());
+    return launch_chunk_merge<D>(P.ws_m, P.ws_l, P.ws_o, tokens, layer->q_heads, layer->kv_heads, P.mtiles, P.ksplit, layer->dtype, out,
+                                 part_m, part_l, part_o, s);
+}
+
+}  // namespace kvb

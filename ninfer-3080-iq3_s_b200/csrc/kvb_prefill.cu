@@ -20,6 +20,7 @@
 // through the normal exit (TMEM is freed).
 #include <climits>
 
+#include "kvb_chunk_merge.cuh"
 #include "kvb_common.cuh"
 #include "kvb_tcgen05.cuh"
 
@@ -62,8 +63,6 @@ struct __align__(1024) PrefillSmem {
 __device__ __forceinline__ uint32_t tile_off(int row, int col) {
     return (col >> 6) * 16384 + (row >> 3) * 1024 + (row & 7) * 128 + ((((col & 63) >> 3) ^ (row & 7)) << 4) + (col & 7) * 2;
 }
-// Position of dim d inside its group of eight: order 0,4,1,5,2,6,3,7.
-__device__ __forceinline__ int dim_slot(int d) { return (d & ~7) | ((d & 3) << 1) | ((d >> 2) & 1); }
 
 __device__ __forceinline__ uint32_t hfma2_u32(uint32_t a, uint32_t b, uint32_t c) {
     uint32_t r;
@@ -723,83 +722,6 @@ __global__ void __launch_bounds__(kThreads, 2) verify_kernel(const PrefillParams
     if (warp == 0) tc::tmem_dealloc(sm.tmem_base, kTmemCols);
 }
 
-// Merge the key ranges of one query row, normalise, undo the tile dim order, rotate back, store -- or, for a cache
-// that holds only a range of the sequence, export the merged partial instead (m in natural-log units, l, o in the
-// rotated domain and natural dim order, not normalised).
-// One CTA of 8 warps per row: warp w takes ranges w, w+8, ..; lane l owns dims l + 32 j.  The loop is pure load
-// latency, so it is unrolled to keep several ranges in flight; the warp sums meet in shared memory.
-template <int kPer>  // ranges per warp: ksplit <= 8 kPer
-__global__ void __launch_bounds__(256) prefill_merge_kernel(const float* __restrict__ ws_m, const float* __restrict__ ws_l,
-                                                            const float* __restrict__ ws_o, int T, int q_heads, int kv_heads,
-                                                            int mtiles, int ksplit, int dtype, uint16_t* __restrict__ out,
-                                                            float* __restrict__ part_m, float* __restrict__ part_l,
-                                                            float* __restrict__ part_o) {
-    __shared__ float so[8][D];
-    __shared__ float sl[8], smx[8];
-    const int row = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int G = q_heads / kv_heads, tq = row / q_heads, qh = row % q_heads, head = qh / G, R = tq * G + qh % G;
-    const int64_t base = ((static_cast<int64_t>(head) * mtiles + R / kM) * ksplit) * kM + R % kM;
-    // Warp w merges ranges w, w + 8, .. (kPer of them; at most 16: ksplit <= 128) relative to their own maximum, every
-    // load issued before the first use: one trip to memory for the whole row; the eight warp results meet in shared
-    // memory.  kPer is a template parameter so that a chunk (a few ranges, tens of thousands of rows) keeps the
-    // registers low and the occupancy high.
-    float pm[kPer], pl[kPer], po[kPer][4];
-#pragma unroll
-    for (int k = 0; k < kPer; ++k) {
-        const int z = warp + 8 * k;
-        const bool on = z < ksplit;
-        const int64_t i = base + static_cast<int64_t>(on ? z : 0) * kM;
-        pm[k] = on ? ws_m[i] : -INFINITY;
-        pl[k] = on ? ws_l[i] : 0.0f;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) po[k][j] = on ? ws_o[i * D + dim_slot(lane + 32 * j)] : 0.0f;
-    }
-    float mw = -INFINITY;
-#pragma unroll
-    for (int k = 0; k < kPer; ++k) mw = fmaxf(mw, pm[k]);
-    float l = 0.0f, o[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    if (mw != -INFINITY) {
-#pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-            const float w = fast_exp2(pm[k] - mw);  // 0 for a range that is not there
-            l += w * pl[k];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) o[j] += w * po[k][j];
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) so[warp][lane + 32 * j] = o[j];
-    if (lane == 0) { sl[warp] = l; smx[warp] = mw; }
-    __syncthreads();
-    if (warp != 0) return;
-    float m = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) m = fmaxf(m, smx[w]);
-    l = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) o[j] = 0.0f;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) {
-        const float wt = smx[w] == -INFINITY ? 0.0f : fast_exp2(smx[w] - m);
-        l += wt * sl[w];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) o[j] += wt * so[w][lane + 32 * j];
-    }
-    if (part_m != nullptr) {
-        if (lane == 0) { part_m[row] = m * 0.6931471805599453f; part_l[row] = l; }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) part_o[static_cast<int64_t>(row) * D + lane + 32 * j] = o[j];
-        return;
-    }
-    const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) o[j] *= inv;
-    hadamard_warp<D>(o, lane);
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-        out[static_cast<int64_t>(row) * D + lane + 32 * j] = dtype == KVB_DTYPE_BF16 ? f32_to_out<true>(o[j]) : f32_to_out<false>(o[j]);
-}
-
 int prefill_sm_count() { return device_sm_count(); }
 
 void prefill_shape(int kv_len_max, int kv_heads, int q_heads, int tokens, int* mtiles, int* ksplit) {
@@ -819,11 +741,10 @@ void prefill_shape(int kv_len_max, int kv_heads, int q_heads, int tokens, int* m
 }  // namespace kvb
 
 namespace kvb {
-// kvb_attn_general.cu: head_dim 256 and caches written with Sinkhorn iterations > 0
-size_t general_workspace_bytes(int kv_len_max, int q_heads, int head_dim, int rows);
-int launch_general_attention(const kvb_layer* layer, const void* q, const int32_t* pos_dev, const int32_t* total_pos_dev, int T,
-                             float scale, int kv_len_max, int key_begin, int key_end, void* workspace, void* out, float* part_m,
-                             float* part_l, float* part_o, cudaStream_t stream);
+// kvb_chunk256.cu: the same for head_dim 256
+size_t chunk256_workspace_bytes(int kv_len_max, int kv_heads, int q_heads, int tokens);
+int launch_chunk_attention_256(const kvb_layer* layer, const void* q, const int32_t* positions_dev, int tokens, float scale,
+                               int kv_len_max, void* workspace, void* out, cudaStream_t s, float* part_m, float* part_l, float* part_o);
 }  // namespace kvb
 
 extern "C" size_t kvb_prefill_workspace_bytes(int kv_len_max, int kv_heads, int q_heads, int head_dim, int tokens) {
@@ -831,8 +752,8 @@ extern "C" size_t kvb_prefill_workspace_bytes(int kv_len_max, int kv_heads, int 
     int mtiles, ksplit;
     kvb::prefill_shape(kv_len_max, kv_heads, q_heads, tokens, &mtiles, &ksplit);
     const size_t tuned = static_cast<size_t>(kv_heads) * mtiles * ksplit * kvb::kM * (head_dim + 2) * sizeof(float);
-    const size_t general = kvb::general_workspace_bytes(kv_len_max, q_heads, head_dim, tokens);  // head_dim 256, Sinkhorn caches
-    return tuned > general ? tuned : general;
+    const size_t wide = head_dim == 256 ? kvb::chunk256_workspace_bytes(kv_len_max, kv_heads, q_heads, tokens) : 0;
+    return tuned > wide ? tuned : wide;
 }
 
 namespace kvb {
@@ -877,13 +798,8 @@ int launch_chunk_attention(const kvb_layer* layer, const void* q, const int32_t*
         prefill_kernel<false><<<dim3(P.mtiles, layer->kv_heads, P.ksplit), kThreads, smem, s>>>(P);
     }
     KVB_CUDA_OK(cudaGetLastError());
-    const int total_rows = tokens * layer->q_heads;
-    auto merge = P.ksplit <= 16 ? prefill_merge_kernel<2> : P.ksplit <= 32 ? prefill_merge_kernel<4> : P.ksplit <= 64 ? prefill_merge_kernel<8>
-                                                                                                                      : prefill_merge_kernel<16>;
-    merge<<<total_rows, 256, 0, s>>>(P.ws_m, P.ws_l, P.ws_o, tokens, layer->q_heads, layer->kv_heads, P.mtiles, P.ksplit, layer->dtype,
-                                     static_cast<uint16_t*>(out), part_m, part_l, part_o);
-    KVB_CUDA_OK(cudaGetLastError());
-    return KVB_OK;
+    return launch_chunk_merge<D>(P.ws_m, P.ws_l, P.ws_o, tokens, layer->q_heads, layer->kv_heads, P.mtiles, P.ksplit, layer->dtype, out,
+                                 part_m, part_l, part_o, s);
 }
 }  // namespace kvb
 
@@ -897,9 +813,9 @@ extern "C" int kvb_attn_prefill(const kvb_layer* layer, const void* q, const voi
     if (layer->stage == nullptr) return fail(KVB_EINVAL, "kvb_attn_prefill: layer has no stage buffer");
     if (tokens > 65535) return fail(KVB_ERANGE, "kvb_attn_prefill: %d tokens in one chunk (at most 65535)", tokens);
     if (int st = kvb_append(layer, k, v, positions_dev, tokens, stream)) return st;
-    if (layer->head_dim != 128)  // two slices per key: general kernel, same semantics
-        return launch_general_attention(layer, q, positions_dev, positions_dev + (tokens - 1), tokens, scale, kv_len_max, 0, INT_MAX,
-                                        workspace, out, nullptr, nullptr, nullptr, static_cast<cudaStream_t>(stream));
+    if (layer->head_dim != 128)
+        return launch_chunk_attention_256(layer, q, positions_dev, tokens, scale, kv_len_max, workspace, out, static_cast<cudaStream_t>(stream),
+                                          nullptr, nullptr, nullptr);
     return launch_chunk_attention(layer, q, positions_dev, tokens, scale, kv_len_max, workspace, out, static_cast<cudaStream_t>(stream),
                                   nullptr, nullptr, nullptr, nullptr);
 }

@@ -91,6 +91,20 @@ __device__ __forceinline__ void named_barrier_sync(int id, int threads) {
     asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// The same barrier, and one verdict for all its threads: whether any of them came with `mine` set.
+__device__ __forceinline__ bool named_barrier_or(int id, int threads, bool mine) {
+    uint32_t any;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %3, 0;\n\t"
+        "barrier.cta.red.or.pred q, %1, %2, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(any)
+        : "r"(id), "r"(threads), "r"(static_cast<uint32_t>(mine))
+        : "memory");
+    return any != 0;
+}
+
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
     uint32_t r;
     asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));

@@ -49,3 +49,44 @@ def test_decode_and_verify(H, QH, T, iters):
         ok, msg = attn_close(out.float().cpu().numpy(), want, MAX_ABS, REL_L2)
         assert ok, "verify of %d rows: %s" % (width, msg)
     assert tw.gpu.errors() == 0
+
+
+# tokens in the cache before the chunk, tokens of the chunk: one row tile and several (128 rows of G heads), ragged ends of
+# pages and tiles, an open tile, an empty prefix, several key ranges
+@pytest.mark.parametrize("H,QH,ctx,T,iters", [(4, 24, 0, 9, 0), (4, 24, 0, 64, 16), (2, 16, 0, 65, 0), (4, 24, 127, 21, 16), (4, 24, 128, 22, 0), (1, 7, 191, 300, 16),
+                                              (8, 8, 1000, 129, 0), (4, 24, 3000, 40, 16), (4, 4, 4096, 128, 0)])
+def test_chunk(H, QH, ctx, T, iters):
+    """The tcgen05 chunk kernel: operands of 22 significant bits and fp32 sums leave the rounding of the output."""
+    import torch
+
+    D, scale = 256, 1.0 / 16.0
+    tw = Twin(D=D, H=H, QH=QH, capacity_tokens=ctx + T, seed=ctx + T, iters=iters)
+    k, v = orc.synth_kv(T, ctx + T, H, D, 1), orc.synth_kv(T, ctx + T, H, D, 2)
+    q = orc.synth_q(T, T, QH, D)
+    gk, gv, gq = (torch.from_numpy(x).to(tw.dev) for x in (k, v, q))
+    at = torch.arange(ctx + T, dtype=torch.int32, device=tw.dev)
+    if ctx:
+        tw.gpu.append(gk[:ctx], gv[:ctx], at[:ctx])
+    out = tw.gpu.attn_prefill(gq, gk[ctx:], gv[ctx:], at[ctx:], scale, ctx + T)
+    want = cpu_twin_of(tw.gpu).attention(q, np.arange(ctx, ctx + T, dtype=np.int32), scale, QH, threads=4, kv_total=ctx + T)
+    assert tw.gpu.errors() == 0
+    ok, msg = attn_close(out.float().cpu().numpy(), want, MAX_ABS, REL_L2)
+    assert ok, msg
+
+
+def test_chunk_far_from_one():
+    """Scales of 2^-10 in K, 2^11 in V and one row of the open tile 2^4 above the rest: the split operands follow them."""
+    import torch
+
+    D, H, QH, T, scale = 256, 2, 8, 300, 16.0
+    tw = Twin(D=D, H=H, QH=QH, capacity_tokens=T, seed=3)
+    k = (orc.synth_kv(1, T, H, D, 1).astype(np.float32) * 2.0 ** -10).astype(np.float16)
+    v = (np.clip(orc.synth_kv(1, T, H, D, 2).astype(np.float32), -2, 2) * 2.0 ** 9).astype(np.float16)
+    v[T - 7] *= 4
+    q = orc.synth_q(1, T, QH, D)
+    at = torch.arange(T, dtype=torch.int32, device=tw.dev)
+    out = tw.gpu.attn_prefill(*(torch.from_numpy(x).to(tw.dev) for x in (q, k, v)), at, scale, T)
+    want = cpu_twin_of(tw.gpu).attention(q, np.arange(T, dtype=np.int32), scale, QH, threads=4, kv_total=T)
+    assert tw.gpu.errors() == 0
+    ok, msg = attn_close(out.float().cpu().numpy(), want, MAX_ABS, REL_L2)
+    assert ok, msg
