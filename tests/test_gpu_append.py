@@ -135,3 +135,18 @@ def test_bad_inputs_set_the_error_word_and_do_not_fault():
     torch.cuda.synchronize()
     assert tw.gpu.errors() & capi.ERR_PAGE_RANGE
     assert not tw.gpu.k_code.any()
+
+
+@pytest.mark.parametrize("D", [128, 256])
+@pytest.mark.parametrize("first,n", [(1, 255), (1, 256), (60, 200), (127, 258), (60, 400), (100, 1000), (128, 300)])
+def test_stage_of_the_last_two_tiles(D, first, n):
+    """One append over three tiles and more that begins inside a tile (or, last case, at its edge): codes and scales of every
+    tile, and the stage rows of the last two tiles, whichever of them shares the slot the first tile is read from."""
+    H, T = 2, first + n
+    tw = Twin(D=D, H=H, QH=2 * H, capacity_tokens=T, seed=n)
+    k, v = orc.synth_kv(n, T, H, D, 1), orc.synth_kv(n, T, H, D, 2)
+    tw.append(k[:first], v[:first])
+    tw.append(k[first:], v[first:])
+    _check_planes(tw)
+    tile = T // 128 - 1  # the sealed tile before the open one: a roll-back may re-open it
+    assert np.array_equal(tw.stage_np()[:, tile & 1], tw.cpu.stage[:, tile & 1])
