@@ -18,6 +18,7 @@
 // phases (de-quantisation, softmax) overlap the other's MMAs.
 // Every wait on an mbarrier is bounded; a wait that gives up sets KVB_ERR_WAIT_TIMEOUT and the CTA leaves
 // through the normal exit (TMEM is freed).
+#include <algorithm>
 #include <climits>
 
 #include "kvb_chunk_merge.cuh"
@@ -728,12 +729,22 @@ void prefill_shape(int kv_len_max, int kv_heads, int q_heads, int tokens, int* m
     const int rows = tokens * (q_heads / kv_heads);
     *mtiles = (rows + kM - 1) / kM;
     const int ctas = *mtiles * kv_heads, ntiles = (kv_len_max + kN - 1) / kN;
-    // two CTAs share an SM: about six waves of CTAs for a chunk, rounded down so that the last wave is full (measured on
-    // 1,024 x 262,144: 9 key ranges 4.94 ms, 7: 5.19, 10: 5.03, 12: 4.98, 14: 5.25); one wave for a few rows (verify),
-    // where every extra key range costs a partial per row
-    int ks = ctas >= 64 ? (6 * 2 * prefill_sm_count()) / ctas : (2 * prefill_sm_count() + ctas - 1) / ctas;
+    // Two CTAs share an SM.  A few rows (verify): one wave, every further key range costs a partial per row.  A chunk: the
+    // number of ranges (at most about six waves) with the lowest (waves x CTA), a CTA costing its tiles plus about five
+    // tiles' worth of set-up (Q tile) and epilogue.  Measured (always six waves in brackets): 1,024 tokens over 262,144, 3
+    // ranges, 4.40 ms (4.52, 9 ranges); 777 tokens alone, 2 ranges, 28 us (46, 3 ranges: a second, nearly empty wave).
+    const int slots = 2 * prefill_sm_count();
+    int ks = (slots + ctas - 1) / ctas;
+    if (ctas >= 64) {
+        int64_t best = INT64_MAX;
+        const int most = std::max(1, std::min(6 * slots / ctas, ntiles / 2));
+        for (int n = 1; n <= most; ++n) {
+            const int64_t cost = static_cast<int64_t>((ctas * n + slots - 1) / slots) * (5 + (ntiles + n - 1) / n);
+            if (cost < best) { best = cost; ks = n; }
+        }
+    }
     if (ks > ntiles / 2) ks = ntiles / 2;
-    if (ks > 128) ks = 128;
+    if (ks > kMaxKeyRanges) ks = kMaxKeyRanges;
     *ksplit = ks < 1 ? 1 : ks;
 }
 
