@@ -8,19 +8,20 @@
 // to a largest magnitude of 2^14 .. 2^15 and their exponents return in the logits (a thread owns a row), V follows the
 // largest page seen so far and O is rescaled, exactly, when that grows.
 //
-// Roles (13 warps, one CTA per SM):
-//   warps 4-11   de-quantise K(i), then V(i-1): code -> fp32 (code * scale + zp) * other -> high | low, 64 KB a page each, in
-//                128-byte-swizzled tiles; thread = one key and 64 dims; codes and scales are fetched a page ahead;
-//   warp 12      issues S(i) = Q K(i)^T, then O += P(i-1) V(i-1);
+// Roles (24 warps, one CTA per SM, registers re-divided by role):
+//   warps 4-11   de-quantise K(i): code -> fp32 (code * scale + zp) * other -> high | low, 64 KB a page, in 128-byte-swizzled
+//                tiles; thread = one key and 64 dims; codes and scales are fetched a page ahead;
+//   warps 12-19  the same for V(i): two chains beside each other instead of one after the other;
+//   warp 20      issues S(i) = Q K(i)^T, then O += P(i-1) V(i-1);
 //   warps 0-3    softmax of S(i), thread = row: P (high | low) over S in tensor memory, O rescaled lazily.
 // K(i+1) is written while P V(i-1) runs, V(i) while Q K(i+1)^T runs.  Tensor memory (512 columns): two S buffers of
 // 64, the high part of Q (128, the A operand of two of the three Q K products), O (256).  The low part of Q stays in
 // shared memory (64 KB), beside one K and one V buffer.
 //
-// Bound by the chain of a page's hand-offs (de-quantise, MMA, softmax and back), with the tensor pipe (48 MMAs of 128x64x16
-// and 12 of 128x256x16 a page, about 3,300 cycles) and shared-memory traffic (MMA operands, 128 KB of tiles written a page)
-// close behind.  Measured on B200, 24 / 4 heads, 1,024 tokens over a prefix of 16,384, balanced bf16 cache: 1.5 ms (280
-// TFLOP/s of attention, 840 of MMA) against 69.8 ms for one warp per key on fp32 FMAs.
+// Bound by the chain of a page: K is de-quantised (about 2,800 cycles), then multiplied (48 MMAs of 128x64x16, 3,100: a
+// 64-key MMA takes as long as a 128-key one), hand-offs 700; P V, V and the softmax run beside it.  Measured on B200, 24 / 4
+// heads, 1,024 tokens over a prefix of 16,384, balanced bf16 cache: 1.26 ms (340 TFLOP/s of attention) against 69.8 ms for
+// one warp per key on fp32 FMAs, 1.40 ms with eight warps for K and V in turn, 1.38 ms with sixteen in turn.
 // Accuracy: against float64 the un-normalised sums are off by 4e-7 .. 6e-6 (fp32 FMAs: 2e-7 .. 1.1e-5, sizes of 32 .. 65,576
 // keys), the fp16 / bf16 outputs by their rounding alone (2.09e-4 and 1.70e-3, as before).
 #include <climits>
@@ -35,8 +36,9 @@ namespace {
 constexpr int D = 256;
 constexpr int kM = 128;   // query rows per CTA
 constexpr int kN = 64;    // keys per step: one page
-constexpr int kSoftWarps = 4, kDqWarps = 8, kMmaWarp = kSoftWarps + kDqWarps, kThreads = 32 * (kMmaWarp + 1);
-constexpr int kDqThreads = 32 * kDqWarps;
+constexpr int kSoftWarps = 4, kDqWarps = 8, kMmaWarp = kSoftWarps + 2 * kDqWarps, kWarps = kMmaWarp + 4, kThreads = 32 * kWarps;
+// Registers per thread: 80 at launch (61,440 a CTA), then by role 128 x 144 + 512 x 72 + 128 x 48 = 61,440.
+constexpr int kSoftRegs = 144, kDqRegs = 72, kMmaRegs = 48;
 constexpr int kKvBlock = kN * 128;       // one 64-dim block of a K or V tile: 64 rows of 128 bytes
 constexpr int kKvTile = 4 * kKvBlock;
 constexpr int kQBlock = kM * 128;        // one 64-dim block of the Q tile
@@ -61,16 +63,15 @@ struct __align__(1024) Chunk256Smem {
     uint8_t q_lo[4 * kQBlock];
     uint8_t k[2][kKvTile];     // high, low part; holds the high part of Q before the walk
     uint8_t v[2][kKvTile];
-    float ks[2][D], kz[2][D];            // per-dim factors of K by page parity; ks is divided by 16^(nibble position)
-    float vo[kSlotsMeta][D];             // per-dim factors of V (used a step later than those of K)
-    uint32_t red[2][kDqWarps][4];        // partial maxima: |K before other_K|, |other_K|, |other_V|, |V before other_V| (float bits)
-    uint32_t poison[kSlotsMeta][kDqWarps];  // keys with a non-finite V (ballots of the warps)
+    float ks[2][D], kz[2][D], vo[2][D];  // per-dim factors by page parity; ks is divided by 16^(nibble position)
+    alignas(16) uint2 red[2][2][kDqWarps];  // partial maxima (float bits) of K, of V: per-dim and per-key factors
+    alignas(16) uint32_t poison[kSlotsMeta][kDqWarps];  // keys with a non-finite V (ballots of the warps)
     float k_unit[kSlotsMeta];            // page i: K = k_unit * (high + low)
     int v_exp[kSlotsMeta];               // exponent of V and O as of page i
     int bad_page[kSlotsMeta];
     int row_pos[kM];
     float row_unit[kM];                  // q' = row_unit * (high + low)
-    uint64_t s_full[2], p_full[2], k_full, v_full, o_done, drain;
+    uint64_t s_full[2], p_full[2], v_meta[2], k_full, v_full, o_done, drain;
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -160,6 +161,183 @@ __device__ __forceinline__ void unpack_f32(uint32_t w, F2 (&n)[4]) {
 }
 __device__ __forceinline__ constexpr int nibble_shift(int d) { return 4 * ((d & 7) < 5 ? (d & 7) : (d & 7) - 5); }
 
+// One de-quantising role (eight warps, thread dt): K or V of the CTA's n pages p0 .. p1 - 1.
+template <bool kValue, bool kOther>
+__device__ __forceinline__ bool dequant_role(Chunk256Smem& sm, const LayerView& L, int head, int dt, int p0, int p1, int kv_total) {
+    const int lane = dt & 31, dw = dt >> 5;                    // dt: also the dim whose factors this thread fetches
+    const int quarter = dw & 3, key = 32 * (dw >> 2) + lane;   // 64 dims of one key of the page
+    const int s = quarter >> 1, n = p1 - p0, sealed_pages = 2 * (kv_total / kTile);
+    const uint32_t row_off = quarter * kKvBlock + key * 128;
+    uint8_t (&tile)[2][kKvTile] = kValue ? sm.v : sm.k;
+    const uint8_t* plane = kValue ? L.v_code : L.k_code;
+    const int32_t* tbl = L.table();
+    struct Meta {
+        __half d0, d1, t0, t1;  // K: scale, zero point of the dim; other_K of the key.  V: other_V of the dim; scale, zero point of the key
+        int32_t page;           // -1: unusable; the page is masked
+        uint4 code[2];
+    };
+    int32_t entry = LayerView::kNoEntry;  // table entry of the page the next fetch asks for, requested a page earlier
+    auto lookup = [&](int p) { entry = p < p1 && p < sealed_pages ? L.page_entry(tbl, p) : LayerView::kNoEntry; };
+    auto fetch = [&](Meta& m) {
+        m.page = L.checked_page(entry);
+        m.d0 = m.d1 = m.t0 = m.t1 = __ushort_as_half(0);
+        m.code[0] = m.code[1] = make_uint4(0u, 0u, 0u, 0u);
+        if (m.page >= 0) {
+            if constexpr (kValue) {
+                const __half* vsp = L.v_scale + page_head_offset(8, L.kv_heads, m.page, head);
+                m.d0 = vsp[8 * (dt >> 2) + (dt & 3)];
+                m.t0 = vsp[8 * key + 4 + s];
+                m.t1 = vsp[8 * key + 6 + s];
+            } else {
+                const __half* ksp = L.k_scale + page_head_offset(10, L.kv_heads, m.page, head);
+                m.d0 = ksp[10 * (dt >> 2) + (dt & 3)];
+                m.d1 = ksp[10 * (dt >> 2) + 4 + (dt & 3)];
+                m.t0 = ksp[10 * key + 8 + s];
+            }
+            const uint4* src = reinterpret_cast<const uint4*>(plane + page_head_offset(128, L.kv_heads, m.page, head) + key * 128 + quarter * 32);
+            m.code[0] = src[0];
+            m.code[1] = src[1];
+        }
+    };
+    Meta m, nxt;  // the next page's is requested at the top of a step: a step hides the trip to memory
+    if (n > 0) {
+        lookup(p0);
+        fetch(nxt);
+        lookup(p0 + 1);
+    }
+    bool failed = false;
+    int v_run = INT_MIN;  // exponent of V so far
+    for (int i = 0; i < n; ++i) {
+        const int p = p0 + i, par = i & 1, slot = i & (kSlotsMeta - 1);
+        const bool sealed = p < sealed_pages;
+        m = nxt;
+        fetch(nxt);
+        lookup(p + 2);
+        const __half* row = nullptr;  // open tile: this key's un-quantised row
+        bool live = true;
+        float d0 = __half2float(m.d0), t0 = __half2float(m.t0), t1 = __half2float(m.t1);
+        // ---- per-dim tables of the page, and the largest magnitudes that decide its scale
+        uint32_t db, tb;
+        if constexpr (kValue) {
+            db = abs_bits(d0);
+            tb = max(abs_bits(t1), abs_bits(fmaf(15.0f, t0, t1)));
+        } else {
+            const float d1 = __half2float(m.d1);
+            db = max(abs_bits(d1), abs_bits(fmaf(15.0f, d0, d1)));
+            sm.ks[par][dt] = d0 * pow2i(-nibble_shift(dt));
+            sm.kz[par][dt] = d1;
+        }
+        if (!sealed) {
+            const int first = (p & 1) * kPage + key;
+            row = L.stage_row(kValue ? 1 : 0, (kv_total / kTile) & 1, head, first) + 64 * quarter;
+            live = p * kN + key < kv_total;
+            uint32_t top = 0;
+            if (live) {
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const uint4 a = reinterpret_cast<const uint4*>(row)[c];
+                    const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float2 f = unpack_half2(w[e]);
+                        top = max(top, max(abs_bits(f.x), abs_bits(f.y)));
+                    }
+                }
+            }
+            if constexpr (kValue) {
+                db = __float_as_uint(1.0f);
+                tb = top;
+            } else {
+                db = top;
+                t0 = 1.0f;
+            }
+        }
+        if constexpr (kValue) {  // a key whose V is not finite is left out of the product, see the softmax
+            const bool bad_key = tb >= 0x7F800000u;
+            if (bad_key) { t0 = t1 = 0.0f; tb = 0u; live = false; }
+            const uint32_t bad = __ballot_sync(0xffffffffu, bad_key);
+            if (lane == 0) sm.poison[slot][dw] = bad;
+            if constexpr (kOther) sm.vo[par][dt] = db >= 0x7F800000u ? 0.0f : d0;
+        } else {
+            tb = abs_bits(t0);
+        }
+        db = __reduce_max_sync(0xffffffffu, db);
+        tb = __reduce_max_sync(0xffffffffu, tb);
+        if (lane == 0) sm.red[par][kValue ? 1 : 0][dw] = make_uint2(db, tb);
+        if (named_barrier_or(kValue ? 2 : 1, 32 * kDqWarps, failed)) return true;
+#pragma unroll
+        for (int w = 0; w < kDqWarps; w += 2) {
+            const uint4 r = *reinterpret_cast<const uint4*>(&sm.red[par][kValue ? 1 : 0][w]);
+            db = max(db, max(r.x, r.z));
+            tb = max(tb, max(r.y, r.w));
+        }
+        float unit;  // 1 / scale of the page
+        if constexpr (kValue) {
+            const bool bad_dim = db >= 0x7F800000u;  // of every key
+            const float top = __uint_as_float(tb) * (bad_dim ? 1.0f : __uint_as_float(db));
+            if (top > 0.0f) v_run = max(v_run, scale_exponent(__float_as_uint(top)));
+            const int v_exp = v_run == INT_MIN ? 0 : v_run;
+            unit = pow2i(-v_exp);
+            if (lane == 0) {
+                if (dw == 0) sm.v_exp[slot] = v_exp;
+                if (bad_dim) sm.poison[slot][dw] = 0xffffffffu;
+                mbar_arrive(&sm.v_meta[par]);
+            }
+            // the buffer is free once P V(i-1) has completed
+            if (i > 0 && !chunk_wait(&sm.o_done, (i - 1) & 1, &sm.abort_flag)) { failed = true; continue; }
+        } else {
+            const int k_exp = scale_exponent(__float_as_uint(__uint_as_float(db) * __uint_as_float(tb)));
+            unit = t0 * pow2i(-k_exp);
+            if (dt == 0) {
+                sm.k_unit[slot] = pow2i(k_exp);
+                sm.bad_page[slot] = sealed && m.page < 0;
+            }
+            // the buffer is free once S(i-1) has completed
+            if (i > 0 && !chunk_wait(&sm.s_full[(i - 1) & 1], ((i - 1) >> 1) & 1, &sm.abort_flag)) { failed = true; continue; }
+        }
+        const F2 unit2(unit, unit);
+        if (sealed) {
+            const float z = t1 * unit, v0 = t0 * unit, v1 = v0 * 0.0625f, v2 = v1 * 0.0625f, v3 = v2 * 0.0625f, v4 = v3 * 0.0625f;
+            const F2 z2(z, z), sc[4] = {F2(v0, v1), F2(v2, v3), F2(v4, v0), F2(v1, v2)};  // V: scale / 16^(nibble position)
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const uint4 cc = m.code[c >> 2];
+                F2 x[4];
+                unpack_f32((c & 3) == 0 ? cc.x : (c & 3) == 1 ? cc.y : (c & 3) == 2 ? cc.z : cc.w, x);
+                const int at = 64 * quarter + 8 * c;
+                if constexpr (kValue) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) x[e] = fma2(x[e], sc[e], z2);
+                    if constexpr (kOther) {
+                        const ulonglong2* ot = reinterpret_cast<const ulonglong2*>(&sm.vo[par][at]);
+                        const ulonglong2 o0 = ot[0], o1 = ot[1];
+                        x[0] = mul2(x[0], F2(o0.x)); x[1] = mul2(x[1], F2(o0.y));
+                        x[2] = mul2(x[2], F2(o1.x)); x[3] = mul2(x[3], F2(o1.y));
+                    }
+                } else {
+                    const ulonglong2* st = reinterpret_cast<const ulonglong2*>(&sm.ks[par][at]);
+                    const ulonglong2* zt = reinterpret_cast<const ulonglong2*>(&sm.kz[par][at]);
+                    const ulonglong2 s0 = st[0], s1 = st[1], z0 = zt[0], z1 = zt[1];
+                    x[0] = mul2(fma2(x[0], F2(s0.x), F2(z0.x)), unit2); x[1] = mul2(fma2(x[1], F2(s0.y), F2(z0.y)), unit2);
+                    x[2] = mul2(fma2(x[2], F2(s1.x), F2(z1.x)), unit2); x[3] = mul2(fma2(x[3], F2(s1.y), F2(z1.y)), unit2);
+                }
+                split_store(x, tile[0], tile[1], row_off + ((c ^ (key & 7)) << 4));
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                F2 x[4];
+                widen(live ? reinterpret_cast<const uint4*>(row)[c] : make_uint4(0u, 0u, 0u, 0u), unit2, x);
+                split_store(x, tile[0], tile[1], row_off + ((c ^ (key & 7)) << 4));
+            }
+        }
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(kValue ? &sm.v_full : &sm.k_full);
+    }
+    return failed;
+}
+
 template <bool kOther>
 __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Params P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -175,6 +353,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Par
         for (int b = 0; b < 2; ++b) {
             mbar_init(&sm.s_full[b], 1);
             mbar_init(&sm.p_full[b], kSoftWarps);
+            mbar_init(&sm.v_meta[b], kDqWarps);
         }
         mbar_init(&sm.k_full, kDqWarps);
         mbar_init(&sm.v_full, kDqWarps);
@@ -185,12 +364,12 @@ __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Par
     }
     // ---- Q: rows rotated, scaled, split; one warp per row, lane l holds dims l + 32 j, the loads of four rows in flight
     constexpr int kQBatch = 4;
-    for (int r0 = warp; r0 < kM; r0 += kQBatch * (kMmaWarp + 1)) {
+    for (int r0 = warp; r0 < kM; r0 += kQBatch * kWarps) {
         uint16_t raw[kQBatch][8];
         int rp[kQBatch];
 #pragma unroll
         for (int u = 0; u < kQBatch; ++u) {
-            const int r = r0 + u * (kMmaWarp + 1), R = mt * kM + r, tq = R / G, gq = R % G;
+            const int r = r0 + u * kWarps, R = mt * kM + r, tq = R / G, gq = R % G;
             rp[u] = -1;
 #pragma unroll
             for (int j = 0; j < 8; ++j) raw[u][j] = 0;
@@ -203,7 +382,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Par
         }
 #pragma unroll
         for (int u = 0; u < kQBatch; ++u) {
-            const int r = r0 + u * (kMmaWarp + 1);
+            const int r = r0 + u * kWarps;
             if (r >= kM) break;
             float v[8];
             uint32_t top = 0;
@@ -268,207 +447,17 @@ __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Par
     const int p0 = static_cast<int>(static_cast<int64_t>(npages) * zs / P.ksplit);
     const int p1 = static_cast<int>(static_cast<int64_t>(npages) * (zs + 1) / P.ksplit);
     const int n = p1 - p0;
-    const int sealed_pages = 2 * (kv_total / kTile);
     bool failed = false;
 
     if (warp >= kSoftWarps && warp < kMmaWarp) {
-        // =========================== de-quantise ===========================
-        const int dt = tid - 32 * kSoftWarps, dw = dt >> 5;        // dt: also the dim whose factors this thread fetches
-        const int quarter = dw & 3, key = 32 * (dw >> 2) + lane;   // 64 dims of one key of the page
-        const int s = quarter >> 1;
-        const uint32_t row_off = quarter * kKvBlock + key * 128;
-        const int32_t* tbl = L.table();
-        struct Meta {
-            __half ks, kz, vo, ko, sv, zp;
-            int32_t page;  // -1: unusable; the page is masked
-            bool sealed;
-        };
-        uint4 kcode[2], vcode[2];
-        int32_t pid_next = -1;  // page id of the page the next fetch asks for, looked up a page earlier
-        auto lookup = [&](int p) { pid_next = p < p1 && p < sealed_pages ? L.page_of(tbl, p) : -1; };
-        auto fetch_meta = [&](int p, Meta& m) {
-            m.sealed = p < sealed_pages;
-            m.page = pid_next;
-            m.ks = m.kz = m.vo = m.ko = m.sv = m.zp = __ushort_as_half(0);
-            if (p < p1 && m.page >= 0) {
-                const __half* ksp = L.k_scale + page_head_offset(10, L.kv_heads, m.page, head);
-                const __half* vsp = L.v_scale + page_head_offset(8, L.kv_heads, m.page, head);
-                m.ks = ksp[10 * (dt >> 2) + (dt & 3)];
-                m.kz = ksp[10 * (dt >> 2) + 4 + (dt & 3)];
-                m.ko = ksp[10 * key + 8 + s];
-                m.vo = vsp[8 * (dt >> 2) + (dt & 3)];
-                m.sv = vsp[8 * key + 4 + s];
-                m.zp = vsp[8 * key + 6 + s];
-            }
-        };
-        auto fetch_codes = [&](const uint8_t* plane, int32_t page, uint4 (&c)[2]) {
-            if (page >= 0) {
-                const uint4* src = reinterpret_cast<const uint4*>(plane + page_head_offset(128, L.kv_heads, page, head) + key * 128 + quarter * 32);
-                c[0] = src[0];
-                c[1] = src[1];
-            } else {
-                c[0] = c[1] = make_uint4(0u, 0u, 0u, 0u);
-            }
-        };
-        Meta cur, nxt;
-        if (n > 0) {
-            lookup(p0);
-            fetch_meta(p0, nxt);
-            fetch_codes(L.k_code, nxt.page, kcode);
-            fetch_codes(L.v_code, nxt.page, vcode);
-            lookup(p0 + 1);
-        }
-        int v_run = INT_MIN;  // exponent of V so far
-        // what V(i-1) needs: its page is de-quantised a step after K of the same page
-        struct {
-            float sv, zp, unit;
-            const __half* row;  // open tile: the un-quantised row of this thread's key (null: de-quantise)
-            bool live;
-        } vprev{};
-        for (int i = 0; i <= n; ++i) {
-            const int p = p0 + i, par = i & 1, slot = i & (kSlotsMeta - 1);
-            auto vnow = vprev;
-            if (i < n) {
-                cur = nxt;
-                const __half* krow = nullptr;  // open tile: this key's un-quantised row
-                float ko = __half2float(cur.ko);
-                vnow.sv = __half2float(cur.sv);
-                vnow.zp = __half2float(cur.zp);
-                vnow.row = nullptr;
-                vnow.live = true;
-                // ---- per-dim tables of the page, and the largest magnitudes that decide its scales
-                {
-                    const float ks = __half2float(cur.ks), kz = __half2float(cur.kz), vo = __half2float(cur.vo);
-                    uint32_t kb = max(abs_bits(kz), abs_bits(fmaf(15.0f, ks, kz))), vb = max(abs_bits(vnow.zp), abs_bits(fmaf(15.0f, vnow.sv, vnow.zp)));
-                    uint32_t ob = abs_bits(vo);
-                    if (!cur.sealed) {
-                        const int tile = kv_total / kTile, first = (p & 1) * kPage + key;
-                        krow = L.stage_row(0, tile & 1, head, first) + 64 * quarter;
-                        vnow.row = L.stage_row(1, tile & 1, head, first) + 64 * quarter;
-                        vnow.live = p * kN + key < kv_total;
-                        ob = __float_as_uint(1.0f);
-                        if (vnow.live) {
-#pragma unroll
-                            for (int c = 0; c < 8; ++c) {
-                                const uint4 a = reinterpret_cast<const uint4*>(vnow.row)[c], b = reinterpret_cast<const uint4*>(krow)[c];
-                                const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, wb[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-                                for (int e = 0; e < 4; ++e) {
-                                    const float2 fa = unpack_half2(wa[e]), fb = unpack_half2(wb[e]);
-                                    vb = max(vb, max(abs_bits(fa.x), abs_bits(fa.y)));
-                                    kb = max(kb, max(abs_bits(fb.x), abs_bits(fb.y)));
-                                }
-                            }
-                        }
-                        ko = 1.0f;
-                    }
-                    const bool bad_key = vb >= 0x7F800000u;
-                    if (bad_key) { vnow.sv = vnow.zp = 0.0f; vb = 0u; vnow.live = false; }
-                    const uint32_t bad = __ballot_sync(0xffffffffu, bad_key);
-                    sm.ks[par][dt] = ks * pow2i(-nibble_shift(dt));
-                    sm.kz[par][dt] = kz;
-                    if constexpr (kOther) sm.vo[slot][dt] = ob >= 0x7F800000u ? 0.0f : vo;
-                    const uint32_t mk = __reduce_max_sync(0xffffffffu, kb), mo = __reduce_max_sync(0xffffffffu, abs_bits(ko));
-                    const uint32_t mov = __reduce_max_sync(0xffffffffu, ob), mv = __reduce_max_sync(0xffffffffu, vb);
-                    if (lane == 0) {
-                        *reinterpret_cast<uint4*>(sm.red[par][dw]) = make_uint4(mk, mo, mov, mv);
-                        sm.poison[slot][dw] = bad;
-                    }
-                }
-                if (named_barrier_or(1, kDqThreads, failed)) { failed = true; break; }
-                uint32_t mk = 0, mo = 0, mov = 0, mv = 0;
-#pragma unroll
-                for (int w = 0; w < kDqWarps; ++w) {
-                    const uint4 r = *reinterpret_cast<const uint4*>(sm.red[par][w]);
-                    mk = max(mk, r.x); mo = max(mo, r.y); mov = max(mov, r.z); mv = max(mv, r.w);
-                }
-                const int k_exp = scale_exponent(__float_as_uint(__uint_as_float(mk) * __uint_as_float(mo)));
-                const float vtop = __uint_as_float(mv) * (mov >= 0x7F800000u ? 1.0f : __uint_as_float(mov));
-                if (vtop > 0.0f) v_run = max(v_run, scale_exponent(__float_as_uint(vtop)));
-                const int v_exp = v_run == INT_MIN ? 0 : v_run;
-                vnow.unit = pow2i(-v_exp);
-                if (dt == 0) {
-                    sm.k_unit[slot] = pow2i(k_exp);
-                    sm.v_exp[slot] = v_exp;
-                    sm.bad_page[slot] = cur.sealed && cur.page < 0;
-                }
-                if (mov >= 0x7F800000u && lane == 0) sm.poison[slot][dw] = 0xffffffffu;  // a dim of every key
-                // ---- K(i): the buffer is free once S(i-1) has completed
-                if (i > 0 && !chunk_wait(&sm.s_full[(i - 1) & 1], ((i - 1) >> 1) & 1, &sm.abort_flag)) { failed = true; continue; }
-                const float kf = ko * pow2i(-k_exp);
-                const F2 kf2(kf, kf);
-                if (cur.sealed) {
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        const uint4 cc = kcode[c >> 2];
-                        const ulonglong2* st = reinterpret_cast<const ulonglong2*>(&sm.ks[par][64 * quarter + 8 * c]);
-                        const ulonglong2* zt = reinterpret_cast<const ulonglong2*>(&sm.kz[par][64 * quarter + 8 * c]);
-                        const ulonglong2 s0 = st[0], s1 = st[1], z0 = zt[0], z1 = zt[1];
-                        F2 x[4];
-                        unpack_f32((c & 3) == 0 ? cc.x : (c & 3) == 1 ? cc.y : (c & 3) == 2 ? cc.z : cc.w, x);
-                        x[0] = mul2(fma2(x[0], F2(s0.x), F2(z0.x)), kf2);
-                        x[1] = mul2(fma2(x[1], F2(s0.y), F2(z0.y)), kf2);
-                        x[2] = mul2(fma2(x[2], F2(s1.x), F2(z1.x)), kf2);
-                        x[3] = mul2(fma2(x[3], F2(s1.y), F2(z1.y)), kf2);
-                        split_store(x, sm.k[0], sm.k[1], row_off + ((c ^ (key & 7)) << 4));
-                    }
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        F2 x[4];
-                        widen(p * kN + key < kv_total ? reinterpret_cast<const uint4*>(krow)[c] : make_uint4(0u, 0u, 0u, 0u), kf2, x);
-                        split_store(x, sm.k[0], sm.k[1], row_off + ((c ^ (key & 7)) << 4));
-                    }
-                }
-                fence_proxy_async();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&sm.k_full);
-                fetch_meta(p + 1, nxt);
-                fetch_codes(L.k_code, nxt.page, kcode);
-                lookup(p + 2);
-            }
-            if (i > 0) {
-                // ---- V(i-1): the buffer is free once P V(i-2) has completed
-                const int vslot = (i - 1) & (kSlotsMeta - 1);
-                if (i > 1 && !chunk_wait(&sm.o_done, i & 1, &sm.abort_flag)) { failed = true; continue; }
-                if (vprev.row == nullptr) {
-                    const float z = vprev.zp * vprev.unit, s0 = vprev.sv * vprev.unit, s1 = s0 * 0.0625f, s2 = s1 * 0.0625f, s3 = s2 * 0.0625f, s4 = s3 * 0.0625f;
-                    const F2 z2(z, z), sc[4] = {F2(s0, s1), F2(s2, s3), F2(s4, s0), F2(s1, s2)};
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        const uint4 cc = vcode[c >> 2];
-                        F2 x[4];
-                        unpack_f32((c & 3) == 0 ? cc.x : (c & 3) == 1 ? cc.y : (c & 3) == 2 ? cc.z : cc.w, x);
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) x[e] = fma2(x[e], sc[e], z2);
-                        if constexpr (kOther) {
-                            const ulonglong2* ot = reinterpret_cast<const ulonglong2*>(&sm.vo[vslot][64 * quarter + 8 * c]);
-                            const ulonglong2 o0 = ot[0], o1 = ot[1];
-                            x[0] = mul2(x[0], F2(o0.x));
-                            x[1] = mul2(x[1], F2(o0.y));
-                            x[2] = mul2(x[2], F2(o1.x));
-                            x[3] = mul2(x[3], F2(o1.y));
-                        }
-                        split_store(x, sm.v[0], sm.v[1], row_off + ((c ^ (key & 7)) << 4));
-                    }
-                } else {
-                    const F2 unit2(vprev.unit, vprev.unit);
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        F2 x[4];
-                        widen(vprev.live ? reinterpret_cast<const uint4*>(vprev.row)[c] : make_uint4(0u, 0u, 0u, 0u), unit2, x);
-                        split_store(x, sm.v[0], sm.v[1], row_off + ((c ^ (key & 7)) << 4));
-                    }
-                }
-                fence_proxy_async();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&sm.v_full);
-                if (i < n) fetch_codes(L.v_code, cur.page, vcode);
-            }
-            vprev = vnow;
-        }
-    } else if (warp == kMmaWarp) {
-        // =========================== MMA issue ===========================
+        tc::regs_dec<kDqRegs>();
+        const int dt = tid - 32 * kSoftWarps;
+        if (dt < 32 * kDqWarps) failed = dequant_role<false, kOther>(sm, L, head, dt, p0, p1, kv_total);
+        else failed = dequant_role<true, kOther>(sm, L, head, dt - 32 * kDqWarps, p0, p1, kv_total);
+    } else if (warp >= kMmaWarp) {
+        // =========================== MMA issue (one warp; the three beside it complete the warpgroup) ===========================
+        tc::regs_dec<kMmaRegs>();
+        if (warp == kMmaWarp) {
         constexpr uint32_t idesc_qk = tc::idesc_f16(kM, kN, false, false), idesc_pv = tc::idesc_f16(kM, D, false, true);
         const uint32_t q_addr = smem_u32(sm.q_lo), k_hi = smem_u32(sm.k[0]), k_lo = smem_u32(sm.k[1]), v_hi = smem_u32(sm.v[0]), v_lo = smem_u32(sm.v[1]);
         for (int i = 0; i <= n && !failed; ++i) {
@@ -477,17 +466,22 @@ __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Par
                 if (!chunk_wait(&sm.k_full, i & 1, &sm.abort_flag) || (i > 1 && !chunk_wait(&sm.o_done, i & 1, &sm.abort_flag))) { failed = true; break; }
                 tc::fence_after_sync();
                 const uint32_t s = tmem + 64 * (i & 1);
+#pragma unroll 1
+                for (int b = 0; b < 4; ++b)  // 64 dims at a time (all of them at once cost more registers than this role has)
 #pragma unroll
-                for (int kk = 0; kk < 16; ++kk) {
-                    const uint32_t ko = (kk >> 2) * kKvBlock + (kk & 3) * 32;
-                    tc::mma_f16_ss(s, tc::smem_desc(q_addr + (kk >> 2) * kQBlock + (kk & 3) * 32, 16, 1024), tc::smem_desc(k_hi + ko, 16, 1024), idesc_qk, kk > 0);
-                }
+                    for (int kk = 0; kk < 4; ++kk)
+                        tc::mma_f16_ss(s, tc::smem_desc(q_addr + b * kQBlock + kk * 32, 16, 1024), tc::smem_desc(k_hi + b * kKvBlock + kk * 32, 16, 1024), idesc_qk,
+                                       b > 0 || kk > 0);
+#pragma unroll 1
+                for (int b = 0; b < 4; ++b)
 #pragma unroll
-                for (int kk = 0; kk < 16; ++kk)
-                    tc::mma_f16_ts(s, tmem + kColQ + 8 * kk, tc::smem_desc(k_lo + (kk >> 2) * kKvBlock + (kk & 3) * 32, 16, 1024), idesc_qk, true);
+                    for (int kk = 0; kk < 4; ++kk)
+                        tc::mma_f16_ts(s, tmem + kColQ + 32 * b + 8 * kk, tc::smem_desc(k_lo + b * kKvBlock + kk * 32, 16, 1024), idesc_qk, true);
+#pragma unroll 1
+                for (int b = 0; b < 4; ++b)
 #pragma unroll
-                for (int kk = 0; kk < 16; ++kk)
-                    tc::mma_f16_ts(s, tmem + kColQ + 8 * kk, tc::smem_desc(k_hi + (kk >> 2) * kKvBlock + (kk & 3) * 32, 16, 1024), idesc_qk, true);
+                    for (int kk = 0; kk < 4; ++kk)
+                        tc::mma_f16_ts(s, tmem + kColQ + 32 * b + 8 * kk, tc::smem_desc(k_hi + b * kKvBlock + kk * 32, 16, 1024), idesc_qk, true);
                 tc::commit(&sm.s_full[i & 1]);
             }
             if (i > 0) {
@@ -511,8 +505,10 @@ __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Par
             tc::commit(&sm.drain);
             mbar_wait_bounded(&sm.drain, 0);
         }
+        }
     } else {
         // =========================== softmax ===========================
+        tc::regs_inc<kSoftRegs>();
         const uint32_t lane_base = static_cast<uint32_t>(32 * warp) << 16;
         const int my_pos = sm.row_pos[tid];
         const float row_unit = sm.row_unit[tid];
@@ -522,7 +518,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Par
         bool poisoned = false;
         for (int i = 0; i < n; ++i) {
             const int base = (p0 + i) * kN, slot = i & (kSlotsMeta - 1);
-            if (!chunk_wait(&sm.s_full[i & 1], (i >> 1) & 1, &sm.abort_flag)) { failed = true; break; }
+            if (!chunk_wait(&sm.v_meta[i & 1], (i >> 1) & 1, &sm.abort_flag) || !chunk_wait(&sm.s_full[i & 1], (i >> 1) & 1, &sm.abort_flag)) { failed = true; break; }
             tc::fence_after_sync();
             if (warp_has_rows) {
                 const uint32_t ts = tmem + 64 * (i & 1) + lane_base;

@@ -69,6 +69,17 @@ struct LayerView {
         if (p < 0 || p >= pages) { flag(KVB_ERR_PAGE_RANGE); return -1; }
         return p;
     }
+    // page_of in two halves, for callers that ask a step ahead: the check needs the value and would wait for the load.
+    static constexpr int32_t kNoEntry = INT32_MIN;
+    __device__ __forceinline__ int32_t page_entry(const int32_t* tbl, int logical) const {
+        if (logical < 0 || logical >= table_len) { flag(KVB_ERR_TABLE_RANGE); return kNoEntry; }
+        return tbl[logical];
+    }
+    __device__ __forceinline__ int32_t checked_page(int32_t entry) const {
+        if (entry >= 0 && entry < pages) return entry;
+        if (entry != kNoEntry) flag(KVB_ERR_PAGE_RANGE);
+        return -1;
+    }
     __device__ __forceinline__ __half* stage_row(int which, int slot, int head, int tok) const {
         const int64_t plane = static_cast<int64_t>(2) * kv_heads * kTile * head_dim;
         return stage + which * plane + ((static_cast<int64_t>(slot) * kv_heads + head) * kTile + tok) * head_dim;

@@ -218,19 +218,19 @@ __global__ void __launch_bounds__(kThreads, 2) prefill_kernel(const PrefillParam
     // The physical pages of a tile are looked up one step before its codes are requested (ids_a / ids_b: pages of the
     // tile the next fetch_k asks for): page id -> code address is a dependent trip to L2 that would otherwise stall
     // every step for about 0.3 us.
-    int32_t ids_a = -1, ids_b = -1;
+    int32_t ids_a = LayerView::kNoEntry, ids_b = LayerView::kNoEntry;
     auto lookup = [&](int t) {
-        ids_a = ids_b = -1;
+        ids_a = ids_b = LayerView::kNoEntry;
         if (t < t1 && t * kN + kN <= kv_total) {
-            ids_a = L.page_of(tbl, 2 * t);
-            ids_b = L.page_of(tbl, 2 * t + 1);
+            ids_a = L.page_entry(tbl, 2 * t);
+            ids_b = L.page_entry(tbl, 2 * t + 1);
         }
     };
     auto fetch_k = [&](int t, KFetch& f) {  // uses the pages `lookup(t)` found, then looks up those of tile t + 1
         f.sealed = t * kN + kN <= kv_total;
         f.ok = t < t1;
         f.page = -1;
-        const int32_t pg0 = ids_a, pg1 = ids_b;
+        const int32_t pg0 = L.checked_page(ids_a), pg1 = L.checked_page(ids_b);
         lookup(t + 1);
         if (!f.ok || !f.sealed) return;
         if (pg0 < 0 || pg1 < 0) { f.ok = false; return; }  // reported in the error word; every thread skips the tile alike
@@ -500,17 +500,17 @@ __global__ void __launch_bounds__(kThreads, 2) verify_kernel(const PrefillParams
             __half ks[2], kz[2], ko[2], vo[2];
             bool bad;
         };
-        int32_t ids_a = -1, ids_b = -1;  // pages of the tile the next fetch asks for, looked up a step earlier
+        int32_t ids_a = LayerView::kNoEntry, ids_b = LayerView::kNoEntry;  // pages of the tile the next fetch asks for, looked up a step earlier
         auto sealed_tile = [&](int t) { return t * kN + kN <= kv_total; };
         auto lookup = [&](int t) {
-            ids_a = ids_b = -1;
+            ids_a = ids_b = LayerView::kNoEntry;
             if (t < t1 && sealed_tile(t)) {
-                ids_a = L.page_of(tbl, 2 * t);
-                ids_b = L.page_of(tbl, 2 * t + 1);
+                ids_a = L.page_entry(tbl, 2 * t);
+                ids_b = L.page_entry(tbl, 2 * t + 1);
             }
         };
         auto fetch = [&](int t, Fetch& f) {
-            int32_t pg[2] = {ids_a, ids_b};
+            int32_t pg[2] = {L.checked_page(ids_a), L.checked_page(ids_b)};
             lookup(t + 1);
             f.bad = false;
             if (t >= t1 || !sealed_tile(t)) return;
