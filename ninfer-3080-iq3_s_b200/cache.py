@@ -6,6 +6,7 @@ kvarn128_launch.h:40-58 and the attention launchers of patches/0003, lines 2362,
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import math
 
 import torch
@@ -16,11 +17,23 @@ TILE, PAGE = 128, 64
 
 
 def _ptr(t):
-    return None if t is None else C.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # the current stream of the current device, without the Stream object torch.cuda.current_stream() would make
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+# Workspace sizes are functions of the shape (and of the device's SM count): a step asks for the same one in every layer.
+@functools.lru_cache(maxsize=256)
+def _workspace_bytes(device, kv_len_max, kv_heads, q_heads, head_dim, rows):
+    return capi.load().kvb_workspace_bytes(kv_len_max, kv_heads, q_heads, head_dim, rows, 1)
+
+
+@functools.lru_cache(maxsize=256)
+def _prefill_workspace_bytes(device, kv_len_max, kv_heads, q_heads, head_dim, tokens):
+    return capi.load().kvb_prefill_workspace_bytes(kv_len_max, kv_heads, q_heads, head_dim, tokens)
 
 
 class KvarnLayer:
@@ -53,6 +66,9 @@ class KvarnLayer:
         self._ws = None
         self._pws = None
 
+    def _device_key(self) -> int:
+        return torch._C._cuda_getDevice() if self.device.type == "cuda" else -1
+
     # ---- kv_cache_append_kvarn128_launch
     def append(self, k: torch.Tensor, v: torch.Tensor, positions: torch.Tensor) -> None:
         """k, v: [tokens, kv_heads, head_dim]; positions: int32 [tokens] on the device, contiguous."""
@@ -69,13 +85,13 @@ class KvarnLayer:
         """Scratch for attention calls of up to `rows` query tokens at up to `kv_len_max` keys.  One buffer per
         layer that only ever grows: a CUDA graph that captured its address stays valid as long as the first call
         (made before the capture) asked for the largest shape the graph uses."""
-        n = capi.load().kvb_workspace_bytes(kv_len_max, self.kv_heads, self.q_heads, self.head_dim, rows, 1)
+        n = _workspace_bytes(self._device_key(), kv_len_max, self.kv_heads, self.q_heads, self.head_dim, rows)
         if self._ws is None or self._ws.numel() * 4 < n:
             self._ws = torch.empty((n + 3) // 4, dtype=torch.float32, device=self.device)
         return self._ws
 
     def prefill_workspace(self, kv_len_max: int, tokens: int) -> torch.Tensor:
-        n = capi.load().kvb_prefill_workspace_bytes(kv_len_max, self.kv_heads, self.q_heads, self.head_dim, tokens)
+        n = _prefill_workspace_bytes(self._device_key(), kv_len_max, self.kv_heads, self.q_heads, self.head_dim, tokens)
         if self._pws is None or self._pws.numel() * 4 < n:
             self._pws = torch.empty((n + 3) // 4, dtype=torch.float32, device=self.device)
         return self._pws

@@ -11,6 +11,7 @@
 //   scale = fmaxf((hi - lo) / 15, 1e-10f);  q = clamp(roundf((x - lo) / scale), 0, 15)
 //   scale_axis = fp16(best_row * scale);  zp_axis = fp16(best_row * lo);  other_axis = fp16(best_col)
 #include "kvb_common.cuh"
+#include "kvb_ptx.cuh"
 
 namespace kvb {
 namespace {
@@ -320,6 +321,7 @@ __global__ void __launch_bounds__(kThreads, 1) append_kernel(LayerView L, const 
     AppendSmem& sm = *reinterpret_cast<AppendSmem*>(smem_raw);
     using G = Geo<D>;
     constexpr int S = G::S;
+    grid_dependency_wait();  // launched while its predecessor still runs: nothing is read or written before it is over
     const int pos0 = positions[0], last = positions[tokens - 1];
     if (pos0 < 0 || last - pos0 != tokens - 1) {  // positions must be contiguous and non-negative
         if (threadIdx.x == 0) L.flag(KVB_ERR_POSITIONS);
@@ -457,8 +459,8 @@ int launch_append(const LayerView& V, const void* k, const void* v, const int32_
         KVB_CUDA_OK(cudaFuncSetAttribute(append_kernel<D, kBf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     }
     const dim3 grid(tokens / kTile + 2, V.kv_heads, 2 * Geo<D>::S);
-    append_kernel<D, kBf16><<<grid, kThreads, smem, stream>>>(V, static_cast<const uint16_t*>(k), static_cast<const uint16_t*>(v), positions, tokens);
-    KVB_CUDA_OK(cudaGetLastError());
+    KVB_CUDA_OK(launch_early(append_kernel<D, kBf16>, grid, dim3(kThreads), smem, stream, V, static_cast<const uint16_t*>(k), static_cast<const uint16_t*>(v),
+                             positions, tokens));
     return KVB_OK;
 }
 
