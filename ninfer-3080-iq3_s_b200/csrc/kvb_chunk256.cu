@@ -96,33 +96,6 @@ __device__ __forceinline__ int scale_exponent(uint32_t bits) {
 __device__ __forceinline__ float pow2i(int e) { return __uint_as_float(static_cast<uint32_t>(e + 127) << 23); }  // |e| <= 126
 __device__ __forceinline__ uint32_t abs_bits(float x) { return __float_as_uint(x) & 0x7FFFFFFFu; }
 
-// Two fp32 values in one register pair: half the issue slots of the scalar forms.
-struct F2 {
-    uint64_t v;
-    __device__ __forceinline__ F2() {}
-    __device__ __forceinline__ explicit F2(uint64_t x) : v(x) {}
-    __device__ __forceinline__ F2(float a, float b) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b)); }
-    __device__ __forceinline__ float2 get() const {
-        float2 r;
-        asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-        return r;
-    }
-};
-__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
-    F2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-    return r;
-}
-__device__ __forceinline__ F2 add2(F2 a, F2 b) {
-    F2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-    return r;
-}
-__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
-    F2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-    return r;
-}
 // x = high + low in fp16 (22 significant bits)
 __device__ __forceinline__ void split2(F2 x, uint32_t& hi, uint32_t& lo) {
     const float2 f = x.get();

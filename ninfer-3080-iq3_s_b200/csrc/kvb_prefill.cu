@@ -1,23 +1,23 @@
-// kvb_prefill.cu -- prefill-chunk attention over the quantised cache on the 5th-generation tensor cores.
+// kvb_prefill.cu -- chunk attention (prefill chunks, wide verify steps) over head_dim-128 caches on the 5th-generation
+// tensor cores.
 //
-// The chunk's (token, q head) rows of one KV head are GQA-packed into tiles of 128 rows; a CTA owns one such
-// tile, one KV head and one range of 128-key tiles, and walks its keys flash-attention style:
+// The chunk's (token, q head) rows of one KV head are GQA-packed into row tiles of 128.  A CTA runs two streams, each with
+// its own S, P and O in tensor memory and its own softmax warps, over 128-key tiles:
 //   S = Q K^T   tcgen05.mma, A = Q tile and B = de-quantised K tile in shared memory (K-major, 128-byte swizzle),
 //               accumulator S[128 x 128] fp32 in tensor memory;
-//   softmax     thread r owns row r (= TMEM lane r): loads S with tcgen05.ld, running max / sum in registers,
-//               writes P (fp16) over the K tile (S is complete by then), rescales the O accumulator in TMEM only
-//               when a row maximum moved;
-//   O += P V    tcgen05.mma, A = P tile (K-major over keys), B = de-quantised V tile (MN-major: one 128-byte row
-//               of 64 dims per key), accumulator O[128 x 128] fp32 in tensor memory.
-// K and V tiles are de-quantised by the CUDA cores straight from the planes (thread = key): nibbles -> fp16 with
-// the exact unpack of the decode kernel, then one fused multiply-add with the tile's per-dim (K) or the key's
-// (V) fp16 scale and zero point.  Dims inside every group of eight are kept in the order the unpack yields
-// (0,4,1,5,2,6,3,7); Q is written in the same order, so the contraction is unaffected, and the merge kernel
+//   softmax     thread r owns row r (= TMEM lane r): reads S in halves with tcgen05.ld, running max / sum in registers,
+//               writes P (fp16) over the columns of S it has read, rescales O in tensor memory only when a row maximum moved;
+//   O += P V    tcgen05.mma, A = P in tensor memory, B = de-quantised V tile (MN-major: one 128-byte row of 64 dims per key),
+//               accumulator O[128 x 128] fp32 in tensor memory.
+// kSplit false: the streams are two row tiles over the same keys (a de-quantised tile serves 256 rows).  kSplit true: one
+// row tile, the streams take the even and the odd key tiles of the CTA's range and leave a partial each.
+// One stream's MMAs run while the other's softmax does.  Sixteen warps de-quantise K and V straight from the planes into
+// two-stage rings (thread = one key, 64 dims): nibbles -> fp16 with the exact unpack, then one fused multiply-add with the
+// tile's per-dim (K) or the key's (V) fp16 scale and zero point.  Dims inside every group of eight are kept in the order the
+// unpack yields (0,4,1,5,2,6,3,7); Q is written in the same order, so the contraction is unaffected, and the merge kernel
 // puts the output dims back.  Keys of the open tile come un-quantised from the stage.
-// Three 32 KB tiles (Q, K/P, V) and 256 TMEM columns per CTA let two CTAs share an SM, so one CTA's CUDA-core
-// phases (de-quantisation, softmax) overlap the other's MMAs.
-// Every wait on an mbarrier is bounded; a wait that gives up sets KVB_ERR_WAIT_TIMEOUT and the CTA leaves
-// through the normal exit (TMEM is freed).
+// Every wait on an mbarrier is bounded and also watches the CTA's abort flag; a wait that gives up sets
+// KVB_ERR_WAIT_TIMEOUT and the CTA leaves through the normal exit (its MMAs are over, TMEM is freed).
 #include <algorithm>
 #include <climits>
 
@@ -29,18 +29,31 @@ namespace kvb {
 namespace {
 
 constexpr int D = 128;
-constexpr int kM = 128;        // query rows per CTA
+constexpr int kM = 128;        // rows per row tile
 constexpr int kN = 128;        // keys per step = one quantisation tile
-constexpr int kThreads = 128;  // thread r <-> query row r <-> TMEM lane r
+constexpr int kStreams = 2;
+// How the 28 warps are divided.  Two row tiles: the softmax is the longer part, its rows are cut into two column halves (a
+// warp for each), eight warps de-quantise.  Split keys (a few rows): the de-quantising is, it gets sixteen warps.
+template <bool kSplit> struct Roles {
+    static constexpr int kHalves = kSplit ? 1 : 2;       // softmax warps per 32 rows of a stream, 128 / kHalves columns each
+    static constexpr int kSoft = 4 * kHalves;            // softmax warps per stream
+    static constexpr int kDq = kSplit ? 8 : 4;           // for K, and again for V
+    static constexpr int kDqWarp = kStreams * kSoft, kMmaWarp = kDqWarp + 2 * kDq;
+    // Registers per thread: 72 at launch (64,512 a CTA), then by role 256 x 112 + 512 x 56 + 128 x 48 = 63,488 (split keys) or
+    // 512 x 80 + 256 x 64 + 128 x 48 = 63,488.
+    static constexpr int kSoftRegs = kSplit ? 112 : 80, kDqRegs = kSplit ? 56 : 64, kMmaRegs = 48;
+};
+constexpr int kWarps = 28, kThreads = 32 * kWarps;
 constexpr int kTileBytes = kM * D * 2;
-constexpr uint32_t kTmemCols = 256;  // S at columns [0,128), O at [128,256)
+constexpr uint32_t kTmemCols = 512, kColO = 256;  // S of stream u at column 128 u, O at 256 + 128 u
+constexpr int kSlotsMeta = 8;  // per-tile words handed to the softmax warps: a writer is at most six tiles ahead of a reader
 
 struct PrefillParams {
     LayerView L;
     const uint16_t* q;         // [T][q_heads][D]
     const int32_t* pos;        // [T]
     const int32_t* total_pos;  // newest position in the cache
-    int T, mtiles, ksplit;
+    int T, mtiles, ksplit;     // ksplit: partials per row
     float scale_log2;
     float* ws_m;               // [H][mtiles][ksplit][128]
     float* ws_l;
@@ -48,16 +61,28 @@ struct PrefillParams {
 };
 
 struct __align__(1024) PrefillSmem {
-    uint8_t q[kTileBytes];
-    uint8_t k[kTileBytes];  // the K tile, then -- once S = Q K^T has completed -- the P tile of the same step
-    uint8_t v[kTileBytes];
-    __half ks[D], kz[D];  // per-dim scale / zero point of the K tile, in tile dim order
-    __half vo[D];         // per-dim other_V of the tile (balanced caches), in tile dim order
-    uint64_t bar_s, bar_o;
+    uint8_t q[kStreams][kTileBytes];
+    uint8_t k[2][kTileBytes];
+    uint8_t v[2][kTileBytes];
+    __half ks[2][D], kz[2][D], vo[2][D];  // per-dim factors by tile parity, in tile dim order
+    uint64_t k_full[2], k_free[2], v_full[2], v_free[2], s_full[kStreams], p_full[kStreams], o_done[kStreams], drain;
     uint32_t tmem_base;
-    int row_pos[kM];
-    int flags[4];
+    int bad_tile[kSlotsMeta];
+    int row_pos[kStreams][kM];
+    float row_top[kStreams][2][kM];  // maximum of a row's column half, exchanged between its two softmax warps
+    int abort_flag;
 };
+
+__device__ __forceinline__ bool chunk_wait(uint64_t* bar, uint32_t parity, int* abort_flag) {
+    bool ok = false;
+    for (uint32_t i = 0; i < kSpinLimit && !ok; ++i) {
+        ok = mbar_try_wait(bar, parity);
+        if (!ok && *reinterpret_cast<volatile int*>(abort_flag) != 0) break;
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) *reinterpret_cast<volatile int*>(abort_flag) = 1;
+    return ok;
+}
 
 // Byte offset of element (row, col) in a [128 rows][128 cols] fp16 tile stored as two 64-column blocks of
 // 128-byte rows, 8-row groups 1024 bytes apart, 16-byte chunks XOR-swizzled with the row (128-byte swizzle).
@@ -76,676 +101,451 @@ __device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
     return r;
 }
 
-// De-quantise one key row (64 code bytes) into the tile: out = code * scale + zp, pairs (d, d+4).
-// kPerDim: scale / zp pairs come from the per-dim tables (K); otherwise s2 / z2 hold the key's pair (V).
-// `other` (caches written with variance balancing): the result is multiplied by the key's other_K (K: o2, both halves)
-// or by the per-dim other_V table (V), reference kvarn128_codec.cuh:331-347; fp16 like the rest of this kernel.
-// ks / kz / vo: the per-dim tables of the tile in shared memory (tile dim order).
-template <bool kPerDim, bool other>
-__device__ __forceinline__ void dequant_row(const uint4 (&codes)[4], uint8_t* tile, int row, const __half* ks, const __half* kz,
-                                            const __half* vo, uint32_t s2, uint32_t z2, uint32_t o2) {
+// One de-quantising role (kDqWarps warps, thread dt): K or V of the CTA's n tiles t0 .. t0 + n - 1, tile j into ring stage j & 1.
+// `other` (caches written with variance balancing): K is multiplied by the key's other_K, V by the per-dim other_V,
+// reference kvarn128_codec.cuh:331-347; fp16 like the rest of this kernel.
+template <bool kValue, bool kOther, int kDqWarps>
+__device__ __forceinline__ bool dequant_role(PrefillSmem& sm, const LayerView& L, int head, int dt, int t0, int n, int kv_total) {
+    // 64 dims of one key per thread with eight warps, all 128 with four; threads 0..127 also fetch the factors of dim dt
+    constexpr int kWords = 64 / kDqWarps;  // 16-byte chunks of the tile row a thread writes
+    const int lane = dt & 31, key = dt & 127, first = kDqWarps == 8 ? 64 * (dt >> 7) : 0;
+    const int32_t* tbl = L.table();
+    const uint8_t* const plane = kValue ? L.v_code : L.k_code;
+    const int sealed_tiles = kv_total / kN;
+    constexpr bool kTables = !kValue || kOther;
+    struct Fetch {
+        uint4 code[kWords / 4];
+        __half d0, d1, t0, t1;  // K: scale, zero point of the dim; other_K of the key.  V: other_V of the dim; scale, zero point of the key
+        bool bad;
+    };
+    // where this thread reads in page 0 of this head, and the page strides
+    const uint8_t* const code_at = plane + page_head_offset(64, L.kv_heads, 0, head) + (key & 63) * 64 + first / 2;
+    constexpr int kLead = kValue ? 4 : 5;  // halves per scale row
+    const __half* const scales = (kValue ? L.v_scale : L.k_scale) + page_head_offset(kLead, L.kv_heads, 0, head);
+    const __half* const tok_at = scales + (key & 63) * kLead + (kValue ? 2 : 4);       // V: scale, zero point of the key; K: other_K
+    const __half* const dim_at = scales + ((dt & 127) >> 1) * kLead + (dt & 1);        // V: other_V of the dim; K: its scale, zero point 2 further
+    const int code_stride = 64 * kPage * L.kv_heads, scale_stride = kLead * kPage * L.kv_heads;
+    int32_t ids[2] = {LayerView::kNoEntry, LayerView::kNoEntry};  // table entries of the tile the next fetch asks for, requested a tile earlier
+    auto lookup = [&](int j) {
+        ids[0] = ids[1] = LayerView::kNoEntry;
+        if (j < n && t0 + j < sealed_tiles) {
+            ids[0] = L.page_entry(tbl, 2 * (t0 + j));
+            ids[1] = L.page_entry(tbl, 2 * (t0 + j) + 1);
+        }
+    };
+    auto fetch = [&](int j, Fetch& f) {
+        const int32_t pg0 = L.checked_page(ids[0]), pg1 = L.checked_page(ids[1]);
+        const bool here = pg0 >= 0 && pg1 >= 0;
+        f.bad = !here && j < n && t0 + j < sealed_tiles;  // reported in the error word; the tile is masked
 #pragma unroll
-    for (int v4 = 0; v4 < 4; ++v4) {
-        const uint4 pk = codes[v4];
-        const uint32_t w[4] = {pk.x, pk.y, pk.z, pk.w};
+        for (int c = 0; c < kWords / 4; ++c) f.code[c] = make_uint4(0u, 0u, 0u, 0u);
+        f.d0 = f.d1 = f.t0 = f.t1 = __ushort_as_half(0);
+        if (here) {
+            const int32_t page = key < kPage ? pg0 : pg1;
+            const uint4* src = reinterpret_cast<const uint4*>(code_at + static_cast<int64_t>(page) * code_stride);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int chunk = v4 * 4 + i;  // dims 8 chunk .. 8 chunk + 7
-            uint32_t u[4];
-            unpack8(w[i], u);
-            uint4 out;
-            if constexpr (kPerDim) {
-                const uint4 sc = *reinterpret_cast<const uint4*>(&ks[8 * chunk]);
-                const uint4 zp = *reinterpret_cast<const uint4*>(&kz[8 * chunk]);
-                out = make_uint4(hfma2_u32(u[0], sc.x, zp.x), hfma2_u32(u[1], sc.y, zp.y), hfma2_u32(u[2], sc.z, zp.z),
-                                 hfma2_u32(u[3], sc.w, zp.w));
-                if constexpr (other) out = make_uint4(hmul2_u32(out.x, o2), hmul2_u32(out.y, o2), hmul2_u32(out.z, o2), hmul2_u32(out.w, o2));
+            for (int c = 0; c < kWords / 4; ++c) f.code[c] = src[c];
+            const __half* tok = tok_at + static_cast<int64_t>(page) * scale_stride;
+            const __half* dim = dim_at + static_cast<int64_t>(pg0) * scale_stride;
+            if constexpr (kValue) {
+                const __half2 sz = *reinterpret_cast<const __half2*>(tok);
+                f.t0 = __low2half(sz);
+                f.t1 = __high2half(sz);
+                if (kOther && dt < D) f.d0 = dim[0];
             } else {
-                out = make_uint4(hfma2_u32(u[0], s2, z2), hfma2_u32(u[1], s2, z2), hfma2_u32(u[2], s2, z2), hfma2_u32(u[3], s2, z2));
-                if constexpr (other) {
-                    const uint4 ot = *reinterpret_cast<const uint4*>(&vo[8 * chunk]);
-                    out = make_uint4(hmul2_u32(out.x, ot.x), hmul2_u32(out.y, ot.y), hmul2_u32(out.z, ot.z), hmul2_u32(out.w, ot.w));
+                if (dt < D) {
+                    f.d0 = dim[0];
+                    f.d1 = dim[2];
+                }
+                if constexpr (kOther) f.t0 = tok[0];
+            }
+        }
+    };
+    Fetch cur, nxt;
+    if (n > 0) {
+        lookup(0);
+        fetch(0, nxt);
+        lookup(1);
+    }
+    bool failed = false;
+    for (int j = 0; j < n; ++j) {
+        const int st = j & 1;
+        const bool sealed = t0 + j < sealed_tiles;
+        cur = nxt;
+        fetch(j + 1, nxt);
+        lookup(j + 2);
+        if constexpr (kTables) {
+            if (dt < D) {
+                if constexpr (kValue) {
+                    sm.vo[st][dim_slot(dt)] = cur.d0;
+                } else {
+                    sm.ks[st][dim_slot(dt)] = cur.d0;
+                    sm.kz[st][dim_slot(dt)] = cur.d1;
                 }
             }
-            *reinterpret_cast<uint4*>(tile + tile_off(row, 8 * chunk)) = out;
+            if (!kValue && dt == 0) sm.bad_tile[j & (kSlotsMeta - 1)] = cur.bad;
+            if (named_barrier_or(kValue ? 2 : 1, 32 * kDqWarps, failed)) return true;
         }
-    }
-}
-
-// Copy one un-quantised fp16 row of the stage into the tile (dims re-ordered inside every group of eight).
-__device__ __forceinline__ void stage_row_to_tile(const __half* __restrict__ src, uint8_t* tile, int row, bool live) {
+        // the stage is free once the MMAs of tile j - 2 have completed
+        if (j > 1 && !chunk_wait(kValue ? &sm.v_free[st] : &sm.k_free[st], ((j >> 1) + 1) & 1, &sm.abort_flag)) {
+            failed = true;
+            if constexpr (!kTables) return true;
+            continue;
+        }
+        uint8_t* tile = kValue ? sm.v[st] : sm.k[st];
+        if (sealed) {
+            const uint32_t s2 = __half_as_ushort(cur.t0) * 0x10001u, z2 = __half_as_ushort(cur.t1) * 0x10001u;
 #pragma unroll
-    for (int chunk = 0; chunk < 16; ++chunk) {
-        uint4 r = live ? reinterpret_cast<const uint4*>(src)[chunk] : make_uint4(0, 0, 0, 0);
-        *reinterpret_cast<uint4*>(tile + tile_off(row, 8 * chunk)) =
-            make_uint4(prmt(r.x, r.z, 0x5410), prmt(r.x, r.z, 0x7632), prmt(r.y, r.w, 0x5410), prmt(r.y, r.w, 0x7632));
-    }
-}
-
-// The Q tile of a CTA: rows (token, q head of this KV head) `first_row` .. + 127 rotated, scaled, rounded to fp16 and
-// stored in tile dim order; rows beyond the chunk are zeros.  One warp per row, lane l holds dims l + 32 j; the rows of
-// a warp are taken eight at a time with every global load issued before the first rotation (a row per iteration cost
-// one memory latency each: 32 us per CTA with four warps).
-__device__ __forceinline__ void build_q_tile(const PrefillParams& P, const LayerView& L, int first_row, int head, int G, uint8_t* q_tile,
-                                             int* row_pos, int warp, int lane) {
-    constexpr int kWarps = kThreads / 32, kBatch = 8;
-    for (int j0 = 0; j0 < kM / kWarps; j0 += kBatch) {
-        uint16_t raw[kBatch][4];
-        int rp[kBatch];
+            for (int c = 0; c < kWords; ++c) {
+                const uint4 cc = cur.code[c >> 2];
+                uint32_t u[4];
+                unpack8((c & 3) == 0 ? cc.x : (c & 3) == 1 ? cc.y : (c & 3) == 2 ? cc.z : cc.w, u);
+                const int at = first + 8 * c;
+                uint4 out;
+                if constexpr (kValue) {
+                    out = make_uint4(hfma2_u32(u[0], s2, z2), hfma2_u32(u[1], s2, z2), hfma2_u32(u[2], s2, z2), hfma2_u32(u[3], s2, z2));
+                    if constexpr (kOther) {
+                        const uint4 ot = *reinterpret_cast<const uint4*>(&sm.vo[st][at]);
+                        out = make_uint4(hmul2_u32(out.x, ot.x), hmul2_u32(out.y, ot.y), hmul2_u32(out.z, ot.z), hmul2_u32(out.w, ot.w));
+                    }
+                } else {
+                    const uint4 sc = *reinterpret_cast<const uint4*>(&sm.ks[st][at]), zp = *reinterpret_cast<const uint4*>(&sm.kz[st][at]);
+                    out = make_uint4(hfma2_u32(u[0], sc.x, zp.x), hfma2_u32(u[1], sc.y, zp.y), hfma2_u32(u[2], sc.z, zp.z), hfma2_u32(u[3], sc.w, zp.w));
+                    if constexpr (kOther) out = make_uint4(hmul2_u32(out.x, s2), hmul2_u32(out.y, s2), hmul2_u32(out.z, s2), hmul2_u32(out.w, s2));
+                }
+                *reinterpret_cast<uint4*>(tile + tile_off(key, at)) = out;
+            }
+        } else {  // un-quantised fp16 rows of the stage (dims re-ordered inside every group of eight)
+            const int t = t0 + j;
+            const uint4* src = reinterpret_cast<const uint4*>(L.stage_row(kValue ? 1 : 0, t & 1, head, key) + first);
+            const bool live = t * kN + key < kv_total;
 #pragma unroll
-        for (int jj = 0; jj < kBatch; ++jj) {
-            const int r = warp + kWarps * (j0 + jj), R = first_row + r, tq = R / G, gq = R % G;
-            rp[jj] = -1;
-            raw[jj][0] = raw[jj][1] = raw[jj][2] = raw[jj][3] = 0;
-            if (tq < P.T) {
-                const uint16_t* qrow = P.q + (static_cast<int64_t>(tq) * L.q_heads + head * G + gq) * D;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) raw[jj][j] = qrow[lane + 32 * j];
-                rp[jj] = P.pos[tq];
+            for (int c = 0; c < kWords; ++c) {
+                const uint4 r = live ? src[c] : make_uint4(0u, 0u, 0u, 0u);
+                *reinterpret_cast<uint4*>(tile + tile_off(key, first + 8 * c)) =
+                    make_uint4(prmt(r.x, r.z, 0x5410), prmt(r.x, r.z, 0x7632), prmt(r.y, r.w, 0x5410), prmt(r.y, r.w, 0x7632));
             }
         }
-#pragma unroll
-        for (int jj = 0; jj < kBatch; ++jj) {
-            const int r = warp + kWarps * (j0 + jj);
-            float v[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = L.dtype == KVB_DTYPE_BF16 ? in_to_f32<true>(raw[jj][j]) : in_to_f32<false>(raw[jj][j]);
-            if (rp[jj] >= 0) hadamard_warp<D>(v, lane);  // warp-uniform: a row is real or not for the whole warp
-            if (lane == 0) row_pos[r] = rp[jj];
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                *reinterpret_cast<__half*>(q_tile + tile_off(r, dim_slot(lane + 32 * j))) = __float2half_rn(v[j] * P.scale_log2);
-        }
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(kValue ? &sm.v_full[st] : &sm.k_full[st]);
     }
+    return failed;
 }
 
-// kOther: the cache carries balancing factors different from 1 (Sinkhorn iterations > 0).
-template <bool kOther>
-__global__ void __launch_bounds__(kThreads, 2) prefill_kernel(const PrefillParams P) {
+template <bool kSplit, bool kOther>
+__global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     // the swizzled tiles need a 1024-byte aligned base; the launch reserves 1024 spare bytes for this
     PrefillSmem& sm = *reinterpret_cast<PrefillSmem*>(smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u));
-    const LayerView& L = P.L;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int mt = blockIdx.x, head = blockIdx.y, zs = blockIdx.z;
-    const int G = L.q_heads / L.kv_heads;
-    const int kv_total = *P.total_pos + 1;
-
-    if (warp == 0) tc::tmem_alloc(&sm.tmem_base, kTmemCols);
-    if (tid == 0) {
-        mbar_init(&sm.bar_s, 1);
-        mbar_init(&sm.bar_o, 1);
-        mbar_fence_init();
-        sm.flags[0] = 0;
-    }
-    build_q_tile(P, L, mt * kM, head, G, sm.q, sm.row_pos, warp, lane);
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
-    const uint32_t tmem_s = sm.tmem_base, tmem_o = sm.tmem_base + kN;
-    const uint32_t lane_base = static_cast<uint32_t>(32 * warp) << 16;
-
-    int max_pos = -1, min_pos = INT_MAX;
-    for (int r = 0; r < kM; ++r) {
-        const int p = sm.row_pos[r];
-        if (p >= 0) { max_pos = max(max_pos, p); min_pos = min(min_pos, p); }
-    }
-    const int my_pos = sm.row_pos[tid];
-    // key tiles this CTA walks: those a row of the tile can see, cut into ksplit ranges
-    const int ntiles = max_pos < 0 ? 0 : min((kv_total + kN - 1) / kN, max_pos / kN + 1);
-    const int t0 = static_cast<int>(static_cast<int64_t>(ntiles) * zs / P.ksplit);
-    const int t1 = static_cast<int>(static_cast<int64_t>(ntiles) * (zs + 1) / P.ksplit);
-    const int32_t* tbl = L.table();
-    constexpr bool other = kOther;
-    const uint32_t idesc_qk = tc::idesc_f16(kM, kN, false, false), idesc_pv = tc::idesc_f16(kM, D, false, true);
-    const uint32_t q_addr = smem_u32(sm.q), k_addr = smem_u32(sm.k), v_addr = smem_u32(sm.v);
-
-    float m_run = -INFINITY, l_run = 0.0f;
-    bool have_o = false, failed = false;
-    uint32_t it = 0;
-    const bool warp_has_rows = __any_sync(0xffffffffu, my_pos >= 0);  // warps without a valid row skip the softmax
-
-    // Everything a tile needs from global memory before its K side can be de-quantised; fetched one tile ahead
-    // so that the page-table lookup and the load latency hide behind the previous tile's softmax.
-    struct KFetch {
-        uint4 codes[4], vcodes[4];
-        uint32_t vsz;
-        __half ks, kz;
-        __half ko, vo;  // balanced caches: other_K of this thread's key, other_V of this thread's dim
-        int32_t page;  // page of this thread's key (-1: tile unusable)
-        bool sealed, ok;
-    };
-    // The physical pages of a tile are looked up one step before its codes are requested (ids_a / ids_b: pages of the
-    // tile the next fetch_k asks for): page id -> code address is a dependent trip to L2 that would otherwise stall
-    // every step for about 0.3 us.
-    int32_t ids_a = LayerView::kNoEntry, ids_b = LayerView::kNoEntry;
-    auto lookup = [&](int t) {
-        ids_a = ids_b = LayerView::kNoEntry;
-        if (t < t1 && t * kN + kN <= kv_total) {
-            ids_a = L.page_entry(tbl, 2 * t);
-            ids_b = L.page_entry(tbl, 2 * t + 1);
-        }
-    };
-    auto fetch_k = [&](int t, KFetch& f) {  // uses the pages `lookup(t)` found, then looks up those of tile t + 1
-        f.sealed = t * kN + kN <= kv_total;
-        f.ok = t < t1;
-        f.page = -1;
-        const int32_t pg0 = L.checked_page(ids_a), pg1 = L.checked_page(ids_b);
-        lookup(t + 1);
-        if (!f.ok || !f.sealed) return;
-        if (pg0 < 0 || pg1 < 0) { f.ok = false; return; }  // reported in the error word; every thread skips the tile alike
-        f.page = tid < 64 ? pg0 : pg1;
-        const uint4* kc = reinterpret_cast<const uint4*>(L.k_code + page_head_offset(64, L.kv_heads, f.page, head) + (tid & 63) * 64);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) f.codes[i] = kc[i];
-        const uint4* vc = reinterpret_cast<const uint4*>(L.v_code + page_head_offset(64, L.kv_heads, f.page, head) + (tid & 63) * 64);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) f.vcodes[i] = vc[i];
-        f.vsz = *reinterpret_cast<const uint32_t*>(L.v_scale + page_head_offset(4, L.kv_heads, f.page, head) + (tid & 63) * 4 + 2);
-        // per-dim scale / zero point of the tile (stored in both pages): page row d/2 = [s s z z other]
-        const __half* ksp = L.k_scale + page_head_offset(5, L.kv_heads, pg0, head);
-        f.ks = ksp[(tid >> 1) * 5 + (tid & 1)];
-        f.kz = ksp[(tid >> 1) * 5 + 2 + (tid & 1)];
-        if constexpr (other) {  // K scale row of a token ends with its other_K; V scale row d / 2 starts with other_V(d), other_V(d + 1)
-            f.ko = L.k_scale[page_head_offset(5, L.kv_heads, f.page, head) + (tid & 63) * 5 + 4];
-            f.vo = L.v_scale[page_head_offset(4, L.kv_heads, pg0, head) + (tid >> 1) * 4 + (tid & 1)];
-        }
-    };
-    KFetch cur, nxt;
-    lookup(t0);
-    fetch_k(t0, nxt);
-    bool tables_ready = false;  // the scale tables of this tile were written during the previous step (saves a barrier)
-    for (int t = t0; t < t1; ++t) {
-        cur = nxt;
-        const int base = t * kN;
-        const bool sealed = cur.sealed;
-        if (!cur.ok) { fetch_k(t + 1, nxt); tables_ready = false; continue; }
-        if (!tables_ready) {
-            if (sealed) {
-                sm.ks[dim_slot(tid)] = cur.ks;
-                sm.kz[dim_slot(tid)] = cur.kz;
-                if constexpr (other) sm.vo[dim_slot(tid)] = cur.vo;
-            }
-            __syncthreads();  // scale tables visible
-        }
-        // ---- K tile -> shared memory (the previous P V does not touch the K buffer: P lives in tensor memory)
-        if (sealed) {
-            dequant_row<true, other>(cur.codes, sm.k, tid, sm.ks, sm.kz, sm.vo, 0, 0, other ? __half_as_ushort(cur.ko) * 0x10001u : 0u);
-        } else {
-            stage_row_to_tile(L.stage_row(0, t & 1, head, tid), sm.k, tid, base + tid < kv_total);
-        }
-        // ---- the previous P V reads P from the columns S = Q K^T is about to overwrite, and the V buffer: drain it
-        if (have_o && !mbar_wait_bounded(&sm.bar_o, (it - 1) & 1)) { failed = true; }
-        fence_proxy_async();
-        __syncthreads();
-        if (warp == 0) {  // the whole warp computes the (warp-uniform) operands, one elected lane issues
-            tc::fence_after_sync();
-#pragma unroll
-            for (int kk = 0; kk < 8; ++kk) {
-                const uint32_t o = (kk >> 2) * 16384 + (kk & 3) * 32;
-                tc::mma_f16_ss(tmem_s, tc::smem_desc(q_addr + o, 16, 1024), tc::smem_desc(k_addr + o, 16, 1024), idesc_qk, kk > 0);
-            }
-            tc::commit(&sm.bar_s);
-        }
-        // ---- V tile -> shared memory (overlaps the QK MMA), then start fetching the next tile
-        if (sealed) {
-            dequant_row<false, other>(cur.vcodes, sm.v, tid, sm.ks, sm.kz, sm.vo, prmt(cur.vsz, cur.vsz, 0x1010), prmt(cur.vsz, cur.vsz, 0x3232), 0u);
-        } else {
-            stage_row_to_tile(L.stage_row(1, t & 1, head, tid), sm.v, tid, base + tid < kv_total);
-        }
-        fetch_k(t + 1, nxt);  // (issuing this at the top of the step was measured slower)
-        // ---- softmax of row `tid`
-        if (!mbar_wait_bounded(&sm.bar_s, it & 1)) { failed = true; }  // a warp that gave up reads stale S; the CTA agrees below
-        tc::fence_after_sync();
-        if (warp_has_rows) {
-        float s[kN];
-        {  // the four loads are in flight together: one round trip to tensor memory, not four
-            uint32_t r0[32], r1[32], r2[32], r3[32];
-            tc::tmem_ld32(tmem_s + lane_base, r0);
-            tc::tmem_ld32(tmem_s + lane_base + 32, r1);
-            tc::tmem_ld32(tmem_s + lane_base + 64, r2);
-            tc::tmem_ld32(tmem_s + lane_base + 96, r3);
-            tc::tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                s[j] = __uint_as_float(r0[j]);
-                s[32 + j] = __uint_as_float(r1[j]);
-                s[64 + j] = __uint_as_float(r2[j]);
-                s[96 + j] = __uint_as_float(r3[j]);
-            }
-        }
-        if (base + kN - 1 > min_pos || !sealed) {
-#pragma unroll
-            for (int j = 0; j < kN; ++j)
-                if (base + j > my_pos || base + j >= kv_total) s[j] = -INFINITY;
-        }
-        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // four chains: two warps per scheduler hide little latency
-#pragma unroll
-        for (int j = 0; j < kN; ++j) mx4[j & 3] = fmaxf(mx4[j & 3], s[j]);
-        const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-        // The reference point of the row's exponentials follows the running maximum lazily: it moves only when the
-        // maximum has grown by more than 2^kLazy, so P stays below 2^kLazy (exact enough in fp16, whose precision is
-        // relative) and the O accumulator is rescaled a few times per walk instead of at every new maximum.
-        constexpr float kLazy = 8.0f;
-        const bool grown = mx > m_run + kLazy || (m_run == -INFINITY && mx > -INFINITY);
-        const float m_new = grown ? mx : m_run;
-        const float m_use = m_new == -INFINITY ? 0.0f : m_new;
-        const float alpha = grown ? fast_exp2(m_run - m_use) : 1.0f;
-        const bool moved = have_o && grown;
-        m_run = m_new;
-        float sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        // P stays in tensor memory: fp16 pairs over the first 64 columns of S (already in registers), the A operand
-        // of the P V product -- no shared-memory round trip for P
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            uint32_t pk[32];
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                const float p0 = fast_exp2(s[64 * c + 2 * j] - m_use), p1 = fast_exp2(s[64 * c + 2 * j + 1] - m_use);
-                sum4[j & 3] += p0 + p1;
-                pk[j] = pack_half2(p0, p1);
-            }
-            tc::tmem_st32(tmem_s + lane_base + 32 * c, pk);
-        }
-        tc::tmem_st_wait();
-        l_run = l_run * alpha + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
-        if (__any_sync(0xffffffffu, moved)) {  // rescale this warp's 32 rows of O (alpha = 1 for rows that did not move)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                uint32_t r[32];
-                tc::tmem_ld32(tmem_o + lane_base + 32 * c, r);
-                tc::tmem_ld_wait();
-#pragma unroll
-                for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * alpha);
-                tc::tmem_st32(tmem_o + lane_base + 32 * c, r);
-            }
-            tc::tmem_st_wait();
-        }
-        }  // warp_has_rows (rows of the other warps are never read: their P and O may hold anything)
-        // the scale tables of the next tile: this tile's K rows were de-quantised two barriers ago
-        tables_ready = nxt.ok;
-        if (nxt.ok && nxt.sealed) {
-            sm.ks[dim_slot(tid)] = nxt.ks;
-            sm.kz[dim_slot(tid)] = nxt.kz;
-        }
-        // ---- O += P V (every warp has its V rows in shared memory and its P rows in tensor memory; any failed wait ends the walk)
-        fence_proxy_async();
-        tc::fence_before_sync();
-        if (__syncthreads_or(failed)) { failed = true; break; }
-        if constexpr (other) {
-            if (nxt.ok && nxt.sealed) sm.vo[dim_slot(tid)] = nxt.vo;  // every thread is past this tile's V rows
-        }
-        if (warp == 0) {  // the whole warp computes the (warp-uniform) operands, one elected lane issues
-            tc::fence_after_sync();
-#pragma unroll
-            for (int kk = 0; kk < 8; ++kk) {
-                tc::mma_f16_ts(tmem_o, tmem_s + 8 * kk, tc::smem_desc(v_addr + kk * 2048, 16384, 1024), idesc_pv, have_o || kk > 0);  // 16 keys = 8 columns of P
-            }
-            tc::commit(&sm.bar_o);
-        }
-        have_o = true;
-        ++it;
-    }
-    if (have_o && !failed && !mbar_wait_bounded(&sm.bar_o, (it - 1) & 1)) failed = true;
-    if (failed && tid == 0) L.flag(KVB_ERR_WAIT_TIMEOUT);
-    tc::fence_after_sync();
-
-    // ---- partial of this (row tile, key range): m (log2 units), l, o in tile dim order
-    const int64_t idx = ((static_cast<int64_t>(head) * P.mtiles + mt) * P.ksplit + zs) * kM + tid;
-    if (my_pos >= 0) {
-        P.ws_m[idx] = failed ? -INFINITY : m_run;
-        P.ws_l[idx] = failed ? 0.0f : l_run;
-    }
-    float* orow = P.ws_o + idx * D;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        if (!warp_has_rows) break;
-        uint32_t r[32];
-        if (have_o) {
-            tc::tmem_ld32(tmem_o + lane_base + 32 * c, r);
-            tc::tmem_ld_wait();
-        }
-        if (my_pos < 0) continue;
-#pragma unroll
-        for (int j = 0; j < 32; j += 4)
-            *reinterpret_cast<float4*>(orow + 32 * c + j) =
-                have_o && !failed ? make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]))
-                                  : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    tc::fence_before_sync();
-    __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(sm.tmem_base, kTmemCols);
-}
-
-// ---------------------------------------------------------------------------------------------------------
-// verify_kernel: the same attention for a verify step (at most 64 GQA-merged rows: 8 tokens x 8 query heads per KV
-// head), with the two halves of the CTA given different work.  Only TMEM lanes 0-63 hold rows, so only warps 0 and 1
-// have a softmax to do; in prefill_kernel warps 2 and 3 idle through it and every warp de-quantises a quarter of
-// each tile in between.  Here
-//   warps 2, 3   de-quantise: K(t+1) into the K buffer as soon as S(t) = Q K(t)^T has completed -- while warps 0, 1
-//                are busy with the softmax of step t -- and V(t+1) as soon as P V(t) has completed; thread = one key
-//                row of each page of the tile; codes fetched a tile ahead;
-//   warps 0, 1   softmax of their rows; warp 0 also issues the MMAs (one elected lane): Q K^T when the K tile is
-//                ready, P V when both warps have stored P and the V tile is ready.
-// The chain of a step shrinks from de-quantise + issue + softmax + issue to issue + softmax + issue.  Hand-offs are
-// mbarriers (bounded waits that also watch a CTA-wide abort flag); the two warps of a half meet at a named barrier
-// once per step, and a warp whose wait gave up still goes to that barrier before it leaves, so nobody is left waiting.
-struct __align__(1024) VerifySmem {
-    uint8_t q[kTileBytes];
-    uint8_t k[kTileBytes];
-    uint8_t v[kTileBytes];
-    __half ks[2][D], kz[2][D], vo[2][D];  // per-dim tables of the tile, by step parity
-    uint64_t bar_s, bar_o, k_ready, v_ready;
-    uint32_t tmem_base;
-    int row_pos[kM];
-    int abort_flag, bad_tile;
-};
-
-__device__ __forceinline__ bool verify_wait(uint64_t* bar, uint32_t parity, VerifySmem& sm) {
-    bool ok = false;
-    for (uint32_t i = 0; i < kSpinLimit && !ok; ++i) {
-        ok = mbar_try_wait(bar, parity);
-        if (!ok && *reinterpret_cast<volatile int*>(&sm.abort_flag) != 0) break;
-    }
-    ok = __all_sync(0xffffffffu, ok);
-    if (!ok) *reinterpret_cast<volatile int*>(&sm.abort_flag) = 1;
-    return ok;
-}
-
-template <bool kOther>
-__global__ void __launch_bounds__(kThreads, 2) verify_kernel(const PrefillParams P) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    VerifySmem& sm = *reinterpret_cast<VerifySmem*>(smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u));
+    using Ro = Roles<kSplit>;
     const LayerView& L = P.L;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int head = blockIdx.y, zs = blockIdx.z;
+    constexpr int kDqWarps = Ro::kDq, kDqWarp = Ro::kDqWarp, kMmaWarp = Ro::kMmaWarp;
+    static_assert(kMmaWarp + 4 == kWarps, "roles");
+    constexpr int kRowTiles = kSplit ? 1 : 2;
+    const int mt = kRowTiles * blockIdx.x;
     const int G = L.q_heads / L.kv_heads;
     const int kv_total = *P.total_pos + 1;
 
-    if (warp == 0) tc::tmem_alloc(&sm.tmem_base, kTmemCols);
+    if (warp == kMmaWarp) tc::tmem_alloc(&sm.tmem_base, kTmemCols);
     if (tid == 0) {
-        mbar_init(&sm.bar_s, 1);
-        mbar_init(&sm.bar_o, 1);
-        mbar_init(&sm.k_ready, 2);  // lane 0 of each de-quantising warp
-        mbar_init(&sm.v_ready, 2);
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&sm.k_full[b], kDqWarps);
+            mbar_init(&sm.v_full[b], kDqWarps);
+            mbar_init(&sm.k_free[b], 1);
+            mbar_init(&sm.v_free[b], 1);
+            mbar_init(&sm.s_full[b], 1);
+            mbar_init(&sm.p_full[b], Ro::kSoft);
+            mbar_init(&sm.o_done[b], 1);
+        }
+        mbar_init(&sm.drain, 1);
         mbar_fence_init();
         sm.abort_flag = 0;
-        sm.bad_tile = 0;
     }
-    build_q_tile(P, L, 0, head, G, sm.q, sm.row_pos, warp, lane);  // rows beyond the step's are zeros; the MMA reads all 128
+    // ---- Q: rows rotated, scaled, rounded to fp16, in tile dim order; rows beyond the chunk are zeros.  One warp per row, lane l
+    //      holds dims l + 32 j, the loads of four rows in flight.
+    constexpr int kQBatch = 4, kRows = kRowTiles * kM;
+    for (int r0 = warp; r0 < kRows; r0 += kQBatch * kWarps) {
+        uint16_t raw[kQBatch][4];
+        int rp[kQBatch];
+#pragma unroll
+        for (int u = 0; u < kQBatch; ++u) {
+            const int r = r0 + u * kWarps, R = mt * kM + r, tq = R / G, gq = R % G;
+            rp[u] = -1;
+            raw[u][0] = raw[u][1] = raw[u][2] = raw[u][3] = 0;
+            if (r < kRows && tq < P.T) {
+                const uint16_t* qrow = P.q + (static_cast<int64_t>(tq) * L.q_heads + head * G + gq) * D;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) raw[u][j] = qrow[lane + 32 * j];
+                rp[u] = P.pos[tq];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kQBatch; ++u) {
+            const int r = r0 + u * kWarps;
+            if (r >= kRows) break;
+            float v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = L.dtype == KVB_DTYPE_BF16 ? in_to_f32<true>(raw[u][j]) : in_to_f32<false>(raw[u][j]);
+            if (rp[u] >= 0) hadamard_warp<D>(v, lane);  // warp-uniform: a row is real or not for the whole warp
+            if (lane == 0) sm.row_pos[r >> 7][r & 127] = rp[u];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                *reinterpret_cast<__half*>(sm.q[r >> 7] + tile_off(r & 127, dim_slot(lane + 32 * j))) = __float2half_rn(v[j] * P.scale_log2);
+        }
+    }
     fence_proxy_async();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    const uint32_t tmem_s = sm.tmem_base, tmem_o = sm.tmem_base + kN;
-    int max_pos = -1, min_pos = INT_MAX;
-    for (int r = 0; r < 64; ++r) {
-        const int p = sm.row_pos[r];
-        if (p >= 0) { max_pos = max(max_pos, p); min_pos = min(min_pos, p); }
-    }
+    const uint32_t tmem = sm.tmem_base;
+    int max_pos = -1;
+    for (int i = lane; i < kRows; i += 32) max_pos = max(max_pos, sm.row_pos[i >> 7][i & 127]);
+    max_pos = __reduce_max_sync(0xffffffffu, max_pos);
+    // key tiles this CTA walks: those a row can see, cut into ranges
+    const int ranges = kSplit ? P.ksplit / 2 : P.ksplit;
     const int ntiles = max_pos < 0 ? 0 : min((kv_total + kN - 1) / kN, max_pos / kN + 1);
-    const int t0 = static_cast<int>(static_cast<int64_t>(ntiles) * zs / P.ksplit);
-    const int t1 = static_cast<int>(static_cast<int64_t>(ntiles) * (zs + 1) / P.ksplit);
-    const int n = t1 - t0;
+    const int t0 = static_cast<int>(static_cast<int64_t>(ntiles) * zs / ranges);
+    const int n = static_cast<int>(static_cast<int64_t>(ntiles) * (zs + 1) / ranges) - t0;
+    // stream u takes tiles u, u + 2, .. of the range (kSplit) or all of them for its row tile (none if it has no rows)
+    auto steps_of = [&](int u) { return kSplit ? (n + 1 - u) / 2 : u == 0 || (mt + 1) * kM < P.T * G ? n : 0; };
     bool failed = false;
-    volatile int* abort_flag = &sm.abort_flag;
 
-    if (warp >= 2) {
+    if (warp >= kDqWarp && warp < kMmaWarp) {
         // =========================== de-quantise ===========================
-        const int dt = tid - 64;  // key rows dt of both pages of the tile (tile rows dt and dt + 64); dims dt and dt + 64
-        const int32_t* tbl = L.table();
-        struct Fetch {
-            uint4 codes[2][4], vcodes[2][4];
-            uint32_t vsz[2];
-            __half ks[2], kz[2], ko[2], vo[2];
-            bool bad;
-        };
-        int32_t ids_a = LayerView::kNoEntry, ids_b = LayerView::kNoEntry;  // pages of the tile the next fetch asks for, looked up a step earlier
-        auto sealed_tile = [&](int t) { return t * kN + kN <= kv_total; };
-        auto lookup = [&](int t) {
-            ids_a = ids_b = LayerView::kNoEntry;
-            if (t < t1 && sealed_tile(t)) {
-                ids_a = L.page_entry(tbl, 2 * t);
-                ids_b = L.page_entry(tbl, 2 * t + 1);
-            }
-        };
-        auto fetch = [&](int t, Fetch& f) {
-            int32_t pg[2] = {L.checked_page(ids_a), L.checked_page(ids_b)};
-            lookup(t + 1);
-            f.bad = false;
-            if (t >= t1 || !sealed_tile(t)) return;
-            if (pg[0] < 0 || pg[1] < 0) { f.bad = true; pg[0] = pg[1] = 0; }  // reported in the error word; the tile is masked
+        tc::regs_dec<Ro::kDqRegs>();
+        const int dt = tid - 32 * kDqWarp;
+        if (dt < 32 * kDqWarps) failed = dequant_role<false, kOther, kDqWarps>(sm, L, head, dt, t0, n, kv_total);
+        else failed = dequant_role<true, kOther, kDqWarps>(sm, L, head, dt - 32 * kDqWarps, t0, n, kv_total);
+    } else if (warp >= kMmaWarp) {
+        // =========================== MMA issue (one warp; the three beside it complete the warpgroup) ===========================
+        tc::regs_dec<Ro::kMmaRegs>();
+        if (warp == kMmaWarp) {
+            constexpr uint32_t idesc_qk = tc::idesc_f16(kM, kN, false, false), idesc_pv = tc::idesc_f16(kM, D, false, true);
+            const int steps[kStreams] = {steps_of(0), steps_of(1)};
+            for (int i = 0; i <= steps[0] && !failed; ++i) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint4* kc = reinterpret_cast<const uint4*>(L.k_code + page_head_offset(64, L.kv_heads, pg[h], head) + dt * 64);
-                const uint4* vc = reinterpret_cast<const uint4*>(L.v_code + page_head_offset(64, L.kv_heads, pg[h], head) + dt * 64);
+                for (int u = 0; u < kStreams; ++u) {
+                    if (i > steps[u]) continue;
+                    // V of step i - 1 and K of step i are there well before P: waited for first, off the chain P -> PV -> S
+                    if (i < steps[u]) {
+                        const int j = kSplit ? 2 * i + u : i;
+                        if (!chunk_wait(&sm.k_full[j & 1], (j >> 1) & 1, &sm.abort_flag)) { failed = true; break; }
+                    }
+                    if (i > 0) {  // O_u += P V of the stream's step i - 1
+                        const int j = kSplit ? 2 * (i - 1) + u : i - 1;
+                        if (!chunk_wait(&sm.v_full[j & 1], (j >> 1) & 1, &sm.abort_flag) || !chunk_wait(&sm.p_full[u], (i - 1) & 1, &sm.abort_flag)) { failed = true; break; }
+                        tc::fence_after_sync();
+                        const uint32_t v_addr = smem_u32(sm.v[j & 1]);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    f.codes[h][i] = kc[i];
-                    f.vcodes[h][i] = vc[i];
+                        for (int kk = 0; kk < 8; ++kk)  // 16 keys = 8 columns of P
+                            tc::mma_f16_ts(tmem + kColO + 128 * u, tmem + 128 * u + (Ro::kHalves == 2 && kk >= 4 ? 64 - 32 : 0) + 8 * kk, tc::smem_desc(v_addr + kk * 2048, 16384, 1024), idesc_pv, i > 1 || kk > 0);
+                        tc::commit(&sm.o_done[u]);
+                        if (kSplit || u == 1 || steps[1] == 0) tc::commit(&sm.v_free[j & 1]);
+                        // the next S_u is written over this P
+                        if (!chunk_wait(&sm.o_done[u], (i - 1) & 1, &sm.abort_flag)) { failed = true; break; }
+                    }
+                    if (i < steps[u]) {
+                        const int j = kSplit ? 2 * i + u : i;
+                        tc::fence_after_sync();
+                        const uint32_t q_addr = smem_u32(sm.q[kSplit ? 0 : u]), k_addr = smem_u32(sm.k[j & 1]);
+#pragma unroll
+                        for (int kk = 0; kk < 8; ++kk) {
+                            const uint32_t o = (kk >> 2) * 16384 + (kk & 3) * 32;
+                            tc::mma_f16_ss(tmem + 128 * u, tc::smem_desc(q_addr + o, 16, 1024), tc::smem_desc(k_addr + o, 16, 1024), idesc_qk, kk > 0);
+                        }
+                        tc::commit(&sm.s_full[u]);
+                        if (kSplit || u == 1 || steps[1] == 0) tc::commit(&sm.k_free[j & 1]);
+                    }
                 }
-                f.vsz[h] = *reinterpret_cast<const uint32_t*>(L.v_scale + page_head_offset(4, L.kv_heads, pg[h], head) + dt * 4 + 2);
-                // per-dim entries of the tile (stored in both pages): this thread's dims are dt and dt + 64
-                const int d = dt + 64 * h;
-                const __half* ksp = L.k_scale + page_head_offset(5, L.kv_heads, pg[0], head);
-                f.ks[h] = ksp[(d >> 1) * 5 + (d & 1)];
-                f.kz[h] = ksp[(d >> 1) * 5 + 2 + (d & 1)];
-                if constexpr (kOther) {
-                    f.ko[h] = L.k_scale[page_head_offset(5, L.kv_heads, pg[h], head) + dt * 5 + 4];
-                    f.vo[h] = L.v_scale[page_head_offset(4, L.kv_heads, pg[0], head) + (d >> 1) * 4 + (d & 1)];
-                }
             }
-        };
-        Fetch cur, nxt;
-        if (n > 0) {
-            lookup(t0);
-            fetch(t0, nxt);
-        }
-        for (int i = 0; i < n; ++i) {
-            const int t = t0 + i, base = t * kN, par = i & 1;
-            const bool sealed = sealed_tile(t);
-            cur = nxt;
-            // ---- K: the buffer (and the tables of this parity) are free once S(i-1) has completed
-            if (!failed && i > 0 && !verify_wait(&sm.bar_s, (i - 1) & 1, sm)) failed = true;
-            if (!failed && sealed) {
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    sm.ks[par][dim_slot(dt + 64 * h)] = cur.ks[h];
-                    sm.kz[par][dim_slot(dt + 64 * h)] = cur.kz[h];
-                    if constexpr (kOther) sm.vo[par][dim_slot(dt + 64 * h)] = cur.vo[h];
-                }
-                if (dt == 0 && cur.bad) sm.bad_tile = 1;  // sticky: the error word is set, the result is void anyway
+            if (failed) {  // nothing of this CTA may still run when its tensor memory is given back
+                tc::commit(&sm.drain);
+                mbar_wait_bounded(&sm.drain, 0);
             }
-            named_barrier_sync(2, 64);  // tables visible to both warps; a warp that gave up meets its partner here
-            if (*abort_flag) break;
-            if (sealed) {
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-                    dequant_row<true, kOther>(cur.codes[h], sm.k, dt + 64 * h, sm.ks[par], sm.kz[par], sm.vo[par], 0, 0,
-                                              kOther ? __half_as_ushort(cur.ko[h]) * 0x10001u : 0u);
-            } else {
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-                    stage_row_to_tile(L.stage_row(0, t & 1, head, dt + 64 * h), sm.k, dt + 64 * h, base + dt + 64 * h < kv_total);
-            }
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.k_ready);
-            fetch(t + 1, nxt);
-            // ---- V: the buffer is free once P V(i-1) has completed
-            if (i > 0 && !verify_wait(&sm.bar_o, (i - 1) & 1, sm)) { failed = true; continue; }
-            if (sealed) {
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-                    dequant_row<false, kOther>(cur.vcodes[h], sm.v, dt + 64 * h, sm.ks[par], sm.kz[par], sm.vo[par],
-                                               prmt(cur.vsz[h], cur.vsz[h], 0x1010), prmt(cur.vsz[h], cur.vsz[h], 0x3232), 0u);
-            } else {
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-                    stage_row_to_tile(L.stage_row(1, t & 1, head, dt + 64 * h), sm.v, dt + 64 * h, base + dt + 64 * h < kv_total);
-            }
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.v_ready);
         }
     } else {
-        // =========================== softmax (warps 0, 1) and MMA issue (warp 0) ===========================
-        const uint32_t lane_base = static_cast<uint32_t>(32 * warp) << 16;
-        const int my_pos = sm.row_pos[tid];
+        // =========================== softmax of stream u ===========================
+        tc::regs_inc<Ro::kSoftRegs>();
+        const int u = warp / Ro::kSoft, half = (warp % Ro::kSoft) >> 2, row = tid & 127;
+        const uint32_t lane_base = static_cast<uint32_t>(32 * (warp & 3)) << 16;
+        constexpr int kCols = kN / Ro::kHalves;  // columns of S (and of O) this warp works on, from column kCols * half
+        // P of a column half lies over the first half of its own columns of S: no warp writes over what another still reads
+        const uint32_t ts = tmem + 128 * u + kCols * half + lane_base, to = tmem + kColO + 128 * u + kCols * half + lane_base;
+        const int my_pos = kSplit ? sm.row_pos[0][row] : sm.row_pos[u][row];
         const bool warp_has_rows = __any_sync(0xffffffffu, my_pos >= 0);
-        const uint32_t idesc_qk = tc::idesc_f16(kM, kN, false, false), idesc_pv = tc::idesc_f16(kM, D, false, true);
-        const uint32_t q_addr = smem_u32(sm.q), k_addr = smem_u32(sm.k), v_addr = smem_u32(sm.v);
+        const int min_pos = __reduce_min_sync(0xffffffffu, my_pos < 0 ? INT_MAX : my_pos);
+        const int steps = steps_of(u);
         float m_run = -INFINITY, l_run = 0.0f;
-        for (int i = 0; i < n; ++i) {
-            const int base = (t0 + i) * kN;
-            const bool sealed = base + kN <= kv_total;
-            if (warp == 0 && !failed) {  // S(i) = Q K(i)^T: the K tile is ready; P V(i-1), which reads P from the columns of S, has completed
-                if (!verify_wait(&sm.k_ready, i & 1, sm) || (i > 0 && !verify_wait(&sm.bar_o, (i - 1) & 1, sm))) {
-                    failed = true;
-                } else {
-                    tc::fence_after_sync();
-#pragma unroll
-                    for (int kk = 0; kk < 8; ++kk) {
-                        const uint32_t o = (kk >> 2) * 16384 + (kk & 3) * 32;
-                        tc::mma_f16_ss(tmem_s, tc::smem_desc(q_addr + o, 16, 1024), tc::smem_desc(k_addr + o, 16, 1024), idesc_qk, kk > 0);
-                    }
-                    tc::commit(&sm.bar_s);
-                }
-            }
-            if (!failed && !verify_wait(&sm.bar_s, i & 1, sm)) failed = true;
+        for (int i = 0; i < steps; ++i) {
+            const int j = kSplit ? 2 * i + u : i, base = (t0 + j) * kN + kCols * half;
+            if (!chunk_wait(&sm.s_full[u], i & 1, &sm.abort_flag)) failed = true;
+            // (two warps that share rows leave together: the one that gave up still meets the other at their barrier below)
+            if (failed && (Ro::kHalves == 1 || !warp_has_rows)) break;
             tc::fence_after_sync();
-            if (!failed && warp_has_rows) {
-                const bool all_masked = *reinterpret_cast<volatile int*>(&sm.bad_tile) != 0;
-                float s[kN];
-                {
-                    uint32_t r0[32], r1[32], r2[32], r3[32];
-                    tc::tmem_ld32(tmem_s + lane_base, r0);
-                    tc::tmem_ld32(tmem_s + lane_base + 32, r1);
-                    tc::tmem_ld32(tmem_s + lane_base + 64, r2);
-                    tc::tmem_ld32(tmem_s + lane_base + 96, r3);
-                    tc::tmem_ld_wait();
+            if (warp_has_rows) {
+                const bool bad_tile = sm.bad_tile[j & (kSlotsMeta - 1)] != 0;
+                const bool masked = base + kCols - 1 > min_pos || base + kCols > kv_total || bad_tile;
+                const int lim = bad_tile ? -1 : min(my_pos, kv_total - 1) - base;  // last visible of this warp's keys
+                auto mask = [&](uint32_t (&s)[32], int first) {                    // keys the row may not see at -inf
+                    if (masked) {
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        s[j] = __uint_as_float(r0[j]);
-                        s[32 + j] = __uint_as_float(r1[j]);
-                        s[64 + j] = __uint_as_float(r2[j]);
-                        s[96 + j] = __uint_as_float(r3[j]);
+                        for (int e = 0; e < 32; ++e)
+                            if (first + e > lim) s[e] = 0xFF800000u;
                     }
-                }
-                if (base + kN - 1 > min_pos || !sealed || all_masked) {
+                };
+                auto top = [&](const uint32_t (&s)[32]) {
+                    float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-                    for (int j = 0; j < kN; ++j)
-                        if (base + j > my_pos || base + j >= kv_total || all_masked) s[j] = -INFINITY;
+                    for (int e = 0; e < 32; ++e) mx[e & 3] = fmaxf(mx[e & 3], __uint_as_float(s[e]));
+                    return fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+                };
+                // A row of S is read twice, 32 columns at a time: for its maximum, and for the exponentials.  What is read last for
+                // the maximum stays in registers and is exponentiated first: P goes over columns already read.
+                uint32_t s0[32], s1[32];
+                float mx;
+                if constexpr (Ro::kHalves == 1) {
+                    tc::tmem_ld32(ts + 64, s0);
+                    tc::tmem_ld32(ts + 96, s1);
+                    tc::tmem_ld_wait();
+                    mask(s0, 64);
+                    mask(s1, 96);
+                    mx = fmaxf(top(s0), top(s1));
+                    tc::tmem_ld32(ts, s0);
+                    tc::tmem_ld32(ts + 32, s1);
+                    tc::tmem_ld_wait();
+                    mask(s0, 0);
+                    mask(s1, 32);
+                    mx = fmaxf(mx, fmaxf(top(s0), top(s1)));
+                } else {
+                    tc::tmem_ld32(ts + 32, s0);
+                    tc::tmem_ld_wait();
+                    mask(s0, 32);
+                    mx = top(s0);
+                    tc::tmem_ld32(ts, s0);
+                    tc::tmem_ld_wait();
+                    mask(s0, 0);
+                    mx = fmaxf(mx, top(s0));
+                    sm.row_top[u][half][row] = mx;
+                    if (named_barrier_or(3 + 4 * u + (warp & 3), 64, failed)) { failed = true; break; }  // the two warps of these 32 rows
+                    mx = fmaxf(mx, sm.row_top[u][half ^ 1][row]);
                 }
-                float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-                for (int j = 0; j < kN; ++j) mx4[j & 3] = fmaxf(mx4[j & 3], s[j]);
-                const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-                constexpr float kLazy = 8.0f;  // lazy reference point, as in prefill_kernel
+                // The reference point of the row's exponentials follows the running maximum lazily: it moves only when the
+                // maximum has grown by more than 2^kLazy, so P stays below 2^kLazy (exact enough in fp16, whose precision is
+                // relative) and the O accumulator is rescaled a few times per walk instead of at every new maximum.
+                constexpr float kLazy = 8.0f;
                 const bool grown = mx > m_run + kLazy || (m_run == -INFINITY && mx > -INFINITY);
                 const float m_new = grown ? mx : m_run;
                 const float m_use = m_new == -INFINITY ? 0.0f : m_new;
                 const float alpha = grown ? fast_exp2(m_run - m_use) : 1.0f;
-                const bool moved = i > 0 && grown;
                 m_run = m_new;
-                float sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                F2 sum[2] = {F2(0.0f, 0.0f), F2(0.0f, 0.0f)};
+                const F2 off(-m_use, -m_use);
+                auto weights = [&](const uint32_t (&s)[32], int c) {  // exponentials of columns 32 c .. -> 16 columns of P
+                    uint32_t pk[16];
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    uint32_t pk[32];
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        const float p0 = fast_exp2(s[64 * c + 2 * j] - m_use), p1 = fast_exp2(s[64 * c + 2 * j + 1] - m_use);
-                        sum4[j & 3] += p0 + p1;
-                        pk[j] = pack_half2(p0, p1);
+                    for (int e = 0; e < 16; ++e) {
+                        const float2 a = add2(F2(__uint_as_float(s[2 * e]), __uint_as_float(s[2 * e + 1])), off).get();
+                        const float p0 = fast_exp2(a.x), p1 = fast_exp2(a.y);
+                        sum[e & 1] = add2(sum[e & 1], F2(p0, p1));
+                        pk[e] = pack_half2(p0, p1);
                     }
-                    tc::tmem_st32(tmem_s + lane_base + 32 * c, pk);
+                    tc::tmem_st16(ts + 16 * c, pk);
+                };
+                weights(s0, 0);
+                if constexpr (Ro::kHalves == 1) weights(s1, 1);
+#pragma unroll 1
+                for (int c = 2 / Ro::kHalves; c < 4 / Ro::kHalves; ++c) {  // (unrolled, the two loads cost spills)
+                    tc::tmem_ld32(ts + 32 * c, s0);
+                    tc::tmem_ld_wait();
+                    mask(s0, 32 * c);
+                    weights(s0, c);
                 }
-                tc::tmem_st_wait();
-                l_run = l_run * alpha + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
-                if (__any_sync(0xffffffffu, moved)) {  // P V(i-1) completed before S(i) was issued: O may be rescaled
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
+                const float2 sum2 = add2(sum[0], sum[1]).get();
+                l_run = l_run * alpha + (sum2.x + sum2.y);
+                if (i > 0 && __any_sync(0xffffffffu, grown)) {  // P V of step i - 1 completed before S of step i was issued
+#pragma unroll 1
+                    for (int c = 0; c < kCols / 32; ++c) {
                         uint32_t r[32];
-                        tc::tmem_ld32(tmem_o + lane_base + 32 * c, r);
+                        tc::tmem_ld32(to + 32 * c, r);
                         tc::tmem_ld_wait();
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * alpha);
-                        tc::tmem_st32(tmem_o + lane_base + 32 * c, r);
+                        for (int e = 0; e < 32; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * alpha);
+                        tc::tmem_st32(to + 32 * c, r);
                     }
-                    tc::tmem_st_wait();
                 }
+                tc::tmem_st_wait();
             }
             tc::fence_before_sync();
-            named_barrier_sync(1, 64);  // P of both warps is in tensor memory; a warp that gave up meets its partner here
-            if (*abort_flag) { failed = true; break; }
-            if (warp == 0) {  // O += P V(i)
-                if (!verify_wait(&sm.v_ready, i & 1, sm)) {
-                    failed = true;
-                } else {
-                    tc::fence_after_sync();
-#pragma unroll
-                    for (int kk = 0; kk < 8; ++kk)
-                        tc::mma_f16_ts(tmem_o, tmem_s + 8 * kk, tc::smem_desc(v_addr + kk * 2048, 16384, 1024), idesc_pv, i > 0 || kk > 0);
-                    tc::commit(&sm.bar_o);
-                }
-            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.p_full[u]);
         }
-        // ---- partial of this key range: m (log2 units), l, o in tile dim order
-        if (n > 0 && !failed && !verify_wait(&sm.bar_o, (n - 1) & 1, sm)) failed = true;
-        if (*abort_flag) failed = true;
+        // ---- partial of this (row tile, key range): m (log2 units), l, o in tile dim order
+        if (steps > 0 && !failed && !chunk_wait(&sm.o_done[u], (steps - 1) & 1, &sm.abort_flag)) failed = true;
         tc::fence_after_sync();
-        const bool have = n > 0 && !failed;
-        const int64_t idx = (static_cast<int64_t>(head) * P.ksplit + zs) * kM + tid;
-        if (my_pos >= 0) {
+        if constexpr (Ro::kHalves == 2) {  // a row's sum has two halves; a warp that gave up comes here too
+            sm.row_top[u][half][row] = l_run;
+            named_barrier_sync(3 + 4 * u + (warp & 3), 64);
+            l_run += sm.row_top[u][half ^ 1][row];
+        }
+        const bool have = steps > 0 && !failed;
+        const int tile = kSplit ? mt : mt + u, part = kSplit ? 2 * zs + u : zs;
+        const int64_t idx = ((static_cast<int64_t>(head) * P.mtiles + tile) * P.ksplit + part) * kM + row;
+        if (my_pos >= 0 && half == 0) {
             P.ws_m[idx] = have ? m_run : -INFINITY;
             P.ws_l[idx] = have ? l_run : 0.0f;
         }
-        float* orow = P.ws_o + idx * D;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        float* orow = P.ws_o + idx * D + kCols * half;
+#pragma unroll 1
+        for (int c = 0; c < kCols / 32; ++c) {
             if (!warp_has_rows) break;
             uint32_t r[32];
             if (have) {
-                tc::tmem_ld32(tmem_o + lane_base + 32 * c, r);
+                tc::tmem_ld32(to + 32 * c, r);
                 tc::tmem_ld_wait();
             }
             if (my_pos < 0) continue;
 #pragma unroll
-            for (int j = 0; j < 32; j += 4)
-                *reinterpret_cast<float4*>(orow + 32 * c + j) =
-                    have ? make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]))
+            for (int e = 0; e < 32; e += 4)
+                *reinterpret_cast<float4*>(orow + 32 * c + e) =
+                    have ? make_float4(__uint_as_float(r[e]), __uint_as_float(r[e + 1]), __uint_as_float(r[e + 2]), __uint_as_float(r[e + 3]))
                          : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     }
-    if ((failed || *abort_flag) && lane == 0) L.flag(KVB_ERR_WAIT_TIMEOUT);
+    if (failed && lane == 0) L.flag(KVB_ERR_WAIT_TIMEOUT);
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(sm.tmem_base, kTmemCols);
+    if (warp == kMmaWarp) tc::tmem_dealloc(tmem, kTmemCols);
 }
 
-int prefill_sm_count() { return device_sm_count(); }
-
-void prefill_shape(int kv_len_max, int kv_heads, int q_heads, int tokens, int* mtiles, int* ksplit) {
-    const int rows = tokens * (q_heads / kv_heads);
-    *mtiles = (rows + kM - 1) / kM;
-    const int ctas = *mtiles * kv_heads, ntiles = (kv_len_max + kN - 1) / kN;
-    // Two CTAs share an SM.  A few rows (verify): one wave, every further key range costs a partial per row.  A chunk: the
-    // number of ranges (at most about six waves) with the lowest (waves x CTA), a CTA costing its tiles plus about five
-    // tiles' worth of set-up (Q tile) and epilogue.  Measured (always six waves in brackets): 1,024 tokens over 262,144, 3
-    // ranges, 4.40 ms (4.52, 9 ranges); 777 tokens alone, 2 ranges, 28 us (46, 3 ranges: a second, nearly empty wave).
-    const int slots = 2 * prefill_sm_count();
-    int ks = (slots + ctas - 1) / ctas;
-    if (ctas >= 64) {
-        int64_t best = INT64_MAX;
-        const int most = std::max(1, std::min(6 * slots / ctas, ntiles / 2));
-        for (int n = 1; n <= most; ++n) {
-            const int64_t cost = static_cast<int64_t>((ctas * n + slots - 1) / slots) * (5 + (ntiles + n - 1) / n);
-            if (cost < best) { best = cost; ks = n; }
+struct ChunkShape {
+    bool split;             // one row tile per CTA, its streams split the keys
+    int mtiles, ksplit;     // row tiles; partials per row
+    int ranges;             // key ranges (grid z)
+};
+constexpr int kWaves = 4;   // at most four waves of CTAs
+// The cheapest (waves x CTA), one CTA per SM, in fifths of the time a row tile takes for a key tile with two row tiles a CTA
+// (1.3 us, measured at 1,024 tokens over 262,144; with split keys 1.8 us): a step of two row tiles costs 10, one with split
+// keys 7, set-up and epilogue about 18 and 13 us.  Measured: 1,024 tokens over 262,144 3.46 ms with two row tiles, 4.76 ms
+// with split keys; 777 tokens alone 36 and 25 us.
+ChunkShape prefill_shape(int kv_len_max, int kv_heads, int q_heads, int tokens) {
+    const int rows = tokens * (q_heads / kv_heads), mtiles = (rows + kM - 1) / kM, ntiles = (kv_len_max + kN - 1) / kN, sms = device_sm_count();
+    ChunkShape best{};
+    int64_t best_cost = INT64_MAX;
+    for (int split = mtiles == 1 ? 1 : 0; split < 2; ++split) {
+        const int ctas = (split ? mtiles : (mtiles + 1) / 2) * kv_heads, per = split ? 2 : 1;
+        for (int r = 1; per * r <= kMaxKeyRanges && (r == 1 || (2 * r <= ntiles && ctas * r <= kWaves * sms)); ++r) {
+            const int64_t steps = (ntiles + r - 1) / r;
+            const int64_t cost = static_cast<int64_t>((ctas * r + sms - 1) / sms) * (split ? 50 + 7 * steps : 70 + 10 * steps);
+            if (cost < best_cost) {
+                best_cost = cost;
+                best = {split != 0, mtiles, per * r, r};
+            }
         }
     }
-    if (ks > ntiles / 2) ks = ntiles / 2;
-    if (ks > kMaxKeyRanges) ks = kMaxKeyRanges;
-    *ksplit = ks < 1 ? 1 : ks;
+    return best;
 }
 
 }  // namespace
@@ -760,9 +560,11 @@ int launch_chunk_attention_256(const kvb_layer* layer, const void* q, const int3
 
 extern "C" size_t kvb_prefill_workspace_bytes(int kv_len_max, int kv_heads, int q_heads, int head_dim, int tokens) {
     if (kv_heads < 1 || q_heads < kv_heads || tokens < 1) return 0;
-    int mtiles, ksplit;
-    kvb::prefill_shape(kv_len_max, kv_heads, q_heads, tokens, &mtiles, &ksplit);
-    const size_t tuned = static_cast<size_t>(kv_heads) * mtiles * ksplit * kvb::kM * (head_dim + 2) * sizeof(float);
+    // The most partials a call of up to this many tokens and keys can have (a shorter one may be cut into more ranges).
+    const size_t tiles = static_cast<size_t>((tokens * (q_heads / kv_heads) + kvb::kM - 1) / kvb::kM) * kv_heads, ntiles = (kv_len_max + kvb::kN - 1) / kvb::kN;
+    const size_t cap = static_cast<size_t>(kvb::kWaves) * kvb::device_sm_count();
+    const size_t partials = 2 * std::max(tiles, std::min(cap, tiles * std::max<size_t>(1, ntiles / 2)));
+    const size_t tuned = partials * kvb::kM * (head_dim + 2) * sizeof(float);
     const size_t wide = head_dim == 256 ? kvb::chunk256_workspace_bytes(kv_len_max, kv_heads, q_heads, tokens) : 0;
     return tuned > wide ? tuned : wide;
 }
@@ -778,7 +580,9 @@ int launch_chunk_attention(const kvb_layer* layer, const void* q, const int32_t*
     P.pos = positions_dev;
     P.total_pos = total_pos_dev != nullptr ? total_pos_dev : positions_dev + (tokens - 1);
     P.T = tokens;
-    prefill_shape(kv_len_max, layer->kv_heads, layer->q_heads, tokens, &P.mtiles, &P.ksplit);
+    const ChunkShape shape = prefill_shape(kv_len_max, layer->kv_heads, layer->q_heads, tokens);
+    P.mtiles = shape.mtiles;
+    P.ksplit = shape.ksplit;
     P.scale_log2 = scale * 1.4426950408889634f;
     const size_t rows = static_cast<size_t>(layer->kv_heads) * P.mtiles * P.ksplit * kM;
     P.ws_m = static_cast<float*>(workspace);
@@ -787,27 +591,15 @@ int launch_chunk_attention(const kvb_layer* layer, const void* q, const int32_t*
     const int smem = static_cast<int>(sizeof(PrefillSmem)) + 1024;  // room to align the tiles to 1024 bytes
     static unsigned long long opted = 0;
     if (first_call_on_device(opted)) {
-        KVB_CUDA_OK(cudaFuncSetAttribute(prefill_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        KVB_CUDA_OK(cudaFuncSetAttribute(prefill_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        KVB_CUDA_OK(cudaFuncSetAttribute(chunk_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        KVB_CUDA_OK(cudaFuncSetAttribute(chunk_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        KVB_CUDA_OK(cudaFuncSetAttribute(chunk_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        KVB_CUDA_OK(cudaFuncSetAttribute(chunk_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     }
-    const bool few_rows = tokens * (layer->q_heads / layer->kv_heads) <= 64;  // a verify step: the role-split kernel
-    if (few_rows) {
-        const int vsmem = static_cast<int>(sizeof(VerifySmem)) + 1024;
-        static unsigned long long vopted = 0;
-        if (first_call_on_device(vopted)) {
-            KVB_CUDA_OK(cudaFuncSetAttribute(verify_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, vsmem));
-            KVB_CUDA_OK(cudaFuncSetAttribute(verify_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, vsmem));
-        }
-        if (layer->sinkhorn_iters > 0) {
-            verify_kernel<true><<<dim3(1, layer->kv_heads, P.ksplit), kThreads, vsmem, s>>>(P);
-        } else {
-            verify_kernel<false><<<dim3(1, layer->kv_heads, P.ksplit), kThreads, vsmem, s>>>(P);
-        }
-    } else if (layer->sinkhorn_iters > 0) {
-        prefill_kernel<true><<<dim3(P.mtiles, layer->kv_heads, P.ksplit), kThreads, smem, s>>>(P);
-    } else {
-        prefill_kernel<false><<<dim3(P.mtiles, layer->kv_heads, P.ksplit), kThreads, smem, s>>>(P);
-    }
+    const bool other = layer->sinkhorn_iters > 0;
+    const auto kernel = shape.split ? (other ? chunk_kernel<true, true> : chunk_kernel<true, false>) : (other ? chunk_kernel<false, true> : chunk_kernel<false, false>);
+    const dim3 grid(shape.split ? shape.mtiles : (shape.mtiles + 1) / 2, layer->kv_heads, shape.ranges);
+    kernel<<<grid, kThreads, smem, s>>>(P);
     KVB_CUDA_OK(cudaGetLastError());
     return launch_chunk_merge<D>(P.ws_m, P.ws_l, P.ws_o, tokens, layer->q_heads, layer->kv_heads, P.mtiles, P.ksplit, layer->dtype, out,
                                  part_m, part_l, part_o, s);

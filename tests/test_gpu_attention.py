@@ -592,3 +592,26 @@ def test_batched_decode_refuses_bad_arguments():
     assert st == capi.KVB_ERANGE
     st = lib.kvb_attn_decode_batch(fake, 2, 4, 24, 128, 0, fake, fake, 0.1, bounds, None, fake, None)
     assert st == capi.KVB_EINVAL
+
+
+# 1,000 tokens and more of 24 / 4 heads run with two row tiles per CTA (an odd number of tiles: the last CTA has one), fewer
+# with the keys split between the two streams of a CTA; ranges of one, two and more key tiles, open tiles, several key ranges
+@pytest.mark.parametrize("H,QH,ctx,T,iters", [(4, 24, 0, 1000, 16), (4, 24, 200, 1003, 0), (4, 24, 0, 43, 0), (4, 24, 85, 43, 16), (2, 16, 640, 17, 0),
+                                              (1, 8, 5000, 33, 16), (8, 8, 130, 700, 0)])
+def test_chunk_shapes(H, QH, ctx, T, iters):
+    import torch
+    from helpers import PREFILL_MAX_ABS, PREFILL_REL_L2
+
+    D, scale = 128, 1.0 / np.sqrt(128.0)
+    tw = Twin(D=D, H=H, QH=QH, capacity_tokens=ctx + T, seed=ctx + T, iters=iters)
+    k, v = orc.synth_kv(T, ctx + T, H, D, 1), orc.synth_kv(T, ctx + T, H, D, 2)
+    q = orc.synth_q(T, T, QH, D)
+    gk, gv, gq = (torch.from_numpy(x).to(tw.dev) for x in (k, v, q))
+    at = torch.arange(ctx + T, dtype=torch.int32, device=tw.dev)
+    if ctx:
+        tw.gpu.append(gk[:ctx], gv[:ctx], at[:ctx])
+    out = tw.gpu.attn_prefill(gq, gk[ctx:], gv[ctx:], at[ctx:], scale, ctx + T)
+    want = cpu_twin_of(tw.gpu).attention(q, np.arange(ctx, ctx + T, dtype=np.int32), scale, QH, threads=4, kv_total=ctx + T)
+    assert tw.gpu.errors() == 0
+    ok, msg = attn_close(out.float().cpu().numpy(), want, PREFILL_MAX_ABS, PREFILL_REL_L2)
+    assert ok, msg
