@@ -611,7 +611,7 @@ def measure_append(E, args):
             "unit": "GB/s", "frac": nbytes / (us * 1e-6) / 1e9 / peak, "peak": peak, "peak_kind": kind, "bound": "hbm",
             "algorithmic_bytes_per_launch": nbytes, "tokens_per_s": T / (us * 1e-6), "layers": layers_n,
             "graph_captured": graphed, "error_words": errs, "clocks": clk.summary(),
-            "gpu_launches": args.steps * layers_n * (2 if T > 128 else 1)}
+            "gpu_launches": args.steps * layers_n}
 
 
 def measure_verify(E, args):
