@@ -1303,14 +1303,8 @@ __global__ void __launch_bounds__(kReduceWarps * 32) reduce_kernel(const float* 
         }
         return;
     }
-    if (part_m != nullptr) {
-        if (lane == 0) { part_m[row] = m * kLn2; part_l[row] = l; }
-#pragma unroll
-        for (int s = 0; s < S; ++s) *reinterpret_cast<float4*>(part_o + static_cast<int64_t>(row) * D + 128 * s + 4 * lane) = acc[s];
-        return;
-    }
-    const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-    // the rotation wants lane l to hold dims l + 32 j: re-distribute through shared memory
+    const float inv = part_m != nullptr ? 1.0f : l > 0.0f ? 1.0f / l : 0.0f;
+    // the rotation (and a store to 4-byte aligned memory) wants lane l to hold dims l + 32 j: re-distribute through shared memory
 #pragma unroll
     for (int s = 0; s < S; ++s) so[0][s][lane] = make_float4(acc[s].x * inv, acc[s].y * inv, acc[s].z * inv, acc[s].w * inv);
     __syncwarp();
@@ -1318,6 +1312,12 @@ __global__ void __launch_bounds__(kReduceWarps * 32) reduce_kernel(const float* 
     float o[4 * S];
 #pragma unroll
     for (int j = 0; j < 4 * S; ++j) o[j] = flat[lane + 32 * j];
+    if (part_m != nullptr) {  // 4-byte stores: in a packed buffer m | l | o, o starts 2 * rows floats behind the base
+        if (lane == 0) { part_m[row] = m * kLn2; part_l[row] = l; }
+#pragma unroll
+        for (int j = 0; j < 4 * S; ++j) part_o[static_cast<int64_t>(row) * D + lane + 32 * j] = o[j];
+        return;
+    }
     hadamard_warp<D>(o, lane);
 #pragma unroll
     for (int j = 0; j < 4 * S; ++j)
