@@ -12,6 +12,8 @@
  *   - calls are asynchronous on `stream`; none synchronises, none allocates.
  *   - no exceptions cross the ABI: functions return a kvb_status; kvb_last_error_string()
  *     gives the text of the calling thread's last failure.
+ *   - planes and stage start at 16-byte boundaries; k, v, q, out, positions, partials and workspaces need no more than
+ *     the alignment of their elements (workspace sizes include room to round the start up).
  *   - positions and block tables are read on the device only (the reference's hard rule,
  *     LAUNCH.cu:5-11): the host never dereferences them.
  *

@@ -1463,7 +1463,7 @@ int launch_attention(const kvb_layer* layer, const void* q, const int32_t* pos_d
     P.key_begin = key_begin;
     P.key_end = key_end;
     const size_t rows = static_cast<size_t>(layer->kv_heads) * Z * parts * kRows;
-    P.ws_m = static_cast<float*>(workspace);
+    P.ws_m = workspace_base(workspace);
     P.ws_l = P.ws_m + rows;
     P.ws_o = P.ws_l + rows;
     const bool upper = plan.nb == 2;
@@ -1515,7 +1515,7 @@ static size_t workspace_bytes_for_rows(int kv_len_max, int kv_heads, int q_heads
     for (int block_rows = 8; block_rows <= 16; block_rows += 8) {  // either cut of the rows into blocks (plan_rows)
         const int Z = kvb::zblocks_of(q_heads, kv_heads, r, block_rows);
         const size_t parts = kvb::split_count(kv_len_max, kv_heads, Z);
-        bytes = std::max(bytes, static_cast<size_t>(kv_heads) * Z * parts * kvb::kRows * (head_dim + 2) * sizeof(float));
+        bytes = std::max(bytes, static_cast<size_t>(kv_heads) * Z * parts * kvb::kRows * (head_dim + 2) * sizeof(float) + kvb::kWorkspaceSlack);
     }
     if (r > 8 || r * (q_heads / kv_heads) >= kDenseRows) {  // steps this wide run on the chunk-attention kernels
         const size_t dense = kvb_prefill_workspace_bytes(kv_len_max, kv_heads, q_heads, head_dim, r);
@@ -1709,7 +1709,7 @@ extern "C" size_t kvb_batch_workspace_bytes(const int32_t* kv_len_max, int batch
         if (kv_len_max[b] < 1) return 0;
     BatchPlan plan;
     const size_t rows = static_cast<size_t>(kv_heads) * plan_batch(kv_len_max, batch, kv_heads, plan) * kRows;
-    return rows * (2 + head_dim) * sizeof(float);
+    return rows * (2 + head_dim) * sizeof(float) + kWorkspaceSlack;
 }
 
 extern "C" int kvb_attn_decode_batch(const kvb_layer* layers_dev, int batch, int kv_heads, int q_heads, int head_dim, int dtype,
@@ -1735,7 +1735,7 @@ extern "C" int kvb_attn_decode_batch(const kvb_layer* layers_dev, int batch, int
     B.kv_heads = kv_heads;
     B.q_heads = q_heads;
     B.dtype = dtype;
-    B.ws_m = static_cast<float*>(workspace);
+    B.ws_m = workspace_base(workspace);
     B.ws_l = B.ws_m + rows;
     B.ws_o = B.ws_l + rows;
     constexpr int smem1 = static_cast<int>(sizeof(AttnSmem<1, kWarpsDecode>)), smem2 = static_cast<int>(sizeof(AttnSmem<1, kWarpsWide>));

@@ -645,7 +645,7 @@ int launch_chunk_attention_256(const kvb_layer* layer, const void* q, const int3
     chunk256_shape(kv_len_max, layer->kv_heads, layer->q_heads, tokens, &P.mtiles, &P.ksplit);
     P.scale_log2 = scale * 1.4426950408889634f;
     const size_t rows = static_cast<size_t>(layer->kv_heads) * P.mtiles * P.ksplit * kM;
-    P.ws_m = static_cast<float*>(workspace);
+    P.ws_m = workspace_base(workspace);
     P.ws_l = P.ws_m + rows;
     P.ws_o = P.ws_l + rows;
     const int smem = static_cast<int>(sizeof(Chunk256Smem)) + 1024;  // room to align the tiles to 1024 bytes

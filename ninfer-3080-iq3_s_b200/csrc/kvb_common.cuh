@@ -124,6 +124,11 @@ inline int device_sm_count() {
     return n;
 }
 
+// Workspaces may start at any 4-byte boundary; the kernels' vector accesses start at the next 16-byte one, for which every size
+// query keeps kWorkspaceSlack bytes.
+constexpr size_t kWorkspaceSlack = 16;
+inline float* workspace_base(void* workspace) { return reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(workspace) + 15) & ~static_cast<uintptr_t>(15)); }
+
 LayerView make_view(const kvb_layer& L);
 int check_layer(const kvb_layer* L, const char* who);
 

@@ -566,7 +566,7 @@ extern "C" size_t kvb_prefill_workspace_bytes(int kv_len_max, int kv_heads, int 
     const size_t partials = 2 * std::max(tiles, std::min(cap, tiles * std::max<size_t>(1, ntiles / 2)));
     const size_t tuned = partials * kvb::kM * (head_dim + 2) * sizeof(float);
     const size_t wide = head_dim == 256 ? kvb::chunk256_workspace_bytes(kv_len_max, kv_heads, q_heads, tokens) : 0;
-    return tuned > wide ? tuned : wide;
+    return (tuned > wide ? tuned : wide) + kvb::kWorkspaceSlack;
 }
 
 namespace kvb {
@@ -585,7 +585,7 @@ int launch_chunk_attention(const kvb_layer* layer, const void* q, const int32_t*
     P.ksplit = shape.ksplit;
     P.scale_log2 = scale * 1.4426950408889634f;
     const size_t rows = static_cast<size_t>(layer->kv_heads) * P.mtiles * P.ksplit * kM;
-    P.ws_m = static_cast<float*>(workspace);
+    P.ws_m = workspace_base(workspace);
     P.ws_l = P.ws_m + rows;
     P.ws_o = P.ws_l + rows;
     const int smem = static_cast<int>(sizeof(PrefillSmem)) + 1024;  // room to align the tiles to 1024 bytes

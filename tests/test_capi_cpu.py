@@ -86,3 +86,12 @@ def test_null_arguments_and_ranges():
     assert lib.kvb_merge_partials(None, 16, 16, 2, 24, 128, 0, 16, None) == capi.KVB_EINVAL
     with pytest.raises(capi.KvarnError):
         capi.check(capi.KVB_EINVAL)
+
+
+def test_workspace_sizes_leave_room_to_round_the_start_up():
+    """Partials of kv_heads x row blocks x splits x 16 rows of (head_dim + 2) floats, and 16 bytes for a start at any float."""
+    lib = pkg().capi.load()
+    for D in (128, 256):
+        parts = lib.kvb_split_capacity(9000, 4, 24, 1, 1)
+        assert lib.kvb_workspace_bytes(9000, 4, 24, D, 1, 1) >= 4 * parts * 16 * (D + 2) * 4 + 12
+    assert lib.kvb_batch_workspace_bytes((C.c_int32 * 1)(128), 1, 1, 1, 128) == 16 * (128 + 2) * 4 + 16

@@ -51,3 +51,37 @@ def test_packed_partials_of_an_odd_number_of_rows(D, H, QH, tokens):
     ref = cpu_twin_of(tw.gpu).attention(q.cpu().numpy(), np.arange(T - tokens, T, dtype=np.int32), 1.0 / np.sqrt(D), QH, threads=4, kv_total=T)
     ok, msg = attn_close(out.float().cpu().numpy().reshape(ref.shape), ref, *((PREFILL_MAX_ABS, PREFILL_REL_L2) if D == 128 and tokens * QH // H >= 32 else (ATTN_MAX_ABS, ATTN_REL_L2)))
     assert ok, msg
+
+
+@pytest.mark.parametrize("D", [128, 256])
+@pytest.mark.parametrize("op,tokens", [("decode", 1), ("verify", 3), ("verify", 8), ("prefill", 40)])
+def test_workspace_at_any_float(D, op, tokens):
+    """A workspace of the queried size that starts 4, 8 or 12 bytes behind a 16-byte boundary: the same bits, and nothing
+    written outside it."""
+    import torch
+
+    H, QH, T, scale = 4, 24, 700, 1.0 / np.sqrt(D)
+    tw = _filled(D, H, QH, T, room=64)
+    lib, capi = pkg().capi.load(), pkg().capi
+    q = torch.from_numpy(orc.synth_q(3, tokens, QH, D)).to(tw.dev)
+    k, v = (torch.from_numpy(orc.synth_kv(4, tokens, H, D, i)).to(tw.dev) for i in (1, 2))
+    pos = torch.arange(T, T + tokens, dtype=torch.int32, device=tw.dev)
+    rows = min(tokens, 8)
+    need = lib.kvb_prefill_workspace_bytes(T + tokens, H, QH, D, tokens) if op == "prefill" else lib.kvb_workspace_bytes(T + tokens, H, QH, D, rows, 1)
+    outs = []
+    for shift in (0, 1, 2, 3):
+        buf = torch.full((need // 4 + 16,), 7.0, device=tw.dev)
+        ws, out = buf[4 + shift:], torch.empty_like(q)
+        ptr = [C.c_void_p(x.data_ptr()) for x in (q, k, v, pos, ws, out)]
+        if op == "decode":
+            tw.gpu.append(k, v, pos)
+            capi.check(lib.kvb_attn_decode(C.byref(tw.gpu.c), ptr[0], ptr[3], scale, T + tokens, ptr[4], ptr[5], None))
+        elif op == "verify":
+            capi.check(lib.kvb_attn_verify(C.byref(tw.gpu.c), *ptr[:4], tokens, scale, T + tokens, ptr[4], ptr[5], None))
+        else:
+            capi.check(lib.kvb_attn_prefill(C.byref(tw.gpu.c), *ptr[:4], tokens, scale, T + tokens, ptr[4], ptr[5], None))
+        torch.cuda.synchronize()
+        assert torch.all(buf[:4 + shift] == 7.0) and torch.all(buf[4 + shift + need // 4:] == 7.0)
+        outs.append(out)
+    assert all(torch.equal(outs[0], x) for x in outs[1:])
+    assert tw.gpu.errors() == 0
