@@ -417,7 +417,7 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
     for (int i = 0; i < kQIter; ++i) {
 #pragma unroll
         for (int j = 0; j < 4 * S; ++j) qraw[i][j] = 0;
-        qpos[i] = -1;
+        qpos[i] = INT_MAX;  // no such row: never masked, never stored
         const int r = warp + W * i;
         if (r < 8 * NB) {
             const int Rr = zb * P.block_rows + r, tq = Rr / G, gq = Rr % G;
@@ -529,8 +529,7 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
         row_lim[nb][0] = sm.row_pos[8 * nb + 2 * t];
         row_lim[nb][1] = sm.row_pos[8 * nb + 2 * t + 1];
     }
-    for (int r = 0; r < 8 * NB; ++r)
-        if (sm.row_pos[r] >= 0) min_lim = min(min_lim, sm.row_pos[r]);
+    for (int r = 0; r < 8 * NB; ++r) min_lim = min(min_lim, sm.row_pos[r]);  // (a negative position: a row that sees no key)
 
     Acc<S, NB> acc;
 #pragma unroll

@@ -343,14 +343,14 @@ __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Par
 #pragma unroll
         for (int u = 0; u < kQBatch; ++u) {
             const int r = r0 + u * kWarps, R = mt * kM + r, tq = R / G, gq = R % G;
-            rp[u] = -1;
+            rp[u] = kNoRow;
 #pragma unroll
             for (int j = 0; j < 8; ++j) raw[u][j] = 0;
             if (r < kM && tq < P.T) {
                 const uint16_t* qrow = P.q + (static_cast<int64_t>(tq) * L.q_heads + head * G + gq) * D;
 #pragma unroll
                 for (int j = 0; j < 8; ++j) raw[u][j] = qrow[lane + 32 * j];
-                rp[u] = P.pos[tq];
+                rp[u] = max(P.pos[tq], -1);
             }
         }
 #pragma unroll
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Par
     for (int i = 0; i < kM / 32; ++i) {
         const int p = sm.row_pos[lane + 32 * i];
         max_pos = max(max_pos, p);
-        if (p >= 0) min_pos = min(min_pos, p);
+        if (p != kNoRow) min_pos = min(min_pos, p);
     }
     max_pos = __reduce_max_sync(0xffffffffu, max_pos);
     min_pos = __reduce_min_sync(0xffffffffu, min_pos);
@@ -485,7 +485,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Par
         const uint32_t lane_base = static_cast<uint32_t>(32 * warp) << 16;
         const int my_pos = sm.row_pos[tid];
         const float row_unit = sm.row_unit[tid];
-        const bool warp_has_rows = __any_sync(0xffffffffu, my_pos >= 0);
+        const bool is_row = my_pos != kNoRow, warp_has_rows = __any_sync(0xffffffffu, is_row);
         float m_run = -INFINITY, l_run = 0.0f;
         int v_exp = 0;
         bool poisoned = false;
@@ -579,11 +579,11 @@ __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Par
         if (n > 1 && !failed && !chunk_wait(&sm.o_done, n & 1, &sm.abort_flag)) failed = true;
         if (n > 0 && !failed && !chunk_wait(&sm.o_done, (n - 1) & 1, &sm.abort_flag)) failed = true;
         tc::fence_after_sync();
-        const bool have = n > 0 && !failed;
+        const bool have = n > 0 && !failed && __any_sync(0xffffffffu, m_run != -INFINITY), seen = have && m_run != -INFINITY;
         const int64_t idx = ((static_cast<int64_t>(head) * P.mtiles + mt) * P.ksplit + zs) * kM + tid;
-        if (my_pos >= 0) {
-            P.ws_m[idx] = have && m_run != -INFINITY ? m_run - kPBoost : -INFINITY;
-            P.ws_l[idx] = have ? l_run : 0.0f;
+        if (is_row) {
+            P.ws_m[idx] = seen ? m_run - kPBoost : -INFINITY;
+            P.ws_l[idx] = seen ? l_run : 0.0f;
         }
         const float unit = poisoned ? __uint_as_float(0x7FC00000u) : pow2i(v_exp);
         float* orow = P.ws_o + idx * D;
@@ -595,11 +595,11 @@ __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Par
                 tc::tmem_ld32(tmem + kColO + lane_base + 32 * c, r);
                 tc::tmem_ld_wait();
             }
-            if (my_pos < 0) continue;
+            if (!is_row) continue;
 #pragma unroll
             for (int j = 0; j < 32; j += 4)
                 *reinterpret_cast<float4*>(orow + 32 * c + j) =
-                    have ? make_float4(__uint_as_float(r[j]) * unit, __uint_as_float(r[j + 1]) * unit, __uint_as_float(r[j + 2]) * unit, __uint_as_float(r[j + 3]) * unit)
+                    seen ? make_float4(__uint_as_float(r[j]) * unit, __uint_as_float(r[j + 1]) * unit, __uint_as_float(r[j + 2]) * unit, __uint_as_float(r[j + 3]) * unit)
                          : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     }

@@ -1,6 +1,8 @@
 // kvb_chunk_merge.cuh -- the last step of chunk attention: the partials of a row's key ranges become its output.
 #pragma once
 
+#include <climits>
+
 #include "kvb_common.cuh"
 #include "kvb_ptx.cuh"
 
@@ -9,6 +11,7 @@ namespace {
 
 constexpr int kRowTile = 128;       // rows per row tile of the partials
 constexpr int kMaxKeyRanges = 128;  // what the merge kernel holds
+constexpr int kNoRow = INT_MIN;     // position of a row of a tile that the chunk does not have (a row that sees no key: -1)
 
 // Position of dim d inside its group of eight: order 0,4,1,5,2,6,3,7.
 __device__ __forceinline__ int dim_slot(int d) { return (d & ~7) | ((d & 3) << 1) | ((d >> 2) & 1); }

@@ -273,13 +273,13 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
 #pragma unroll
         for (int u = 0; u < kQBatch; ++u) {
             const int r = r0 + u * kWarps, R = mt * kM + r, tq = R / G, gq = R % G;
-            rp[u] = -1;
+            rp[u] = kNoRow;
             raw[u][0] = raw[u][1] = raw[u][2] = raw[u][3] = 0;
             if (r < kRows && tq < P.T) {
                 const uint16_t* qrow = P.q + (static_cast<int64_t>(tq) * L.q_heads + head * G + gq) * D;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) raw[u][j] = qrow[lane + 32 * j];
-                rp[u] = P.pos[tq];
+                rp[u] = max(P.pos[tq], -1);
             }
         }
 #pragma unroll
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
             float v[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) v[j] = L.dtype == KVB_DTYPE_BF16 ? in_to_f32<true>(raw[u][j]) : in_to_f32<false>(raw[u][j]);
-            if (rp[u] >= 0) hadamard_warp<D>(v, lane);  // warp-uniform: a row is real or not for the whole warp
+            if (rp[u] != kNoRow) hadamard_warp<D>(v, lane);  // warp-uniform: a row is real or not for the whole warp
             if (lane == 0) sm.row_pos[r >> 7][r & 127] = rp[u];
 #pragma unroll
             for (int j = 0; j < 4; ++j)
@@ -375,8 +375,8 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
         // P of a column half lies over the first half of its own columns of S: no warp writes over what another still reads
         const uint32_t ts = tmem + 128 * u + kCols * half + lane_base, to = tmem + kColO + 128 * u + kCols * half + lane_base;
         const int my_pos = kSplit ? sm.row_pos[0][row] : sm.row_pos[u][row];
-        const bool warp_has_rows = __any_sync(0xffffffffu, my_pos >= 0);
-        const int min_pos = __reduce_min_sync(0xffffffffu, my_pos < 0 ? INT_MAX : my_pos);
+        const bool is_row = my_pos != kNoRow, warp_has_rows = __any_sync(0xffffffffu, is_row);
+        const int min_pos = __reduce_min_sync(0xffffffffu, is_row ? my_pos : INT_MAX);
         const int steps = steps_of(u);
         float m_run = -INFINITY, l_run = 0.0f;
         for (int i = 0; i < steps; ++i) {
@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
             if (warp_has_rows) {
                 const bool bad_tile = sm.bad_tile[j & (kSlotsMeta - 1)] != 0;
                 const bool masked = base + kCols - 1 > min_pos || base + kCols > kv_total || bad_tile;
-                const int lim = bad_tile ? -1 : min(my_pos, kv_total - 1) - base;  // last visible of this warp's keys
+                const int lim = bad_tile || !is_row ? -1 : min(my_pos, kv_total - 1) - base;  // last visible of this warp's keys
                 auto mask = [&](uint32_t (&s)[32], int first) {                    // keys the row may not see at -inf
                     if (masked) {
 #pragma unroll
@@ -490,12 +490,12 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
             named_barrier_sync(3 + 4 * u + (warp & 3), 64);
             l_run += sm.row_top[u][half ^ 1][row];
         }
-        const bool have = steps > 0 && !failed;
+        const bool have = steps > 0 && !failed && __any_sync(0xffffffffu, m_run != -INFINITY), seen = have && m_run != -INFINITY;
         const int tile = kSplit ? mt : mt + u, part = kSplit ? 2 * zs + u : zs;
         const int64_t idx = ((static_cast<int64_t>(head) * P.mtiles + tile) * P.ksplit + part) * kM + row;
-        if (my_pos >= 0 && half == 0) {
-            P.ws_m[idx] = have ? m_run : -INFINITY;
-            P.ws_l[idx] = have ? l_run : 0.0f;
+        if (is_row && half == 0) {
+            P.ws_m[idx] = seen ? m_run : -INFINITY;
+            P.ws_l[idx] = seen ? l_run : 0.0f;
         }
         float* orow = P.ws_o + idx * D + kCols * half;
 #pragma unroll 1
@@ -506,11 +506,11 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
                 tc::tmem_ld32(to + 32 * c, r);
                 tc::tmem_ld_wait();
             }
-            if (my_pos < 0) continue;
+            if (!is_row) continue;
 #pragma unroll
             for (int e = 0; e < 32; e += 4)
                 *reinterpret_cast<float4*>(orow + 32 * c + e) =
-                    have ? make_float4(__uint_as_float(r[e]), __uint_as_float(r[e + 1]), __uint_as_float(r[e + 2]), __uint_as_float(r[e + 3]))
+                    seen ? make_float4(__uint_as_float(r[e]), __uint_as_float(r[e + 1]), __uint_as_float(r[e + 2]), __uint_as_float(r[e + 3]))
                          : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     }

@@ -85,3 +85,35 @@ def test_workspace_at_any_float(D, op, tokens):
         outs.append(out)
     assert all(torch.equal(outs[0], x) for x in outs[1:])
     assert tw.gpu.errors() == 0
+
+
+@pytest.mark.parametrize("D", [128, 256])
+@pytest.mark.parametrize("tokens", [1, 4, 8, 9, 40])
+def test_rows_without_a_key(D, tokens):
+    """A position of -1 (a rank whose range of a sharded sequence is empty passes it for every row): the row's partial is that of
+    no key at all, whatever the workspace held before, and the rows beside it are as without it."""
+    import torch
+
+    H, QH = 4, 24
+    q = torch.from_numpy(orc.synth_q(5, tokens, QH, D)).to("cuda")
+    none = torch.full((tokens,), -1, dtype=torch.int32, device="cuda")
+    n = tokens * QH * (D + 2)
+
+    def run(tw, pos, kv_len):
+        for ws in (tw.gpu.workspace(kv_len, min(tokens, 8)), tw.gpu.prefill_workspace(kv_len, tokens)):
+            ws.fill_(3.0)
+        return [x.clone() for x in _partial(tw, q, pos, kv_len, torch.full((n,), 7.0, device="cuda"))]
+
+    tw = _filled(D, H, QH, 0)
+    m, l, o = run(tw, none, 128)
+    assert torch.all(m == float("-inf")) and torch.all(l == 0) and torch.all(o == 0)
+    T = 700
+    tw = _filled(D, H, QH, T)
+    pos = torch.arange(T - tokens, T, dtype=torch.int32, device="cuda")
+    want = run(tw, pos, T)
+    pos[:tokens // 2] = -1
+    got = run(tw, pos, T)
+    cut = tokens // 2 * QH
+    assert torch.all(got[0][:cut] == float("-inf")) and torch.all(got[1][:cut] == 0) and torch.all(got[2][:cut] == 0)
+    assert all(torch.equal(a[cut:], b[cut:]) for a, b in zip(got, want))
+    assert tw.gpu.errors() == 0
