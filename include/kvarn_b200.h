@@ -69,6 +69,9 @@ typedef struct kvb_layer {
     int32_t head_dim;            /* 128 or 256 */
     int32_t dtype;               /* KVB_DTYPE_* of k, v, q and out */
     int32_t sinkhorn_iters;      /* 0 = bit-exact regime; the reference engine's default is 16 */
+                                  /* attention at head_dim 128 reads the balancing factors (other_axis) of the planes only when
+                                     this is not 0: a cache must be read with 0 only if it was written with 0.  At head_dim 256
+                                     (and in kvb_decode_tile) they are always applied. */
     uint32_t* error_word;        /* optional device word: kernels OR in a code instead of faulting */
 } kvb_layer;
 

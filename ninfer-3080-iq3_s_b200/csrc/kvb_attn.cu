@@ -1467,12 +1467,9 @@ int launch_attention(const kvb_layer* layer, const void* q, const int32_t* pos_d
     P.ws_o = P.ws_l + rows;
     const bool upper = plan.nb == 2;
     const dim3 grid(parts, layer->kv_heads, Z);
-    if (layer->head_dim != 128) {  // two slices per head: twice the accumulators and the wider integers leave room for 8 warps
-        if (layer->sinkhorn_iters != 0) {
-            KVB_CUDA_OK((launch_attn<2, 1, kWarpsWide, true>(grid, stream, P)));
-        } else {
-            KVB_CUDA_OK((launch_attn<2, 1, kWarpsWide>(grid, stream, P)));
-        }
+    if (layer->head_dim != 128) {  // two slices per head: twice the accumulators and the wider integers leave room for 8 warps.  The
+        // factors of balanced caches are applied whatever the descriptor says: at this head dim a reader need not know the count
+        KVB_CUDA_OK((launch_attn<2, 1, kWarpsWide, true>(grid, stream, P)));
     } else if (layer->sinkhorn_iters != 0) {  // balanced caches: other_K per key, other_V per dim (more registers: 8 warps)
         if (upper) {
             KVB_CUDA_OK((launch_attn<1, 2, kWarpsWide, true>(grid, stream, P)));

@@ -135,7 +135,7 @@ __device__ __forceinline__ void unpack_f32(uint32_t w, F2 (&n)[4]) {
 __device__ __forceinline__ constexpr int nibble_shift(int d) { return 4 * ((d & 7) < 5 ? (d & 7) : (d & 7) - 5); }
 
 // One de-quantising role (eight warps, thread dt): K or V of the CTA's n pages p0 .. p1 - 1.
-template <bool kValue, bool kOther>
+template <bool kValue>
 __device__ __forceinline__ bool dequant_role(Chunk256Smem& sm, const LayerView& L, int head, int dt, int p0, int p1, int kv_total) {
     const int lane = dt & 31, dw = dt >> 5;                    // dt: also the dim whose factors this thread fetches
     const int quarter = dw & 3, key = 32 * (dw >> 2) + lane;   // 64 dims of one key of the page
@@ -230,7 +230,7 @@ __device__ __forceinline__ bool dequant_role(Chunk256Smem& sm, const LayerView& 
             if (bad_key) { t0 = t1 = 0.0f; tb = 0u; live = false; }
             const uint32_t bad = __ballot_sync(0xffffffffu, bad_key);
             if (lane == 0) sm.poison[slot][dw] = bad;
-            if constexpr (kOther) sm.vo[par][dt] = db >= 0x7F800000u ? 0.0f : d0;
+            sm.vo[par][dt] = db >= 0x7F800000u ? 0.0f : d0;
         } else {
             tb = abs_bits(t0);
         }
@@ -281,12 +281,10 @@ __device__ __forceinline__ bool dequant_role(Chunk256Smem& sm, const LayerView& 
                 if constexpr (kValue) {
 #pragma unroll
                     for (int e = 0; e < 4; ++e) x[e] = fma2(x[e], sc[e], z2);
-                    if constexpr (kOther) {
-                        const ulonglong2* ot = reinterpret_cast<const ulonglong2*>(&sm.vo[par][at]);
-                        const ulonglong2 o0 = ot[0], o1 = ot[1];
-                        x[0] = mul2(x[0], F2(o0.x)); x[1] = mul2(x[1], F2(o0.y));
-                        x[2] = mul2(x[2], F2(o1.x)); x[3] = mul2(x[3], F2(o1.y));
-                    }
+                    const ulonglong2* ot = reinterpret_cast<const ulonglong2*>(&sm.vo[par][at]);
+                    const ulonglong2 o0 = ot[0], o1 = ot[1];
+                    x[0] = mul2(x[0], F2(o0.x)); x[1] = mul2(x[1], F2(o0.y));
+                    x[2] = mul2(x[2], F2(o1.x)); x[3] = mul2(x[3], F2(o1.y));
                 } else {
                     const ulonglong2* st = reinterpret_cast<const ulonglong2*>(&sm.ks[par][at]);
                     const ulonglong2* zt = reinterpret_cast<const ulonglong2*>(&sm.kz[par][at]);
@@ -311,7 +309,6 @@ __device__ __forceinline__ bool dequant_role(Chunk256Smem& sm, const LayerView& 
     return failed;
 }
 
-template <bool kOther>
 __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Params P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Chunk256Smem& sm = *reinterpret_cast<Chunk256Smem*>(smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u));
@@ -425,8 +422,8 @@ __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Par
     if (warp >= kSoftWarps && warp < kMmaWarp) {
         tc::regs_dec<kDqRegs>();
         const int dt = tid - 32 * kSoftWarps;
-        if (dt < 32 * kDqWarps) failed = dequant_role<false, kOther>(sm, L, head, dt, p0, p1, kv_total);
-        else failed = dequant_role<true, kOther>(sm, L, head, dt - 32 * kDqWarps, p0, p1, kv_total);
+        if (dt < 32 * kDqWarps) failed = dequant_role<false>(sm, L, head, dt, p0, p1, kv_total);
+        else failed = dequant_role<true>(sm, L, head, dt - 32 * kDqWarps, p0, p1, kv_total);
     } else if (warp >= kMmaWarp) {
         // =========================== MMA issue (one warp; the three beside it complete the warpgroup) ===========================
         tc::regs_dec<kMmaRegs>();
@@ -651,12 +648,10 @@ int launch_chunk_attention_256(const kvb_layer* layer, const void* q, const int3
     const int smem = static_cast<int>(sizeof(Chunk256Smem)) + 1024;  // room to align the tiles to 1024 bytes
     static unsigned long long opted = 0;
     if (first_call_on_device(opted)) {
-        KVB_CUDA_OK(cudaFuncSetAttribute(chunk256_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        KVB_CUDA_OK(cudaFuncSetAttribute(chunk256_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        KVB_CUDA_OK(cudaFuncSetAttribute(chunk256_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     }
     const dim3 grid(P.mtiles, layer->kv_heads, P.ksplit);
-    if (layer->sinkhorn_iters > 0) chunk256_kernel<true><<<grid, kThreads, smem, s>>>(P);
-    else chunk256_kernel<false><<<grid, kThreads, smem, s>>>(P);
+    chunk256_kernel<<<grid, kThreads, smem, s>>>(P);
     KVB_CUDA_OK(cudaGetLastError());
     return launch_chunk_merge<D>(P.ws_m, P.ws_l, P.ws_o, tokens, layer->q_heads, layer->kv_heads, P.mtiles, P.ksplit, layer->dtype, out,
                                  part_m, part_l, part_o, s);

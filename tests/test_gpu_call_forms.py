@@ -117,3 +117,23 @@ def test_rows_without_a_key(D, tokens):
     assert torch.all(got[0][:cut] == float("-inf")) and torch.all(got[1][:cut] == 0) and torch.all(got[2][:cut] == 0)
     assert all(torch.equal(a[cut:], b[cut:]) for a, b in zip(got, want))
     assert tw.gpu.errors() == 0
+
+
+@pytest.mark.parametrize("T,tokens", [(300, 1), (900, 5), (130, 8), (500, 40)])
+def test_a_balanced_cache_of_256_dims_read_without_the_count(T, tokens):
+    """At head_dim 256 the balancing factors lie in the planes and are applied whatever sinkhorn_iters the reader gives."""
+    import torch
+
+    H, QH, D, scale = 4, 24, 256, 1.0 / 16.0
+    tw = _filled(D, H, QH, T, iters=16)
+    q = torch.from_numpy(orc.synth_q(6, tokens, QH, D)).to(tw.dev)
+    pos = torch.arange(T - tokens, T, dtype=torch.int32, device=tw.dev)
+    n = tokens * QH * (D + 2)
+    want = _partial(tw, q, pos, T, torch.empty(n, device=tw.dev))
+    tw.gpu.c.sinkhorn_iters = 0
+    got = _partial(tw, q, pos, T, torch.empty(n, device=tw.dev))
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    out = pkg().merge_partials(*(x.unsqueeze(0) for x in got))
+    ref = cpu_twin_of(tw.gpu).attention(q.cpu().numpy(), pos.cpu().numpy(), scale, QH, threads=4, kv_total=T)
+    ok, msg = attn_close(out.float().cpu().numpy().reshape(ref.shape), ref, ATTN_MAX_ABS, ATTN_REL_L2)
+    assert ok, msg
