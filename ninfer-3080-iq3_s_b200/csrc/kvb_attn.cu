@@ -100,6 +100,7 @@ template <int S, int W> struct __align__(128) AttnSmem {
     WarpRing<S> ring[W];
     float4 qfrag[2 / S][8 * S][32];  // q' in per-lane fragment order: [row half][8 slice + j][lane] = dims 128 slice + 32t+4j..+3 of row g(+8)
     int row_pos[kRows];
+    int poison[2][kRows];    // 256 dims: the row sees a key whose V (in this slice) is not finite
 };
 
 // Per-thread state of the running softmax.  Lane (g, t) owns query rows 8 nb + 2t, 2t+1 of n-block nb and dims
@@ -288,11 +289,60 @@ __device__ __forceinline__ void rescale(Acc<S, NB>& acc, const float (&alpha)[NB
     }
 }
 
+// Values that are not finite (head_dim 256).  A weight of zero does not keep an infinite V away from the rows that may not see its
+// key: V enters the products clamped to finite values, and the rows that do see such a key are marked and end as NaN.
+__device__ __forceinline__ bool nonfinite_half2(uint32_t w) { return (((w & 0x7C007C00u) + 0x04000400u) & 0x80008000u) != 0u; }
+__device__ __forceinline__ uint32_t finite_half2(uint32_t w) {  // the same bits, or +-65504 in the place of an infinity or a NaN
+    asm("max.f16x2 %0, %0, %1;" : "+r"(w) : "r"(0xFBFFFBFFu));
+    asm("min.f16x2 %0, %0, %1;" : "+r"(w) : "r"(0x7BFF7BFFu));
+    return w;
+}
+// Marks the rows that see one of the keys first + i, bit i of `keys`, i < 64.
+__device__ __forceinline__ void poison_rows(int* poison, const int* row_pos, int lane, uint64_t keys, int first, int key_begin, int key_end) {
+    if (lane >= kRows) return;
+    const int lo = max(key_begin - first, 0), hi = min(min(key_end - 1, row_pos[lane]) - first, 63);
+    if (lo <= hi && ((keys >> lo) << (63 - hi + lo)) != 0) poison[lane] = 1;
+}
+// The V scale rows of a page (a key's row: other_V of four dims | its scales | its zero points), some of them not finite: such keys
+// and dims leave the page.  A call: what happens never stays out of the loop's instructions and registers.
+__device__ __noinline__ void sanitize_page(uint4* rows, int (*poison)[kRows], const int* row_pos, int lane, int first, int key_begin, int key_end) {
+    key_end = min(key_end, first + kPage);
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+        uint4 r = rows[lane + 32 * h];
+        const bool dims = nonfinite_half2(r.x) || nonfinite_half2(r.y);
+        if (dims) r.x = r.y = 0u;
+        for (int s = 0; s < 2; ++s) {
+            const uint32_t keep = s ? 0x0000FFFFu : 0xFFFF0000u;
+            const bool key = nonfinite_half2(r.z & ~keep) || nonfinite_half2(r.w & ~keep);
+            if (key) { r.z &= keep; r.w &= keep; }
+            const uint32_t keys = __ballot_sync(0xffffffffu, key);
+            poison_rows(poison[s], row_pos, lane, static_cast<uint64_t>(keys) << (32 * h), first, key_begin, key_end);
+        }
+        if (__any_sync(0xffffffffu, dims)) poison_rows(poison[h], row_pos, lane, ~0ull, first, key_begin, key_end);  // rows 0 .. 31: dims of slice 0
+        rows[lane + 32 * h] = r;
+    }
+    fence_proxy_async();
+    __syncwarp();
+}
+// The same for 16 V rows of the open tile (256 dims; lanes 0 .. 15 look at slice 0, 16 .. 31 at slice 1).
+__device__ __noinline__ void poison_stage_group(const __half* vrow, int (*poison)[kRows], const int* row_pos, int lane, int first, int kv_total, int key_begin, int key_end) {
+    uint32_t keys[2] = {0u, 0u};
+#pragma unroll 1
+    for (int key = 0; key < 16 && first + key < kv_total; ++key) {
+        const uint4 r = *reinterpret_cast<const uint4*>(vrow + key * 256 + 8 * lane);
+        const uint32_t hit = __ballot_sync(0xffffffffu, nonfinite_half2(r.x) || nonfinite_half2(r.y) || nonfinite_half2(r.z) || nonfinite_half2(r.w));
+        if (hit & 0x0000FFFFu) keys[0] |= 1u << key;
+        if (hit & 0xFFFF0000u) keys[1] |= 1u << key;
+    }
+    for (int s = 0; s < 2; ++s) poison_rows(poison[s], row_pos, lane, keys[s], first, key_begin, key_end);
+}
+
 // 16 keys of the open tile, read un-quantised (fp16, rotated) straight from the stage.
 // krow/vrow point at the first of the 16 stage rows of this head (row stride D halves).
 // At 256 dims the weights enter as an fp16 high and low part, like the query.
-template <int S, int NB>
-__device__ __forceinline__ void process_stage_group(const __half* krow, const __half* vrow, const QFrag<S, NB>& qf,
+template <int S, int NB, typename Smem>
+__device__ __forceinline__ void process_stage_group(Smem& sm, const __half* krow, const __half* vrow, const QFrag<S, NB>& qf,
                                                     Acc<S, NB>& acc, int lane, int first_pos, int kv_total,
                                                     const int (&row_lim)[NB][2], int key_begin, int key_end) {
     constexpr int D = Shape<S>::kDim;
@@ -360,7 +410,8 @@ __device__ __forceinline__ void process_stage_group(const __half* krow, const __
         }
     }
     // A = V^T: the lane supplies dims 32 db + 4g .. +3 of keys 2t, 2t+1, 2t+8, 2t+9.  Keys at or beyond kv_total hold
-    // stale rows: their p is exactly 0; zero V there so 0 * inf cannot appear.
+    // stale rows: their p is exactly 0; zero V there so 0 * inf cannot appear.  (At 256 dims V is clamped: see finite_half2.)
+    uint32_t odd = 0;
 #pragma unroll
     for (int db = 0; db < 4 * S; ++db) {
         uint2 v[4];
@@ -369,6 +420,11 @@ __device__ __forceinline__ void process_stage_group(const __half* krow, const __
             const int key = 2 * t + (kk & 1) + (kk >> 1) * 8;
             const bool live = first_pos + key < kv_total;
             v[kk] = live ? *reinterpret_cast<const uint2*>(vrow + key * D + 32 * db + 4 * g) : make_uint2(0u, 0u);
+            if constexpr (S == 2) {
+                const uint2 f = make_uint2(finite_half2(v[kk].x), finite_half2(v[kk].y));
+                odd |= (f.x ^ v[kk].x) | (f.y ^ v[kk].y);
+                v[kk] = f;
+            }
         }
         const uint32_t x0 = prmt(v[0].x, v[1].x, 0x5410), x1 = prmt(v[0].y, v[1].y, 0x5410);  // dims 4g, 4g+2 of keys 2t, 2t+1
         const uint32_t x2 = prmt(v[2].x, v[3].x, 0x5410), x3 = prmt(v[2].y, v[3].y, 0x5410);  // ... of keys 2t+8, 2t+9
@@ -383,6 +439,9 @@ __device__ __forceinline__ void process_stage_group(const __half* krow, const __
                 mma16816(acc.o[nb][db][1], y0, y1, y2, y3, c0[nb], c1[nb]);
             }
         }
+    }
+    if constexpr (S == 2) {
+        if (__any_sync(0xffffffffu, odd != 0u)) poison_stage_group(vrow, sm.poison, sm.row_pos, lane, first_pos, kv_total, key_begin, key_end);
     }
 }
 
@@ -433,6 +492,7 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
     const int key_end = min(P.key_end, kv_total), key_begin = max(P.key_begin, 0);
     const int sealed_pages = 2 * (kv_total / kTile);
 
+    if (S == 2 && threadIdx.x < 2 * kRows) (&sm.poison[0][0])[threadIdx.x] = 0;
     if (lane == 0) {
 #pragma unroll
         for (int s = 0; s < kSlots; ++s) mbar_init(&R.bars[s], 1);
@@ -555,7 +615,7 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
             if (first < key_end && first + 16 > key_begin && first < kv_total) {
                 QFrag<S, NB> qf;
                 build_qfrag<S, NB>(sm, lane, qf);
-                process_stage_group<S, NB>(L.stage_row(0, tile & 1, head, 16 * grp), L.stage_row(1, tile & 1, head, 16 * grp), qf,
+                process_stage_group<S, NB>(sm, L.stage_row(0, tile & 1, head, 16 * grp), L.stage_row(1, tile & 1, head, 16 * grp), qf,
                                         acc, lane, first, kv_total, row_lim, key_begin, key_end);
             }
         }
@@ -604,6 +664,21 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
         // ---- K chunk + header
         wait_slot(slot);
         const uint8_t* hdr = R.hdr[pi % kHdrs];
+        uint32_t sc = 0;  // 256 dims: the lane's largest scales of V, one slice a half
+        if constexpr (S == 2) {
+            uint4* rows = reinterpret_cast<uint4*>(R.hdr[pi % kHdrs]);
+            constexpr uint32_t kAbs = 0x7FFF7FFFu;
+            auto look = [&]() {  // whether a factor of V is not finite
+                const uint4 a = rows[lane], b = rows[lane + 32];
+                sc = __vmaxu2(a.z & kAbs, b.z & kAbs);
+                const uint32_t all = __vmaxu2(__vmaxu2(__vmaxu2(a.x & kAbs, b.x & kAbs), __vmaxu2(a.y & kAbs, b.y & kAbs)), __vmaxu2(__vmaxu2(a.w & kAbs, b.w & kAbs), sc));
+                return __any_sync(0xffffffffu, nonfinite_half2(all));
+            };
+            if (look()) {
+                sanitize_page(rows, sm.poison, sm.row_pos, lane, lp * kPage, key_begin, key_end);
+                sc = __vmaxu2(rows[lane].z & kAbs, rows[lane + 32].z & kAbs);
+            }
+        }
         if ((lp >> 1) != cur_tile) {  // per-dim scale / zero point of K belong to the tile
             cur_tile = lp >> 1;
             __syncwarp();
@@ -615,8 +690,7 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
                 for (int db = 0; db < Sh::kBlocks; ++db)
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        const int at = S == 1 ? (16 * db + 2 * g + h) * 8 : (8 * db + g) * 16 + 4 * h;
-                        const float2 o2 = unpack_half2(*reinterpret_cast<const uint32_t*>(hdr + at));
+                        const float2 o2 = unpack_half2(*reinterpret_cast<const uint32_t*>(hdr + (S == 1 ? (16 * db + 2 * g + h) * 8 : (8 * db + g) * 16 + 4 * h)));
                         ov[db][0][h] = o2.x;
                         ov[db][1][h] = o2.y;
                     }
@@ -718,14 +792,20 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
         {
             // per-key scale of V: the largest of the page bounds p * scale_V; one factor for all rows
             float F[S], invF[S];
-#pragma unroll
-            for (int s = 0; s < S; ++s) {
-                float svmax = fmaxf(fabsf(__half2float(*reinterpret_cast<const __half*>(hdr + lane * 8 * S + 4 * S + 2 * s))),
-                                    fabsf(__half2float(*reinterpret_cast<const __half*>(hdr + (lane + 32) * 8 * S + 4 * S + 2 * s))));
+            if constexpr (S == 1) {
+                float svmax = fmaxf(fabsf(__half2float(*reinterpret_cast<const __half*>(hdr + lane * 8 + 4))),
+                                    fabsf(__half2float(*reinterpret_cast<const __half*>(hdr + (lane + 32) * 8 + 4))));
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) svmax = fmaxf(svmax, __shfl_xor_sync(0xffffffffu, svmax, o));
-                F[s] = svmax > 0.0f ? Sh::kPMax / svmax : 0.0f;
-                invF[s] = svmax * (1.0f / Sh::kPMax);
+                F[0] = svmax > 0.0f ? Sh::kPMax / svmax : 0.0f;
+                invF[0] = svmax * (1.0f / Sh::kPMax);
+            } else {
+#pragma unroll
+                for (int s = 0; s < S; ++s) {
+                    const float svmax = __half2float(__ushort_as_half(static_cast<uint16_t>(__reduce_max_sync(0xffffffffu, s ? sc >> 16 : sc & 0xFFFFu))));
+                    F[s] = svmax > 0.0f ? Sh::kPMax / svmax : 0.0f;
+                    invF[s] = svmax * (1.0f / Sh::kPMax);
+                }
             }
             float alpha[NB][2], wpass[NB][2], cst[NB][2];
             bool moved = false;
@@ -998,6 +1078,7 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
                 o.x += wt * (v.x + z); o.y += wt * (v.y + z); o.z += wt * (v.z + z); o.w += wt * (v.w + z);
             }
         }
+        if (S == 2 && sm.poison[d / 128][row] != 0) o.x = o.y = o.z = o.w = __uint_as_float(0x7FC00000u);
         *reinterpret_cast<float4*>(P.ws_o + (pidx + row) * D + d) = o;
         if (d == 0) { P.ws_m[pidx + row] = m; P.ws_l[pidx + row] = l; }
     }

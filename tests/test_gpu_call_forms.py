@@ -137,3 +137,76 @@ def test_a_balanced_cache_of_256_dims_read_without_the_count(T, tokens):
     ref = cpu_twin_of(tw.gpu).attention(q.cpu().numpy(), pos.cpu().numpy(), scale, QH, threads=4, kv_total=T)
     ok, msg = attn_close(out.float().cpu().numpy().reshape(ref.shape), ref, ATTN_MAX_ABS, ATTN_REL_L2)
     assert ok, msg
+
+
+def _causal_run(tw, q, k, v, T, entry):
+    import torch
+
+    pos = torch.arange(T, T + q.shape[0], dtype=torch.int32, device=tw.dev)
+    return getattr(tw.gpu, entry)(q, k, v, pos, 1.0 / np.sqrt(tw.D), T + q.shape[0])
+
+
+@pytest.mark.parametrize("T,tokens,at,entry", [(300, 5, 2, "attn_verify"), (125, 5, 1, "attn_verify"), (255, 8, 7, "attn_verify"), (120, 8, 0, "attn_verify"),
+                                               (300, 40, 17, "attn_prefill"), (100, 60, 30, "attn_prefill")])
+def test_non_finite_v_reaches_the_rows_that_see_it(T, tokens, at, entry):
+    """One row of a step at head_dim 256 overflows in V, in the open tile or in one that the step seals: the rows before it are as
+    if that key's V were zero, the rows from it on are not a number."""
+    import torch
+
+    H, QH, D = 4, 24, 256
+    q, k, v = (torch.from_numpy(x).cuda() for x in (orc.synth_q(7, tokens, QH, D), orc.synth_kv(8, tokens, H, D, 1), orc.synth_kv(8, tokens, H, D, 2)))
+    out = {}
+    for name, value in (("zero", 0.0), ("inf", float("inf")), ("nan", float("nan"))):
+        tw = _filled(D, H, QH, T, room=64)
+        v[at] = 0.0
+        v[at, 1:3, 77] = value
+        out[name] = _causal_run(tw, q, k, v, T, entry).float().view(tokens, H, QH // H, D)
+        assert tw.gpu.errors() == 0
+    assert torch.isfinite(out["zero"]).all()
+    for name in ("inf", "nan"):
+        hit, ref = out[name], out["zero"]
+        assert torch.equal(hit[:at], ref[:at]) and torch.equal(hit[:, [0, 3]], ref[:, [0, 3]])
+        assert torch.isnan(hit[at:, 1:3]).all()
+
+
+@pytest.mark.parametrize("what", ["scale", "zero point", "dim"])
+def test_non_finite_factors_of_a_page(what):
+    """A V factor of tile 1 (of token 150, or of a dim) is infinite in the planes, slice 1 only: key ranges without that token (that
+    tile) are unaffected, ranges with it are not a number in that slice."""
+    import torch
+
+    H, QH, D, T = 4, 24, 256, 400
+    tw = _filled(D, H, QH, T)
+    q = torch.from_numpy(orc.synth_q(9, 1, QH, D)[0]).to(tw.dev)
+    pos = torch.tensor([T - 1], dtype=torch.int32, device=tw.dev)
+
+    def ranges():
+        return [[x.clone() for x in tw.gpu.attn_decode_partial(q, pos, 1.0 / 16.0, T, a, b)] for a, b in ((0, 128), (128, 150), (150, 151), (140, 170), (256, T), (0, T))]
+
+    def row(token):
+        return tw.gpu.v_scale[int(tw.table[token // 64]), :, token % 64]
+
+    if what == "dim":  # dim 200: entry 0 of scale row 50 of either page
+        for page in (2, 3):
+            row(64 * page + 50)[:, 0] = 0.0
+    else:
+        row(150)[:, 5 if what == "scale" else 7] = 0.0
+    want = ranges()
+    if what == "dim":
+        for page in (2, 3):
+            row(64 * page + 50)[:, 0] = float("inf")
+        hit = [False, True, True, True, False, True]
+    else:
+        row(150)[:, 5 if what == "scale" else 7] = float("-inf")
+        if what == "zero point":  # the whole factor leaves with it
+            row(150)[:, 5] = 0.0
+        hit = [False, False, True, True, False, True]
+    got = ranges()
+    for g, w, h in zip(got, want, hit):
+        assert torch.equal(g[0], w[0]) and torch.equal(g[1], w[1])
+        if h:
+            assert torch.isnan(g[2][:, 128:]).all() and torch.isfinite(g[2][:, :128]).all()
+        elif what == "dim":
+            assert torch.equal(g[2], w[2])
+        else:
+            assert torch.allclose(g[2], w[2], rtol=0, atol=float(w[2].abs().max()) * 2.0 ** -21)  # another largest scale of the page
