@@ -453,11 +453,9 @@ template <int D, bool kBf16>
 int launch_append(const LayerView& V, const void* k, const void* v, const int32_t* positions, int tokens,
                   cudaStream_t stream) {
     static_assert(sizeof(AppendSmem) <= 227 * 1024, "shared memory");
-    static unsigned long long opted = 0;  // per template instance; setting the attribute again is harmless
+    static OncePerDevice opted;  // per template instance
     const int smem = static_cast<int>(sizeof(AppendSmem));
-    if (first_call_on_device(opted)) {
-        KVB_CUDA_OK(cudaFuncSetAttribute(append_kernel<D, kBf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    }
+    KVB_CUDA_OK(allow_smem(opted, append_kernel<D, kBf16>, smem));
     const dim3 grid(tokens / kTile + 2, V.kv_heads, 2 * Geo<D>::S);
     KVB_CUDA_OK(launch_early(append_kernel<D, kBf16>, grid, dim3(kThreads), smem, stream, V, static_cast<const uint16_t*>(k), static_cast<const uint16_t*>(v),
                              positions, tokens));

@@ -1466,11 +1466,8 @@ namespace {
 template <int S, int NB, int W, bool kOther = false>
 cudaError_t launch_attn(dim3 grid, cudaStream_t stream, const AttnParams& P) {
     constexpr int smem = static_cast<int>(sizeof(AttnSmem<S, W>));
-    static unsigned long long opted = 0;
-    if (first_call_on_device(opted)) {
-        const cudaError_t e = cudaFuncSetAttribute(attn_kernel<S, NB, W, kOther>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return e;
-    }
+    static OncePerDevice opted;
+    if (const cudaError_t e = allow_smem(opted, attn_kernel<S, NB, W, kOther>, smem)) return e;
     return launch_early(attn_kernel<S, NB, W, kOther>, grid, dim3(W * 32), smem, stream, P);
 }
 
@@ -1816,11 +1813,9 @@ extern "C" int kvb_attn_decode_batch(const kvb_layer* layers_dev, int batch, int
     B.ws_l = B.ws_m + rows;
     B.ws_o = B.ws_l + rows;
     constexpr int smem1 = static_cast<int>(sizeof(AttnSmem<1, kWarpsDecode>)), smem2 = static_cast<int>(sizeof(AttnSmem<1, kWarpsWide>));
-    static unsigned long long opted = 0;
-    if (first_call_on_device(opted)) {
-        KVB_CUDA_OK(cudaFuncSetAttribute(attn_batch_kernel<1, kWarpsDecode>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem1));
-        KVB_CUDA_OK(cudaFuncSetAttribute(attn_batch_kernel<2, kWarpsWide>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2));
-    }
+    static OncePerDevice opted1, opted2;
+    KVB_CUDA_OK(allow_smem(opted1, attn_batch_kernel<1, kWarpsDecode>, smem1));
+    KVB_CUDA_OK(allow_smem(opted2, attn_batch_kernel<2, kWarpsWide>, smem2));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (q_heads / kv_heads > 8) KVB_CUDA_OK(launch_early(attn_batch_kernel<2, kWarpsWide>, dim3(total, kv_heads, 1), dim3(kWarpsWide * 32), smem2, st, B));
     else KVB_CUDA_OK(launch_early(attn_batch_kernel<1, kWarpsDecode>, dim3(total, kv_heads, 1), dim3(kWarpsDecode * 32), smem1, st, B));

@@ -646,10 +646,8 @@ int launch_chunk_attention_256(const kvb_layer* layer, const void* q, const int3
     P.ws_l = P.ws_m + rows;
     P.ws_o = P.ws_l + rows;
     const int smem = static_cast<int>(sizeof(Chunk256Smem)) + 1024;  // room to align the tiles to 1024 bytes
-    static unsigned long long opted = 0;
-    if (first_call_on_device(opted)) {
-        KVB_CUDA_OK(cudaFuncSetAttribute(chunk256_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    }
+    static OncePerDevice opted;
+    KVB_CUDA_OK(allow_smem(opted, chunk256_kernel, smem));
     const dim3 grid(P.mtiles, layer->kv_heads, P.ksplit);
     chunk256_kernel<<<grid, kThreads, smem, s>>>(P);
     KVB_CUDA_OK(cudaGetLastError());

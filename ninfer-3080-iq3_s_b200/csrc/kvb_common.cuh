@@ -5,10 +5,12 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
 
 #include "../../include/kvarn_b200.h"
+#include "kvb_once.hpp"
 
 namespace kvb {
 
@@ -103,24 +105,24 @@ inline cudaError_t launch_early(void (*kernel)(KArgs...), dim3 grid, dim3 block,
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-// True the first time it is called on the current device for this `seen` mask: for set-up CUDA keeps per device
-// (the opt-in to large dynamic shared memory).  Not synchronised -- two threads making the first call at once
-// both do the set-up, which is harmless.
-inline bool first_call_on_device(unsigned long long& seen) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return true;
-    const unsigned long long bit = 1ull << (dev & 63);
-    if (seen & bit) return false;
-    seen |= bit;
-    return true;
+inline int current_device() {  // -1: unknown
+    int dev = -1;
+    return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
+}
+// Lets a kernel take more dynamic shared memory than a launch may by default (CUDA keeps this per device).
+template <typename K> cudaError_t allow_smem(OncePerDevice& once, K* kernel, int bytes) {
+    return once.run(current_device(), [&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); });
 }
 // SM count of the current device (cached per device; 148 if the query fails).
 inline int device_sm_count() {
-    static int cache[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 148;
-    int& n = cache[dev & 63];
-    if (n <= 0 && (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)) n = 148;
+    static std::atomic<int> cache[64];
+    const int dev = current_device();
+    if (dev < 0) return 148;
+    int n = cache[dev & 63].load(std::memory_order_relaxed);
+    if (n <= 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+        cache[dev & 63].store(n, std::memory_order_relaxed);
+    }
     return n;
 }
 

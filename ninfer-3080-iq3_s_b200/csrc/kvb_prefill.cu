@@ -589,15 +589,10 @@ int launch_chunk_attention(const kvb_layer* layer, const void* q, const int32_t*
     P.ws_l = P.ws_m + rows;
     P.ws_o = P.ws_l + rows;
     const int smem = static_cast<int>(sizeof(PrefillSmem)) + 1024;  // room to align the tiles to 1024 bytes
-    static unsigned long long opted = 0;
-    if (first_call_on_device(opted)) {
-        KVB_CUDA_OK(cudaFuncSetAttribute(chunk_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        KVB_CUDA_OK(cudaFuncSetAttribute(chunk_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        KVB_CUDA_OK(cudaFuncSetAttribute(chunk_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        KVB_CUDA_OK(cudaFuncSetAttribute(chunk_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    }
     const bool other = layer->sinkhorn_iters > 0;
     const auto kernel = shape.split ? (other ? chunk_kernel<true, true> : chunk_kernel<true, false>) : (other ? chunk_kernel<false, true> : chunk_kernel<false, false>);
+    static OncePerDevice opted[4];
+    KVB_CUDA_OK(allow_smem(opted[2 * shape.split + other], kernel, smem));
     const dim3 grid(shape.split ? shape.mtiles : (shape.mtiles + 1) / 2, layer->kv_heads, shape.ranges);
     kernel<<<grid, kThreads, smem, s>>>(P);
     KVB_CUDA_OK(cudaGetLastError());

@@ -46,3 +46,17 @@ def test_engine_shim_on_the_gpu_equals_the_c_abi(tmp_path):
     r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
     assert "engine shim on the GPU: ok" in r.stdout
+
+
+def _run_host_check(tmp_path, name):
+    exe = str(tmp_path / name)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", "-I", os.path.join(ROOT, "ninfer-3080-iq3_s_b200", "csrc"),
+                    os.path.join(ROOT, "tests", "cpp", name + ".cpp"), "-o", exe], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+    return r.stdout
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs a C++ compiler")
+def test_device_setup_is_done_before_any_thread_goes_on(tmp_path):
+    assert "once per device: ok" in _run_host_check(tmp_path, "once_check")
