@@ -1471,6 +1471,23 @@ cudaError_t launch_attn(dim3 grid, cudaStream_t stream, const AttnParams& P) {
     return launch_early(attn_kernel<S, NB, W, kOther>, grid, dim3(W * 32), smem, stream, P);
 }
 
+// The merge asks for as little shared memory as an SM can be set to.  Left to itself the driver sets an SM up for as many of its
+// CTAs as the registers allow (four: 64 KB), and the SM's change between that and the attention kernel's 132 KB or more lies
+// between the two in a chain of layers.  Measured on B200 in graph replay, a decode call at 16,384 / 32,768 / 131,072 tokens:
+// 9.4 / 12.0 / 23.1 us left to the driver, 8.6 / 11.2 / 22.2 with 0, 9.7 / 12.3 / 23.3 with both kernels asking for all of it.
+template <int S, bool kPush>
+cudaError_t launch_reduce(int rows, cudaStream_t stream, const float* ws_m, const float* ws_l, const float* ws_o, int parts, int T, int q_heads, int kv_heads,
+                          int zblocks, int block_rows, int dtype, uint16_t* out, float* part_m, float* part_l, float* part_o, const PushTarget& push,
+                          const BatchPlan& plan) {
+    static OncePerDevice set;
+    const cudaError_t e = set.run(current_device(), [] {
+        return cudaFuncSetAttribute(reduce_kernel<S, kPush>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1);
+    });
+    if (e != cudaSuccess) return e;
+    return launch_early(reduce_kernel<S, kPush>, dim3(rows), dim3(kReduceWarps * 32), 0, stream, ws_m, ws_l, ws_o, parts, T, q_heads, kv_heads, zblocks,
+                        block_rows, dtype, out, part_m, part_l, part_o, push, plan);
+}
+
 // Warps per CTA for a decode call: 8, 12 or 16 (whole warp quartets: an SM hands registers and issue slots out per
 // quartet; 10 or 14 warps measured no faster per warp than 12 or 16).  A warp works on whole pages, so a CTA with n
 // pages needs ceil(n / W) rounds; a round and the fixed part (set-up, merge of the warps) take longer the more warps
@@ -1564,8 +1581,8 @@ int launch_attention(const kvb_layer* layer, const void* q, const int32_t* pos_d
         }
     }
     const int total_rows = T * layer->q_heads;
-    const auto reduce = layer->head_dim != 128 ? reduce_kernel<2, false> : push != nullptr ? reduce_kernel<1, true> : reduce_kernel<1, false>;
-    KVB_CUDA_OK(launch_early(reduce, dim3(total_rows), dim3(kReduceWarps * 32), 0, stream, P.ws_m, P.ws_l, P.ws_o, parts, T,
+    const auto launch = layer->head_dim != 128 ? launch_reduce<2, false> : push != nullptr ? launch_reduce<1, true> : launch_reduce<1, false>;
+    KVB_CUDA_OK(launch(total_rows, stream, P.ws_m, P.ws_l, P.ws_o, parts, T,
                              layer->q_heads, layer->kv_heads, Z, plan.block_rows, layer->dtype, static_cast<uint16_t*>(out), part_m, part_l, part_o,
                              push != nullptr ? *push : PushTarget{}, BatchPlan{}));
     return KVB_OK;
@@ -1819,9 +1836,8 @@ extern "C" int kvb_attn_decode_batch(const kvb_layer* layers_dev, int batch, int
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (q_heads / kv_heads > 8) KVB_CUDA_OK(launch_early(attn_batch_kernel<2, kWarpsWide>, dim3(total, kv_heads, 1), dim3(kWarpsWide * 32), smem2, st, B));
     else KVB_CUDA_OK(launch_early(attn_batch_kernel<1, kWarpsDecode>, dim3(total, kv_heads, 1), dim3(kWarpsDecode * 32), smem1, st, B));
-    KVB_CUDA_OK(launch_early(reduce_kernel<1, false>, dim3(batch * q_heads), dim3(kReduceWarps * 32), 0, st, B.ws_m, B.ws_l, B.ws_o, 0, batch, q_heads,
-                             kv_heads, 1, kRows, dtype, static_cast<uint16_t*>(out), static_cast<float*>(nullptr), static_cast<float*>(nullptr),
-                             static_cast<float*>(nullptr), PushTarget{}, B.plan));
+    KVB_CUDA_OK((launch_reduce<1, false>(batch * q_heads, st, B.ws_m, B.ws_l, B.ws_o, 0, batch, q_heads, kv_heads, 1, kRows, dtype, static_cast<uint16_t*>(out),
+                                         nullptr, nullptr, nullptr, PushTarget{}, B.plan)));
     return KVB_OK;
 }
 
