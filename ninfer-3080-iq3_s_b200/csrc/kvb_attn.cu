@@ -1605,7 +1605,7 @@ static size_t workspace_bytes_for_rows(int kv_len_max, int kv_heads, int q_heads
         const size_t parts = kvb::split_count(kv_len_max, kv_heads, Z);
         bytes = std::max(bytes, static_cast<size_t>(kv_heads) * Z * parts * kvb::kRows * (head_dim + 2) * sizeof(float) + kvb::kWorkspaceSlack);
     }
-    if (r > 8 || r * (q_heads / kv_heads) >= kDenseRows) {  // steps this wide run on the chunk-attention kernels
+    if (r > 8 || (head_dim == 128 && r * (q_heads / kv_heads) >= kDenseRows)) {  // steps this wide run on the chunk-attention kernels
         const size_t dense = kvb_prefill_workspace_bytes(kv_len_max, kv_heads, q_heads, head_dim, r);
         if (dense > bytes) bytes = dense;
     }

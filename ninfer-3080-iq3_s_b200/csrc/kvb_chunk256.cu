@@ -606,29 +606,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Par
     if (warp == kMmaWarp) tc::tmem_dealloc(tmem, kTmemCols);
 }
 
-// Row tiles and key ranges of a call.  One CTA per SM; a CTA costs its pages plus about six pages' worth of set-up and
-// epilogue, and every further range a partial per row: the number of ranges (at most four waves' worth, at least four
-// pages each) with the lowest (waves x CTA) is taken.
-void chunk256_shape(int kv_len_max, int kv_heads, int q_heads, int tokens, int* mtiles, int* ksplit) {
-    const int rows = tokens * (q_heads / kv_heads), sms = device_sm_count(), pages = (kv_len_max + kN - 1) / kN;
-    *mtiles = (rows + kM - 1) / kM;
-    const int ctas = *mtiles * kv_heads;
-    int best = 1;
-    int64_t best_cost = INT64_MAX;
-    for (int ks = 1; ks <= kMaxKeyRanges && (ks == 1 || (4 * ks <= pages && ctas * ks <= 4 * sms)); ++ks) {
-        const int64_t cost = static_cast<int64_t>((ctas * ks + sms - 1) / sms) * (6 + (pages + ks - 1) / ks);
-        if (cost < best_cost) { best_cost = cost; best = ks; }
-    }
-    *ksplit = best;
-}
-
 }  // namespace
-
-size_t chunk256_workspace_bytes(int kv_len_max, int kv_heads, int q_heads, int tokens) {
-    int mtiles, ksplit;
-    chunk256_shape(kv_len_max, kv_heads, q_heads, tokens, &mtiles, &ksplit);
-    return static_cast<size_t>(kv_heads) * mtiles * ksplit * kM * (D + 2) * sizeof(float);
-}
 
 // Chunk attention of `tokens` rows that are already appended, over a head_dim-256 cache.
 int launch_chunk_attention_256(const kvb_layer* layer, const void* q, const int32_t* positions_dev, int tokens, float scale,
@@ -639,7 +617,9 @@ int launch_chunk_attention_256(const kvb_layer* layer, const void* q, const int3
     P.pos = positions_dev;
     P.total_pos = positions_dev + (tokens - 1);
     P.T = tokens;
-    chunk256_shape(kv_len_max, layer->kv_heads, layer->q_heads, tokens, &P.mtiles, &P.ksplit);
+    const ChunkShape shape = chunk_shape_256(kv_len_max, layer->kv_heads, layer->q_heads, tokens, device_sm_count());
+    P.mtiles = shape.mtiles;
+    P.ksplit = shape.ksplit;
     P.scale_log2 = scale * 1.4426950408889634f;
     const size_t rows = static_cast<size_t>(layer->kv_heads) * P.mtiles * P.ksplit * kM;
     P.ws_m = workspace_base(workspace);

@@ -3,14 +3,13 @@
 
 #include <climits>
 
+#include "kvb_chunk_shape.hpp"
 #include "kvb_common.cuh"
 #include "kvb_ptx.cuh"
 
 namespace kvb {
 namespace {
 
-constexpr int kRowTile = 128;       // rows per row tile of the partials
-constexpr int kMaxKeyRanges = 128;  // what the merge kernel holds
 constexpr int kNoRow = INT_MIN;     // position of a row of a tile that the chunk does not have (a row that sees no key: -1)
 
 // Position of dim d inside its group of eight: order 0,4,1,5,2,6,3,7.

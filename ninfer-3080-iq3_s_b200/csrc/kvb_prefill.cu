@@ -18,7 +18,6 @@
 // puts the output dims back.  Keys of the open tile come un-quantised from the stage.
 // Every wait on an mbarrier is bounded and also watches the CTA's abort flag; a wait that gives up sets
 // KVB_ERR_WAIT_TIMEOUT and the CTA leaves through the normal exit (its MMAs are over, TMEM is freed).
-#include <algorithm>
 #include <climits>
 
 #include "kvb_chunk_merge.cuh"
@@ -520,53 +519,18 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
     if (warp == kMmaWarp) tc::tmem_dealloc(tmem, kTmemCols);
 }
 
-struct ChunkShape {
-    bool split;             // one row tile per CTA, its streams split the keys
-    int mtiles, ksplit;     // row tiles; partials per row
-    int ranges;             // key ranges (grid z)
-};
-constexpr int kWaves = 4;   // at most four waves of CTAs
-// The cheapest (waves x CTA), one CTA per SM, in fifths of the time a row tile takes for a key tile with two row tiles a CTA
-// (1.3 us, measured at 1,024 tokens over 262,144; with split keys 1.8 us): a step of two row tiles costs 10, one with split
-// keys 7, set-up and epilogue about 18 and 13 us.  Measured: 1,024 tokens over 262,144 3.46 ms with two row tiles, 4.76 ms
-// with split keys; 777 tokens alone 36 and 25 us.
-ChunkShape prefill_shape(int kv_len_max, int kv_heads, int q_heads, int tokens) {
-    const int rows = tokens * (q_heads / kv_heads), mtiles = (rows + kM - 1) / kM, ntiles = (kv_len_max + kN - 1) / kN, sms = device_sm_count();
-    ChunkShape best{};
-    int64_t best_cost = INT64_MAX;
-    for (int split = mtiles == 1 ? 1 : 0; split < 2; ++split) {
-        const int ctas = (split ? mtiles : (mtiles + 1) / 2) * kv_heads, per = split ? 2 : 1;
-        for (int r = 1; per * r <= kMaxKeyRanges && (r == 1 || (2 * r <= ntiles && ctas * r <= kWaves * sms)); ++r) {
-            const int64_t steps = (ntiles + r - 1) / r;
-            const int64_t cost = static_cast<int64_t>((ctas * r + sms - 1) / sms) * (split ? 50 + 7 * steps : 70 + 10 * steps);
-            if (cost < best_cost) {
-                best_cost = cost;
-                best = {split != 0, mtiles, per * r, r};
-            }
-        }
-    }
-    return best;
-}
-
 }  // namespace
 }  // namespace kvb
 
 namespace kvb {
 // kvb_chunk256.cu: the same for head_dim 256
-size_t chunk256_workspace_bytes(int kv_len_max, int kv_heads, int q_heads, int tokens);
 int launch_chunk_attention_256(const kvb_layer* layer, const void* q, const int32_t* positions_dev, int tokens, float scale,
                                int kv_len_max, void* workspace, void* out, cudaStream_t s, float* part_m, float* part_l, float* part_o);
 }  // namespace kvb
 
 extern "C" size_t kvb_prefill_workspace_bytes(int kv_len_max, int kv_heads, int q_heads, int head_dim, int tokens) {
     if (kv_heads < 1 || q_heads < kv_heads || tokens < 1) return 0;
-    // The most partials a call of up to this many tokens and keys can have (a shorter one may be cut into more ranges).
-    const size_t tiles = static_cast<size_t>((tokens * (q_heads / kv_heads) + kvb::kM - 1) / kvb::kM) * kv_heads, ntiles = (kv_len_max + kvb::kN - 1) / kvb::kN;
-    const size_t cap = static_cast<size_t>(kvb::kWaves) * kvb::device_sm_count();
-    const size_t partials = 2 * std::max(tiles, std::min(cap, tiles * std::max<size_t>(1, ntiles / 2)));
-    const size_t tuned = partials * kvb::kM * (head_dim + 2) * sizeof(float);
-    const size_t wide = head_dim == 256 ? kvb::chunk256_workspace_bytes(kv_len_max, kv_heads, q_heads, tokens) : 0;
-    return (tuned > wide ? tuned : wide) + kvb::kWorkspaceSlack;
+    return kvb::partials_bytes(kvb::most_partials(head_dim, kv_len_max, kv_heads, q_heads, tokens, kvb::device_sm_count()), head_dim) + kvb::kWorkspaceSlack;
 }
 
 namespace kvb {
@@ -580,7 +544,7 @@ int launch_chunk_attention(const kvb_layer* layer, const void* q, const int32_t*
     P.pos = positions_dev;
     P.total_pos = total_pos_dev != nullptr ? total_pos_dev : positions_dev + (tokens - 1);
     P.T = tokens;
-    const ChunkShape shape = prefill_shape(kv_len_max, layer->kv_heads, layer->q_heads, tokens);
+    const ChunkShape shape = chunk_shape_128(kv_len_max, layer->kv_heads, layer->q_heads, tokens, device_sm_count());
     P.mtiles = shape.mtiles;
     P.ksplit = shape.ksplit;
     P.scale_log2 = scale * 1.4426950408889634f;

@@ -60,3 +60,19 @@ def _run_host_check(tmp_path, name):
 @pytest.mark.skipif(shutil.which("g++") is None, reason="needs a C++ compiler")
 def test_device_setup_is_done_before_any_thread_goes_on(tmp_path):
     assert "once per device: ok" in _run_host_check(tmp_path, "once_check")
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs a C++ compiler")
+def test_chunk_workspaces_cover_every_smaller_call(tmp_path):
+    assert "chunk shapes: ok" in _run_host_check(tmp_path, "chunk_shape_check")
+
+
+def test_chunk_workspaces_are_what_a_call_can_use():
+    """24 / 4 heads, 148 SMs: an 8-row verify step takes 74 partials a row at 128 dims and the narrow kernel's at 256; a short prompt
+    takes one key range, a chunk at 256 dims three."""
+    lib = pkg().capi.load()
+    part = {D: 128 * (D + 2) * 4 for D in (128, 256)}
+    assert lib.kvb_workspace_bytes(131072, 4, 24, 128, 8, 1) <= 4 * 74 * part[128] + 64
+    assert lib.kvb_workspace_bytes(131072, 4, 24, 256, 8, 1) <= 4 * 37 * 16 * 258 * 4 + 64
+    assert lib.kvb_prefill_workspace_bytes(777, 4, 24, 128, 777) <= 4 * 37 * 2 * part[128] + 64
+    assert lib.kvb_prefill_workspace_bytes(17408, 4, 24, 256, 1024) <= 1.1 * 4 * 48 * 3 * part[256]
