@@ -518,6 +518,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Par
                     if ((lo | hi) != 0u && !bad_page) {
                         for (int j = 0; j < kN; ++j)
                             if (((j < 32 ? lo : hi) >> (j & 31) & 1u) && base + j <= my_pos && base + j < kv_total) poisoned = true;
+                        __syncwarp();
                     }
                 }
                 float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -587,17 +588,19 @@ __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Par
 #pragma unroll 1
         for (int c = 0; c < D / 32; ++c) {
             if (!warp_has_rows) break;
+            __syncwarp();  // the load is the whole warp's: lanes without a row are back from the stores
             uint32_t r[32];
             if (have) {
                 tc::tmem_ld32(tmem + kColO + lane_base + 32 * c, r);
                 tc::tmem_ld_wait();
             }
-            if (!is_row) continue;
+            if (is_row) {
 #pragma unroll
-            for (int j = 0; j < 32; j += 4)
-                *reinterpret_cast<float4*>(orow + 32 * c + j) =
-                    seen ? make_float4(__uint_as_float(r[j]) * unit, __uint_as_float(r[j + 1]) * unit, __uint_as_float(r[j + 2]) * unit, __uint_as_float(r[j + 3]) * unit)
-                         : make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int j = 0; j < 32; j += 4)
+                    *reinterpret_cast<float4*>(orow + 32 * c + j) =
+                        seen ? make_float4(__uint_as_float(r[j]) * unit, __uint_as_float(r[j + 1]) * unit, __uint_as_float(r[j + 2]) * unit, __uint_as_float(r[j + 3]) * unit)
+                             : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
         }
     }
     if (failed && lane == 0) L.flag(KVB_ERR_WAIT_TIMEOUT);

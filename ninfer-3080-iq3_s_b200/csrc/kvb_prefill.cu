@@ -500,17 +500,19 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
 #pragma unroll 1
         for (int c = 0; c < kCols / 32; ++c) {
             if (!warp_has_rows) break;
+            __syncwarp();  // the load is the whole warp's: lanes without a row are back from the stores
             uint32_t r[32];
             if (have) {
                 tc::tmem_ld32(to + 32 * c, r);
                 tc::tmem_ld_wait();
             }
-            if (!is_row) continue;
+            if (is_row) {
 #pragma unroll
-            for (int e = 0; e < 32; e += 4)
-                *reinterpret_cast<float4*>(orow + 32 * c + e) =
-                    seen ? make_float4(__uint_as_float(r[e]), __uint_as_float(r[e + 1]), __uint_as_float(r[e + 2]), __uint_as_float(r[e + 3]))
-                         : make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int e = 0; e < 32; e += 4)
+                    *reinterpret_cast<float4*>(orow + 32 * c + e) =
+                        seen ? make_float4(__uint_as_float(r[e]), __uint_as_float(r[e + 1]), __uint_as_float(r[e + 2]), __uint_as_float(r[e + 3]))
+                             : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
         }
     }
     if (failed && lane == 0) L.flag(KVB_ERR_WAIT_TIMEOUT);
