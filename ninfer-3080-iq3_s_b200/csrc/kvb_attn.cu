@@ -1451,9 +1451,6 @@ int split_count(int kv_len_max, int kv_heads, int zblocks) {
 }  // namespace kvb
 
 namespace kvb {
-namespace {
-
-}  // namespace
 // kvb_chunk256.cu
 int launch_chunk_attention_256(const kvb_layer* layer, const void* q, const int32_t* positions_dev, int tokens, float scale,
                                int kv_len_max, void* workspace, void* out, cudaStream_t s, float* part_m, float* part_l, float* part_o);

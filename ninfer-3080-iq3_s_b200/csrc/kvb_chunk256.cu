@@ -42,7 +42,9 @@ constexpr int kSoftRegs = 144, kDqRegs = 72, kMmaRegs = 48;
 constexpr int kKvBlock = kN * 128;       // one 64-dim block of a K or V tile: 64 rows of 128 bytes
 constexpr int kKvTile = 4 * kKvBlock;
 constexpr int kQBlock = kM * 128;        // one 64-dim block of the Q tile
-constexpr int kSlotsMeta = 4;            // per-page words handed to the softmax warps: a writer is at most 2 pages ahead of a reader
+// Per-page words handed to the softmax warps.  A writer is at most 3 pages ahead of a reader: the K role writes those of page i once
+// S(i-2) is complete, which was issued after P V(i-4) but not after the softmax of page i-3.  No slot to spare.
+constexpr int kSlotsMeta = 4;
 constexpr uint32_t kTmemCols = 512, kColQ = 128, kColO = 256;  // S buffers at columns 0 and 64
 constexpr int kTop = 14;                 // scaled operands reach 2^14 .. 2^15
 constexpr float kPBoost = 4.0f;          // P is taken 2^4 above the row's reference point (and stays below 2^12): more bits of small weights survive
@@ -75,17 +77,6 @@ struct __align__(1024) Chunk256Smem {
     uint32_t tmem_base;
     int abort_flag;
 };
-
-__device__ __forceinline__ bool chunk_wait(uint64_t* bar, uint32_t parity, int* abort_flag) {
-    bool ok = false;
-    for (uint32_t i = 0; i < kSpinLimit && !ok; ++i) {
-        ok = mbar_try_wait(bar, parity);
-        if (!ok && *reinterpret_cast<volatile int*>(abort_flag) != 0) break;
-    }
-    ok = __all_sync(0xffffffffu, ok);
-    if (!ok) *reinterpret_cast<volatile int*>(abort_flag) = 1;
-    return ok;
-}
 
 // Largest power of two that keeps values of magnitude `bits` (a non-negative float) below 2^(kTop + 1): exponent of the
 // scale that was taken out.  Zero and non-finite magnitudes: 0.

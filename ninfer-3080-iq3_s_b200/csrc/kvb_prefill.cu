@@ -72,17 +72,6 @@ struct __align__(1024) PrefillSmem {
     int abort_flag;
 };
 
-__device__ __forceinline__ bool chunk_wait(uint64_t* bar, uint32_t parity, int* abort_flag) {
-    bool ok = false;
-    for (uint32_t i = 0; i < kSpinLimit && !ok; ++i) {
-        ok = mbar_try_wait(bar, parity);
-        if (!ok && *reinterpret_cast<volatile int*>(abort_flag) != 0) break;
-    }
-    ok = __all_sync(0xffffffffu, ok);
-    if (!ok) *reinterpret_cast<volatile int*>(abort_flag) = 1;
-    return ok;
-}
-
 // Byte offset of element (row, col) in a [128 rows][128 cols] fp16 tile stored as two 64-column blocks of
 // 128-byte rows, 8-row groups 1024 bytes apart, 16-byte chunks XOR-swizzled with the row (128-byte swizzle).
 __device__ __forceinline__ uint32_t tile_off(int row, int col) {

@@ -56,6 +56,18 @@ __device__ __forceinline__ bool mbar_wait_lane_bounded(uint64_t* bar, uint32_t p
     return false;
 }
 
+// The same wait of a whole warp of a CTA whose warps give up together: it also watches the CTA's abort flag, and raises it.
+__device__ __forceinline__ bool chunk_wait(uint64_t* bar, uint32_t parity, int* abort_flag) {
+    bool ok = false;
+    for (uint32_t i = 0; i < kSpinLimit && !ok; ++i) {
+        ok = mbar_try_wait(bar, parity);
+        if (!ok && *reinterpret_cast<volatile int*>(abort_flag) != 0) break;
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) *reinterpret_cast<volatile int*>(abort_flag) = 1;
+    return ok;
+}
+
 // Generic-proxy accesses to shared memory made before this fence are ordered before later async-proxy
 // (bulk copy) accesses: needed before a buffer that was read with ld.shared is refilled by a bulk copy.
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
