@@ -210,3 +210,111 @@ def test_non_finite_factors_of_a_page(what):
             assert torch.equal(g[2], w[2])
         else:
             assert torch.allclose(g[2], w[2], rtol=0, atol=float(w[2].abs().max()) * 2.0 ** -21)  # another largest scale of the page
+
+
+def _chunk_reference(tw, q_bits, at, T, dtype=0, without=None):
+    """The oracle's attention over the bytes of the GPU's cache, the keys [a, b) of `without` left out."""
+    cpu, scale = cpu_twin_of(tw.gpu), 1.0 / np.sqrt(tw.D)
+    if without is None:
+        return cpu.attention(q_bits, at, scale, tw.QH, dtype=dtype, threads=8, kv_total=T)
+    parts = [cpu.attention(q_bits, at, scale, tw.QH, dtype=dtype, threads=8, kv_total=T, key_begin=a, key_end=b, want_partials=True)[1:]
+             for a, b in ((0, without[0]), (without[1], T))]
+    return np.stack([orc.merge_partials(*(np.stack([p[i][t] for p in parts]) for i in range(3))) for t in range(len(at))])
+
+
+@pytest.mark.parametrize("entry,T,tokens", [("attn_decode", 700, 1), ("attn_verify", 300, 5), ("attn_verify", 125, 8), ("attn_prefill", 0, 64), ("attn_prefill", 700, 40)])
+@pytest.mark.parametrize("iters", [0, 16])
+def test_bf16_rows_of_256_dims(entry, T, tokens, iters):
+    """The engine's own type and geometry.  What is left is the rounding of the output: 2^-9 of a value at most, 10 % on top."""
+    import torch
+
+    from helpers import from_bits, to_bits
+
+    H, QH, D, end = 4, 24, 256, T + tokens
+    tw = Twin(D=D, H=H, QH=QH, capacity_tokens=end, seed=T, dtype=1, iters=iters)
+    kb, vb = (to_bits(orc.synth_kv(13, end, H, D, i), 1) for i in (1, 2))
+    qb = to_bits(orc.synth_q(13, tokens, QH, D), 1)
+    k, v, q = (from_bits(x, 1).to(tw.dev) for x in (kb, vb, qb))
+    pos = torch.arange(end, dtype=torch.int32, device=tw.dev)
+    if T:
+        tw.gpu.append(k[:T], v[:T], pos[:T])
+    if entry == "attn_decode":
+        tw.gpu.append(k[T:], v[T:], pos[T:])
+        out = tw.gpu.attn_decode(q[0], pos[T:], 1.0 / 16.0, end).unsqueeze(0)
+    else:
+        out = getattr(tw.gpu, entry)(q, k[T:], v[T:], pos[T:], 1.0 / 16.0, end)
+    assert out.dtype == torch.bfloat16 and tw.gpu.errors() == 0
+    want = _chunk_reference(tw, qb, np.arange(T, end, dtype=np.int32), end, dtype=1)
+    ok, msg = attn_close(out.float().cpu().numpy(), want, 1.1 * 2.0 ** -8, 1.1 * 2.0 ** -8 / 3 ** 0.5)
+    assert ok, msg
+
+
+# key ranges per row 17 .. 32, 33 .. 64, 65 .. 128: a CTA per row merges them
+@pytest.mark.parametrize("H,QH,ctx,tokens", [(8, 8, 12000, 9), (4, 4, 16300, 9), (2, 4, 33000, 9), (4, 24, 16384, 32)])
+@pytest.mark.parametrize("D", [128, 256])
+def test_chunks_over_many_key_ranges(D, H, QH, ctx, tokens):
+    """... as output and as the merged partial of a chunk."""
+    import torch
+
+    T, scale = ctx + tokens, 1.0 / np.sqrt(D)
+    tw = _filled(D, H, QH, T, room=0, seed=14)
+    qn = orc.synth_q(15, tokens, QH, D)
+    q, at = torch.from_numpy(qn).to(tw.dev), np.arange(ctx, T, dtype=np.int32)
+    pos = torch.from_numpy(at).to(tw.dev)
+    m, l, o = _partial(tw, q, pos, T, torch.empty(tokens * QH * (D + 2), device=tw.dev))
+    merged = pkg().merge_partials(m[None], l[None], o[None]).view(tokens, QH, D)
+    k, v = (torch.from_numpy(orc.synth_kv(14, T, H, D, i)[ctx:]).to(tw.dev) for i in (1, 2))
+    out = tw.gpu.attn_prefill(q, k, v, pos, scale, T)
+    assert tw.gpu.errors() == 0
+    want = _chunk_reference(tw, qn, at, T)
+    tol = (PREFILL_MAX_ABS, PREFILL_REL_L2) if D == 128 else (ATTN_MAX_ABS, ATTN_REL_L2)
+    for what, x in (("output", out), ("partial", merged)):
+        ok, msg = attn_close(x.float().cpu().numpy(), want, *tol)
+        assert ok, what + ": " + msg
+
+
+@pytest.mark.parametrize("D,H,QH,ctx,tokens,cuts", [(256, 4, 24, 900, 3, (128, 512)), (256, 4, 24, 900, 8, (200, 450)), (256, 4, 24, 900, 50, (128, 512)), (256, 2, 16, 500, 200, (100, 300)),
+                                                    (128, 4, 24, 900, 50, (128, 512))])
+def test_chunk_partials_of_tile_ranges(D, H, QH, ctx, tokens, cuts):
+    """The rows of a chunk over three caches that hold consecutive tile ranges (the last one also the rows themselves): the merged
+    partials are the attention over the whole sequence."""
+    import torch
+
+    T = ctx + tokens
+    k, v, qn = orc.synth_kv(16, T, H, D, 1), orc.synth_kv(16, T, H, D, 2), orc.synth_q(16, tokens, QH, D)
+    cuts = [0] + [c // 128 * 128 for c in cuts] + [T]
+    whole = _filled(D, H, QH, 0, room=T)
+    whole.gpu.append(*(torch.from_numpy(x).to(whole.dev) for x in (k, v)), torch.arange(T, dtype=torch.int32, device=whole.dev))
+    parts = []
+    for i, (a, b) in enumerate(zip(cuts, cuts[1:])):
+        tw = _filled(D, H, QH, 0, room=b - a + 128, seed=i)
+        if b > a:
+            tw.gpu.append(*(torch.from_numpy(x[a:b].copy()).to(tw.dev) for x in (k, v)), torch.arange(b - a, dtype=torch.int32, device=tw.dev))
+        last = i == len(cuts) - 2
+        at = torch.arange(ctx - a, T - a, dtype=torch.int32, device=tw.dev) if last else torch.full((tokens,), b - a - 1, dtype=torch.int32, device=tw.dev)
+        parts.append([x.clone() for x in _partial(tw, torch.from_numpy(qn).to(tw.dev), at, max(b - a, 1), torch.empty(tokens * QH * (D + 2), device=tw.dev))])
+    out = pkg().merge_partials(*(torch.stack(x) for x in zip(*parts))).view(tokens, QH, D)
+    want = _chunk_reference(whole, qn, np.arange(ctx, T, dtype=np.int32), T)
+    ok, msg = attn_close(out.float().cpu().numpy(), want, *((PREFILL_MAX_ABS, PREFILL_REL_L2) if D == 128 else (ATTN_MAX_ABS, ATTN_REL_L2)))
+    assert ok, msg
+
+
+@pytest.mark.parametrize("D,H,QH,ctx,tokens", [(128, 4, 24, 900, 8), (128, 4, 24, 900, 40), (128, 8, 64, 600, 300), (256, 4, 24, 900, 5), (256, 4, 24, 900, 40), (256, 2, 16, 500, 90)])
+@pytest.mark.parametrize("bad", [-7, 1 << 20])
+def test_bad_page_in_the_prefix_of_a_chunk(D, H, QH, ctx, tokens, bad):
+    """A table entry outside the pool: reported in the error word, and the keys of its page (at 128 dims from 32 rows on: of its
+    tile) are left out."""
+    import torch
+
+    T, page = ctx + tokens, 5
+    tw = _filled(D, H, QH, T, room=0, seed=17)
+    tw.gpu.table[page] = bad
+    qn, at = orc.synth_q(18, tokens, QH, D), np.arange(ctx, T, dtype=np.int32)
+    m, l, o = _partial(tw, torch.from_numpy(qn).to(tw.dev), torch.from_numpy(at).to(tw.dev), T, torch.empty(tokens * QH * (D + 2), device=tw.dev))
+    out = pkg().merge_partials(m[None], l[None], o[None]).view(tokens, QH, D)
+    assert tw.gpu.errors() == pkg().capi.ERR_PAGE_RANGE
+    tw.gpu.table[page] = 0  # for the oracle: a page it may read (its keys are left out)
+    tile = D == 128 and tokens * QH // H >= 32
+    want = _chunk_reference(tw, qn, at, T, without=(page // 2 * 128, (page // 2 + 1) * 128) if tile else (64 * page, 64 * (page + 1)))
+    ok, msg = attn_close(out.float().cpu().numpy(), want, *((PREFILL_MAX_ABS, PREFILL_REL_L2) if tile else (ATTN_MAX_ABS, ATTN_REL_L2)))
+    assert ok, msg
