@@ -26,10 +26,11 @@
 //     enter the running fp32 accumulators with the weight exp2(page max - running max).
 // The page-local reference keeps 16 significant bits below each page's own maximum, whatever the global one is.
 // At head_dim 256 each slice has its own query integers (one scale_K, zp_K table per slice) and weights (scale_V per slice),
-// with a third byte each; the slices meet in the fp32 logits.  Bound by instruction issue like the 128-dim form (a 16 KB
-// page costs about as much as two 8 KB ones).  Measured on B200, 24 / 4 heads, balanced bf16 cache: decode at 30,011
-// tokens 21.4 us against 148.6 us for one warp per key on fp32 FMAs, a 5-row verify step at 20,000 tokens 35.7 against
-// 454 us (the whole difference: no per-element de-quantisation, rows of a KV head share every code read).
+// with a third byte each; the slices meet in the fp32 logits.  Bound by latency, most of it of instructions: eight warps, two a
+// scheduler, run thousands of instructions a page once or twice (a 16 KB page costs about as much as two 8 KB ones).  Measured on
+// B200 in graph replay, 24 / 4 heads, balanced bf16 cache: decode at 30,011 tokens 23.2 us a layer against 178 for one warp per key
+// on fp32 FMAs, a 5-row verify step at 20,000 tokens 41.5 against 486 (no per-element de-quantisation, rows of a KV head share
+// every code read); the look for factors that are not finite is 0.4 and 1.0 us of it.
 #include <algorithm>
 #include <climits>
 #include <cstddef>
@@ -1585,8 +1586,10 @@ int launch_attention(const kvb_layer* layer, const void* q, const int32_t* pos_d
 }  // namespace
 }  // namespace kvb
 
-// From this many GQA-merged query rows per KV head on, the tcgen05 kernel wins (measured at 131,072 tokens: widths 4-5 of a
-// 24/4-head model are faster on the warp-level kernel, widths 6-8 on this one).
+// From this many GQA-merged query rows per KV head on, steps run on the tcgen05 kernel.  Measured on B200 in graph replay, 24 / 4
+// heads, 131,072 tokens, us a layer for widths 3 .. 8 (18 .. 48 rows) on the warp-level kernel and on this one: unbalanced
+// 55.4 54.7 69.7 86.9 101.5 99.0 against 65.3 66.7 67.2 67.8 69.7 70.0, balanced 76.7 76.6 77.2 104.8 105.3 103.7 against 71.3 72.6
+// 73.1 73.7 75.6 75.8.
 static constexpr int kDenseRows = 32;
 extern "C" int kvb_split_capacity(int kv_len_max, int kv_heads, int q_heads, int rows, int batch) {
     (void)batch;

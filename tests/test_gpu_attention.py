@@ -318,10 +318,10 @@ def _sync_cpu_from_gpu(tw):
 
 
 @pytest.mark.parametrize("D,H,QH,iters,T", [(256, 4, 24, 0, 700), (256, 2, 4, 0, 333), (128, 4, 24, 16, 600), (256, 2, 8, 16, 300)])
-def test_general_kernel_head_dim_256_and_sinkhorn(D, H, QH, iters, T):
-    """The reference engine's own geometry (head_dim 256, with and without Sinkhorn iterations) runs on the general
-    kernel, a balanced head_dim-128 cache on the tuned kernels: decode, a 4-row verify step and a small prefill chunk,
-    against the oracle on the same cache bytes."""
+def test_head_dim_256_and_balanced_caches(D, H, QH, iters, T):
+    """The reference engine's own geometry (head_dim 256, with and without Sinkhorn iterations: the int8 kernel with two slices,
+    chunks on its tcgen05 kernel) and a balanced head_dim-128 cache: decode, a 4-row verify step and a small prefill chunk, against
+    the oracle on the same cache bytes."""
     import torch
 
     tw = Twin(D=D, H=H, QH=QH, capacity_tokens=T + 40, seed=101, iters=iters)
