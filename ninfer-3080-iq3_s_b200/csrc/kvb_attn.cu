@@ -991,11 +991,14 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
 #pragma unroll
                     for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
-                        for (int n = 0; n < 2 * kDigits; ++n) {  // all digits of x, then of y (in turn: 4-row verify steps 0.4 % longer)
-                            const int xy = n / kDigits, d = n % kDigits;
-                            const uint32_t a0 = xy ? ay0 : ax0, a1 = xy ? ay1 : ax1, a2 = xy ? ay2 : ax2, a3 = xy ? ay3 : ax3;
-                            if (c == 0) imma_uu0(ix[nb][xy][d], a0, a1, a2, a3, bw[s][nb][d][0], bw[s][nb][d][1]);
-                            else imma_uu(ix[nb][xy][d], a0, a1, a2, a3, bw[s][nb][d][2], bw[s][nb][d][3]);
+                        for (int d = 0; d < kDigits; ++d) {
+                            if (c == 0) {
+                                imma_uu0(ix[nb][0][d], ax0, ax1, ax2, ax3, bw[s][nb][d][0], bw[s][nb][d][1]);
+                                imma_uu0(ix[nb][1][d], ay0, ay1, ay2, ay3, bw[s][nb][d][0], bw[s][nb][d][1]);
+                            } else {
+                                imma_uu(ix[nb][0][d], ax0, ax1, ax2, ax3, bw[s][nb][d][2], bw[s][nb][d][3]);
+                                imma_uu(ix[nb][1][d], ay0, ay1, ay2, ay3, bw[s][nb][d][2], bw[s][nb][d][3]);
+                            }
                         }
                 }
                 // ---- integer sums of the page -> running fp32 accumulators
