@@ -1193,7 +1193,8 @@ __device__ __forceinline__ bool ring_arrived(const uint4& w, uint32_t call) { re
 
 // kPush: the ring exchange of a sharded decode (head_dim 128), compiled out of the other calls' kernel (it needs 242
 // registers per thread, the plain merge 72).
-template <int S, bool kPush>
+// kMany: a name of its own for calls with many rows, see launch_reduce.
+template <int S, bool kPush, bool kMany>
 __global__ void __launch_bounds__(kReduceWarps * 32) reduce_kernel(const float* __restrict__ ws_m, const float* __restrict__ ws_l,
                                                                   const float* __restrict__ ws_o, int parts, int T, int q_heads,
                                                                   int kv_heads, int zblocks, int block_rows, int dtype, uint16_t* __restrict__ out,
@@ -1473,16 +1474,21 @@ cudaError_t launch_attn(dim3 grid, cudaStream_t stream, const AttnParams& P) {
 // CTAs as the registers allow (four: 64 KB), and the SM's change between that and the attention kernel's 132 KB or more lies
 // between the two in a chain of layers.  Measured on B200 in graph replay, a decode call at 16,384 / 32,768 / 131,072 tokens:
 // 9.4 / 12.0 / 23.1 us left to the driver, 8.6 / 11.2 / 22.2 with 0, 9.7 / 12.3 / 23.3 with both kernels asking for all of it.
+// The least there is holds one CTA an SM: with more rows than SMs (a batch: 768) the driver's choice is the better one
+// (32 sequences, 315 us against 320).
 template <int S, bool kPush>
 cudaError_t launch_reduce(int rows, cudaStream_t stream, const float* ws_m, const float* ws_l, const float* ws_o, int parts, int T, int q_heads, int kv_heads,
                           int zblocks, int block_rows, int dtype, uint16_t* out, float* part_m, float* part_l, float* part_o, const PushTarget& push,
                           const BatchPlan& plan) {
     static OncePerDevice set;
-    const cudaError_t e = set.run(current_device(), [] {
-        return cudaFuncSetAttribute(reduce_kernel<S, kPush>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1);
-    });
-    if (e != cudaSuccess) return e;
-    return launch_early(reduce_kernel<S, kPush>, dim3(rows), dim3(kReduceWarps * 32), 0, stream, ws_m, ws_l, ws_o, parts, T, q_heads, kv_heads, zblocks,
+    const bool many = rows > device_sm_count();
+    if (!many) {
+        const cudaError_t e = set.run(current_device(), [] {
+            return cudaFuncSetAttribute(reduce_kernel<S, kPush, false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1);
+        });
+        if (e != cudaSuccess) return e;
+    }
+    return launch_early(many ? reduce_kernel<S, kPush, true> : reduce_kernel<S, kPush, false>, dim3(rows), dim3(kReduceWarps * 32), 0, stream, ws_m, ws_l, ws_o, parts, T, q_heads, kv_heads, zblocks,
                         block_rows, dtype, out, part_m, part_l, part_o, push, plan);
 }
 
