@@ -1,0 +1,46 @@
+"""Chunks whose rows see one key range are finished in chunk_kernel itself (head_dim 128): no partials, no merge kernel.  Compared
+with the merge kernel's route -- taken by an output that starts at no 16-byte boundary -- and with the oracle."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from helpers import PREFILL_MAX_ABS, PREFILL_REL_L2, Twin, attn_close, cpu_twin_of, orc, pkg
+
+pytestmark = pytest.mark.gpu
+
+
+# split walks of one and several key tiles, the second stream without a tile, ragged row tiles; two row tiles a CTA, the last one
+# alone or with few rows; rows of a group that end inside a row tile (7 and 3 query heads a KV head)
+@pytest.mark.parametrize("H,QH,ctx,tokens,dtype,iters", [(4, 24, 0, 780, 0, 0), (8, 64, 0, 128, 0, 16), (8, 64, 0, 290, 1, 0), (4, 28, 5, 680, 0, 16), (4, 24, 0, 1024, 0, 0),
+                                                         (8, 24, 130, 1000, 1, 16), (8, 64, 0, 1023, 0, 0), (1, 3, 0, 20, 0, 0), (2, 16, 0, 8, 1, 0)])
+def test_finished_rows(H, QH, ctx, tokens, dtype, iters):
+    import torch
+
+    D, T = 128, ctx + tokens
+    scale = 1.0 / np.sqrt(D)
+    k, v, qn = orc.synth_kv(T, T, H, D, 1), orc.synth_kv(T, T, H, D, 2), orc.synth_q(T, tokens, QH, D)
+    got = []
+    for shift in (0, 1):  # elements
+        tw = Twin(D=D, H=H, QH=QH, capacity_tokens=T, seed=T, dtype=dtype, iters=iters)
+        kd, vd, q = (torch.from_numpy(x).to(tw.dev).to(tw.gpu.dtype) for x in (k, v, qn))
+        at = torch.arange(T, dtype=torch.int32, device=tw.dev)
+        if ctx:
+            tw.gpu.append(kd[:ctx], vd[:ctx], at[:ctx])
+        ws = tw.gpu.prefill_workspace(T, tokens).fill_(float("nan"))
+        buf = torch.full((q.numel() + 16,), 7.0, dtype=q.dtype, device=tw.dev)
+        out = buf[8 + shift:8 + shift + q.numel()]
+        args = [C.c_void_p(x.data_ptr()) for x in (q, kd[ctx:], vd[ctx:], at[ctx:])]
+        pkg().capi.check(pkg().capi.load().kvb_attn_prefill(C.byref(tw.gpu.c), *args, tokens, scale, T, C.c_void_p(ws.data_ptr()), C.c_void_p(out.data_ptr()), None))
+        torch.cuda.synchronize()
+        assert torch.all(buf[:8 + shift] == 7.0) and torch.all(buf[8 + shift + q.numel():] == 7.0)
+        assert tw.gpu.errors() == 0
+        got.append(out.view(tokens, QH, D).float().cpu().numpy())
+    # both routes round the same sums (fp32 sums in another order) to the output type
+    assert np.abs(got[0] - got[1]).max() <= np.abs(got[1]).max() * (2.0 ** -8 if dtype else 2.0 ** -11)
+    rows = np.unique(np.concatenate([np.arange(0, tokens, max(1, tokens // 6)), [tokens - 1]]))
+    bits = q.view(torch.int16).cpu().numpy().view(np.uint16)[rows] if dtype else qn[rows]
+    want = cpu_twin_of(tw.gpu).attention(bits, np.arange(ctx, T, dtype=np.int32)[rows], scale, QH, dtype=dtype, threads=8, kv_total=T)
+    tol = (PREFILL_MAX_ABS, PREFILL_REL_L2) if dtype == 0 else (2.0 ** -7, 2.0 ** -7)  # bf16: half a unit of the output, 2^-9 of a value, and of P's, K's and V's rounding
+    ok, msg = attn_close(got[0][rows], want, *tol)
+    assert ok, msg
