@@ -322,6 +322,10 @@ __global__ void __launch_bounds__(kThreads, 1) append_kernel(LayerView L, const 
     using G = Geo<D>;
     constexpr int S = G::S;
     grid_dependency_wait();  // launched while its predecessor still runs: nothing is read or written before it is over
+    // The attention of a step starts beside the append, and what of it reads the rows written here waits for the append's end.
+    // Measured on B200, a step of one layer: 32,768 tokens 13.8 -> 13.4 us, 8-row verify of 100,003 67.6 -> 63.6 us, a prompt of 777
+    // 35.9 -> 33.0 us.  Not for several rows of a verify step at 256 dims, whose four row blocks share their pages through L2: 41.2 -> 42.5.
+    if (D == 128 || tokens == 1 || tokens > 8) launch_dependents();
     const int pos0 = positions[0], last = positions[tokens - 1];
     if (pos0 < 0 || last - pos0 != tokens - 1) {  // positions must be contiguous and non-negative
         if (threadIdx.x == 0) L.flag(KVB_ERR_POSITIONS);

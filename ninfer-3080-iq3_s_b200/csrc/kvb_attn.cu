@@ -85,6 +85,7 @@ struct AttnParams {
     int nsplit;          // CTAs over the sealed tiles of a head; the last one also reads the open tile
     int block_rows;      // GQA-merged query rows per row block (grid z): 8 (one 8-row block per warp) or 16 (two)
     int key_begin, key_end;
+    bool after_append;   // launched behind the append of the rows at pos[0] ..: only the CTAs that read what it writes wait for it
     float* ws_m;         // [H][Z][nsplit][16]
     float* ws_l;
     float* ws_o;         // [H][Z][nsplit][16][D]
@@ -509,6 +510,8 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
         const int c1 = pb + static_cast<int>(static_cast<int64_t>(n) * (split + 1) / P.nsplit);
         w0 = c0 + (c1 - c0) * warp / kWarps;
         w1 = c0 + (c1 - c0) * (warp + 1) / kWarps;
+        // the stage, and tiles from that of the first appended row on
+        if (P.after_append && (split == P.nsplit - 1 || c1 * kPage > P.pos[0] / kTile * kTile)) grid_dependency_wait();
     }
     const int npages = w1 - w0, nchunks = 2 * npages;
     // ---- the refill side of the ring.  Chunk n of this warp is page w0 + n / 2: even n = K codes + header, odd n = V
@@ -1087,7 +1090,8 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
 
 template <int S, int NB, int W, bool kOther = false>
 __global__ void __launch_bounds__(W * 32, 1) attn_kernel(const AttnParams P) {
-    grid_dependency_wait();  // q, the positions and the cache come from the kernels before this one
+    // q, the positions and the cache come from the kernels before this one; an append has waited for those before it
+    if (!P.after_append) grid_dependency_wait();
     const int head = blockIdx.y, zb = blockIdx.z, split = blockIdx.x;
     attn_cta<S, NB, W, kOther>(P, split, head, zb, ((static_cast<int64_t>(head) * gridDim.z + zb) * P.nsplit + split) * kRows);
 }
@@ -1149,6 +1153,7 @@ __global__ void __launch_bounds__(W * 32, 1) attn_batch_kernel(const BatchParams
     P.block_rows = kRows;
     P.key_begin = 0;
     P.key_end = INT_MAX;
+    P.after_append = false;
     P.ws_m = B.ws_m;
     P.ws_l = B.ws_l;
     P.ws_o = B.ws_o;
@@ -1458,7 +1463,7 @@ int split_count(int kv_len_max, int kv_heads, int zblocks) {
 namespace kvb {
 // kvb_chunk256.cu
 int launch_chunk_attention_256(const kvb_layer* layer, const void* q, const int32_t* positions_dev, int tokens, float scale,
-                               int kv_len_max, void* workspace, void* out, cudaStream_t s, float* part_m, float* part_l, float* part_o);
+                               int kv_len_max, void* workspace, void* out, cudaStream_t s, float* part_m, float* part_l, float* part_o, bool after_append);
 namespace {
 
 // One attention launch with W warps per CTA (the opt-in to large dynamic shared memory is made once per device and W).
@@ -1538,7 +1543,7 @@ RowPlan plan_rows(int kv_len_max, int kv_heads, int q_heads, int head_dim, int T
 int launch_attention(const kvb_layer* layer, const void* q, const int32_t* pos_dev, const int32_t* total_pos_dev, int T,
                      float scale, int kv_len_max,
                      int key_begin, int key_end, void* workspace, void* out, float* part_m, float* part_l,
-                     float* part_o, cudaStream_t stream, const char* who, const PushTarget* push = nullptr) {
+                     float* part_o, cudaStream_t stream, const char* who, const PushTarget* push = nullptr, bool after_append = false) {
     if (int st = check_layer(layer, who)) return st;
     if (q == nullptr || pos_dev == nullptr || workspace == nullptr) return fail(KVB_EINVAL, "%s: null q / positions / workspace", who);
     if (out == nullptr && part_m == nullptr && push == nullptr) return fail(KVB_EINVAL, "%s: null output", who);
@@ -1560,6 +1565,7 @@ int launch_attention(const kvb_layer* layer, const void* q, const int32_t* pos_d
     P.block_rows = plan.block_rows;
     P.key_begin = key_begin;
     P.key_end = key_end;
+    P.after_append = after_append;
     const size_t rows = static_cast<size_t>(layer->kv_heads) * Z * parts * kRows;
     P.ws_m = workspace_base(workspace);
     P.ws_l = P.ws_m + rows;
@@ -1745,11 +1751,11 @@ extern "C" int kvb_append_decode(const kvb_layer* layer, const void* q, const vo
     if (int st = kvb_append(layer, k, v, pos_dev, 1, stream)) return st;
     if (ring == nullptr)
         return launch_attention(layer, q, pos_dev, pos_dev, 1, scale, kv_len_max, 0, INT_MAX, workspace, out, nullptr, nullptr, nullptr,
-                                static_cast<cudaStream_t>(stream), "kvb_append_decode");
+                                static_cast<cudaStream_t>(stream), "kvb_append_decode", nullptr, true);
     PushTarget push{};
     if (int st = make_push_target(layer, ring, out, "kvb_append_decode", push)) return st;
     return launch_attention(layer, q, pos_dev, pos_dev, 1, scale, kv_len_max, 0, INT_MAX, workspace, out, nullptr, nullptr, nullptr,
-                            static_cast<cudaStream_t>(stream), "kvb_append_decode", &push);
+                            static_cast<cudaStream_t>(stream), "kvb_append_decode", &push, true);
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -1850,7 +1856,7 @@ extern "C" int kvb_attn_decode_batch(const kvb_layer* layers_dev, int batch, int
 namespace kvb {
 int launch_chunk_attention(const kvb_layer* layer, const void* q, const int32_t* positions_dev, int tokens, float scale,
                            int kv_len_max, void* workspace, void* out, cudaStream_t s, float* part_m, float* part_l,
-                           float* part_o, const int32_t* total_pos_dev);  // kvb_prefill.cu
+                           float* part_o, const int32_t* total_pos_dev, bool after_append);  // kvb_prefill.cu
 }
 
 extern "C" int kvb_attn_verify(const kvb_layer* layer, const void* q, const void* k, const void* v,
@@ -1862,10 +1868,10 @@ extern "C" int kvb_attn_verify(const kvb_layer* layer, const void* q, const void
     if (width * (layer->q_heads / layer->kv_heads) >= kDenseRows && layer->head_dim == 128) {
         if (q == nullptr || workspace == nullptr || out == nullptr) return kvb::fail(KVB_EINVAL, "kvb_attn_verify: null q / workspace / out");
         return kvb::launch_chunk_attention(layer, q, positions_dev, width, scale, kv_len_max, workspace, out, static_cast<cudaStream_t>(stream),
-                                           nullptr, nullptr, nullptr, nullptr);
+                                           nullptr, nullptr, nullptr, nullptr, true);
     }
     return kvb::launch_attention(layer, q, positions_dev, positions_dev + (width - 1), width, scale, kv_len_max, 0, INT_MAX, workspace, out, nullptr, nullptr,
-                                 nullptr, static_cast<cudaStream_t>(stream), "kvb_attn_verify");
+                                 nullptr, static_cast<cudaStream_t>(stream), "kvb_attn_verify", nullptr, layer->head_dim == 128);
 }
 
 // Causal attention of `tokens` already-appended (or foreign) query rows over THIS cache alone, exported as log-sum-exp
@@ -1885,8 +1891,8 @@ extern "C" int kvb_attn_chunk_partial(const kvb_layer* layer, const void* q, con
         return launch_attention(layer, q, positions_dev, positions_dev + (tokens - 1), tokens, scale, kv_len_max, 0, INT_MAX, workspace, nullptr,
                                 part_m, part_l, part_o, st, "kvb_attn_chunk_partial");
     if (layer->head_dim != 128)
-        return launch_chunk_attention_256(layer, q, positions_dev, tokens, scale, kv_len_max, workspace, nullptr, st, part_m, part_l, part_o);
-    return launch_chunk_attention(layer, q, positions_dev, tokens, scale, kv_len_max, workspace, nullptr, st, part_m, part_l, part_o, nullptr);
+        return launch_chunk_attention_256(layer, q, positions_dev, tokens, scale, kv_len_max, workspace, nullptr, st, part_m, part_l, part_o, false);
+    return launch_chunk_attention(layer, q, positions_dev, tokens, scale, kv_len_max, workspace, nullptr, st, part_m, part_l, part_o, nullptr, false);
 }
 
 // Causal attention of 1..8 query rows whose K/V rows are already in the cache -- a verify step without its append, for
@@ -1901,7 +1907,7 @@ extern "C" int kvb_attn_rows(const kvb_layer* layer, const void* q, const int32_
     if (rows * (layer->q_heads / layer->kv_heads) >= kDenseRows && layer->head_dim == 128) {
         if (q == nullptr || positions_dev == nullptr || workspace == nullptr || out == nullptr)
             return fail(KVB_EINVAL, "kvb_attn_rows: null q / positions / workspace / out");
-        return launch_chunk_attention(layer, q, positions_dev, rows, scale, kv_len_max, workspace, out, st, nullptr, nullptr, nullptr, total_pos_dev);
+        return launch_chunk_attention(layer, q, positions_dev, rows, scale, kv_len_max, workspace, out, st, nullptr, nullptr, nullptr, total_pos_dev, false);
     }
     return launch_attention(layer, q, positions_dev, total_pos_dev, rows, scale, kv_len_max, 0, INT_MAX, workspace, out, nullptr, nullptr, nullptr,
                             st, "kvb_attn_rows");

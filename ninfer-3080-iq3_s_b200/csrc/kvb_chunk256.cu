@@ -55,6 +55,7 @@ struct Chunk256Params {
     const int32_t* pos;        // [T]
     const int32_t* total_pos;  // newest position in the cache
     int T, mtiles, ksplit;
+    bool after_append;         // launched behind the append of the rows: only the readers of the planes and the stage wait for it
     float scale_log2;
     float* ws_m;               // [H][mtiles][ksplit][128]
     float* ws_l;
@@ -307,6 +308,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Par
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int mt = blockIdx.x, head = blockIdx.y, zs = blockIdx.z;
     const int G = L.q_heads / L.kv_heads;
+    if (!P.after_append) grid_dependency_wait();
     const int kv_total = *P.total_pos + 1;
 
     if (warp == kMmaWarp) tc::tmem_alloc(&sm.tmem_base, kTmemCols);
@@ -412,6 +414,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Par
 
     if (warp >= kSoftWarps && warp < kMmaWarp) {
         tc::regs_dec<kDqRegs>();
+        if (P.after_append) grid_dependency_wait();
         const int dt = tid - 32 * kSoftWarps;
         if (dt < 32 * kDqWarps) failed = dequant_role<false>(sm, L, head, dt, p0, p1, kv_total);
         else failed = dequant_role<true>(sm, L, head, dt - 32 * kDqWarps, p0, p1, kv_total);
@@ -604,8 +607,9 @@ __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Par
 
 // Chunk attention of `tokens` rows that are already appended, over a head_dim-256 cache.
 int launch_chunk_attention_256(const kvb_layer* layer, const void* q, const int32_t* positions_dev, int tokens, float scale,
-                               int kv_len_max, void* workspace, void* out, cudaStream_t s, float* part_m, float* part_l, float* part_o) {
+                               int kv_len_max, void* workspace, void* out, cudaStream_t s, float* part_m, float* part_l, float* part_o, bool after_append) {
     Chunk256Params P;
+    P.after_append = after_append;
     P.L = make_view(*layer);
     P.q = static_cast<const uint16_t*>(q);
     P.pos = positions_dev;
@@ -623,8 +627,7 @@ int launch_chunk_attention_256(const kvb_layer* layer, const void* q, const int3
     static OncePerDevice opted;
     KVB_CUDA_OK(allow_smem(opted, chunk256_kernel, smem));
     const dim3 grid(P.mtiles, layer->kv_heads, P.ksplit);
-    chunk256_kernel<<<grid, kThreads, smem, s>>>(P);
-    KVB_CUDA_OK(cudaGetLastError());
+    KVB_CUDA_OK(launch_early(chunk256_kernel, grid, dim3(kThreads), smem, s, P));
     return launch_chunk_merge<D>(P.ws_m, P.ws_l, P.ws_o, tokens, layer->q_heads, layer->kv_heads, P.mtiles, P.ksplit, layer->dtype, out,
                                  part_m, part_l, part_o, s);
 }

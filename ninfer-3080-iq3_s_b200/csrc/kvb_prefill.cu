@@ -55,6 +55,7 @@ struct PrefillParams {
     const int32_t* pos;        // [T]
     const int32_t* total_pos;  // newest position in the cache
     int T, mtiles, ksplit;     // ksplit: partials per row
+    bool after_append;         // launched behind the append of the rows: only the readers of the planes and the stage wait for it
     float scale_log2;
     uint16_t* out;             // one key range: the finished rows [T][q_heads][D]; else null, and
     float* ws_m;               // [H][mtiles][ksplit][128]
@@ -332,6 +333,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
     constexpr int kRowTiles = kSplit ? 1 : 2;
     const int mt = kRowTiles * blockIdx.x;
     const int G = L.q_heads / L.kv_heads;
+    if (!P.after_append) grid_dependency_wait();
     const int kv_total = *P.total_pos + 1;
 
     if (warp == kMmaWarp) tc::tmem_alloc(&sm.tmem_base, kTmemCols);
@@ -401,6 +403,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
     if (warp >= kDqWarp && warp < kMmaWarp) {
         // =========================== de-quantise ===========================
         tc::regs_dec<Ro::kDqRegs>();
+        if (P.after_append) grid_dependency_wait();
         const int dt = tid - 32 * kDqWarp;
         if (dt < 32 * kDqWarps) failed = dequant_role<false, kOther, kDqWarps>(sm, L, head, dt, t0, n, kv_total);
         else failed = dequant_role<true, kOther, kDqWarps>(sm, L, head, dt - 32 * kDqWarps, t0, n, kv_total);
@@ -617,7 +620,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
 namespace kvb {
 // kvb_chunk256.cu: the same for head_dim 256
 int launch_chunk_attention_256(const kvb_layer* layer, const void* q, const int32_t* positions_dev, int tokens, float scale,
-                               int kv_len_max, void* workspace, void* out, cudaStream_t s, float* part_m, float* part_l, float* part_o);
+                               int kv_len_max, void* workspace, void* out, cudaStream_t s, float* part_m, float* part_l, float* part_o, bool after_append);
 }  // namespace kvb
 
 extern "C" size_t kvb_prefill_workspace_bytes(int kv_len_max, int kv_heads, int q_heads, int head_dim, int tokens) {
@@ -629,8 +632,9 @@ namespace kvb {
 // Chunk attention of `tokens` rows that are already appended (shared by the prefill and the verify entry points).
 int launch_chunk_attention(const kvb_layer* layer, const void* q, const int32_t* positions_dev, int tokens, float scale,
                            int kv_len_max, void* workspace, void* out, cudaStream_t s, float* part_m, float* part_l,
-                           float* part_o, const int32_t* total_pos_dev) {
+                           float* part_o, const int32_t* total_pos_dev, bool after_append) {
     PrefillParams P;
+    P.after_append = after_append;
     P.L = make_view(*layer);
     P.q = static_cast<const uint16_t*>(q);
     P.pos = positions_dev;
@@ -652,8 +656,7 @@ int launch_chunk_attention(const kvb_layer* layer, const void* q, const int32_t*
     static OncePerDevice opted[4];
     KVB_CUDA_OK(allow_smem(opted[2 * shape.split + other], kernel, smem));
     const dim3 grid(shape.split ? shape.mtiles : (shape.mtiles + 1) / 2, layer->kv_heads, shape.ranges);
-    kernel<<<grid, kThreads, smem, s>>>(P);
-    KVB_CUDA_OK(cudaGetLastError());
+    KVB_CUDA_OK(launch_early(kernel, grid, dim3(kThreads), smem, s, P));
     if (P.out != nullptr) return KVB_OK;
     return launch_chunk_merge<D>(P.ws_m, P.ws_l, P.ws_o, tokens, layer->q_heads, layer->kv_heads, P.mtiles, P.ksplit, layer->dtype, out,
                                  part_m, part_l, part_o, s);
@@ -672,7 +675,7 @@ extern "C" int kvb_attn_prefill(const kvb_layer* layer, const void* q, const voi
     if (int st = kvb_append(layer, k, v, positions_dev, tokens, stream)) return st;
     if (layer->head_dim != 128)
         return launch_chunk_attention_256(layer, q, positions_dev, tokens, scale, kv_len_max, workspace, out, static_cast<cudaStream_t>(stream),
-                                          nullptr, nullptr, nullptr);
+                                          nullptr, nullptr, nullptr, true);
     return launch_chunk_attention(layer, q, positions_dev, tokens, scale, kv_len_max, workspace, out, static_cast<cudaStream_t>(stream),
-                                  nullptr, nullptr, nullptr, nullptr);
+                                  nullptr, nullptr, nullptr, nullptr, true);
 }
