@@ -423,50 +423,59 @@ __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Par
         tc::regs_dec<kMmaRegs>();
         if (warp == kMmaWarp) {
         constexpr uint32_t idesc_qk = tc::idesc_f16(kM, kN, false, false), idesc_pv = tc::idesc_f16(kM, D, false, true);
-        const uint32_t q_addr = smem_u32(sm.q_lo), k_hi = smem_u32(sm.k[0]), k_lo = smem_u32(sm.k[1]), v_hi = smem_u32(sm.v[0]), v_lo = smem_u32(sm.v[1]);
+        const uint64_t q0 = tc::smem_desc(smem_u32(sm.q_lo), 16, 1024), k_hi = tc::smem_desc(smem_u32(sm.k[0]), 16, 1024), k_lo = tc::smem_desc(smem_u32(sm.k[1]), 16, 1024);
+        const uint64_t v_hi = tc::smem_desc(smem_u32(sm.v[0]), kKvBlock, 1024), v_lo = tc::smem_desc(smem_u32(sm.v[1]), kKvBlock, 1024);
         for (int i = 0; i <= n && !failed; ++i) {
             if (i < n) {
                 // S(i) goes where P(i-2) was: P V(i-2) has to be over
                 if (!chunk_wait(&sm.k_full, i & 1, &sm.abort_flag) || (i > 1 && !chunk_wait(&sm.o_done, i & 1, &sm.abort_flag))) { failed = true; break; }
                 tc::fence_after_sync();
-                const uint32_t s = tmem + 64 * (i & 1);
-#pragma unroll 1
-                for (int b = 0; b < 4; ++b)  // 64 dims at a time (all of them at once cost more registers than this role has)
+                if (tc::elect_one()) {
+                    const uint32_t s = tmem + 64 * (i & 1);
+                    const uint64_t q = tc::desc_here(q0), kh = tc::desc_here(k_hi), kl = tc::desc_here(k_lo);
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk)
-                        tc::mma_f16_ss(s, tc::smem_desc(q_addr + b * kQBlock + kk * 32, 16, 1024), tc::smem_desc(k_hi + b * kKvBlock + kk * 32, 16, 1024), idesc_qk,
-                                       b > 0 || kk > 0);
-#pragma unroll 1
-                for (int b = 0; b < 4; ++b)
+                    for (int b = 0; b < 4; ++b)  // 64 dims at a time
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk)
-                        tc::mma_f16_ts(s, tmem + kColQ + 32 * b + 8 * kk, tc::smem_desc(k_lo + b * kKvBlock + kk * 32, 16, 1024), idesc_qk, true);
-#pragma unroll 1
-                for (int b = 0; b < 4; ++b)
+                        for (int kk = 0; kk < 4; ++kk)
+                            tc::mma_f16_ss(s, tc::desc_at(q, b * kQBlock + kk * 32), tc::desc_at(kh, b * kKvBlock + kk * 32), idesc_qk, b > 0 || kk > 0);
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk)
-                        tc::mma_f16_ts(s, tmem + kColQ + 32 * b + 8 * kk, tc::smem_desc(k_hi + b * kKvBlock + kk * 32, 16, 1024), idesc_qk, true);
-                tc::commit(&sm.s_full[i & 1]);
+                    for (int b = 0; b < 4; ++b)
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk)
+                            tc::mma_f16_ts(s, tmem + kColQ + 32 * b + 8 * kk, tc::desc_at(kl, b * kKvBlock + kk * 32), idesc_qk, true);
+#pragma unroll
+                    for (int b = 0; b < 4; ++b)
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk)
+                            tc::mma_f16_ts(s, tmem + kColQ + 32 * b + 8 * kk, tc::desc_at(kh, b * kKvBlock + kk * 32), idesc_qk, true);
+                    tc::commit(&sm.s_full[i & 1]);
+                }
+                __syncwarp();
             }
             if (i > 0) {
                 const int j = i - 1;
                 if (!chunk_wait(&sm.p_full[j & 1], (j >> 1) & 1, &sm.abort_flag) || !chunk_wait(&sm.v_full, j & 1, &sm.abort_flag)) { failed = true; break; }
                 tc::fence_after_sync();
-                const uint32_t p = tmem + 64 * (j & 1);
+                if (tc::elect_one()) {
+                    const uint32_t p = tmem + 64 * (j & 1);
+                    const uint64_t vh = tc::desc_here(v_hi), vl = tc::desc_here(v_lo);
 #pragma unroll
-                for (int kk = 0; kk < 4; ++kk)
-                    tc::mma_f16_ts(tmem + kColO, p + 32 + 8 * kk, tc::smem_desc(v_hi + kk * 2048, kKvBlock, 1024), idesc_pv, j > 0 || kk > 0);
+                    for (int kk = 0; kk < 4; ++kk)
+                        tc::mma_f16_ts(tmem + kColO, p + 32 + 8 * kk, tc::desc_at(vh, kk * 2048), idesc_pv, j > 0 || kk > 0);
 #pragma unroll
-                for (int kk = 0; kk < 4; ++kk)
-                    tc::mma_f16_ts(tmem + kColO, p + 8 * kk, tc::smem_desc(v_lo + kk * 2048, kKvBlock, 1024), idesc_pv, true);
+                    for (int kk = 0; kk < 4; ++kk)
+                        tc::mma_f16_ts(tmem + kColO, p + 8 * kk, tc::desc_at(vl, kk * 2048), idesc_pv, true);
 #pragma unroll
-                for (int kk = 0; kk < 4; ++kk)
-                    tc::mma_f16_ts(tmem + kColO, p + 8 * kk, tc::smem_desc(v_hi + kk * 2048, kKvBlock, 1024), idesc_pv, true);
-                tc::commit(&sm.o_done);
+                    for (int kk = 0; kk < 4; ++kk)
+                        tc::mma_f16_ts(tmem + kColO, p + 8 * kk, tc::desc_at(vh, kk * 2048), idesc_pv, true);
+                    tc::commit(&sm.o_done);
+                }
+                __syncwarp();
             }
         }
         if (failed) {  // nothing of this CTA may still run when its tensor memory is given back
-            tc::commit(&sm.drain);
+            if (tc::elect_one()) tc::commit(&sm.drain);
+            __syncwarp();
             mbar_wait_bounded(&sm.drain, 0);
         }
         }

@@ -413,6 +413,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
         if (warp == kMmaWarp) {
             constexpr uint32_t idesc_qk = tc::idesc_f16(kM, kN, false, false), idesc_pv = tc::idesc_f16(kM, D, false, true);
             const int steps[kStreams] = {steps_of(0), steps_of(1)};
+            const uint64_t q0 = tc::smem_desc(smem_u32(sm.q[0]), 16, 1024), k0 = tc::smem_desc(smem_u32(sm.k[0]), 16, 1024), v0 = tc::smem_desc(smem_u32(sm.v[0]), 16384, 1024);
             for (int i = 0; i <= steps[0] && !failed; ++i) {
 #pragma unroll
                 for (int u = 0; u < kStreams; ++u) {
@@ -426,31 +427,38 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
                         const int j = kSplit ? 2 * (i - 1) + u : i - 1;
                         if (!chunk_wait(&sm.v_full[j & 1], (j >> 1) & 1, &sm.abort_flag) || !chunk_wait(&sm.p_full[u], (i - 1) & 1, &sm.abort_flag)) { failed = true; break; }
                         tc::fence_after_sync();
-                        const uint32_t v_addr = smem_u32(sm.v[j & 1]);
+                        if (tc::elect_one()) {
+                            const uint64_t v = tc::desc_at(tc::desc_here(v0), (j & 1) * kTileBytes);
 #pragma unroll
-                        for (int kk = 0; kk < 8; ++kk)  // 16 keys = 8 columns of P
-                            tc::mma_f16_ts(tmem + kColO + 128 * u, tmem + 128 * u + (Ro::kHalves == 2 && kk >= 4 ? 64 - 32 : 0) + 8 * kk, tc::smem_desc(v_addr + kk * 2048, 16384, 1024), idesc_pv, i > 1 || kk > 0);
-                        tc::commit(&sm.o_done[u]);
-                        if (kSplit || u == 1 || steps[1] == 0) tc::commit(&sm.v_free[j & 1]);
+                            for (int kk = 0; kk < 8; ++kk)  // 16 keys = 8 columns of P
+                                tc::mma_f16_ts(tmem + kColO + 128 * u, tmem + 128 * u + (Ro::kHalves == 2 && kk >= 4 ? 64 - 32 : 0) + 8 * kk, tc::desc_at(v, kk * 2048), idesc_pv, i > 1 || kk > 0);
+                            tc::commit(&sm.o_done[u]);
+                            if (kSplit || u == 1 || steps[1] == 0) tc::commit(&sm.v_free[j & 1]);
+                        }
+                        __syncwarp();
                         // the next S_u is written over this P
                         if (!chunk_wait(&sm.o_done[u], (i - 1) & 1, &sm.abort_flag)) { failed = true; break; }
                     }
                     if (i < steps[u]) {
                         const int j = kSplit ? 2 * i + u : i;
                         tc::fence_after_sync();
-                        const uint32_t q_addr = smem_u32(sm.q[kSplit ? 0 : u]), k_addr = smem_u32(sm.k[j & 1]);
+                        if (tc::elect_one()) {
+                            const uint64_t q = tc::desc_at(tc::desc_here(q0), (kSplit ? 0 : u) * kTileBytes), k = tc::desc_at(tc::desc_here(k0), (j & 1) * kTileBytes);
 #pragma unroll
-                        for (int kk = 0; kk < 8; ++kk) {
-                            const uint32_t o = (kk >> 2) * 16384 + (kk & 3) * 32;
-                            tc::mma_f16_ss(tmem + 128 * u, tc::smem_desc(q_addr + o, 16, 1024), tc::smem_desc(k_addr + o, 16, 1024), idesc_qk, kk > 0);
+                            for (int kk = 0; kk < 8; ++kk) {
+                                const int o = (kk >> 2) * 16384 + (kk & 3) * 32;
+                                tc::mma_f16_ss(tmem + 128 * u, tc::desc_at(q, o), tc::desc_at(k, o), idesc_qk, kk > 0);
+                            }
+                            tc::commit(&sm.s_full[u]);
+                            if (kSplit || u == 1 || steps[1] == 0) tc::commit(&sm.k_free[j & 1]);
                         }
-                        tc::commit(&sm.s_full[u]);
-                        if (kSplit || u == 1 || steps[1] == 0) tc::commit(&sm.k_free[j & 1]);
+                        __syncwarp();
                     }
                 }
             }
             if (failed) {  // nothing of this CTA may still run when its tensor memory is given back
-                tc::commit(&sm.drain);
+                if (tc::elect_one()) tc::commit(&sm.drain);
+                __syncwarp();
                 mbar_wait_bounded(&sm.drain, 0);
             }
         }

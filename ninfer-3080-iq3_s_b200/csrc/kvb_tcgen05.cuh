@@ -43,16 +43,26 @@ __host__ __device__ constexpr uint32_t idesc_f16(int m, int n, bool a_mn_major, 
            (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
 }
 
-// D[tmem] (+)= A[smem] * B[smem].  K = 16 per instruction for 16-bit operands.  Called by a whole, converged warp with
-// warp-uniform operands: one elected lane issues the instruction (always the same lane, so a later commit by the
-// same election covers it); keeping the operand arithmetic warp-uniform lets it run on the uniform datapath, where
-// the instruction takes its operands from.
+// One thread of a whole, converged warp (always the same one): it issues the MMAs below and commits them.  A block of them under one
+// election costs an instruction or two each; an election, a predicate and a descriptor per MMA took longer to issue than to run.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(one));
+    return one != 0u;
+}
+// The same descriptor, as the compiler cannot know: offsets from it are not kept in registers from one step to the next.
+__device__ __forceinline__ uint64_t desc_here(uint64_t desc) {
+    asm volatile("" : "+l"(desc));
+    return desc;
+}
+// A descriptor `bytes` further (a multiple of 16).
+__device__ __forceinline__ uint64_t desc_at(uint64_t desc, int bytes) { return desc + static_cast<uint64_t>(bytes >> 4); }
+// D[tmem] (+)= A[smem] * B[smem].  K = 16 per instruction for 16-bit operands.
 __device__ __forceinline__ void mma_f16_ss(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, bool accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "elect.sync _|q, 0xffffffff;\n\t"
+        "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(static_cast<uint32_t>(accumulate))
         : "memory");
 }
@@ -60,21 +70,15 @@ __device__ __forceinline__ void mma_f16_ss(uint32_t tmem_d, uint64_t desc_a, uin
 // two elements per 32-bit column (even k in the low half), 8 columns per instruction.
 __device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, bool accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "elect.sync _|q, 0xffffffff;\n\t"
+        "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
         ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(static_cast<uint32_t>(accumulate))
         : "memory");
 }
-// All MMAs issued so far by the elected lane of this (whole, converged) warp arrive on `bar` when they have completed
-// (implies the before-sync fence).
+// All MMAs issued so far by this thread arrive on `bar` when they have completed (implies the before-sync fence).
 __device__ __forceinline__ void commit(uint64_t* bar) {
-    asm volatile(
-        "{\n\t.reg .pred q;\n\t"
-        "elect.sync _|q, 0xffffffff;\n\t"
-        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar))
-        : "memory");
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 // ---- TMEM <-> registers: lane = 32 * (warp % 4) + lane id, 32 consecutive 32-bit columns ---------------------
