@@ -95,11 +95,13 @@ template <int S> struct __align__(128) WarpRing {
     uint8_t slots[kSlots][Shape<S>::kSlot];
     uint8_t hdr[kHdrs][Shape<S>::kHdr];
     float scale_k[Shape<S>::kTab], zp_k[Shape<S>::kTab];  // per-dim scale / zero point of K for the tile in work: dim d at d + kTabPad * (d / 32)
-    uint64_t bars[kSlots];      // completes when the copies of the chunk in the slot have landed
 };
 
 template <int S, int W> struct __align__(128) AttnSmem {
-    WarpRing<S> ring[W];
+    WarpRing<S> ring[W];        // in the end the merge buffer of the warps
+    // One per slot: completes when the copies of the chunk in the slot have landed.  Outside the rings: memory that holds an mbarrier
+    // must not be used for anything else while it does.
+    uint64_t bars[W][kSlots];
     float4 qfrag[2 / S][8 * S][32];  // q' in per-lane fragment order: [row half][8 slice + j][lane] = dims 128 slice + 32t+4j..+3 of row g(+8)
     int row_pos[kRows];
     int poison[2][kRows];    // 256 dims: the row sees a key whose V (in this slice) is not finite
@@ -461,13 +463,15 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
     constexpr int kWarps = W, kThreads = W * 32;
     constexpr int kGroups = kPage / 16;            // 16-key groups of a page
     constexpr int kORow = D + 4, kWarpFloats = (2 + S) * kRows + kRows * kORow;  // merge buffer of a warp: m, l, z (per slice) per row, then o
-    static_assert(kWarps * kWarpFloats * 4 <= static_cast<int>(sizeof(WarpRing<S>)) * kWarps, "merge buffer exceeds the rings");
+    using Smem = AttnSmem<S, W>;
+    static_assert(kWarps * kWarpFloats * 4 <= offsetof(Smem, bars), "the merge buffer ends before the barriers");
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    AttnSmem<S, W>& sm = *reinterpret_cast<AttnSmem<S, W>*>(smem_raw);
+    Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
     const LayerView& L = P.L;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int G = L.q_heads / L.kv_heads;
     WarpRing<S>& R = sm.ring[warp];
+    uint64_t (&bars)[kSlots] = sm.bars[warp];
     // ---- order of the first memory requests: the few bytes everything waits for (positions, q rows, page table
     //      entries) go out first, then the first chunk of every warp, then -- after the rotation of q -- the rest of
     //      the ring.
@@ -497,7 +501,7 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
     if (S == 2 && threadIdx.x < 2 * kRows) (&sm.poison[0][0])[threadIdx.x] = 0;
     if (lane == 0) {
 #pragma unroll
-        for (int s = 0; s < kSlots; ++s) mbar_init(&R.bars[s], 1);
+        for (int s = 0; s < kSlots; ++s) mbar_init(&bars[s], 1);
         mbar_fence_init();
     }
     __syncwarp();
@@ -549,17 +553,17 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
             uint8_t* dst = R.slots[slot];
             if (n & 1) {
                 const uint8_t* src = vc + static_cast<size_t>(pid) * code_stride;
-                mbar_expect_tx(&R.bars[slot], kChunkBytes);
+                mbar_expect_tx(&bars[slot], kChunkBytes);
 #pragma unroll
-                for (int a = 0; a < Sh::kSubs; ++a) bulk_g2s(dst + a * Sh::kSubBytes, src + a * 1024, 1024, &R.bars[slot]);
+                for (int a = 0; a < Sh::kSubs; ++a) bulk_g2s(dst + a * Sh::kSubBytes, src + a * 1024, 1024, &bars[slot]);
             } else {
                 const int lp = w0 + (n >> 1);
                 const bool with_k = kOther || (lp & 1) == 0 || lp == w0;  // K scale rows: with the first page of a tile this warp reads (their fifth column is other_K of the page's own keys: always, when it is not 1)
                 uint8_t* hdr = R.hdr[(n >> 1) % kHdrs];
-                mbar_expect_tx(&R.bars[slot], kChunkBytes + kHdrV + (with_k ? kHdrK : 0));
-                bulk_g2s(dst, kc + static_cast<size_t>(pid) * code_stride, kChunkBytes, &R.bars[slot]);
-                bulk_g2s(hdr, vsr + static_cast<size_t>(pid) * (static_cast<uint32_t>(L.kv_heads) * kHdrV), kHdrV, &R.bars[slot]);
-                if (with_k) bulk_g2s(hdr + kHdrV, ksr + static_cast<size_t>(pid) * (static_cast<uint32_t>(L.kv_heads) * kHdrK), kHdrK, &R.bars[slot]);
+                mbar_expect_tx(&bars[slot], kChunkBytes + kHdrV + (with_k ? kHdrK : 0));
+                bulk_g2s(dst, kc + static_cast<size_t>(pid) * code_stride, kChunkBytes, &bars[slot]);
+                bulk_g2s(hdr, vsr + static_cast<size_t>(pid) * (static_cast<uint32_t>(L.kv_heads) * kHdrV), kHdrV, &bars[slot]);
+                if (with_k) bulk_g2s(hdr + kHdrV, ksr + static_cast<size_t>(pid) * (static_cast<uint32_t>(L.kv_heads) * kHdrK), kHdrK, &bars[slot]);
             }
         }
     };
@@ -633,7 +637,7 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
     // the barrier complete as soon as any lane has, so the verdict is the same in every lane without a vote.
     auto wait_slot = [&](int s) {
         if (timed_out) return;
-        if (!mbar_try_wait(&R.bars[s], (phases >> s) & 1u) && !mbar_wait_lane_bounded(&R.bars[s], (phases >> s) & 1u)) timed_out = true;
+        if (!mbar_try_wait(&bars[s], (phases >> s) & 1u) && !mbar_wait_lane_bounded(&bars[s], (phases >> s) & 1u)) timed_out = true;
     };
     auto release_chunk = [&](bool was_live) {  // the chunk in `slot` has been read by every lane: refill the slot, advance
         if (was_live) phases ^= 1u << slot;
@@ -1029,7 +1033,7 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
         if (lane == 0) L.flag(KVB_ERR_WAIT_TIMEOUT);
         // copies already issued must land before the CTA's shared memory is released: one more bounded wait each
         for (int s2 = 0; s2 < kSlots; ++s2)
-            if ((live >> s2) & 1u) mbar_wait_lane_bounded(&R.bars[s2], (phases >> s2) & 1u);
+            if ((live >> s2) & 1u) mbar_wait_lane_bounded(&bars[s2], (phases >> s2) & 1u);
     }
 
     // ---- merge the warps of the CTA (log-sum-exp) and store one partial per row; every slot has been consumed: the
