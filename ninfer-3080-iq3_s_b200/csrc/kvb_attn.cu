@@ -634,10 +634,11 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
     int slot = 0;          // slot of the oldest chunk not yet released
     uint32_t phases = 0;   // bit s: parity the next wait on slot s expects
     // Wait for the chunk in slot s (bounded).  The first probe usually succeeds; a lane that has to keep probing finds
-    // the barrier complete as soon as any lane has, so the verdict is the same in every lane without a vote.
+    // the barrier complete as soon as any lane has, so the verdict is the same in every lane without a vote.  The lanes come
+    // together again behind it: ldmatrix, movmatrix and the MMAs are instructions of a converged warp.
     auto wait_slot = [&](int s) {
-        if (timed_out) return;
-        if (!mbar_try_wait(&bars[s], (phases >> s) & 1u) && !mbar_wait_lane_bounded(&bars[s], (phases >> s) & 1u)) timed_out = true;
+        if (!timed_out && !mbar_try_wait(&bars[s], (phases >> s) & 1u) && !mbar_wait_lane_bounded(&bars[s], (phases >> s) & 1u)) timed_out = true;
+        __syncwarp();
     };
     auto release_chunk = [&](bool was_live) {  // the chunk in `slot` has been read by every lane: refill the slot, advance
         if (was_live) phases ^= 1u << slot;
