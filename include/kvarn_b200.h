@@ -210,8 +210,10 @@ int kvb_attn_rows_sharded(const kvb_layer* layer, const void* q, const int32_t* 
 /* One decode step: append the token at *pos_dev (k, v: [kv_heads][head_dim]), then decode attention of q over the
  * cache including it -- kvb_append followed by kvb_attn_decode (ring == NULL) or kvb_attn_decode_sharded (ring given:
  * the rank that owns the open tile of a range-sharded sequence), same results bit for bit, one host call instead of
- * two; the attention starts beside the append, and only its CTAs that read what the append writes wait for it.  The reference's decode
- * step makes the same pair of calls (kv_cache_append_launch, then causal_attention_cached_small_t_launch, P3:1379, 3612). */
+ * two; the attention starts beside the append, and only its CTAs that read what the append writes wait for it (in this call,
+ * kvb_attn_verify and kvb_attn_prefill alike; where what it writes shares memory with what the append
+ * reads it starts after it).  The reference's decode step makes the same pair of calls (kv_cache_append_launch, then
+ * causal_attention_cached_small_t_launch, P3:1379, 3612). */
 int kvb_append_decode(const kvb_layer* layer, const void* q, const void* k, const void* v, const int32_t* pos_dev, float scale,
                       int kv_len_max, void* workspace, const kvb_peer_ring* ring, void* out, void* stream);
 

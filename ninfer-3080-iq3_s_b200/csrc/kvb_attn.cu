@@ -1468,7 +1468,7 @@ int split_count(int kv_len_max, int kv_heads, int zblocks) {
 namespace kvb {
 // kvb_chunk256.cu
 int launch_chunk_attention_256(const kvb_layer* layer, const void* q, const int32_t* positions_dev, int tokens, float scale,
-                               int kv_len_max, void* workspace, void* out, cudaStream_t s, float* part_m, float* part_l, float* part_o, bool after_append);
+                               int kv_len_max, void* workspace, void* out, cudaStream_t s, float* part_m, float* part_l, float* part_o, const StepAppend* behind);
 namespace {
 
 // One attention launch with W warps per CTA (the opt-in to large dynamic shared memory is made once per device and W).
@@ -1548,7 +1548,7 @@ RowPlan plan_rows(int kv_len_max, int kv_heads, int q_heads, int head_dim, int T
 int launch_attention(const kvb_layer* layer, const void* q, const int32_t* pos_dev, const int32_t* total_pos_dev, int T,
                      float scale, int kv_len_max,
                      int key_begin, int key_end, void* workspace, void* out, float* part_m, float* part_l,
-                     float* part_o, cudaStream_t stream, const char* who, const PushTarget* push = nullptr, bool after_append = false) {
+                     float* part_o, cudaStream_t stream, const char* who, const PushTarget* push = nullptr, const StepAppend* behind = nullptr) {
     if (int st = check_layer(layer, who)) return st;
     if (q == nullptr || pos_dev == nullptr || workspace == nullptr) return fail(KVB_EINVAL, "%s: null q / positions / workspace", who);
     if (out == nullptr && part_m == nullptr && push == nullptr) return fail(KVB_EINVAL, "%s: null output", who);
@@ -1570,11 +1570,11 @@ int launch_attention(const kvb_layer* layer, const void* q, const int32_t* pos_d
     P.block_rows = plan.block_rows;
     P.key_begin = key_begin;
     P.key_end = key_end;
-    P.after_append = after_append;
     const size_t rows = static_cast<size_t>(layer->kv_heads) * Z * parts * kRows;
     P.ws_m = workspace_base(workspace);
     P.ws_l = P.ws_m + rows;
     P.ws_o = P.ws_l + rows;
+    P.after_append = starts_beside(behind, span_of(P.ws_m, rows * (2 + layer->head_dim) * sizeof(float)));
     const bool upper = plan.nb == 2;
     const dim3 grid(parts, layer->kv_heads, Z);
     if (layer->head_dim != 128) {  // two slices per head: twice the accumulators and the wider integers leave room for 8 warps.  The
@@ -1754,13 +1754,14 @@ extern "C" int kvb_append_decode(const kvb_layer* layer, const void* q, const vo
                                  int kv_len_max, void* workspace, const kvb_peer_ring* ring, void* out, void* stream) {
     using namespace kvb;
     if (int st = kvb_append(layer, k, v, pos_dev, 1, stream)) return st;
+    const StepAppend step = step_append(*layer, k, v, pos_dev, 1);
     if (ring == nullptr)
         return launch_attention(layer, q, pos_dev, pos_dev, 1, scale, kv_len_max, 0, INT_MAX, workspace, out, nullptr, nullptr, nullptr,
-                                static_cast<cudaStream_t>(stream), "kvb_append_decode", nullptr, true);
+                                static_cast<cudaStream_t>(stream), "kvb_append_decode", nullptr, &step);
     PushTarget push{};
     if (int st = make_push_target(layer, ring, out, "kvb_append_decode", push)) return st;
     return launch_attention(layer, q, pos_dev, pos_dev, 1, scale, kv_len_max, 0, INT_MAX, workspace, out, nullptr, nullptr, nullptr,
-                            static_cast<cudaStream_t>(stream), "kvb_append_decode", &push, true);
+                            static_cast<cudaStream_t>(stream), "kvb_append_decode", &push, &step);
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -1861,7 +1862,7 @@ extern "C" int kvb_attn_decode_batch(const kvb_layer* layers_dev, int batch, int
 namespace kvb {
 int launch_chunk_attention(const kvb_layer* layer, const void* q, const int32_t* positions_dev, int tokens, float scale,
                            int kv_len_max, void* workspace, void* out, cudaStream_t s, float* part_m, float* part_l,
-                           float* part_o, const int32_t* total_pos_dev, bool after_append);  // kvb_prefill.cu
+                           float* part_o, const int32_t* total_pos_dev, const StepAppend* behind);  // kvb_prefill.cu
 }
 
 extern "C" int kvb_attn_verify(const kvb_layer* layer, const void* q, const void* k, const void* v,
@@ -1870,13 +1871,14 @@ extern "C" int kvb_attn_verify(const kvb_layer* layer, const void* q, const void
     if (width < 1 || width > 8) return kvb::fail(KVB_ERANGE, "kvb_attn_verify: width %d (1..8; the reference rejects more, too)", width);
     if (int st = kvb::check_layer(layer, "kvb_attn_verify")) return st;
     if (int st = kvb_append(layer, k, v, positions_dev, width, stream)) return st;
+    const kvb::StepAppend step = kvb::step_append(*layer, k, v, positions_dev, width);
     if (width * (layer->q_heads / layer->kv_heads) >= kDenseRows && layer->head_dim == 128) {
         if (q == nullptr || workspace == nullptr || out == nullptr) return kvb::fail(KVB_EINVAL, "kvb_attn_verify: null q / workspace / out");
         return kvb::launch_chunk_attention(layer, q, positions_dev, width, scale, kv_len_max, workspace, out, static_cast<cudaStream_t>(stream),
-                                           nullptr, nullptr, nullptr, nullptr, true);
+                                           nullptr, nullptr, nullptr, nullptr, &step);
     }
     return kvb::launch_attention(layer, q, positions_dev, positions_dev + (width - 1), width, scale, kv_len_max, 0, INT_MAX, workspace, out, nullptr, nullptr,
-                                 nullptr, static_cast<cudaStream_t>(stream), "kvb_attn_verify", nullptr, layer->head_dim == 128);
+                                 nullptr, static_cast<cudaStream_t>(stream), "kvb_attn_verify", nullptr, layer->head_dim == 128 ? &step : nullptr);
 }
 
 // Causal attention of `tokens` already-appended (or foreign) query rows over THIS cache alone, exported as log-sum-exp
@@ -1896,8 +1898,8 @@ extern "C" int kvb_attn_chunk_partial(const kvb_layer* layer, const void* q, con
         return launch_attention(layer, q, positions_dev, positions_dev + (tokens - 1), tokens, scale, kv_len_max, 0, INT_MAX, workspace, nullptr,
                                 part_m, part_l, part_o, st, "kvb_attn_chunk_partial");
     if (layer->head_dim != 128)
-        return launch_chunk_attention_256(layer, q, positions_dev, tokens, scale, kv_len_max, workspace, nullptr, st, part_m, part_l, part_o, false);
-    return launch_chunk_attention(layer, q, positions_dev, tokens, scale, kv_len_max, workspace, nullptr, st, part_m, part_l, part_o, nullptr, false);
+        return launch_chunk_attention_256(layer, q, positions_dev, tokens, scale, kv_len_max, workspace, nullptr, st, part_m, part_l, part_o, nullptr);
+    return launch_chunk_attention(layer, q, positions_dev, tokens, scale, kv_len_max, workspace, nullptr, st, part_m, part_l, part_o, nullptr, nullptr);
 }
 
 // Causal attention of 1..8 query rows whose K/V rows are already in the cache -- a verify step without its append, for
@@ -1912,7 +1914,7 @@ extern "C" int kvb_attn_rows(const kvb_layer* layer, const void* q, const int32_
     if (rows * (layer->q_heads / layer->kv_heads) >= kDenseRows && layer->head_dim == 128) {
         if (q == nullptr || positions_dev == nullptr || workspace == nullptr || out == nullptr)
             return fail(KVB_EINVAL, "kvb_attn_rows: null q / positions / workspace / out");
-        return launch_chunk_attention(layer, q, positions_dev, rows, scale, kv_len_max, workspace, out, st, nullptr, nullptr, nullptr, total_pos_dev, false);
+        return launch_chunk_attention(layer, q, positions_dev, rows, scale, kv_len_max, workspace, out, st, nullptr, nullptr, nullptr, total_pos_dev, nullptr);
     }
     return launch_attention(layer, q, positions_dev, total_pos_dev, rows, scale, kv_len_max, 0, INT_MAX, workspace, out, nullptr, nullptr, nullptr,
                             st, "kvb_attn_rows");

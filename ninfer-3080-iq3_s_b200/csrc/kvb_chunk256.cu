@@ -616,9 +616,8 @@ __global__ void __launch_bounds__(kThreads, 1) chunk256_kernel(const Chunk256Par
 
 // Chunk attention of `tokens` rows that are already appended, over a head_dim-256 cache.
 int launch_chunk_attention_256(const kvb_layer* layer, const void* q, const int32_t* positions_dev, int tokens, float scale,
-                               int kv_len_max, void* workspace, void* out, cudaStream_t s, float* part_m, float* part_l, float* part_o, bool after_append) {
+                               int kv_len_max, void* workspace, void* out, cudaStream_t s, float* part_m, float* part_l, float* part_o, const StepAppend* behind) {
     Chunk256Params P;
-    P.after_append = after_append;
     P.L = make_view(*layer);
     P.q = static_cast<const uint16_t*>(q);
     P.pos = positions_dev;
@@ -632,6 +631,7 @@ int launch_chunk_attention_256(const kvb_layer* layer, const void* q, const int3
     P.ws_m = workspace_base(workspace);
     P.ws_l = P.ws_m + rows;
     P.ws_o = P.ws_l + rows;
+    P.after_append = starts_beside(behind, span_of(P.ws_m, partials_bytes(rows / kM, D)));
     const int smem = static_cast<int>(sizeof(Chunk256Smem)) + 1024;  // room to align the tiles to 1024 bytes
     static OncePerDevice opted;
     KVB_CUDA_OK(allow_smem(opted, chunk256_kernel, smem));

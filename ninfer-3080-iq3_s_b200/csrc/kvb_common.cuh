@@ -11,6 +11,7 @@
 
 #include "../../include/kvarn_b200.h"
 #include "kvb_once.hpp"
+#include "kvb_step.hpp"
 
 namespace kvb {
 
@@ -133,6 +134,10 @@ inline float* workspace_base(void* workspace) { return reinterpret_cast<float*>(
 
 LayerView make_view(const kvb_layer& L);
 int check_layer(const kvb_layer* L, const char* who);
+inline StepAppend step_append(const kvb_layer& L, const void* k, const void* v, const int32_t* positions, int tokens) {
+    const size_t bytes = static_cast<size_t>(tokens) * L.kv_heads * L.head_dim * sizeof(uint16_t);
+    return {span_of(k, bytes), span_of(v, bytes), span_of(positions, tokens * sizeof(int32_t))};
+}
 
 // 16-bit input element -> fp32.
 template <bool kBf16> __device__ __forceinline__ float in_to_f32(const uint16_t v) {

@@ -628,7 +628,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
 namespace kvb {
 // kvb_chunk256.cu: the same for head_dim 256
 int launch_chunk_attention_256(const kvb_layer* layer, const void* q, const int32_t* positions_dev, int tokens, float scale,
-                               int kv_len_max, void* workspace, void* out, cudaStream_t s, float* part_m, float* part_l, float* part_o, bool after_append);
+                               int kv_len_max, void* workspace, void* out, cudaStream_t s, float* part_m, float* part_l, float* part_o, const StepAppend* behind);
 }  // namespace kvb
 
 extern "C" size_t kvb_prefill_workspace_bytes(int kv_len_max, int kv_heads, int q_heads, int head_dim, int tokens) {
@@ -640,9 +640,8 @@ namespace kvb {
 // Chunk attention of `tokens` rows that are already appended (shared by the prefill and the verify entry points).
 int launch_chunk_attention(const kvb_layer* layer, const void* q, const int32_t* positions_dev, int tokens, float scale,
                            int kv_len_max, void* workspace, void* out, cudaStream_t s, float* part_m, float* part_l,
-                           float* part_o, const int32_t* total_pos_dev, bool after_append) {
+                           float* part_o, const int32_t* total_pos_dev, const StepAppend* behind) {
     PrefillParams P;
-    P.after_append = after_append;
     P.L = make_view(*layer);
     P.q = static_cast<const uint16_t*>(q);
     P.pos = positions_dev;
@@ -652,12 +651,17 @@ int launch_chunk_attention(const kvb_layer* layer, const void* q, const int32_t*
     P.mtiles = shape.mtiles;
     P.ksplit = shape.ksplit;
     P.scale_log2 = scale * 1.4426950408889634f;
-    // one key range needs no merge; the rows are stored 16 bytes at a time, an output that starts elsewhere takes the merge kernel's route
-    P.out = shape.ranges == 1 && part_m == nullptr && (reinterpret_cast<uintptr_t>(out) & 15u) == 0 ? static_cast<uint16_t*>(out) : nullptr;
     const size_t rows = static_cast<size_t>(layer->kv_heads) * P.mtiles * P.ksplit * kM;
     P.ws_m = workspace_base(workspace);
     P.ws_l = P.ws_m + rows;
     P.ws_o = P.ws_l + rows;
+    // One key range needs no merge.  The rows are stored 16 bytes at a time, and while other CTAs still read q and the positions: an
+    // output that starts elsewhere, or shares memory with them, takes the merge kernel's route.
+    const size_t out_bytes = static_cast<size_t>(tokens) * layer->q_heads * D * sizeof(uint16_t);
+    const bool finish = shape.ranges == 1 && part_m == nullptr && (reinterpret_cast<uintptr_t>(out) & 15u) == 0 &&
+                        stores_beside(span_of(out, out_bytes), span_of(q, out_bytes), span_of(positions_dev, tokens * sizeof(int32_t)), span_of(P.total_pos, sizeof(int32_t)));
+    P.out = finish ? static_cast<uint16_t*>(out) : nullptr;
+    P.after_append = starts_beside(behind, finish ? span_of(out, out_bytes) : span_of(P.ws_m, partials_bytes(rows / kM, D)));
     const int smem = static_cast<int>(sizeof(PrefillSmem)) + 1024;  // room to align the tiles to 1024 bytes
     const bool other = layer->sinkhorn_iters > 0;
     const auto kernel = shape.split ? (other ? chunk_kernel<true, true> : chunk_kernel<true, false>) : (other ? chunk_kernel<false, true> : chunk_kernel<false, false>);
@@ -681,9 +685,10 @@ extern "C" int kvb_attn_prefill(const kvb_layer* layer, const void* q, const voi
     if (layer->stage == nullptr) return fail(KVB_EINVAL, "kvb_attn_prefill: layer has no stage buffer");
     if (tokens > 65535) return fail(KVB_ERANGE, "kvb_attn_prefill: %d tokens in one chunk (at most 65535)", tokens);
     if (int st = kvb_append(layer, k, v, positions_dev, tokens, stream)) return st;
+    const StepAppend step = step_append(*layer, k, v, positions_dev, tokens);
     if (layer->head_dim != 128)
         return launch_chunk_attention_256(layer, q, positions_dev, tokens, scale, kv_len_max, workspace, out, static_cast<cudaStream_t>(stream),
-                                          nullptr, nullptr, nullptr, true);
+                                          nullptr, nullptr, nullptr, &step);
     return launch_chunk_attention(layer, q, positions_dev, tokens, scale, kv_len_max, workspace, out, static_cast<cudaStream_t>(stream),
-                                  nullptr, nullptr, nullptr, nullptr, true);
+                                  nullptr, nullptr, nullptr, nullptr, &step);
 }
