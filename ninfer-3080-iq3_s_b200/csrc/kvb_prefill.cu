@@ -232,7 +232,7 @@ __device__ __forceinline__ bool dequant_role(PrefillSmem& sm, const LayerView& L
 // [dim][row], where the K and V rings were.  Stages and roundings are those of hadamard_warp.
 template <bool kSplit>
 __device__ __forceinline__ void finish_rows(PrefillSmem& sm, const PrefillParams& P, uint32_t to, int u, int half, int row, int mt, int head, int G, bool is_row, bool seen,
-                                            float m_run, float l_run) {
+                                            float m_run, float l_run, bool failed) {
     using Ro = Roles<kSplit>;
     constexpr int kFinishThreads = 32 * kStreams * Ro::kSoft;
     const int h = kSplit ? u : half;
@@ -240,17 +240,26 @@ __device__ __forceinline__ void finish_rows(PrefillSmem& sm, const PrefillParams
         sm.row_top[u][0][row] = seen ? m_run : -INFINITY;
         sm.row_top[u][1][row] = seen ? l_run : 0.0f;
     }
+    const int m = (kSplit ? mt : mt + u) * kM + row, tq = m / G, gq = m % G;
+    uint16_t* const dst = P.out + (static_cast<int64_t>(tq) * P.L.q_heads + head * G + gq) * D + 16 * h;  // dims 16 h .. + 15 of every 32
     tc::fence_before_sync();
-    named_barrier_sync(11, kFinishThreads);  // every P V of the CTA is over
+    // every P V of the CTA is over -- or a wait was given up: sums are missing, the de-quantising warps may still write where the
+    // values would meet, and all rows of the CTA are zeros (the error word says why)
+    if (named_barrier_or(11, kFinishThreads, failed)) {
+#pragma unroll 1
+        for (int c = 0; c < 8; ++c)
+            if (is_row) *reinterpret_cast<uint4*>(dst + 8 * (c & 1) + 32 * (c >> 1)) = make_uint4(0u, 0u, 0u, 0u);
+        return;
+    }
     tc::fence_after_sync();
     float w[2] = {0.0f, 0.0f};  // weights of the streams' sums; a stream that saw no key has none
     bool used[2] = {seen, false};
     if constexpr (kSplit) {
-        const float m0 = sm.row_top[0][0][row], m1 = sm.row_top[1][0][row], m = fmaxf(m0, m1);
+        const float m0 = sm.row_top[0][0][row], m1 = sm.row_top[1][0][row], top = fmaxf(m0, m1);
         used[0] = m0 != -INFINITY;
         used[1] = m1 != -INFINITY;
-        if (used[0]) w[0] = fast_exp2(m0 - m);
-        if (used[1]) w[1] = fast_exp2(m1 - m);
+        if (used[0]) w[0] = fast_exp2(m0 - top);
+        if (used[1]) w[1] = fast_exp2(m1 - top);
         l_run = w[0] * sm.row_top[0][1][row] + w[1] * sm.row_top[1][1][row];
     } else {
         w[0] = 1.0f;
@@ -295,9 +304,7 @@ __device__ __forceinline__ void finish_rows(PrefillSmem& sm, const PrefillParams
         for (int e = 0; e < 32; ++e) mine[(64 * h + 32 * c + e) * kM] = x[e];
     }
     named_barrier_sync(11, kFinishThreads);
-    const int m = (kSplit ? mt : mt + u) * kM + row, tq = m / G, gq = m % G;
     if (!is_row) return;
-    uint16_t* const dst = P.out + (static_cast<int64_t>(tq) * P.L.q_heads + head * G + gq) * D;
 #pragma unroll 1
     for (int c = 0; c < 2; ++c) {  // dims d .. d + 7 and those 32, 64, 96 further
         const int d = 16 * h + 8 * c;
@@ -315,7 +322,7 @@ __device__ __forceinline__ void finish_rows(PrefillSmem& sm, const PrefillParams
             }
         }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4*>(dst + d + 32 * k) = make_uint4(o[k][0], o[k][1], o[k][2], o[k][3]);
+        for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4*>(dst + 8 * c + 32 * k) = make_uint4(o[k][0], o[k][1], o[k][2], o[k][3]);
     }
 }
 
@@ -588,7 +595,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
         }
         const bool have = steps > 0 && !failed && __any_sync(0xffffffffu, m_run != -INFINITY), seen = have && m_run != -INFINITY;
         if (P.out != nullptr) {
-            finish_rows<kSplit>(sm, P, to - kCols * half, u, half, row, mt, head, G, is_row, seen, m_run, l_run);
+            finish_rows<kSplit>(sm, P, to - kCols * half, u, half, row, mt, head, G, is_row, seen, m_run, l_run, failed);
         } else {
         const int tile = kSplit ? mt : mt + u, part = kSplit ? 2 * zs + u : zs;
         const int64_t idx = ((static_cast<int64_t>(head) * P.mtiles + tile) * P.ksplit + part) * kM + row;

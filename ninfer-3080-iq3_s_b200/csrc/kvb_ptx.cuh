@@ -57,9 +57,13 @@ __device__ __forceinline__ bool mbar_wait_lane_bounded(uint64_t* bar, uint32_t p
 }
 
 // The same wait of a whole warp of a CTA whose warps give up together: it also watches the CTA's abort flag, and raises it.
+// (A test builds the chunk kernels with no probe at all: every wait gives up at once.)
+#ifndef KVB_CHUNK_PROBES
+#define KVB_CHUNK_PROBES kSpinLimit
+#endif
 __device__ __forceinline__ bool chunk_wait(uint64_t* bar, uint32_t parity, int* abort_flag) {
     bool ok = false;
-    for (uint32_t i = 0; i < kSpinLimit && !ok; ++i) {
+    for (uint32_t i = 0; i < KVB_CHUNK_PROBES && !ok; ++i) {
         ok = mbar_try_wait(bar, parity);
         if (!ok && *reinterpret_cast<volatile int*>(abort_flag) != 0) break;
     }

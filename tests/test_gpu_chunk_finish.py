@@ -1,11 +1,14 @@
 """Chunks whose rows see one key range are finished in chunk_kernel itself (head_dim 128): no partials, no merge kernel.  Compared
 with the merge kernel's route -- taken by an output that starts at no 16-byte boundary -- and with the oracle."""
 import ctypes as C
+import os
+import shutil
+import subprocess
 
 import numpy as np
 import pytest
 
-from helpers import PREFILL_MAX_ABS, PREFILL_REL_L2, Twin, attn_close, cpu_twin_of, orc, pkg
+from helpers import PREFILL_MAX_ABS, PREFILL_REL_L2, ROOT, Twin, attn_close, cpu_twin_of, orc, pkg
 
 pytestmark = pytest.mark.gpu
 
@@ -44,3 +47,49 @@ def test_finished_rows(H, QH, ctx, tokens, dtype, iters):
     tol = (PREFILL_MAX_ABS, PREFILL_REL_L2) if dtype == 0 else (2.0 ** -7, 2.0 ** -7)  # bf16: half a unit of the output, 2^-9 of a value, and of P's, K's and V's rounding
     ok, msg = attn_close(got[0][rows], want, *tol)
     assert ok, msg
+
+
+@pytest.fixture(scope="module")
+def gives_up(tmp_path_factory):
+    """The chunk kernel built with waits that never look at their barrier: every one of them gives up at once, no MMA is issued."""
+    if shutil.which("nvcc") is None:
+        pytest.skip("needs nvcc on the GPU machine")
+    home = os.path.join(ROOT, "ninfer-3080-iq3_s_b200")
+    pkg().capi.load()
+    lib = str(tmp_path_factory.mktemp("gives_up") / "libchunk.so")
+    subprocess.run(["nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-shared", "-DKVB_CHUNK_PROBES=0u",
+                    os.path.join(home, "csrc", "kvb_prefill.cu"), "-o", lib, "-L", home, "-lkvarn_b200", "-Xlinker", "-rpath", "-Xlinker", home], check=True)
+    return C.CDLL(lib).kvb_attn_prefill
+
+
+# finished in the kernel (two row tiles a CTA, split keys with tiles for both streams and for one), and merged
+@pytest.mark.parametrize("H,QH,ctx,tokens,shift", [(4, 24, 0, 780, 0), (8, 64, 0, 290, 0), (1, 3, 0, 20, 0), (4, 24, 0, 780, 1), (4, 24, 900, 40, 0)])
+def test_a_chunk_that_gives_up(gives_up, H, QH, ctx, tokens, shift):
+    """A wait that runs out is reported, the rows are zeros and nothing beside them is touched; the next call is as if nothing had been."""
+    import torch
+
+    D, T = 128, ctx + tokens
+    k, v, q = orc.synth_kv(T, T, H, D, 1), orc.synth_kv(T, T, H, D, 2), orc.synth_q(T, tokens, QH, D)
+    for call in (gives_up, pkg().capi.load().kvb_attn_prefill):
+        tw = Twin(D=D, H=H, QH=QH, capacity_tokens=T, seed=T)
+        kd, vd, qd = (torch.from_numpy(x).to(tw.dev) for x in (k, v, q))
+        at = torch.arange(T, dtype=torch.int32, device=tw.dev)
+        if ctx:
+            tw.gpu.append(kd[:ctx], vd[:ctx], at[:ctx])
+        ws = tw.gpu.prefill_workspace(T, tokens).fill_(float("nan"))
+        buf = torch.full((qd.numel() + 16,), 7.0, dtype=qd.dtype, device=tw.dev)
+        out = buf[8 + shift:8 + shift + qd.numel()]
+        args = [C.c_void_p(x.data_ptr()) for x in (qd, kd[ctx:], vd[ctx:], at[ctx:])]
+        assert call(C.byref(tw.gpu.c), *args, tokens, C.c_float(1.0 / np.sqrt(D)), T, C.c_void_p(ws.data_ptr()), C.c_void_p(out.data_ptr()), None) == 0
+        torch.cuda.synchronize()
+        assert torch.all(buf[:8 + shift] == 7.0) and torch.all(buf[8 + shift + qd.numel():] == 7.0)
+        if call is gives_up:
+            assert tw.gpu.errors() == pkg().capi.ERR_WAIT_TIMEOUT
+            assert torch.all(out == 0.0)
+        else:
+            assert tw.gpu.errors() == 0
+            got = out.view(tokens, QH, D).float().cpu().numpy()
+            rows = np.array([0, tokens // 2, tokens - 1])
+            want = cpu_twin_of(tw.gpu).attention(q[rows], np.arange(ctx, T, dtype=np.int32)[rows], 1.0 / np.sqrt(D), QH, threads=8, kv_total=T)
+            ok, msg = attn_close(got[rows], want, PREFILL_MAX_ABS, PREFILL_REL_L2)
+            assert ok, msg
