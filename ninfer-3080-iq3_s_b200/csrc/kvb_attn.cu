@@ -1099,6 +1099,7 @@ __global__ void __launch_bounds__(W * 32, 1) attn_kernel(const AttnParams P) {
     if (!P.after_append) grid_dependency_wait();
     const int head = blockIdx.y, zb = blockIdx.z, split = blockIdx.x;
     attn_cta<S, NB, W, kOther>(P, split, head, zb, ((static_cast<int64_t>(head) * gridDim.z + zb) * P.nsplit + split) * kRows);
+    if (P.after_append) grid_dependency_wait();  // nobody leaves before the append is over: what waits for this grid finds both done
 }
 
 // Batched decode: `n` independent sequences (their caches described by device-resident kvb_layer structs, same

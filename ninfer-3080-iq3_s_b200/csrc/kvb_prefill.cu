@@ -623,6 +623,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
         }
         }
     }
+    if (P.after_append) grid_dependency_wait();  // nobody leaves before the append is over: what waits for this grid finds both done
     if (failed && lane == 0) L.flag(KVB_ERR_WAIT_TIMEOUT);
     tc::fence_before_sync();
     __syncthreads();
