@@ -316,16 +316,13 @@ __device__ __forceinline__ void rotate_rows(const uint16_t* __restrict__ src, in
 template <int D, bool kBf16>
 __global__ void __launch_bounds__(kThreads, 1) append_kernel(LayerView L, const uint16_t* __restrict__ k,
                                                              const uint16_t* __restrict__ v,
-                                                             const int32_t* __restrict__ positions, int tokens) {
+                                                             const int32_t* __restrict__ positions, int tokens, bool starts_next) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     AppendSmem& sm = *reinterpret_cast<AppendSmem*>(smem_raw);
     using G = Geo<D>;
     constexpr int S = G::S;
     grid_dependency_wait();  // launched while its predecessor still runs: nothing is read or written before it is over
-    // The attention of a step starts beside the append, and what of it reads the rows written here waits for the append's end.
-    // Measured on B200, a step of one layer: 32,768 tokens 13.8 -> 13.4 us, 8-row verify of 100,003 67.6 -> 63.6 us, a prompt of 777
-    // 35.9 -> 33.0 us.  Not for several rows of a verify step at 256 dims, whose four row blocks share their pages through L2: 41.2 -> 42.5.
-    if (D == 128 || tokens == 1 || tokens > 8) launch_dependents();
+    if (starts_next) launch_dependents();
     const int pos0 = positions[0], last = positions[tokens - 1];
     if (pos0 < 0 || last - pos0 != tokens - 1) {  // positions must be contiguous and non-negative
         if (threadIdx.x == 0) L.flag(KVB_ERR_POSITIONS);
@@ -462,7 +459,7 @@ int launch_append(const LayerView& V, const void* k, const void* v, const int32_
     KVB_CUDA_OK(allow_smem(opted, append_kernel<D, kBf16>, smem));
     const dim3 grid(tokens / kTile + 2, V.kv_heads, 2 * Geo<D>::S);
     KVB_CUDA_OK(launch_early(append_kernel<D, kBf16>, grid, dim3(kThreads), smem, stream, V, static_cast<const uint16_t*>(k), static_cast<const uint16_t*>(v),
-                             positions, tokens));
+                             positions, tokens, append_starts_next(D, tokens)));
     return KVB_OK;
 }
 

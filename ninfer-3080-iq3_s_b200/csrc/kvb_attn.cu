@@ -1879,7 +1879,7 @@ extern "C" int kvb_attn_verify(const kvb_layer* layer, const void* q, const void
                                            nullptr, nullptr, nullptr, nullptr, &step);
     }
     return kvb::launch_attention(layer, q, positions_dev, positions_dev + (width - 1), width, scale, kv_len_max, 0, INT_MAX, workspace, out, nullptr, nullptr,
-                                 nullptr, static_cast<cudaStream_t>(stream), "kvb_attn_verify", nullptr, layer->head_dim == 128 ? &step : nullptr);
+                                 nullptr, static_cast<cudaStream_t>(stream), "kvb_attn_verify", nullptr, &step);
 }
 
 // Causal attention of `tokens` already-appended (or foreign) query rows over THIS cache alone, exported as log-sum-exp

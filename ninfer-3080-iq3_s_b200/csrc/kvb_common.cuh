@@ -136,7 +136,7 @@ LayerView make_view(const kvb_layer& L);
 int check_layer(const kvb_layer* L, const char* who);
 inline StepAppend step_append(const kvb_layer& L, const void* k, const void* v, const int32_t* positions, int tokens) {
     const size_t bytes = static_cast<size_t>(tokens) * L.kv_heads * L.head_dim * sizeof(uint16_t);
-    return {span_of(k, bytes), span_of(v, bytes), span_of(positions, tokens * sizeof(int32_t))};
+    return {append_starts_next(L.head_dim, tokens), span_of(k, bytes), span_of(v, bytes), span_of(positions, tokens * sizeof(int32_t))};
 }
 
 // 16-bit input element -> fp32.

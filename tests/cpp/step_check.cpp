@@ -1,5 +1,6 @@
 // What of a step may run beside what: by the memory its buffers share.
 #include <cstdio>
+#include <initializer_list>
 
 #include "kvb_step.hpp"
 
@@ -17,7 +18,7 @@ int main() {
     expect(overlap(at(0, 100), at(40, 50)) && overlap(at(40, 50), at(0, 100)), true, "inside");
     expect(overlap(at(5, 5), at(5, 5)), false, "nothing");
 
-    const StepAppend step{at(1000, 1512), at(2000, 2512), at(3000, 3032)};
+    const StepAppend step{true, at(1000, 1512), at(2000, 2512), at(3000, 3032)};
     expect(starts_beside(nullptr, at(0, 10)), false, "no append");
     expect(starts_beside(&step, at(0, 1000)) && starts_beside(&step, at(1512, 2000)) && starts_beside(&step, at(2512, 3000)) && starts_beside(&step, at(3032, 4096)), true, "beside what the append reads");
     expect(starts_beside(&step, at(0, 1001)), false, "first byte of k");
@@ -25,6 +26,11 @@ int main() {
     expect(starts_beside(&step, at(2511, 2600)), false, "last byte of v");
     expect(starts_beside(&step, at(3028, 3100)), false, "last position");
     expect(starts_beside(&step, at(0, 4096)), false, "all of them");
+
+    const StepAppend alone{false, step.k, step.v, step.positions};
+    expect(starts_beside(&alone, at(0, 10)), false, "an append that does not let it start");
+    for (int tokens : {1, 2, 8, 9, 1024}) expect(append_starts_next(128, tokens), true, "128 dims");
+    for (int tokens : {1, 2, 8, 9, 1024}) expect(append_starts_next(256, tokens), tokens == 1 || tokens > 8, "256 dims");
 
     const Span q = at(0, 1024), pos = at(2000, 2032), total = at(3000, 3004);
     expect(stores_beside(at(1024, 2000), q, pos, total), true, "an output of its own");
