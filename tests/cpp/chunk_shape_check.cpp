@@ -34,6 +34,16 @@ int main() {
                     }
                 }
             }
+    // the calls of tests/test_gpu_chunk_finish.py: one key range, and the walk they are there for
+    const struct { int kv_heads, q_heads, ctx, tokens; bool split; } one_range[] = {
+        {4, 24, 0, 780, true}, {8, 64, 0, 128, true}, {1, 3, 0, 20, true}, {2, 16, 0, 8, true}, {8, 64, 250, 8, true}, {4, 24, 300, 40, true}, {4, 24, 192, 8, true}, {4, 32, 125, 5, true}, {8, 64, 56, 4, true},
+        {8, 64, 0, 290, false}, {4, 28, 5, 680, false}, {4, 24, 0, 1024, false}, {8, 24, 130, 1000, false}, {8, 64, 0, 1023, false}, {8, 64, 140, 290, false}};
+    for (const auto& c : one_range) {
+        const ChunkShape s = chunk_shape_128(c.ctx + c.tokens, c.kv_heads, c.q_heads, c.tokens, 148);
+        if (s.ranges == 1 && s.split == c.split) continue;
+        std::printf("heads %d/%d ctx %d tokens %d: %d ranges, split %d\n", c.kv_heads, c.q_heads, c.ctx, c.tokens, s.ranges, s.split);
+        ++bad;
+    }
     std::printf(bad ? "chunk shapes: %d wrong\n" : "chunk shapes: ok\n", bad);
     return bad != 0;
 }
