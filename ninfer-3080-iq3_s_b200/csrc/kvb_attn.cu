@@ -28,8 +28,8 @@
 // At head_dim 256 each slice has its own query integers (one scale_K, zp_K table per slice) and weights (scale_V per slice),
 // with a third byte each; the slices meet in the fp32 logits.  Bound by latency, most of it of instructions: eight warps, two a
 // scheduler, run thousands of instructions a page once or twice (a 16 KB page costs about as much as two 8 KB ones).  Measured on
-// B200 in graph replay, 24 / 4 heads, balanced bf16 cache: decode at 30,011 tokens 23.2 us a layer against 178 for one warp per key
-// on fp32 FMAs, a 5-row verify step at 20,000 tokens 41.5 against 486 (no per-element de-quantisation, rows of a KV head share
+// B200 in graph replay, 24 / 4 heads, balanced bf16 cache: decode at 30,011 tokens 22.9 us a layer against 178 for one warp per key
+// on fp32 FMAs, a 5-row verify step at 20,000 tokens 40.0 against 486 (no per-element de-quantisation, rows of a KV head share
 // every code read); the look for factors that are not finite is 0.4 and 1.0 us of it.
 #include <algorithm>
 #include <climits>
@@ -85,7 +85,7 @@ struct AttnParams {
     int nsplit;          // CTAs over the sealed tiles of a head; the last one also reads the open tile
     int block_rows;      // GQA-merged query rows per row block (grid z): 8 (one 8-row block per warp) or 16 (two)
     int key_begin, key_end;
-    bool after_append;   // launched behind the append of the rows at pos[0] ..: only the CTAs that read what it writes wait for it
+    bool after_append;   // beside the append of the rows at pos[0] .. (kvb_step.hpp): only the CTAs that read what it writes wait for it first
     float* ws_m;         // [H][Z][nsplit][16]
     float* ws_l;
     float* ws_o;         // [H][Z][nsplit][16][D]
@@ -1615,8 +1615,8 @@ int launch_attention(const kvb_layer* layer, const void* q, const int32_t* pos_d
 
 // From this many GQA-merged query rows per KV head on, steps run on the tcgen05 kernel.  Measured on B200 in graph replay, 24 / 4
 // heads, 131,072 tokens, us a layer for widths 3 .. 8 (18 .. 48 rows) on the warp-level kernel and on this one: unbalanced
-// 55.4 54.7 69.7 86.9 101.5 99.0 against 65.3 66.7 67.2 67.8 69.7 70.0, balanced 76.7 76.6 77.2 104.8 105.3 103.7 against 71.3 72.6
-// 73.1 73.7 75.6 75.8.
+// 54.3 53.1 69.3 85.6 99.6 96.9 against 64.0 65.2 65.6 66.4 68.3 68.5, balanced 71.8 71.3 71.6 99.7 99.4 97.2 against 70.0 70.3
+// 70.7 71.4 73.2 73.5.  (At 30 rows the tensor cores would be faster, but K and V are rounded to fp16 there.)
 static constexpr int kDenseRows = 32;
 extern "C" int kvb_split_capacity(int kv_len_max, int kv_heads, int q_heads, int rows, int batch) {
     (void)batch;

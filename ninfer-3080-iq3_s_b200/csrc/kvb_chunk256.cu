@@ -18,9 +18,9 @@
 // 64, the high part of Q (128, the A operand of two of the three Q K products), O (256).  The low part of Q stays in
 // shared memory (64 KB), beside one K and one V buffer.
 //
-// Bound by the chain of a page: K is de-quantised (about 2,800 cycles), then multiplied (48 MMAs of 128x64x16, 3,100: a
-// 64-key MMA takes as long as a 128-key one), hand-offs 700; P V, V and the softmax run beside it.  Measured on B200, 24 / 4
-// heads, 1,024 tokens over a prefix of 16,384, balanced bf16 cache: 1.26 ms (340 TFLOP/s of attention) against 69.8 ms for
+// Bound by the chain of a page: K is de-quantised (3,220 cycles), handed over (530), multiplied (48 MMAs of 128x64x16, 2,100 until
+// the buffer is free; 3,100 with an election and a descriptor per MMA); P V, V and the softmax run beside it.  Measured on B200, 24 / 4
+// heads, 1,024 tokens over a prefix of 16,384, balanced bf16 cache: 1.23 ms (346 TFLOP/s of attention) against 69.8 ms for
 // one warp per key on fp32 FMAs, 1.40 ms with eight warps for K and V in turn, 1.38 ms with sixteen in turn.
 // Accuracy: against float64 the un-normalised sums are off by 4e-7 .. 6e-6 (fp32 FMAs: 2e-7 .. 1.1e-5, sizes of 32 .. 65,576
 // keys), the fp16 / bf16 outputs by their rounding alone (2.09e-4 and 1.70e-3, as before).
@@ -55,7 +55,7 @@ struct Chunk256Params {
     const int32_t* pos;        // [T]
     const int32_t* total_pos;  // newest position in the cache
     int T, mtiles, ksplit;
-    bool after_append;         // launched behind the append of the rows: only the readers of the planes and the stage wait for it
+    bool after_append;         // beside the append of the rows (kvb_step.hpp): only the readers of the planes and the stage wait for it first
     float scale_log2;
     float* ws_m;               // [H][mtiles][ksplit][128]
     float* ws_l;

@@ -90,7 +90,8 @@ struct LayerView {
 };
 
 // Launch with programmatic stream serialization: the kernel may become resident while its predecessor in the
-// stream still runs and must call grid_dependency_wait() (kvb_ptx.cuh) before its first global memory access.
+// stream still runs and must call grid_dependency_wait() (kvb_ptx.cuh) before its first global memory access -- all but an
+// attention that starts beside its append: there, what does not depend on the append does not wait for it first (kvb_step.hpp).
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_early(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
     cudaLaunchConfig_t cfg{};

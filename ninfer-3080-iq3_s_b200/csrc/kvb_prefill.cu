@@ -10,12 +10,13 @@
 //   O += P V    tcgen05.mma, A = P in tensor memory, B = de-quantised V tile (MN-major: one 128-byte row of 64 dims per key),
 //               accumulator O[128 x 128] fp32 in tensor memory.
 // kSplit false: the streams are two row tiles over the same keys (a de-quantised tile serves 256 rows).  kSplit true: one
-// row tile, the streams take the even and the odd key tiles of the CTA's range and leave a partial each.
+// row tile, the streams take the even and the odd key tiles of the CTA's range.  A stream leaves a partial for the merge kernel, or,
+// where the rows see one key range only, the CTA finishes them (finish_rows).
 // One stream's MMAs run while the other's softmax does.  Sixteen warps de-quantise K and V straight from the planes into
 // two-stage rings (thread = one key, 64 dims): nibbles -> fp16 with the exact unpack, then one fused multiply-add with the
 // tile's per-dim (K) or the key's (V) fp16 scale and zero point.  Dims inside every group of eight are kept in the order the
-// unpack yields (0,4,1,5,2,6,3,7); Q is written in the same order, so the contraction is unaffected, and the merge kernel
-// puts the output dims back.  Keys of the open tile come un-quantised from the stage.
+// unpack yields (0,4,1,5,2,6,3,7); Q is written in the same order, so the contraction is unaffected, and what finishes a row
+// (the merge kernel, finish_rows) puts the output dims back.  Keys of the open tile come un-quantised from the stage.
 // Every wait on an mbarrier is bounded and also watches the CTA's abort flag; a wait that gives up sets
 // KVB_ERR_WAIT_TIMEOUT and the CTA leaves through the normal exit (its MMAs are over, TMEM is freed).
 #include <climits>
@@ -55,7 +56,7 @@ struct PrefillParams {
     const int32_t* pos;        // [T]
     const int32_t* total_pos;  // newest position in the cache
     int T, mtiles, ksplit;     // ksplit: partials per row
-    bool after_append;         // launched behind the append of the rows: only the readers of the planes and the stage wait for it
+    bool after_append;         // beside the append of the rows (kvb_step.hpp): only the readers of the planes and the stage wait for it first
     float scale_log2;
     uint16_t* out;             // one key range: the finished rows [T][q_heads][D]; else null, and
     float* ws_m;               // [H][mtiles][ksplit][128]
@@ -597,30 +598,30 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
         if (P.out != nullptr) {
             finish_rows<kSplit>(sm, P, to - kCols * half, u, half, row, mt, head, G, is_row, seen, m_run, l_run, failed);
         } else {
-        const int tile = kSplit ? mt : mt + u, part = kSplit ? 2 * zs + u : zs;
-        const int64_t idx = ((static_cast<int64_t>(head) * P.mtiles + tile) * P.ksplit + part) * kM + row;
-        if (is_row && half == 0) {
-            P.ws_m[idx] = seen ? m_run : -INFINITY;
-            P.ws_l[idx] = seen ? l_run : 0.0f;
-        }
-        float* orow = P.ws_o + idx * D + kCols * half;
+            const int tile = kSplit ? mt : mt + u, part = kSplit ? 2 * zs + u : zs;
+            const int64_t idx = ((static_cast<int64_t>(head) * P.mtiles + tile) * P.ksplit + part) * kM + row;
+            if (is_row && half == 0) {
+                P.ws_m[idx] = seen ? m_run : -INFINITY;
+                P.ws_l[idx] = seen ? l_run : 0.0f;
+            }
+            float* orow = P.ws_o + idx * D + kCols * half;
 #pragma unroll 1
-        for (int c = 0; c < kCols / 32; ++c) {
-            if (!warp_has_rows) break;
-            __syncwarp();  // the load is the whole warp's: lanes without a row are back from the stores
-            uint32_t r[32];
-            if (have) {
-                tc::tmem_ld32(to + 32 * c, r);
-                tc::tmem_ld_wait();
-            }
-            if (is_row) {
+            for (int c = 0; c < kCols / 32; ++c) {
+                if (!warp_has_rows) break;
+                __syncwarp();  // the load is the whole warp's: lanes without a row are back from the stores
+                uint32_t r[32];
+                if (have) {
+                    tc::tmem_ld32(to + 32 * c, r);
+                    tc::tmem_ld_wait();
+                }
+                if (is_row) {
 #pragma unroll
-                for (int e = 0; e < 32; e += 4)
-                    *reinterpret_cast<float4*>(orow + 32 * c + e) =
-                        seen ? make_float4(__uint_as_float(r[e]), __uint_as_float(r[e + 1]), __uint_as_float(r[e + 2]), __uint_as_float(r[e + 3]))
-                             : make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int e = 0; e < 32; e += 4)
+                        *reinterpret_cast<float4*>(orow + 32 * c + e) =
+                            seen ? make_float4(__uint_as_float(r[e]), __uint_as_float(r[e + 1]), __uint_as_float(r[e + 2]), __uint_as_float(r[e + 3]))
+                                 : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
             }
-        }
         }
     }
     if (P.after_append) grid_dependency_wait();  // nobody leaves before the append is over: what waits for this grid finds both done

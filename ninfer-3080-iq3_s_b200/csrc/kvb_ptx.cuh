@@ -97,8 +97,9 @@ __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1
 // Programmatic dependent launch.  A kernel launched with the programmatic-stream-serialization attribute may
 // start while its predecessor in the stream still runs (as soon as every CTA of the predecessor has called
 // launch_dependents or exited); it must call grid_dependency_wait() before touching anything the predecessor
-// writes: that returns when the predecessor has completed and its memory is visible.  Both are no-ops in a
-// kernel launched the ordinary way.
+// writes: that returns when the predecessor has completed and its memory is visible.  What the kernels before the predecessor
+// wrote may be read without it only if the predecessor called it ahead of launch_dependents.  Both are no-ops in a kernel
+// launched the ordinary way.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

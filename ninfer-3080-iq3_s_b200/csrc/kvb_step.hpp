@@ -27,8 +27,12 @@ struct StepAppend {
     Span k, v, positions;
 };
 
-// The attention writes (partials, or finished rows) while the append may still read: it starts beside the append unless what it writes
-// shares memory with what the append reads.
+// An attention that starts beside its append (after_append in the kernels' parameters) reads q, the positions and the pages the append
+// leaves alone, and writes, without waiting for it.  That is sound because
+//   - the append is the launch right before it in the stream and waits for all before it ahead of its trigger;
+//   - the CTAs and warps that read what the append writes (the stage, tiles from that of its first row on) wait for its end first;
+//   - what the attention writes shares no memory with what the append reads: checked here;
+//   - every thread waits for the append before it leaves, so that whatever waits for the attention finds both over.
 inline bool starts_beside(const StepAppend* step, Span written) {
     return step != nullptr && step->starts_next && !overlap(written, step->k) && !overlap(written, step->v) && !overlap(written, step->positions);
 }
