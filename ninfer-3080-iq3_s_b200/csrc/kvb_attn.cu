@@ -35,6 +35,7 @@
 #include <climits>
 #include <cstddef>
 #include <cstdlib>
+#include <functional>
 
 #include "kvb_common.cuh"
 #include "kvb_ptx.cuh"
@@ -43,7 +44,6 @@ namespace kvb {
 namespace {
 
 constexpr int D = 128;
-constexpr int kWarpsDecode = 16;    // warps per CTA for up to 8 merged query rows (one N block per warp): 128 registers per thread
 constexpr int kWarpsWide = 8;       // ... for 9..16 merged rows (two N blocks per warp), and at head_dim 256: twice the accumulators, 255 registers
 constexpr int kRows = 16;           // query rows per CTA: one or two 8-row N blocks
 constexpr int kSlots = 2;           // ring slots per warp: the chunk in work and the next one in flight
@@ -1113,6 +1113,7 @@ __global__ void __launch_bounds__(W * 32, 1) attn_kernel(const AttnParams P) {
 // over sealed pages, then its open tile; the number of splits follows the host's bound of its length, so long and
 // short sequences give CTAs of similar size.
 constexpr int kBatchMax = 64;
+constexpr int kBatchPerSm = 2;  // CTAs of 8 warps beside each other on an SM (up to 8 merged rows)
 struct BatchPlan {
     int n;                      // sequences; 0 = not a batched call
     int prefix[kBatchMax + 1];  // parts before sequence b
@@ -1139,8 +1140,8 @@ __device__ __forceinline__ int batch_entry_of(const BatchPlan& plan, int part) {
     return lo;
 }
 
-template <int NB, int W>
-__global__ void __launch_bounds__(W * 32, 1) attn_batch_kernel(const BatchParams B) {
+template <int NB, int W, int kPerSm>
+__global__ void __launch_bounds__(W * 32, kPerSm) attn_batch_kernel(const BatchParams B) {
     constexpr int kThreads = W * 32;
     grid_dependency_wait();
     const int part = blockIdx.x, head = blockIdx.y;
@@ -1782,36 +1783,81 @@ static_assert(sizeof(LayerView) == sizeof(kvb_layer) && offsetof(LayerView, erro
               "the device reads kvb_layer structs as LayerView");
 
 // Parts (splits over the sealed tiles; the last one also reads the open tile) of every sequence from the host's
-// bounds of their lengths: chunks of at least 8 tiles, at most 64 splits per sequence.  The chunk size trades the fixed
-// part of a CTA (about 8.8 us with 16 warps: set-up, first fetch, merge) against the balance of the SMs: the candidates
-// are 2 .. 12 CTAs per SM in total, costed as (CTAs x time of a CTA) / SMs + half a CTA for the ragged end, a CTA taking
-// 8.8 us + 3.93 us per round of 16 pages (the same figures as the single-sequence decode).
-int plan_batch(const int32_t* kv_len_max, int batch, int kv_heads, BatchPlan& plan) {
+// bounds of their lengths: chunks of at least 4 tiles, at most 64 splits per sequence.  A CTA of 8 warps takes `fixed` us (set-up,
+// first fetch, merge) and `round` us per 8 pages; `beside` of them share an SM, so that one's set-up and end lie beside the
+// others' work.  Chunk sizes that make about 1/2 .. 4 waves of CTAs are costed by the work per place plus 0.45 of what the last CTA
+// ends later than that, the CTAs of a head taken in order by its share of the places (a CTA left alone on its SM runs faster, hence not
+// all of it: fitted to sweeps of the chunk size over six batches).  Measured on B200, calls in a row, one CTA of 16 warps an SM with 2 ..
+// 12 CTAs per SM in total against this, us: 32 sequences of up to 131,072 tokens (24 / 4 heads) 317 -> 286, 8 of them 117 -> 84, 48 of
+// 30,000 130 -> 124, 40 of 4,096 34.4 -> 31.5, 24 of 100,000 (32 / 8) 353 -> 342, 20 of 60,000 (16 / 2) 73.5 -> 52.8.
+struct BatchCost {
+    int beside;
+    float fixed, round;
+};
+constexpr int kBatchLeast = 4;     // tiles of a chunk: a page for each of the 8 warps
+constexpr int kBatchPlaces = 512;  // the most places of a head that are modelled
+constexpr BatchCost kBatchNarrow{kBatchPerSm, 3.0f, 4.3f}, kBatchBroad{1, 6.1f, 4.4f};  // up to 8 merged rows, more
+int batch_parts(int kv_len_max, int chunk) { return std::min(std::max((kv_len_max / kTile + chunk - 1) / chunk, 1), kReduceWarps * kMaxPartsPerWarp); }
+int plan_batch_chunk(const int32_t* kv_len_max, int batch, int kv_heads, int sms, const BatchCost& cost) {
+    constexpr int kMost = kReduceWarps * kMaxPartsPerWarp;
     int64_t total_tiles = 0;
-    for (int b = 0; b < batch; ++b) total_tiles += kv_len_max[b] / kTile;
+    int most_tiles = 0;
+    for (int b = 0; b < batch; ++b) {
+        total_tiles += kv_len_max[b] / kTile;
+        most_tiles = std::max(most_tiles, kv_len_max[b] / kTile);
+    }
+    const int places = std::min(std::max(1, cost.beside * sms / kv_heads), kBatchPlaces);  // of a head
+    int best_chunk = kBatchLeast, last_chunk = 0;
+    float best = 1e30f, ends[kBatchPlaces];
+    static const float kWaves[] = {0.5f, 0.98f, 1.48f, 1.95f, 2.45f, 2.9f, 3.9f};
+    for (float waves : kWaves) {
+        const int want = static_cast<int>(static_cast<float>(total_tiles) / (waves * static_cast<float>(places))) + 1;
+        const int chunk = (std::max({kBatchLeast, want, (most_tiles + kMost - 1) / kMost}) + 3) / 4 * 4;
+        if (chunk == last_chunk) continue;
+        last_chunk = chunk;
+        std::fill(ends, ends + places, 0.0f);  // a heap, the earliest end first
+        float work = 0.0f, end = 0.0f;
+        for (int b = 0; b < batch; ++b) {
+            const int parts = batch_parts(kv_len_max[b], chunk);
+            const float t = cost.fixed + cost.round * static_cast<float>(((kv_len_max[b] / kTile + parts - 1) / parts + 3) / 4);
+            work += t * static_cast<float>(parts);
+            for (int i = 0; i < parts; ++i) {
+                std::pop_heap(ends, ends + places, std::greater<float>());
+                ends[places - 1] += t;
+                end = std::max(end, ends[places - 1]);
+                std::push_heap(ends, ends + places, std::greater<float>());
+            }
+        }
+        const float per_place = work / static_cast<float>(places), us = per_place + 0.45f * (end - per_place);
+        if (us < best) {
+            best = us;
+            best_chunk = chunk;
+        }
+    }
+    return best_chunk;
+}
+// The chunk size of the thread's last plan is kept with the numbers it follows from: a serving loop asks for the same ones at
+// every step, and costing them takes up to 0.1 ms.
+int plan_batch(const int32_t* kv_len_max, int batch, int kv_heads, int group, BatchPlan& plan) {
+    struct Last {
+        int32_t bounds[kBatchMax];
+        int batch = 0, kv_heads = 0, sms = 0, chunk = kBatchLeast;
+        bool broad = false;
+    };
+    static thread_local Last last;
+    const bool broad = group > 8;
     const int sms = sm_count();
-    int64_t chunk = 8;
-    float best = 1e30f;
-    static const int kPerSm[] = {2, 3, 4, 6, 8, 12};
-    for (int per_sm : kPerSm) {
-        const int64_t want = std::max<int64_t>(batch, static_cast<int64_t>(per_sm) * sms / kv_heads);
-        const int64_t c = std::max<int64_t>(8, (total_tiles + want - 1) / want);
-        int64_t ctas = 0;
-        for (int b = 0; b < batch; ++b)
-            ctas += std::min<int64_t>(std::max<int64_t>((kv_len_max[b] / kTile + c - 1) / c, 1), kReduceWarps * kMaxPartsPerWarp);
-        ctas *= kv_heads;
-        const float one = 8.8f + 3.93f * static_cast<float>((2 * c + kWarpsDecode - 1) / kWarpsDecode);
-        const float cost = static_cast<float>(ctas) * one / static_cast<float>(sms) + 0.5f * one;
-        if (cost < best) { best = cost; chunk = c; }
+    if (last.batch != batch || last.kv_heads != kv_heads || last.sms != sms || last.broad != broad || !std::equal(kv_len_max, kv_len_max + batch, last.bounds)) {
+        last.chunk = plan_batch_chunk(kv_len_max, batch, kv_heads, sms, broad ? kBatchBroad : kBatchNarrow);
+        std::copy(kv_len_max, kv_len_max + batch, last.bounds);
+        last.batch = batch;
+        last.kv_heads = kv_heads;
+        last.sms = sms;
+        last.broad = broad;
     }
     plan.n = batch;
     plan.prefix[0] = 0;
-    for (int b = 0; b < batch; ++b) {
-        const int64_t tiles = kv_len_max[b] / kTile;
-        int nsplit = static_cast<int>((tiles + chunk - 1) / chunk);
-        nsplit = std::min(std::max(nsplit, 1), kReduceWarps * kMaxPartsPerWarp);
-        plan.prefix[b + 1] = plan.prefix[b] + nsplit;
-    }
+    for (int b = 0; b < batch; ++b) plan.prefix[b + 1] = plan.prefix[b] + batch_parts(kv_len_max[b], last.chunk);
     return plan.prefix[batch];
 }
 
@@ -1824,7 +1870,7 @@ extern "C" size_t kvb_batch_workspace_bytes(const int32_t* kv_len_max, int batch
     for (int b = 0; b < batch; ++b)
         if (kv_len_max[b] < 1) return 0;
     BatchPlan plan;
-    const size_t rows = static_cast<size_t>(kv_heads) * plan_batch(kv_len_max, batch, kv_heads, plan) * kRows;
+    const size_t rows = static_cast<size_t>(kv_heads) * plan_batch(kv_len_max, batch, kv_heads, q_heads / kv_heads, plan) * kRows;
     return rows * (2 + head_dim) * sizeof(float) + kWorkspaceSlack;
 }
 
@@ -1842,7 +1888,7 @@ extern "C" int kvb_attn_decode_batch(const kvb_layer* layers_dev, int batch, int
     for (int b = 0; b < batch; ++b)
         if (kv_len_max[b] < 1) return fail(KVB_EINVAL, "kvb_attn_decode_batch: kv_len_max[%d] = %d", b, kv_len_max[b]);
     BatchParams B;
-    const int total = plan_batch(kv_len_max, batch, kv_heads, B.plan);
+    const int total = plan_batch(kv_len_max, batch, kv_heads, q_heads / kv_heads, B.plan);
     const size_t rows = static_cast<size_t>(kv_heads) * total * kRows;
     B.layers = reinterpret_cast<const LayerView*>(layers_dev);
     B.q = static_cast<const uint16_t*>(q);
@@ -1854,13 +1900,14 @@ extern "C" int kvb_attn_decode_batch(const kvb_layer* layers_dev, int batch, int
     B.ws_m = workspace_base(workspace);
     B.ws_l = B.ws_m + rows;
     B.ws_o = B.ws_l + rows;
-    constexpr int smem1 = static_cast<int>(sizeof(AttnSmem<1, kWarpsDecode>)), smem2 = static_cast<int>(sizeof(AttnSmem<1, kWarpsWide>));
+    constexpr int smem = static_cast<int>(sizeof(AttnSmem<1, kWarpsWide>));
+    static_assert(kBatchPerSm * (smem + 1024) <= 228 * 1024, "CTAs beside each other");
     static OncePerDevice opted1, opted2;
-    KVB_CUDA_OK(allow_smem(opted1, attn_batch_kernel<1, kWarpsDecode>, smem1));
-    KVB_CUDA_OK(allow_smem(opted2, attn_batch_kernel<2, kWarpsWide>, smem2));
+    KVB_CUDA_OK(allow_smem(opted1, attn_batch_kernel<1, kWarpsWide, kBatchPerSm>, smem));
+    KVB_CUDA_OK(allow_smem(opted2, attn_batch_kernel<2, kWarpsWide, 1>, smem));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (q_heads / kv_heads > 8) KVB_CUDA_OK(launch_early(attn_batch_kernel<2, kWarpsWide>, dim3(total, kv_heads, 1), dim3(kWarpsWide * 32), smem2, st, B));
-    else KVB_CUDA_OK(launch_early(attn_batch_kernel<1, kWarpsDecode>, dim3(total, kv_heads, 1), dim3(kWarpsDecode * 32), smem1, st, B));
+    if (q_heads / kv_heads > 8) KVB_CUDA_OK(launch_early(attn_batch_kernel<2, kWarpsWide, 1>, dim3(total, kv_heads, 1), dim3(kWarpsWide * 32), smem, st, B));
+    else KVB_CUDA_OK(launch_early(attn_batch_kernel<1, kWarpsWide, kBatchPerSm>, dim3(total, kv_heads, 1), dim3(kWarpsWide * 32), smem, st, B));
     KVB_CUDA_OK((launch_reduce<1, false>(batch * q_heads, st, B.ws_m, B.ws_l, B.ws_o, 0, batch, q_heads, kv_heads, 1, kRows, dtype, static_cast<uint16_t*>(out),
                                          nullptr, nullptr, nullptr, PushTarget{}, B.plan)));
     return KVB_OK;
