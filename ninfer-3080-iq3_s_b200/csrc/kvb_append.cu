@@ -49,6 +49,7 @@ struct AppendSmem {
     alignas(16) float fac_tok[kTile];              // ... per token
     float best_col[kSlice], best_row[kSlice];      // the factors the codes are made with
     float4 extremes[kSlice / 32];                  // per warp: smallest / largest column, row deviation
+    float2 state_dev[kSlice], state_fac[kSlice];   // a state of the balancing: column and row deviations, factors
     __half ax_scale[kSlice], ax_zp[kSlice], ax_other[kSlice];
 };
 
@@ -73,6 +74,17 @@ __device__ __forceinline__ void load_by_dim(const AppendSmem& sm, float (&x)[kPe
     for (int e = 0; e < kPer; ++e) x[e] = __half2float(sm.rows[(c0 + e) * kRowStride + d]);
 }
 
+// 1 / sqrt(x) and 1 / x for x > 0: the hardware's approximation and a step of Newton's method.
+__device__ __forceinline__ float rsqrt_newton(float x) {
+    const float y = rsqrtf(x), e = fmaf(-x * y, y, 1.0f);
+    return fmaf(0.5f * y, e, y);
+}
+__device__ __forceinline__ float rcp_newton(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return fmaf(y, fmaf(-x, y, 1.0f), y);
+}
+
 // Sinkhorn variance balancing, `iters` rounds, in the reference's order of updates
 // (kvarn128_codec.cuh:104-186 == bee_oracle.cpp:210-255): columns, rows, then "keep the best so far".
 // iters > 0 is the tolerance-checked regime (the reference's own CUDA kernel does not reproduce its host oracle
@@ -80,72 +92,62 @@ __device__ __forceinline__ void load_by_dim(const AppendSmem& sm, float (&x)[kPe
 // takes part, x / (s_col * s_row) becomes x * (1/s_col) * (1/s_row) with the reciprocals taken once per update
 // and the factor of the reduced-over axis pulled out of the sums, and partial sums meet in shared memory.
 // Both views of the matrix stay in registers, so a pass reads only the 128 factors; a row update changes only the factor
-// outside the row sums, so the deviations after it come from the sums before it; threads 0..127 own column i and row i and
-// hold their logs and factors.  Two passes and four barriers a round.  Bound by the chain of barriers, logf / expf and the
-// 32-long sums.  Measured on B200, 1,024 tokens, 4 heads of 256 dims, 16 rounds: 38.9 us a call against 120.8 us with 256
-// threads for both slices, the matrix in shared memory, three passes and twelve barriers a round, and a second launch for
-// the stage.  Every sum keeps its order: codes and axes are the same bytes.
+// outside the row sums, so the deviations after it come from the sums before it.  Threads 0..127 own column i and row i and hold
+// their factors; the reference's running sum of clamped logarithms is kept as the running product it stands for, clamped to the same
+// range, which leaves a reciprocal square root, a few products and a reciprocal between the sums and the next factors.  Threads
+// 128..255 judge the states meanwhile: the extremes of a state's deviations while the rows of the next are updated, the verdict while
+// its columns are.  Two passes (in pairs of elements) and four barriers a round; bound by the chain pass, barrier, factors, barrier: 1.0
+// us a round.  Measured on B200, 1,024 tokens, 4 heads of 256 dims, 16 rounds: 36.3 -> 31.8 us a call (logf and expf per round, the
+// owners judging, single elements before).
 template <bool kValue>
 __device__ void sinkhorn(AppendSmem& sm, const float (&by_token)[kPer], const float (&by_dim)[kPer], int iters) {
-    const int i = threadIdx.x;
-    const bool owner = i < kSlice;
-    auto finish = [](float sum, float sq) {  // sample standard deviation of 128 values from their sum and sum of squares
-        const float mean = sum * (1.0f / 128.0f);
-        return sqrtf(fmaxf((sq - 128.0f * mean * mean) * (1.0f / 127.0f), 0.0f));
-    };
-    auto sums_over_dims = [&]() {
-        const int par = i & 1, t = (i >> 1) & 127, hf = i >> 8;
-        float s = 0.0f, q = 0.0f;
+    const int i = threadIdx.x, j = i & (kSlice - 1);
+    const bool owner = i < kSlice, judge = i >= kSlice && i < 2 * kSlice;
+    auto sums = [&](const float (&x)[kPer], const float* factors, int part, int index) {
+        F2 s(0.0f, 0.0f), q(0.0f, 0.0f);
 #pragma unroll
         for (int e = 0; e < kPer; e += 4) {
-            const float4 f = *reinterpret_cast<const float4*>(&sm.fac_dim[par][hf * kPer + e]);
-            const float fs[4] = {f.x, f.y, f.z, f.w};
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const float a = by_token[e + u] * fs[u];
-                s += a;
-                q = fmaf(a, a, q);
-            }
+            const float4 f = *reinterpret_cast<const float4*>(factors + e);
+            const F2 a = mul2(F2(x[e], x[e + 1]), F2(f.x, f.y)), b = mul2(F2(x[e + 2], x[e + 3]), F2(f.z, f.w));
+            s = add2(s, a);
+            q = fma2(a, a, q);
+            s = add2(s, b);
+            q = fma2(b, b, q);
         }
-        sm.red_lo[(2 * hf + par) * kRedStride + t] = s;
-        sm.red_hi[(2 * hf + par) * kRedStride + t] = q;
+        const float2 s2 = s.get(), q2 = q.get();
+        sm.red_lo[part * kRedStride + index] = s2.x + s2.y;
+        sm.red_hi[part * kRedStride + index] = q2.x + q2.y;
     };
-    auto sums_over_tokens = [&]() {
-        const int d = i & 127, qtr = i >> 7;
-        float s = 0.0f, q = 0.0f;
-#pragma unroll
-        for (int e = 0; e < kPer; e += 4) {
-            const float4 f = *reinterpret_cast<const float4*>(&sm.fac_tok[qtr * kPer + e]);
-            const float fs[4] = {f.x, f.y, f.z, f.w};
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const float a = by_dim[e + u] * fs[u];
-                s += a;
-                q = fmaf(a, a, q);
-            }
-        }
-        sm.red_lo[qtr * kRedStride + d] = s;
-        sm.red_hi[qtr * kRedStride + d] = q;
-    };
+    auto sums_over_dims = [&]() { sums(by_token, &sm.fac_dim[i & 1][(i >> 8) * kPer], 2 * (i >> 8) + (i & 1), (i >> 1) & 127); };
+    auto sums_over_tokens = [&]() { sums(by_dim, &sm.fac_tok[(i >> 7) * kPer], i >> 7, i & 127); };
     auto col_pass = [&]() { if constexpr (kValue) sums_over_tokens(); else sums_over_dims(); };
     auto row_pass = [&]() { if constexpr (kValue) sums_over_dims(); else sums_over_tokens(); };
     auto dim_factor = [&](float f) { sm.fac_dim[i & 1][i >> 1] = f; };
     auto set_col = [&](float f) { if constexpr (kValue) dim_factor(f); else sm.fac_tok[i] = f; };
     auto set_row = [&](float f) { if constexpr (kValue) sm.fac_tok[i] = f; else dim_factor(f); };
     auto total = [&](const float* red) { return (red[i] + red[kRedStride + i]) + (red[2 * kRedStride + i] + red[3 * kRedStride + i]); };
-
-    float log_col = 0.0f, log_row = 0.0f, cur_col = 1.0f, cur_row = 1.0f, rcp_col = 1.0f, rcp_row = 1.0f, std_col = 0.0f, std_row = 0.0f;
-    float best_col = 1.0f, best_row = 1.0f, best = 3.402823466e+38f;
-    auto publish_extremes = [&]() {  // of the current deviations
-        float cmin = fminf(3.402823466e+38f, std_col), cmax = fmaxf(0.0f, std_col), rmin = fminf(3.402823466e+38f, std_row), rmax = fmaxf(0.0f, std_row);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            cmin = fminf(cmin, __shfl_xor_sync(0xffffffffu, cmin, o)); cmax = fmaxf(cmax, __shfl_xor_sync(0xffffffffu, cmax, o));
-            rmin = fminf(rmin, __shfl_xor_sync(0xffffffffu, rmin, o)); rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
-        }
-        if ((i & 31) == 0) sm.extremes[i >> 5] = make_float4(cmin, cmax, rmin, rmax);
+    auto deviation = [&]() {  // sample standard deviation of the 128 values summed last
+        const float sum = total(sm.red_lo), sq = total(sm.red_hi), mean = sum * (1.0f / 128.0f);
+        const float var = fmaxf((sq - 128.0f * mean * mean) * (1.0f / 127.0f), 0.0f);
+        return var > 1e-30f && var < INFINITY ? var * rsqrt_newton(var) : sqrtf(var);
     };
-    auto keep_best = [&](float col, float row) {  // imbalance of the published factors; "<=" lets a later tie win
+    // exp of the reference's clamped sum of logarithms, -0.3 .. 10
+    auto advance = [](float factor, float dev) { return fminf(fmaxf(factor * fminf(fmaxf(dev, 1e-3f), 1e3f), 0.74081822f), 22026.466f); };
+
+    float cur_col = 1.0f, cur_row = 1.0f, rcp_col = 1.0f, rcp_row = 1.0f, dev_col = 0.0f, dev_row = 0.0f;
+    float best_col = 1.0f, best_row = 1.0f, best = 3.402823466e+38f;
+    auto hand_over = [&]() {  // the state the owners leave
+        sm.state_dev[i] = make_float2(dev_col, dev_row);
+        sm.state_fac[i] = make_float2(cur_col, cur_row);
+    };
+    auto look = [&]() {  // a state's extremes; deviations are >= 0, so their bits have their order
+        const float2 d = sm.state_dev[j];
+        const uint32_t c = __float_as_uint(d.x), r = __float_as_uint(d.y);
+        const uint32_t cmin = __reduce_min_sync(0xffffffffu, c), cmax = __reduce_max_sync(0xffffffffu, c), rmin = __reduce_min_sync(0xffffffffu, r), rmax = __reduce_max_sync(0xffffffffu, r);
+        if ((i & 31) == 0) sm.extremes[j >> 5] = make_float4(__uint_as_float(cmin), __uint_as_float(cmax), __uint_as_float(rmin), __uint_as_float(rmax));
+    };
+    float2 seen = make_float2(1.0f, 1.0f);  // the factors of the state that was looked at
+    auto keep_best = [&]() {  // imbalance of that state; "<=" lets a later tie win
         float4 x = sm.extremes[0];
 #pragma unroll
         for (int w = 1; w < kSlice / 32; ++w) {
@@ -153,56 +155,59 @@ __device__ void sinkhorn(AppendSmem& sm, const float (&by_token)[kPer], const fl
             x = make_float4(fminf(x.x, y.x), fmaxf(x.y, y.y), fminf(x.z, y.z), fmaxf(x.w, y.w));
         }
         const float imb = __fadd_rn(__fdiv_rn(x.y, fmaxf(x.x, 1e-8f)), __fdiv_rn(x.w, fmaxf(x.z, 1e-8f)));
-        if (imb <= best) { best = imb; best_col = col; best_row = row; }
+        if (imb <= best) { best = imb; best_col = seen.x; best_row = seen.y; }
     };
 
     if (owner) { set_col(1.0f); set_row(1.0f); }
     __syncthreads();
-    col_pass();
-    __syncthreads();
-    if (owner) std_col = finish(total(sm.red_lo), total(sm.red_hi));
-    __syncthreads();
     row_pass();
     __syncthreads();
-    if (owner) {
-        std_row = finish(total(sm.red_lo), total(sm.red_hi));
-        publish_extremes();
-    }
+    if (owner) dev_row = deviation();
+    __syncthreads();
+    col_pass();
+    __syncthreads();
     for (int it = 0; it < iters; ++it) {
-        const float old_col = cur_col, old_row = cur_row;
         if (owner) {
-            const float c = fminf(fmaxf(std_col, 1e-3f), 1e3f);
-            log_col = fminf(fmaxf(__fadd_rn(log_col, logf(c)), -0.3f), 10.0f);
-            cur_col = expf(log_col);
-            rcp_col = __fdiv_rn(1.0f, cur_col);
+            dev_col = deviation() * rcp_col;
+            hand_over();
+            cur_col = advance(cur_col, dev_col);
+            rcp_col = rcp_newton(cur_col);
             set_col(rcp_col);
         }
+        if (judge && it > 0) keep_best();
         __syncthreads();
         row_pass();
-        if (owner) keep_best(old_col, old_row);
         __syncthreads();
         if (owner) {
-            const float sum = total(sm.red_lo), sq = total(sm.red_hi);
-            const float r = fminf(fmaxf(finish(sum * rcp_row, sq * rcp_row * rcp_row), 1e-3f), 1e3f);
-            log_row = fminf(fmaxf(__fadd_rn(log_row, logf(r)), -0.3f), 10.0f);
-            cur_row = expf(log_row);
-            rcp_row = __fdiv_rn(1.0f, cur_row);
+            const float dev = deviation();
+            cur_row = advance(cur_row, dev * rcp_row);
+            rcp_row = rcp_newton(cur_row);
             set_row(rcp_row);
-            std_row = finish(sum * rcp_row, sq * rcp_row * rcp_row);
+            dev_row = dev * rcp_row;
+        }
+        if (judge) {
+            look();
+            seen = sm.state_fac[j];
         }
         __syncthreads();
         col_pass();
         __syncthreads();
-        if (owner) {
-            std_col = finish(total(sm.red_lo) * rcp_col, total(sm.red_hi) * rcp_col * rcp_col);
-            publish_extremes();
-        }
+    }
+    if (owner) {
+        dev_col = deviation() * rcp_col;
+        hand_over();
+    }
+    if (judge && iters > 0) keep_best();
+    __syncthreads();
+    if (judge) {
+        look();
+        seen = sm.state_fac[j];
     }
     __syncthreads();
-    if (owner) {
-        keep_best(cur_col, cur_row);
-        sm.best_col[i] = best_col;
-        sm.best_row[i] = best_row;
+    if (judge) {
+        keep_best();
+        sm.best_col[j] = best_col;
+        sm.best_row[j] = best_row;
     }
     __syncthreads();
 }
