@@ -24,7 +24,10 @@
 //     unsigned bytes; V codes are transposed to "four keys of one dim per register" by ldmatrix.trans plus one
 //     byte permute and one AND per register; the integer sums of the page are converted once per page and
 //     enter the running fp32 accumulators with the weight exp2(page max - running max).
-// The page-local reference keeps 16 significant bits below each page's own maximum, whatever the global one is.
+// The page-local reference keeps 16 significant bits below each page's own maximum, whatever the global one is.  What is fp32 runs on
+// packed pairs (two keys of a row, two rows of a dim).  Measured on B200 in graph replay against single values, us a layer: decode at
+// 378,944 tokens 47.1 -> 45.1, verify of 2 / 3 / 4 / 5 rows at 131,072 36.9 / 54.5 / 53.4 / 69.6 -> 36.2 / 52.6 / 51.9 / 67.2, 5 rows of 256 dims
+// at 20,000 40.1 -> 39.6.
 // At head_dim 256 each slice has its own query integers (one scale_K, zp_K table per slice) and weights (scale_V per slice),
 // with a third byte each; the slices meet in the fp32 logits.  Bound by latency, most of it of instructions: eight warps, two a
 // scheduler, run thousands of instructions a page once or twice (a 16 KB page costs about as much as two 8 KB ones).  Measured on
@@ -109,10 +112,10 @@ template <int S, int W> struct __align__(128) AttnSmem {
 
 // Per-thread state of the running softmax.  Lane (g, t) owns query rows 8 nb + 2t, 2t+1 of n-block nb and dims
 // 32 db + 4g + i (db < 4 S, i < 4):  o[nb][db][xy][c] is dim 32 db + 4g + xy + 2 (c >> 1), row 8 nb + 2t + (c & 1) -- the
-// accumulator layout of the two MMAs per 32-dim block (xy = 0: even dims, 1: odd dims).  l and z (per slice) are partial
+// accumulator layout of the two MMAs per 32-dim block (xy = 0: even dims, 1: odd dims), kept in pairs of rows [c >> 1].  l and z (per slice) are partial
 // over the lane's keys; everything is relative to the running maximum m (log2 units).
 template <int S, int NB> struct Acc {
-    float o[NB][4 * S][2][4];
+    F2 o[NB][4 * S][2][2];
     float m[NB][2], l[NB][2], z[S][NB][2];
 };
 
@@ -203,19 +206,22 @@ __device__ __forceinline__ void build_qint(const Smem& sm, const WarpRing<S>& R,
     for (int s = 0; s < S; ++s) {
 #pragma unroll
         for (int nb = 0; nb < NB; ++nb) {
-            float qs[32];
-            float qz = 0.0f, amax = 0.0f;
+            F2 qs[16], qz2(0.0f, 0.0f);
+            float amax = 0.0f;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const float4 qv = sm.qfrag[nb][8 * s + j][lane];
                 const float4 ks = *reinterpret_cast<const float4*>(&R.scale_k[(32 + kTabPad) * (4 * s + t) + 4 * j]);
                 const float4 kz = *reinterpret_cast<const float4*>(&R.zp_k[(32 + kTabPad) * (4 * s + t) + 4 * j]);
-                qs[4 * j + 0] = qv.x * ks.x; qs[4 * j + 1] = qv.y * ks.y;
-                qs[4 * j + 2] = qv.z * ks.z; qs[4 * j + 3] = qv.w * ks.w;
-                qz = fmaf(qv.x, kz.x, qz); qz = fmaf(qv.y, kz.y, qz);
-                qz = fmaf(qv.z, kz.z, qz); qz = fmaf(qv.w, kz.w, qz);
-                amax = fmaxf(fmaxf(amax, fmaxf(fabsf(qs[4 * j]), fabsf(qs[4 * j + 1]))), fmaxf(fabsf(qs[4 * j + 2]), fabsf(qs[4 * j + 3])));
+                const F2 q0(qv.x, qv.y), q1(qv.z, qv.w);
+                qs[2 * j] = mul2(q0, F2(ks.x, ks.y));
+                qs[2 * j + 1] = mul2(q1, F2(ks.z, ks.w));
+                qz2 = fma2(q0, F2(kz.x, kz.y), qz2);
+                qz2 = fma2(q1, F2(kz.z, kz.w), qz2);
+                const float2 a = qs[2 * j].get(), b = qs[2 * j + 1].get();
+                amax = fmaxf(fmaxf(amax, fmaxf(fabsf(a.x), fabsf(a.y))), fmaxf(fabsf(b.x), fabsf(b.y)));
             }
+            float qz = qz2.get().x + qz2.get().y;
             qz += __shfl_xor_sync(0xffffffffu, qz, 1);
             qz += __shfl_xor_sync(0xffffffffu, qz, 2);  // every lane of group g now holds qz of row 8 nb + g
             amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
@@ -227,7 +233,11 @@ __device__ __forceinline__ void build_qint(const Smem& sm, const WarpRing<S>& R,
             f.f[s][nb][1] = __shfl_sync(0xffffffffu, fr, 8 * t + 4) * 0.0625f;
             uint32_t x[32];
 #pragma unroll
-            for (int i = 0; i < 32; ++i) x[i] = __float_as_uint(fmaf(qs[i], inv, kMagic));  // low 16 bits (22 at 256 dims): Qi (two's complement)
+            for (int i = 0; i < 16; ++i) {  // low 16 bits (22 at 256 dims): Qi (two's complement)
+                const float2 y = fma2(qs[i], F2(inv, inv), F2(kMagic, kMagic)).get();
+                x[2 * i] = __float_as_uint(y.x);
+                x[2 * i + 1] = __float_as_uint(y.y);
+            }
 #pragma unroll
             for (int kb = 0; kb < 2; ++kb)
 #pragma unroll
@@ -283,7 +293,7 @@ __device__ __forceinline__ void rescale(Acc<S, NB>& acc, const float (&alpha)[NB
 #pragma unroll
             for (int xy = 0; xy < 2; ++xy)
 #pragma unroll
-                for (int c = 0; c < 4; ++c) acc.o[nb][db][xy][c] *= alpha[nb][c & 1];
+                for (int h = 0; h < 2; ++h) acc.o[nb][db][xy][h] = mul2(acc.o[nb][db][xy][h], F2(alpha[nb][0], alpha[nb][1]));
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             acc.l[nb][j] *= alpha[nb][j];
@@ -436,11 +446,22 @@ __device__ __forceinline__ void process_stage_group(Smem& sm, const __half* krow
         const uint32_t y2 = prmt(v[2].x, v[3].x, 0x7632), y3 = prmt(v[2].y, v[3].y, 0x7632);
 #pragma unroll
         for (int nb = 0; nb < NB; ++nb) {
-            mma16816(acc.o[nb][db][0], x0, x1, x2, x3, b0[nb], b1[nb]);
-            mma16816(acc.o[nb][db][1], y0, y1, y2, y3, b0[nb], b1[nb]);
+            float o[2][4];
+#pragma unroll
+            for (int xy = 0; xy < 2; ++xy) {
+                const float2 lo = acc.o[nb][db][xy][0].get(), hi = acc.o[nb][db][xy][1].get();
+                o[xy][0] = lo.x; o[xy][1] = lo.y; o[xy][2] = hi.x; o[xy][3] = hi.y;
+            }
+            mma16816(o[0], x0, x1, x2, x3, b0[nb], b1[nb]);
+            mma16816(o[1], y0, y1, y2, y3, b0[nb], b1[nb]);
             if constexpr (S == 2) {
-                mma16816(acc.o[nb][db][0], x0, x1, x2, x3, c0[nb], c1[nb]);
-                mma16816(acc.o[nb][db][1], y0, y1, y2, y3, c0[nb], c1[nb]);
+                mma16816(o[0], x0, x1, x2, x3, c0[nb], c1[nb]);
+                mma16816(o[1], y0, y1, y2, y3, c0[nb], c1[nb]);
+            }
+#pragma unroll
+            for (int xy = 0; xy < 2; ++xy) {
+                acc.o[nb][db][xy][0] = F2(o[xy][0], o[xy][1]);
+                acc.o[nb][db][xy][1] = F2(o[xy][2], o[xy][3]);
             }
         }
     }
@@ -607,7 +628,7 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
 #pragma unroll
             for (int xy = 0; xy < 2; ++xy)
 #pragma unroll
-                for (int c = 0; c < 4; ++c) acc.o[nb][db][xy][c] = 0.0f;
+                for (int h = 0; h < 2; ++h) acc.o[nb][db][xy][h] = F2(0.0f, 0.0f);
         acc.m[nb][0] = acc.m[nb][1] = -INFINITY;
         acc.l[nb][0] = acc.l[nb][1] = 0.0f;
 #pragma unroll
@@ -808,10 +829,8 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
             // per-key scale of V: the largest of the page bounds p * scale_V; one factor for all rows
             float F[S], invF[S];
             if constexpr (S == 1) {
-                float svmax = fmaxf(fabsf(__half2float(*reinterpret_cast<const __half*>(hdr + lane * 8 + 4))),
-                                    fabsf(__half2float(*reinterpret_cast<const __half*>(hdr + (lane + 32) * 8 + 4))));
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) svmax = fmaxf(svmax, __shfl_xor_sync(0xffffffffu, svmax, o));
+                const uint32_t a = *reinterpret_cast<const uint16_t*>(hdr + lane * 8 + 4) & 0x7FFFu, b = *reinterpret_cast<const uint16_t*>(hdr + (lane + 32) * 8 + 4) & 0x7FFFu;
+                const float svmax = __half2float(__ushort_as_half(static_cast<uint16_t>(__reduce_max_sync(0xffffffffu, max(a, b)))));
                 F[0] = svmax > 0.0f ? Sh::kPMax / svmax : 0.0f;
                 invF[0] = svmax * (1.0f / Sh::kPMax);
             } else {
@@ -896,7 +915,11 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
 #pragma unroll
                     for (int grp = 0; grp < kGroups; ++grp)
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) sl[nb][grp][e] = fmaf(static_cast<float>(tot[nb][grp][e]), qi.f[0][nb][e & 1], cst[nb][e & 1]);
+                        for (int j = 0; j < 2; ++j) {  // the keys of m-rows g and g + 8 of one row
+                            const float2 y = fma2(F2(static_cast<float>(tot[nb][grp][j]), static_cast<float>(tot[nb][grp][2 + j])), F2(qi.f[0][nb][j], qi.f[0][nb][j]), F2(cst[nb][j], cst[nb][j])).get();
+                            sl[nb][grp][j] = y.x;
+                            sl[nb][grp][2 + j] = y.y;
+                        }
                 if (need_mask) {  // ... and get weight exactly zero
 #pragma unroll
                     for (int grp = 0; grp < kGroups; ++grp)
@@ -910,13 +933,15 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
                         }
                 }
             }
-            float lp_[NB][2], zp_[S][NB][2];
+            F2 lp_[NB][2], zp_[S][NB][2];  // per row, the keys of m-rows g and g + 8
 #pragma unroll
-            for (int nb = 0; nb < NB; ++nb) {
-                lp_[nb][0] = lp_[nb][1] = 0.0f;
+            for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
-                for (int s = 0; s < S; ++s) zp_[s][nb][0] = zp_[s][nb][1] = 0.0f;
-            }
+                for (int j = 0; j < 2; ++j) {
+                    lp_[nb][j] = F2(0.0f, 0.0f);
+#pragma unroll
+                    for (int s = 0; s < S; ++s) zp_[s][nb][j] = F2(0.0f, 0.0f);
+                }
             const uint8_t* vs = hdr + key_lo * 8 * S + 4 * S;  // V scale rows per key: 2 S other_V, S scales, S zero points
 #pragma unroll
             for (int grp = 0; grp < kGroups; ++grp) {
@@ -933,21 +958,24 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
                 }
 #pragma unroll
                 for (int nb = 0; nb < NB; ++nb) {
-                    float p[4];
+                    F2 p[2];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        p[e] = fast_exp2(sl[nb][grp][e]);
-                        lp_[nb][e & 1] += p[e];
+                    for (int j = 0; j < 2; ++j) {
+                        p[j] = F2(fast_exp2(sl[nb][grp][j]), fast_exp2(sl[nb][grp][2 + j]));
+                        lp_[nb][j] = add2(lp_[nb][j], p[j]);
                     }
 #pragma unroll
                     for (int s = 0; s < S; ++s) {
-                        zp_[s][nb][0] += p[0] * zz0[s] + p[2] * zz1[s];
-                        zp_[s][nb][1] += p[1] * zz0[s] + p[3] * zz1[s];
                         // accumulator layout (m-row g; rows 2t, 2t+1) -> operand layout (row g; m-rows 2t, 2t+1 | 2t+8, 2t+9)
-                        const float sf0 = sc0[s] * F[s], sf1 = sc1[s] * F[s];
+                        const F2 sf = mul2(F2(sc0[s], sc1[s]), F2(F[s], F[s]));
                         uint32_t w[4];
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) w[e] = __float_as_uint(fmaf(p[e], e < 2 ? sf0 : sf1, Sh::kPMagic));
+                        for (int j = 0; j < 2; ++j) {
+                            zp_[s][nb][j] = fma2(p[j], F2(zz0[s], zz1[s]), zp_[s][nb][j]);
+                            const float2 y = fma2(p[j], sf, F2(Sh::kPMagic, Sh::kPMagic)).get();
+                            w[j] = __float_as_uint(y.x);
+                            w[2 + j] = __float_as_uint(y.y);
+                        }
                         const uint32_t y0 = movmatrix_trans(prmt(w[0], w[1], 0x5410)), y1 = movmatrix_trans(prmt(w[2], w[3], 0x5410));
                         bw[s][nb][kDigits - 1][grp] = prmt(y0, y1, 0x6420);
                         bw[s][nb][kDigits - 2][grp] = prmt(y0, y1, 0x7531);
@@ -962,17 +990,19 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
             for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
-                    acc.l[nb][j] = fmaf(lp_[nb][j], wpass[nb][j], acc.l[nb][j]);
+                    const float2 lp2 = lp_[nb][j].get();
+                    acc.l[nb][j] = fmaf(lp2.x + lp2.y, wpass[nb][j], acc.l[nb][j]);
 #pragma unroll
                     for (int s = 0; s < S; ++s) {
+                        const float2 zp2 = zp_[s][nb][j].get();
                         if constexpr (kOther) {  // the zero-point term takes other_V of the tile per dim: it enters the accumulators with the page
-                            float zs = zp_[s][nb][j];
+                            float zs = zp2.x + zp2.y;
                             zs += __shfl_xor_sync(0xffffffffu, zs, 4);
                             zs += __shfl_xor_sync(0xffffffffu, zs, 8);
                             zs += __shfl_xor_sync(0xffffffffu, zs, 16);
                             zfull[s][nb][j] = zs * wpass[nb][j];
                         } else {
-                            acc.z[s][nb][j] = fmaf(zp_[s][nb][j], wpass[nb][j], acc.z[s][nb][j]);
+                            acc.z[s][nb][j] = fmaf(zp2.x + zp2.y, wpass[nb][j], acc.z[s][nb][j]);
                         }
                     }
                 }
@@ -1019,19 +1049,25 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
 #pragma unroll
                 for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
-                    for (int xy = 0; xy < 2; ++xy)
+                    for (int xy = 0; xy < 2; ++xy) {
+                        const float nibble = xy ? 0.0625f : 1.0f;
+                        const F2 w(wq[s][nb][0] * nibble, wq[s][nb][1] * nibble);
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            float v = static_cast<float>((ix[nb][xy][kDigits - 2][c] << 8) + ix[nb][xy][kDigits - 1][c]);
-                            if constexpr (S == 2) v = fmaf(static_cast<float>(ix[nb][xy][kHi][c]), 65536.0f, v);
-                            const float w = xy ? wq[s][nb][c & 1] * 0.0625f : wq[s][nb][c & 1];
-                            if constexpr (kOther) {  // (sum p code scale_V + sum p zp_V) * other_V(dim)
-                                const float tv = fmaf(v, w, zfull[s][nb][c & 1]);
-                                acc.o[nb][db][xy][c] = fmaf(tv, ov[db][xy][c >> 1], acc.o[nb][db][xy][c]);
-                            } else {
-                                acc.o[nb][db][xy][c] = fmaf(v, w, acc.o[nb][db][xy][c]);
+                        for (int h = 0; h < 2; ++h) {  // a dim, rows 2t and 2t + 1
+                            float v[2];
+#pragma unroll
+                            for (int j = 0; j < 2; ++j) {
+                                const int c = 2 * h + j;
+                                v[j] = static_cast<float>((ix[nb][xy][kDigits - 2][c] << 8) + ix[nb][xy][kDigits - 1][c]);
+                                if constexpr (S == 2) v[j] = fmaf(static_cast<float>(ix[nb][xy][kHi][c]), 65536.0f, v[j]);
                             }
+                            F2& o = acc.o[nb][db][xy][h];
+                            if constexpr (kOther)  // (sum p code scale_V + sum p zp_V) * other_V(dim)
+                                o = fma2(fma2(F2(v[0], v[1]), w, F2(zfull[s][nb][0], zfull[s][nb][1])), F2(ov[db][xy][h], ov[db][xy][h]), o);
+                            else
+                                o = fma2(F2(v[0], v[1]), w, o);
                         }
+                    }
             }
         }
         release_chunk(true);
@@ -1070,7 +1106,8 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
 #pragma unroll
             for (int j = 0; j < 2; ++j) {  // row 8 nb + 2t + j, dims 32 db + 4g .. +3
                 float* dst = mbuf + (2 + S) * kRows + (8 * nb + 2 * t + j) * kORow + 32 * db + 4 * g;
-                *reinterpret_cast<float4*>(dst) = make_float4(acc.o[nb][db][0][j], acc.o[nb][db][1][j], acc.o[nb][db][0][2 + j], acc.o[nb][db][1][2 + j]);
+                const float2 a = acc.o[nb][db][0][0].get(), b = acc.o[nb][db][1][0].get(), c = acc.o[nb][db][0][1].get(), d = acc.o[nb][db][1][1].get();
+                *reinterpret_cast<float4*>(dst) = j ? make_float4(a.y, b.y, c.y, d.y) : make_float4(a.x, b.x, c.x, d.x);
             }
     }
     __syncthreads();

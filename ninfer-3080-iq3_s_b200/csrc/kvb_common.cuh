@@ -159,10 +159,11 @@ template <int D> __device__ __forceinline__ void hadamard_warp(float (&v)[D / 32
     constexpr int R = D / 32;
 #pragma unroll
     for (int stride = 1; stride <= 16; stride <<= 1) {
+        const float sign = (lane & stride) == 0 ? 1.0f : -1.0f;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const float peer = __shfl_xor_sync(0xffffffffu, v[r], stride);
-            v[r] = (lane & stride) == 0 ? __fadd_rn(v[r], peer) : __fsub_rn(peer, v[r]);
+            v[r] = __fmaf_rn(v[r], sign, peer);  // v + peer, peer - v above: exactly the sum or the difference, rounded once
         }
     }
 #pragma unroll
