@@ -53,6 +53,7 @@ constexpr int kSlots = 2;           // ring slots per warp: the chunk in work an
 constexpr int kHdrs = 2;            // header buffers per warp (a header lives from the issue of its page's K chunk to the end of the page)
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kMagic = 12582912.0f;   // 1.5 * 2^23: x + kMagic has round(x) in its low mantissa bits (|x| < 2^22)
+constexpr int kShortSplits = 8;     // most splits of a head that are a cluster, see attn_short_kernel
 constexpr int kTabPad = 4;          // the per-dim tables are padded by 4 floats per 32 dims: the 32-dim chunks a warp reads at once fall in different banks
 
 // What depends on the number of 128-dim slices of a head (head_dim 128 or 256).
@@ -108,6 +109,12 @@ template <int S, int W> struct __align__(128) AttnSmem {
     float4 qfrag[2 / S][8 * S][32];  // q' in per-lane fragment order: [row half][8 slice + j][lane] = dims 128 slice + 32t+4j..+3 of row g(+8)
     int row_pos[kRows];
     int poison[2][kRows];    // 256 dims: the row sees a key whose V (in this slice) is not finite
+};
+
+// The partial of a CTA whose cluster merges it (attn_short_kernel), behind the rest.
+template <int S> struct ClusterPart {
+    float o[kRows][Shape<S>::kDim];
+    float m[kRows], l[kRows];
 };
 
 // Per-thread state of the running softmax.  Lane (g, t) owns query rows 8 nb + 2t, 2t+1 of n-block nb and dims
@@ -477,7 +484,8 @@ __device__ __forceinline__ void process_stage_group(Smem& sm, const __half* krow
 // kOther: the cache was written with variance balancing (Sinkhorn iterations > 0): every key carries a factor other_K on
 // its logits and every dim of a tile a factor other_V on its output (reference kvarn128_codec.cuh:331-347); both are 1
 // otherwise and the arithmetic for them is compiled out.
-template <int S, int NB, int W, bool kOther = false>
+// kCluster: the partial stays in shared memory, for the cluster (attn_short_kernel).
+template <int S, int NB, int W, bool kOther = false, bool kCluster = false>
 __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int head, int zb, int64_t pidx) {
     using Sh = Shape<S>;
     constexpr int D = Sh::kDim, kChunkBytes = Sh::kChunk, kHdrV = Sh::kHdrV, kHdrK = Sh::kHdrK, kDigits = Sh::kDigits;
@@ -1131,8 +1139,14 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
             }
         }
         if (S == 2 && sm.poison[d / 128][row] != 0) o.x = o.y = o.z = o.w = __uint_as_float(0x7FC00000u);
-        *reinterpret_cast<float4*>(P.ws_o + (pidx + row) * D + d) = o;
-        if (d == 0) { P.ws_m[pidx + row] = m; P.ws_l[pidx + row] = l; }
+        if constexpr (kCluster) {
+            ClusterPart<S>& part = *reinterpret_cast<ClusterPart<S>*>(smem_raw + sizeof(Smem));
+            *reinterpret_cast<float4*>(&part.o[row][d]) = o;
+            if (d == 0) { part.m[row] = m; part.l[row] = l; }
+        } else {
+            *reinterpret_cast<float4*>(P.ws_o + (pidx + row) * D + d) = o;
+            if (d == 0) { P.ws_m[pidx + row] = m; P.ws_l[pidx + row] = l; }
+        }
     }
 }
 
@@ -1143,6 +1157,76 @@ __global__ void __launch_bounds__(W * 32, 1) attn_kernel(const AttnParams P) {
     const int head = blockIdx.y, zb = blockIdx.z, split = blockIdx.x;
     attn_cta<S, NB, W, kOther>(P, split, head, zb, ((static_cast<int64_t>(head) * gridDim.z + zb) * P.nsplit + split) * kRows);
     if (P.after_append) grid_dependency_wait();  // nobody leaves before the append is over: what waits for this grid finds both done
+}
+
+// Short contexts: the splits of a head (at most 8) are a cluster, which merges its partials through distributed shared memory: no
+// partials in the workspace, no merge kernel.  CTA c of the cluster finishes rows c, c + n, .., a warp each: every split's partial of the
+// row, in the order and with the roundings of the merge kernel, normalised, rotated back, stored.
+template <int S, int NB, bool kOther>
+__global__ void __launch_bounds__(kWarpsWide * 32, 1) attn_short_kernel(const AttnParams P, uint16_t* __restrict__ out) {
+    constexpr int W = kWarpsWide, D = Shape<S>::kDim;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    using Smem = AttnSmem<S, W>;
+    Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
+    ClusterPart<S>& part = *reinterpret_cast<ClusterPart<S>*>(smem_raw + sizeof(Smem));
+    static_assert(sizeof(Smem) % 16 == 0, "alignment");
+    if (!P.after_append) grid_dependency_wait();
+    const int head = blockIdx.y, zb = blockIdx.z, split = blockIdx.x, n = P.nsplit;
+    attn_cta<S, NB, W, kOther, true>(P, split, head, zb, 0);
+    cluster_sync();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, G = P.L.q_heads / P.L.kv_heads;
+    for (int r = split + n * warp; r < 8 * NB; r += n * W) {
+        const int Rr = zb * P.block_rows + r, tq = Rr / G, gq = Rr % G;
+        if (tq >= P.T) continue;
+        float pm[kShortSplits], pl[kShortSplits];
+        float4 v[kShortSplits][S];
+#pragma unroll
+        for (int p = 0; p < kShortSplits; ++p) {
+            pm[p] = -INFINITY;
+            pl[p] = 0.0f;
+#pragma unroll
+            for (int s = 0; s < S; ++s) v[p][s] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (p < n) {
+                pm[p] = cluster_load(cluster_map(&part.m[r], p));
+                pl[p] = cluster_load(cluster_map(&part.l[r], p));
+#pragma unroll
+                for (int s = 0; s < S; ++s) v[p][s] = cluster_load4(cluster_map(&part.o[r][128 * s + 4 * lane], p));
+            }
+        }
+        float m = -INFINITY, l = 0.0f;
+#pragma unroll
+        for (int p = 0; p < kShortSplits; ++p) m = fmaxf(m, pm[p]);
+        float4 acc[S];
+#pragma unroll
+        for (int s = 0; s < S; ++s) acc[s] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (m != -INFINITY) {
+#pragma unroll
+            for (int p = 0; p < kShortSplits; ++p) {
+                const float w = fast_exp2(pm[p] - m);
+                l = __fadd_rn(l, __fmul_rn(w, pl[p]));
+#pragma unroll
+                for (int s = 0; s < S; ++s) {
+                    acc[s].x = __fadd_rn(acc[s].x, __fmul_rn(w, v[p][s].x)); acc[s].y = __fadd_rn(acc[s].y, __fmul_rn(w, v[p][s].y));
+                    acc[s].z = __fadd_rn(acc[s].z, __fmul_rn(w, v[p][s].z)); acc[s].w = __fadd_rn(acc[s].w, __fmul_rn(w, v[p][s].w));
+                }
+            }
+        }
+        const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+        float4* const so = reinterpret_cast<float4*>(sm.ring) + 32 * S * warp;  // every warp of the CTA is past the merge buffer
+#pragma unroll
+        for (int s = 0; s < S; ++s) so[32 * s + lane] = make_float4(acc[s].x * inv, acc[s].y * inv, acc[s].z * inv, acc[s].w * inv);
+        __syncwarp();
+        float o[4 * S];
+#pragma unroll
+        for (int j = 0; j < 4 * S; ++j) o[j] = reinterpret_cast<const float*>(so)[lane + 32 * j];
+        __syncwarp();
+        hadamard_warp<D>(o, lane);
+        uint16_t* const dst = out + (static_cast<int64_t>(tq) * P.L.q_heads + head * G + gq) * D + lane;
+#pragma unroll
+        for (int j = 0; j < 4 * S; ++j) dst[32 * j] = P.L.dtype == KVB_DTYPE_BF16 ? f32_to_out<true>(o[j]) : f32_to_out<false>(o[j]);
+    }
+    if (P.after_append) grid_dependency_wait();  // nobody leaves before the append is over: what waits for this grid finds both done
+    cluster_sync();                              // ... nor before the others have read its partial
 }
 
 // Batched decode: `n` independent sequences (their caches described by device-resident kvb_layer structs, same
@@ -1547,6 +1631,21 @@ cudaError_t launch_reduce(int rows, cudaStream_t stream, const float* ws_m, cons
                         block_rows, dtype, out, part_m, part_l, part_o, push, plan);
 }
 
+// Up to this many keys, and with up to this many clusters, the splits of a head and row block are a cluster (attn_short_kernel).  Beyond
+// the keys, eight CTAs have more than a round of pages; beyond the clusters, they are not all on the GPU at once.  Measured on B200 in
+// graph replay, append and attention, 24 / 4 heads, merge kernel against clusters, us a layer: 300 tokens 9.0 8.5, 1,500 9.6 9.1, 2,500 9.6
+// 9.2, 4,000 9.0 9.4, 6,000 9.9 12.3; 256 dims 1,500 16.0 14.9, 3,000 16.0 16.0, 4,000 15.7 16.2; verify at 1,500 tokens, 4 rows (12
+// clusters) 9.5 9.2, 5 rows (16) 9.6 16.4.  Launched one by one (3 us of the host each), 16 layers at 1,500 tokens take 206 and 164 us.
+constexpr int kShortKeys = 3072, kShortClusters = 12;
+// The same as clusters: the splits of a head and row block.
+template <int S, int NB, bool kOther>
+cudaError_t launch_short(dim3 grid, cudaStream_t stream, const AttnParams& P, uint16_t* out) {
+    constexpr int smem = static_cast<int>(sizeof(AttnSmem<S, kWarpsWide>) + sizeof(ClusterPart<S>));
+    static OncePerDevice opted;
+    if (const cudaError_t e = allow_smem(opted, attn_short_kernel<S, NB, kOther>, smem)) return e;
+    return launch_early_cluster(attn_short_kernel<S, NB, kOther>, grid, dim3(kWarpsWide * 32), smem, static_cast<int>(grid.x), stream, P, out);
+}
+
 // Warps per CTA for a decode call: 8, 12 or 16 (whole warp quartets: an SM hands registers and issue slots out per
 // quartet; 10 or 14 warps measured no faster per warp than 12 or 16).  A warp works on whole pages, so a CTA with n
 // pages needs ceil(n / W) rounds; a round and the fixed part (set-up, merge of the warps) take longer the more warps
@@ -1602,7 +1701,11 @@ int launch_attention(const kvb_layer* layer, const void* q, const int32_t* pos_d
     if (layer->stage == nullptr) return fail(KVB_EINVAL, "%s: layer has no stage buffer", who);
     if (layer->head_dim != 128 && push != nullptr) return fail(KVB_ERANGE, "%s: the sharded decode covers head_dim 128", who);
     const RowPlan plan = plan_rows(kv_len_max, layer->kv_heads, layer->q_heads, layer->head_dim, T, layer->sinkhorn_iters != 0);
-    const int Z = plan.zblocks, nsplit = plan.nsplit;
+    // The output may be stored while others still read q, the positions and, behind an append, its rows?
+    const size_t out_bytes = static_cast<size_t>(T) * layer->q_heads * layer->head_dim * sizeof(uint16_t);
+    const bool clustered = kv_len_max <= kShortKeys && layer->kv_heads * plan.zblocks <= kShortClusters && out != nullptr && part_m == nullptr && push == nullptr &&
+                           stores_beside(span_of(out, out_bytes), span_of(q, out_bytes), span_of(pos_dev, T * sizeof(int32_t)), span_of(total_pos_dev, sizeof(int32_t)));
+    const int Z = plan.zblocks, nsplit = clustered ? std::min(plan.nsplit, kShortSplits) : plan.nsplit;
     const int parts = nsplit;
     AttnParams P;
     P.L = make_view(*layer);
@@ -1619,9 +1722,18 @@ int launch_attention(const kvb_layer* layer, const void* q, const int32_t* pos_d
     P.ws_m = workspace_base(workspace);
     P.ws_l = P.ws_m + rows;
     P.ws_o = P.ws_l + rows;
-    P.after_append = starts_beside(behind, span_of(P.ws_m, rows * (2 + layer->head_dim) * sizeof(float)));
+    P.after_append = starts_beside(behind, clustered ? span_of(out, out_bytes) : span_of(P.ws_m, rows * (2 + layer->head_dim) * sizeof(float)));
     const bool upper = plan.nb == 2;
     const dim3 grid(parts, layer->kv_heads, Z);
+    if (clustered) {
+        uint16_t* const to = static_cast<uint16_t*>(out);
+        const bool other = layer->sinkhorn_iters != 0;
+        const auto launch = layer->head_dim != 128 ? launch_short<2, 1, true>
+                            : upper                ? (other ? launch_short<1, 2, true> : launch_short<1, 2, false>)
+                                                   : (other ? launch_short<1, 1, true> : launch_short<1, 1, false>);
+        KVB_CUDA_OK(launch(grid, stream, P, to));
+        return KVB_OK;
+    }
     if (layer->head_dim != 128) {  // two slices per head: twice the accumulators and the wider integers leave room for 8 warps.  The
         // factors of balanced caches are applied whatever the descriptor says: at this head dim a reader need not know the count
         KVB_CUDA_OK((launch_attn<2, 1, kWarpsWide, true>(grid, stream, P)));
