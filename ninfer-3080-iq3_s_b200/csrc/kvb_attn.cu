@@ -60,10 +60,6 @@ constexpr int kTabPad = 4;          // the per-dim tables are padded by 4 floats
 template <int S> struct Shape {
     static constexpr int kDim = 128 * S;
     static constexpr int kChunk = kPage * 64 * S;  // the K or the V codes of one page
-    // The V codes lie as 1 KB sub-blocks (16 keys at 128 dims, 8 at 256), each shifted 16 bytes further: the eight rows of
-    // every transposing ldmatrix fall in eight different bank groups.
-    static constexpr int kSubs = 4 * S, kSubBytes = 1024 + 16;
-    static constexpr int kSlot = (kChunk + (kSubs - 1) * 16 + 127) / 128 * 128;
     static constexpr int kHdrV = 512 * S, kHdrK = 640 * S, kHdr = kHdrV + kHdrK;  // V scale rows of the page, then the K scale rows
     static constexpr int kBlocks = 4 * S;          // 32-dim blocks
     static constexpr int kTab = kDim + kBlocks * kTabPad;
@@ -77,6 +73,17 @@ template <int S> struct Shape {
     static constexpr int kKeyH = 2 / S;
     static __device__ __forceinline__ int key_lo(int g) { return S == 1 ? 16 * (g >> 1) + (g & 1) : 8 * g; }
     static __device__ __forceinline__ constexpr int key_grp(int grp) { return (8 / S) * (grp >> 1) + (4 / S) * (grp & 1); }
+};
+
+// The V codes of a page in a slot.  With two row blocks a warp as they lie in the page, one copy; else as 1 KB sub-blocks (16 keys at 128
+// dims, 8 at 256), each shifted 16 bytes further: the eight rows of every transposing ldmatrix then fall in eight different bank groups.
+// The copies cost instructions, the conflicts shared-memory cycles, of which a page of 256 dims and warps with one row block (more of
+// them, or less work a page) have fewer to spare.  Measured on B200, us a layer, shifted against plain: 2 rows at 131,072 tokens 35.9 35.1,
+// balanced 2 / 4 / 5 rows at 100,003 33.3 / 55.0 / 55.2 32.7 / 53.5 / 53.6; one row block, 378,944 tokens 45.1 46.3, a batch of 32 278 282; 256 dims,
+// 131,072 tokens 46.3 50.0.
+template <int S, int NB> struct VSlot {
+    static constexpr int kShift = S == 1 && NB == 2 ? 0 : 16, kSubs = kShift ? 4 * S : 1, kSubBytes = Shape<S>::kChunk / kSubs;
+    static constexpr int kBytes = (Shape<S>::kChunk + (kSubs - 1) * kShift + 127) / 128 * 128;
 };
 
 struct AttnParams {
@@ -95,14 +102,14 @@ struct AttnParams {
     float* ws_o;         // [H][Z][nsplit][16][D]
 };
 
-template <int S> struct __align__(128) WarpRing {
-    uint8_t slots[kSlots][Shape<S>::kSlot];
+template <int S, int NB> struct __align__(128) WarpRing {
+    uint8_t slots[kSlots][VSlot<S, NB>::kBytes];
     uint8_t hdr[kHdrs][Shape<S>::kHdr];
     float scale_k[Shape<S>::kTab], zp_k[Shape<S>::kTab];  // per-dim scale / zero point of K for the tile in work: dim d at d + kTabPad * (d / 32)
 };
 
-template <int S, int W> struct __align__(128) AttnSmem {
-    WarpRing<S> ring[W];        // in the end the merge buffer of the warps
+template <int S, int NB, int W> struct __align__(128) AttnSmem {
+    WarpRing<S, NB> ring[W];        // in the end the merge buffer of the warps
     // One per slot: completes when the copies of the chunk in the slot have landed.  Outside the rings: memory that holds an mbarrier
     // must not be used for anything else while it does.
     uint64_t bars[W][kSlots];
@@ -205,8 +212,8 @@ template <int S, int NB> struct QInt {
     float qz[S][NB][2];  // sum_d q'[row][d] * zp_K[d]
 };
 
-template <int S, int NB, typename Smem>
-__device__ __forceinline__ void build_qint(const Smem& sm, const WarpRing<S>& R, int lane, QInt<S, NB>& f) {
+template <int S, int NB, typename Smem, typename Ring>
+__device__ __forceinline__ void build_qint(const Smem& sm, const Ring& R, int lane, QInt<S, NB>& f) {
     constexpr float kQMax = Shape<S>::kQMax;
     const int t = lane & 3;
 #pragma unroll
@@ -269,8 +276,8 @@ __device__ __forceinline__ void build_qint(const Smem& sm, const WarpRing<S>& R,
 // Scale rows of K -> per-dim tables in natural dim order, fp32; lane l converts rows 2l and 2l+1.
 // 128 dims: a page row is 5 halves [scale(2r) scale(2r+1) zp(2r) zp(2r+1) other(r)]: dims 4l .. 4l+3.
 // 256 dims: 10 halves [scale(4r) .. scale(4r+3) zp(4r) .. zp(4r+3) other(r), other(r) of the second slice]: dims 8l .. 8l+7.
-template <int S>
-__device__ __forceinline__ void transpose_k_scale(const uint8_t* kscale_rows, WarpRing<S>& R, int lane) {
+template <int S, typename Ring>
+__device__ __forceinline__ void transpose_k_scale(const uint8_t* kscale_rows, Ring& R, int lane) {
     const uint32_t* w = reinterpret_cast<const uint32_t*>(kscale_rows + 20 * S * lane);
     if constexpr (S == 1) {
         const uint32_t w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3], w4 = w[4];
@@ -492,14 +499,15 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
     constexpr int kWarps = W, kThreads = W * 32;
     constexpr int kGroups = kPage / 16;            // 16-key groups of a page
     constexpr int kORow = D + 4, kWarpFloats = (2 + S) * kRows + kRows * kORow;  // merge buffer of a warp: m, l, z (per slice) per row, then o
-    using Smem = AttnSmem<S, W>;
+    using Smem = AttnSmem<S, NB, W>;
     static_assert(kWarps * kWarpFloats * 4 <= offsetof(Smem, bars), "the merge buffer ends before the barriers");
     extern __shared__ __align__(128) unsigned char smem_raw[];
     Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
     const LayerView& L = P.L;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int G = L.q_heads / L.kv_heads;
-    WarpRing<S>& R = sm.ring[warp];
+    WarpRing<S, NB>& R = sm.ring[warp];
+    using Vs = VSlot<S, NB>;
     uint64_t (&bars)[kSlots] = sm.bars[warp];
     // ---- order of the first memory requests: the few bytes everything waits for (positions, q rows, page table
     //      entries) go out first, then the first chunk of every warp, then -- after the rotation of q -- the rest of
@@ -584,7 +592,7 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
                 const uint8_t* src = vc + static_cast<size_t>(pid) * code_stride;
                 mbar_expect_tx(&bars[slot], kChunkBytes);
 #pragma unroll
-                for (int a = 0; a < Sh::kSubs; ++a) bulk_g2s(dst + a * Sh::kSubBytes, src + a * 1024, 1024, &bars[slot]);
+                for (int a = 0; a < Vs::kSubs; ++a) bulk_g2s(dst + a * (Vs::kSubBytes + Vs::kShift), src + a * Vs::kSubBytes, Vs::kSubBytes, &bars[slot]);
             } else {
                 const int lp = w0 + (n >> 1);
                 const bool with_k = kOther || (lp & 1) == 0 || lp == w0;  // K scale rows: with the first page of a tile this warp reads (their fifth column is other_K of the page's own keys: always, when it is not 1)
@@ -1024,8 +1032,8 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
         {
             // lane L addresses row L & 7 of matrix L >> 3, shifted with its sub-block
             const int vrow = lane & 7, vmat = lane >> 3;
-            const uint8_t* ch = S == 1 ? R.slots[slot] + (16 * (vrow >> 1) + 2 * vmat + (vrow & 1)) * 64 + 16 * (vrow >> 1)
-                                       : R.slots[slot] + (8 * vrow + vmat) * 128 + 16 * vrow;
+            const uint8_t* ch = S == 1 ? R.slots[slot] + (16 * (vrow >> 1) + 2 * vmat + (vrow & 1)) * 64 + Vs::kShift * (vrow >> 1)
+                                       : R.slots[slot] + (8 * vrow + vmat) * 128 + Vs::kShift * vrow;
             // swept one 32-dim block at a time: a quarter of the integer accumulators live (measured 1.6 % faster than two halves)
 #pragma unroll
             for (int db = 0; db < Sh::kBlocks; ++db) {
@@ -1166,7 +1174,7 @@ template <int S, int NB, bool kOther>
 __global__ void __launch_bounds__(kWarpsWide * 32, 1) attn_short_kernel(const AttnParams P, uint16_t* __restrict__ out) {
     constexpr int W = kWarpsWide, D = Shape<S>::kDim;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    using Smem = AttnSmem<S, W>;
+    using Smem = AttnSmem<S, NB, W>;
     Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
     ClusterPart<S>& part = *reinterpret_cast<ClusterPart<S>*>(smem_raw + sizeof(Smem));
     static_assert(sizeof(Smem) % 16 == 0, "alignment");
@@ -1603,7 +1611,7 @@ namespace {
 // One attention launch with W warps per CTA (the opt-in to large dynamic shared memory is made once per device and W).
 template <int S, int NB, int W, bool kOther = false>
 cudaError_t launch_attn(dim3 grid, cudaStream_t stream, const AttnParams& P) {
-    constexpr int smem = static_cast<int>(sizeof(AttnSmem<S, W>));
+    constexpr int smem = static_cast<int>(sizeof(AttnSmem<S, NB, W>));
     static OncePerDevice opted;
     if (const cudaError_t e = allow_smem(opted, attn_kernel<S, NB, W, kOther>, smem)) return e;
     return launch_early(attn_kernel<S, NB, W, kOther>, grid, dim3(W * 32), smem, stream, P);
@@ -1640,7 +1648,7 @@ constexpr int kShortKeys = 3072, kShortClusters = 12;
 // The same as clusters: the splits of a head and row block.
 template <int S, int NB, bool kOther>
 cudaError_t launch_short(dim3 grid, cudaStream_t stream, const AttnParams& P, uint16_t* out) {
-    constexpr int smem = static_cast<int>(sizeof(AttnSmem<S, kWarpsWide>) + sizeof(ClusterPart<S>));
+    constexpr int smem = static_cast<int>(sizeof(AttnSmem<S, NB, kWarpsWide>) + sizeof(ClusterPart<S>));
     static OncePerDevice opted;
     if (const cudaError_t e = allow_smem(opted, attn_short_kernel<S, NB, kOther>, smem)) return e;
     return launch_early_cluster(attn_short_kernel<S, NB, kOther>, grid, dim3(kWarpsWide * 32), smem, static_cast<int>(grid.x), stream, P, out);
@@ -2049,7 +2057,7 @@ extern "C" int kvb_attn_decode_batch(const kvb_layer* layers_dev, int batch, int
     B.ws_m = workspace_base(workspace);
     B.ws_l = B.ws_m + rows;
     B.ws_o = B.ws_l + rows;
-    constexpr int smem = static_cast<int>(sizeof(AttnSmem<1, kWarpsWide>));
+    constexpr int smem = static_cast<int>(sizeof(AttnSmem<1, 1, kWarpsWide>));
     static_assert(kBatchPerSm * (smem + 1024) <= 228 * 1024, "CTAs beside each other");
     static OncePerDevice opted1, opted2;
     KVB_CUDA_OK(allow_smem(opted1, attn_batch_kernel<1, kWarpsWide, kBatchPerSm>, smem));
