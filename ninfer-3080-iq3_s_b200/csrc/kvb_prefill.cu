@@ -12,7 +12,10 @@
 // kSplit false: the streams are two row tiles over the same keys (a de-quantised tile serves 256 rows).  kSplit true: one
 // row tile, the streams take the even and the odd key tiles of the CTA's range.  A stream leaves a partial for the merge kernel, or,
 // where the rows see one key range only, the CTA finishes them (finish_rows).
-// One stream's MMAs run while the other's softmax does.  Sixteen warps de-quantise K and V straight from the planes into
+// One stream's MMAs run while the other's softmax does; each stream has a warp that issues them (one warp for both, which waited for one
+// stream's hand-overs while the other's were due: 8-row verify step of a balanced cache of 100,003 tokens 62.0 us a layer, now 54.4).  With
+// two row tiles a key tile is two parts of 64 keys, each with its own S and P: a stream's MMAs of one part run beside its softmax of the
+// other (with one part and two issuing warps 1,024 tokens over 262,144 took 3.94 ms against 3.54).  Sixteen warps de-quantise K and V straight from the planes into
 // two-stage rings (thread = one key, 64 dims): nibbles -> fp16 with the exact unpack, then one fused multiply-add with the
 // tile's per-dim (K) or the key's (V) fp16 scale and zero point.  Dims inside every group of eight are kept in the order the
 // unpack yields (0,4,1,5,2,6,3,7); Q is written in the same order, so the contraction is unaffected, and what finishes a row
@@ -37,7 +40,8 @@ constexpr int kStreams = 2;
 // How the 28 warps are divided.  Two row tiles: the softmax is the longer part, its rows are cut into two column halves (a
 // warp for each), eight warps de-quantise.  Split keys (a few rows): the de-quantising is, it gets sixteen warps.
 template <bool kSplit> struct Roles {
-    static constexpr int kHalves = kSplit ? 1 : 2;       // softmax warps per 32 rows of a stream, 128 / kHalves columns each
+    static constexpr int kHalves = kSplit ? 1 : 2;       // softmax warps per 32 rows of a stream, that share the columns of S and of O
+    static constexpr int kParts = kSplit ? 1 : 2;        // parts of a key tile, each with its own S, P and hand-overs
     static constexpr int kSoft = 4 * kHalves;            // softmax warps per stream
     static constexpr int kDq = kSplit ? 8 : 4;           // for K, and again for V
     static constexpr int kDqWarp = kStreams * kSoft, kMmaWarp = kDqWarp + 2 * kDq;
@@ -69,11 +73,11 @@ struct __align__(1024) PrefillSmem {
     uint8_t k[2][kTileBytes];
     uint8_t v[2][kTileBytes];
     __half ks[2][D], kz[2][D], vo[2][D];  // per-dim factors by tile parity, in tile dim order
-    uint64_t k_full[2], k_free[2], v_full[2], v_free[2], s_full[kStreams], p_full[kStreams], o_done[kStreams], drain;
+    uint64_t k_full[2], k_free[2], v_full[2], v_free[2], s_full[kStreams][2], p_full[kStreams][2], o_done[kStreams][2], drain[kStreams];  // [2]: part of a tile
     uint32_t tmem_base;
     int bad_tile[kSlotsMeta];
     int row_pos[kStreams][kM];
-    float row_top[kStreams][2][kM];  // maximum of a row's column half, exchanged between its two softmax warps
+    float row_top[kStreams][2][2][kM];  // [part][half]: maximum of a row's columns, exchanged between its two softmax warps
     int abort_flag;
 };
 
@@ -238,8 +242,8 @@ __device__ __forceinline__ void finish_rows(PrefillSmem& sm, const PrefillParams
     constexpr int kFinishThreads = 32 * kStreams * Ro::kSoft;
     const int h = kSplit ? u : half;
     if constexpr (kSplit) {
-        sm.row_top[u][0][row] = seen ? m_run : -INFINITY;
-        sm.row_top[u][1][row] = seen ? l_run : 0.0f;
+        sm.row_top[u][0][0][row] = seen ? m_run : -INFINITY;
+        sm.row_top[u][0][1][row] = seen ? l_run : 0.0f;
     }
     const int m = (kSplit ? mt : mt + u) * kM + row, tq = m / G, gq = m % G;
     uint16_t* const dst = P.out + (static_cast<int64_t>(tq) * P.L.q_heads + head * G + gq) * D + 16 * h;  // dims 16 h .. + 15 of every 32
@@ -256,12 +260,12 @@ __device__ __forceinline__ void finish_rows(PrefillSmem& sm, const PrefillParams
     float w[2] = {0.0f, 0.0f};  // weights of the streams' sums; a stream that saw no key has none
     bool used[2] = {seen, false};
     if constexpr (kSplit) {
-        const float m0 = sm.row_top[0][0][row], m1 = sm.row_top[1][0][row], top = fmaxf(m0, m1);
+        const float m0 = sm.row_top[0][0][0][row], m1 = sm.row_top[1][0][0][row], top = fmaxf(m0, m1);
         used[0] = m0 != -INFINITY;
         used[1] = m1 != -INFINITY;
         if (used[0]) w[0] = fast_exp2(m0 - top);
         if (used[1]) w[1] = fast_exp2(m1 - top);
-        l_run = w[0] * sm.row_top[0][1][row] + w[1] * sm.row_top[1][1][row];
+        l_run = w[0] * sm.row_top[0][0][1][row] + w[1] * sm.row_top[1][0][1][row];
     } else {
         w[0] = 1.0f;
     }
@@ -346,16 +350,19 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
 
     if (warp == kMmaWarp) tc::tmem_alloc(&sm.tmem_base, kTmemCols);
     if (tid == 0) {
+        const int readers = !kSplit && (mt + 1) * kM < P.T * G ? 2 : 1;  // streams that read a tile
         for (int b = 0; b < 2; ++b) {
             mbar_init(&sm.k_full[b], kDqWarps);
             mbar_init(&sm.v_full[b], kDqWarps);
-            mbar_init(&sm.k_free[b], 1);
-            mbar_init(&sm.v_free[b], 1);
-            mbar_init(&sm.s_full[b], 1);
-            mbar_init(&sm.p_full[b], Ro::kSoft);
-            mbar_init(&sm.o_done[b], 1);
+            mbar_init(&sm.k_free[b], readers);
+            mbar_init(&sm.v_free[b], readers);
+            for (int h = 0; h < 2; ++h) {
+                mbar_init(&sm.s_full[b][h], 1);
+                mbar_init(&sm.p_full[b][h], Ro::kSoft);
+                mbar_init(&sm.o_done[b][h], 1);
+            }
+            mbar_init(&sm.drain[b], 1);
         }
-        mbar_init(&sm.drain, 1);
         mbar_fence_init();
         sm.abort_flag = 0;
     }
@@ -416,58 +423,57 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
         if (dt < 32 * kDqWarps) failed = dequant_role<false, kOther, kDqWarps>(sm, L, head, dt, t0, n, kv_total);
         else failed = dequant_role<true, kOther, kDqWarps>(sm, L, head, dt - 32 * kDqWarps, t0, n, kv_total);
     } else if (warp >= kMmaWarp) {
-        // =========================== MMA issue (one warp; the three beside it complete the warpgroup) ===========================
+        // =========================== MMA issue (a warp a stream; the two beside them complete the warpgroup) ===========================
         tc::regs_dec<Ro::kMmaRegs>();
-        if (warp == kMmaWarp) {
-            constexpr uint32_t idesc_qk = tc::idesc_f16(kM, kN, false, false), idesc_pv = tc::idesc_f16(kM, D, false, true);
-            const int steps[kStreams] = {steps_of(0), steps_of(1)};
-            const uint64_t q0 = tc::smem_desc(smem_u32(sm.q[0]), 16, 1024), k0 = tc::smem_desc(smem_u32(sm.k[0]), 16, 1024), v0 = tc::smem_desc(smem_u32(sm.v[0]), 16384, 1024);
-            for (int i = 0; i <= steps[0] && !failed; ++i) {
+        const int u = warp - kMmaWarp;
+        if (u < kStreams) {
+            constexpr int kPart = kN / Ro::kParts;  // keys
+            constexpr uint32_t idesc_qk = tc::idesc_f16(kM, kPart, false, false), idesc_pv = tc::idesc_f16(kM, D, false, true);
+            const int steps = steps_of(u);
+            const uint64_t q0 = tc::smem_desc(smem_u32(sm.q[kSplit ? 0 : u]), 16, 1024), k0 = tc::smem_desc(smem_u32(sm.k[0]), 16, 1024), v0 = tc::smem_desc(smem_u32(sm.v[0]), 16384, 1024);
+            for (int i = 0; i <= steps && steps > 0 && !failed; ++i) {
+                const int jk = kSplit ? 2 * i + u : i, jv = kSplit ? 2 * (i - 1) + u : i - 1;
+                // V of step i - 1 and K of step i are there well before P: waited for first, off the chain P -> PV -> S
+                if (i < steps && !chunk_wait(&sm.k_full[jk & 1], (jk >> 1) & 1, &sm.abort_flag)) { failed = true; break; }
+                if (i > 0 && !chunk_wait(&sm.v_full[jv & 1], (jv >> 1) & 1, &sm.abort_flag)) { failed = true; break; }
 #pragma unroll
-                for (int u = 0; u < kStreams; ++u) {
-                    if (i > steps[u]) continue;
-                    // V of step i - 1 and K of step i are there well before P: waited for first, off the chain P -> PV -> S
-                    if (i < steps[u]) {
-                        const int j = kSplit ? 2 * i + u : i;
-                        if (!chunk_wait(&sm.k_full[j & 1], (j >> 1) & 1, &sm.abort_flag)) { failed = true; break; }
-                    }
+                for (int h = 0; h < Ro::kParts; ++h) {
+                    const uint32_t s = tmem + 128 * u + kPart * h;  // S of the part, then its P
                     if (i > 0) {  // O_u += P V of the stream's step i - 1
-                        const int j = kSplit ? 2 * (i - 1) + u : i - 1;
-                        if (!chunk_wait(&sm.v_full[j & 1], (j >> 1) & 1, &sm.abort_flag) || !chunk_wait(&sm.p_full[u], (i - 1) & 1, &sm.abort_flag)) { failed = true; break; }
+                        if (!chunk_wait(&sm.p_full[u][h], (i - 1) & 1, &sm.abort_flag)) { failed = true; break; }
                         tc::fence_after_sync();
                         if (tc::elect_one()) {
-                            const uint64_t v = tc::desc_at(tc::desc_here(v0), (j & 1) * kTileBytes);
+                            const uint64_t v = tc::desc_at(tc::desc_here(v0), (jv & 1) * kTileBytes + h * (kPart / 16) * 2048);
 #pragma unroll
-                            for (int kk = 0; kk < 8; ++kk)  // 16 keys = 8 columns of P
-                                tc::mma_f16_ts(tmem + kColO + 128 * u, tmem + 128 * u + (Ro::kHalves == 2 && kk >= 4 ? 64 - 32 : 0) + 8 * kk, tc::desc_at(v, kk * 2048), idesc_pv, i > 1 || kk > 0);
-                            tc::commit(&sm.o_done[u]);
-                            if (kSplit || u == 1 || steps[1] == 0) tc::commit(&sm.v_free[j & 1]);
+                            for (int kk = 0; kk < kPart / 16; ++kk)  // 16 keys = 8 columns of P
+                                tc::mma_f16_ts(tmem + kColO + 128 * u, s + 8 * kk, tc::desc_at(v, kk * 2048), idesc_pv, i > 1 || h > 0 || kk > 0);
+                            tc::commit(&sm.o_done[u][h]);
+                            if (h == Ro::kParts - 1) tc::commit(&sm.v_free[jv & 1]);
                         }
                         __syncwarp();
                         // the next S_u is written over this P
-                        if (!chunk_wait(&sm.o_done[u], (i - 1) & 1, &sm.abort_flag)) { failed = true; break; }
+                        if (!chunk_wait(&sm.o_done[u][h], (i - 1) & 1, &sm.abort_flag)) { failed = true; break; }
                     }
-                    if (i < steps[u]) {
-                        const int j = kSplit ? 2 * i + u : i;
+                    if (i < steps) {
                         tc::fence_after_sync();
                         if (tc::elect_one()) {
-                            const uint64_t q = tc::desc_at(tc::desc_here(q0), (kSplit ? 0 : u) * kTileBytes), k = tc::desc_at(tc::desc_here(k0), (j & 1) * kTileBytes);
+                            const uint64_t q = tc::desc_here(q0), k = tc::desc_at(tc::desc_here(k0), (jk & 1) * kTileBytes + h * kPart * 128);
 #pragma unroll
                             for (int kk = 0; kk < 8; ++kk) {
                                 const int o = (kk >> 2) * 16384 + (kk & 3) * 32;
-                                tc::mma_f16_ss(tmem + 128 * u, tc::desc_at(q, o), tc::desc_at(k, o), idesc_qk, kk > 0);
+                                tc::mma_f16_ss(s, tc::desc_at(q, o), tc::desc_at(k, o), idesc_qk, kk > 0);
                             }
-                            tc::commit(&sm.s_full[u]);
-                            if (kSplit || u == 1 || steps[1] == 0) tc::commit(&sm.k_free[j & 1]);
+                            tc::commit(&sm.s_full[u][h]);
+                            if (h == Ro::kParts - 1) tc::commit(&sm.k_free[jk & 1]);
                         }
                         __syncwarp();
                     }
                 }
             }
             if (failed) {  // nothing of this CTA may still run when its tensor memory is given back
-                if (tc::elect_one()) tc::commit(&sm.drain);
+                if (tc::elect_one()) tc::commit(&sm.drain[u]);
                 __syncwarp();
-                mbar_wait_bounded(&sm.drain, 0);
+                mbar_wait_bounded(&sm.drain[u], 0);
             }
         }
     } else {
@@ -475,124 +481,135 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
         tc::regs_inc<Ro::kSoftRegs>();
         const int u = warp / Ro::kSoft, half = (warp % Ro::kSoft) >> 2, row = tid & 127;
         const uint32_t lane_base = static_cast<uint32_t>(32 * (warp & 3)) << 16;
-        constexpr int kCols = kN / Ro::kHalves;  // columns of S (and of O) this warp works on, from column kCols * half
-        // P of a column half lies over the first half of its own columns of S: no warp writes over what another still reads
-        const uint32_t ts = tmem + 128 * u + kCols * half + lane_base, to = tmem + kColO + 128 * u + kCols * half + lane_base;
+        constexpr int kCols = D / Ro::kHalves;                     // columns of O this warp works on, from column kCols * half
+        constexpr int kKeys = kN / Ro::kParts / Ro::kHalves;       // columns of S of a part, from kKeys * half
+        const uint32_t to = tmem + kColO + 128 * u + kCols * half + lane_base;
         const int my_pos = kSplit ? sm.row_pos[0][row] : sm.row_pos[u][row];
         const bool is_row = my_pos != kNoRow, warp_has_rows = __any_sync(0xffffffffu, is_row);
         const int min_pos = __reduce_min_sync(0xffffffffu, is_row ? my_pos : INT_MAX);
         const int steps = steps_of(u);
         float m_run = -INFINITY, l_run = 0.0f;
-        for (int i = 0; i < steps; ++i) {
-            const int j = kSplit ? 2 * i + u : i, base = (t0 + j) * kN + kCols * half;
-            if (!chunk_wait(&sm.s_full[u], i & 1, &sm.abort_flag)) failed = true;
-            // (two warps that share rows leave together: the one that gave up still meets the other at their barrier below)
-            if (failed && (Ro::kHalves == 1 || !warp_has_rows)) break;
-            tc::fence_after_sync();
-            if (warp_has_rows) {
-                const bool bad_tile = sm.bad_tile[j & (kSlotsMeta - 1)] != 0;
-                const bool masked = base + kCols - 1 > min_pos || base + kCols > kv_total || bad_tile;
-                const int lim = bad_tile || !is_row ? -1 : min(my_pos, kv_total - 1) - base;  // last visible of this warp's keys
-                auto mask = [&](uint32_t (&s)[32], int first) {                    // keys the row may not see at -inf
-                    if (masked) {
-#pragma unroll
-                        for (int e = 0; e < 32; ++e)
-                            if (first + e > lim) s[e] = 0xFF800000u;
-                    }
-                };
-                auto top = [&](const uint32_t (&s)[32]) {
-                    float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-                    for (int e = 0; e < 32; ++e) mx[e & 3] = fmaxf(mx[e & 3], __uint_as_float(s[e]));
-                    return fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-                };
-                // A row of S is read twice, 32 columns at a time: for its maximum, and for the exponentials.  What is read last for
-                // the maximum stays in registers and is exponentiated first: P goes over columns already read.
-                uint32_t s0[32], s1[32];
-                float mx;
-                if constexpr (Ro::kHalves == 1) {
-                    tc::tmem_ld32(ts + 64, s0);
-                    tc::tmem_ld32(ts + 96, s1);
-                    tc::tmem_ld_wait();
-                    mask(s0, 64);
-                    mask(s1, 96);
-                    mx = fmaxf(top(s0), top(s1));
-                    tc::tmem_ld32(ts, s0);
-                    tc::tmem_ld32(ts + 32, s1);
-                    tc::tmem_ld_wait();
-                    mask(s0, 0);
-                    mask(s1, 32);
-                    mx = fmaxf(mx, fmaxf(top(s0), top(s1)));
-                } else {
-                    tc::tmem_ld32(ts + 32, s0);
-                    tc::tmem_ld_wait();
-                    mask(s0, 32);
-                    mx = top(s0);
-                    tc::tmem_ld32(ts, s0);
-                    tc::tmem_ld_wait();
-                    mask(s0, 0);
-                    mx = fmaxf(mx, top(s0));
-                    sm.row_top[u][half][row] = mx;
-                    if (named_barrier_or(3 + 4 * u + (warp & 3), 64, failed)) { failed = true; break; }  // the two warps of these 32 rows
-                    mx = fmaxf(mx, sm.row_top[u][half ^ 1][row]);
-                }
-                // The reference point of the row's exponentials follows the running maximum lazily: it moves only when the
-                // maximum has grown by more than 2^kLazy, so P stays below 2^kLazy (exact enough in fp16, whose precision is
-                // relative) and the O accumulator is rescaled a few times per walk instead of at every new maximum.
-                constexpr float kLazy = 8.0f;
-                const bool grown = mx > m_run + kLazy || (m_run == -INFINITY && mx > -INFINITY);
-                const float m_new = grown ? mx : m_run;
-                const float m_use = m_new == -INFINITY ? 0.0f : m_new;
-                const float alpha = grown ? fast_exp2(m_run - m_use) : 1.0f;
-                m_run = m_new;
-                F2 sum[2] = {F2(0.0f, 0.0f), F2(0.0f, 0.0f)};
-                const F2 off(-m_use, -m_use);
-                auto weights = [&](const uint32_t (&s)[32], int c) {  // exponentials of columns 32 c .. -> 16 columns of P
-                    uint32_t pk[16];
-#pragma unroll
-                    for (int e = 0; e < 16; ++e) {
-                        const float2 a = add2(F2(__uint_as_float(s[2 * e]), __uint_as_float(s[2 * e + 1])), off).get();
-                        const float p0 = fast_exp2(a.x), p1 = fast_exp2(a.y);
-                        sum[e & 1] = add2(sum[e & 1], F2(p0, p1));
-                        pk[e] = pack_half2(p0, p1);
-                    }
-                    tc::tmem_st16(ts + 16 * c, pk);
-                };
-                weights(s0, 0);
-                if constexpr (Ro::kHalves == 1) weights(s1, 1);
+        for (int i = 0; i < steps && !failed; ++i) {
+            const int j = kSplit ? 2 * i + u : i;
 #pragma unroll 1
-                for (int c = 2 / Ro::kHalves; c < 4 / Ro::kHalves; ++c) {  // (unrolled, the two loads cost spills)
-                    tc::tmem_ld32(ts + 32 * c, s0);
-                    tc::tmem_ld_wait();
-                    mask(s0, 32 * c);
-                    weights(s0, c);
-                }
-                const float2 sum2 = add2(sum[0], sum[1]).get();
-                l_run = l_run * alpha + (sum2.x + sum2.y);
-                if (i > 0 && __any_sync(0xffffffffu, grown)) {  // P V of step i - 1 completed before S of step i was issued
-#pragma unroll 1
-                    for (int c = 0; c < kCols / 32; ++c) {
-                        uint32_t r[32];
-                        tc::tmem_ld32(to + 32 * c, r);
+            for (int h = 0; h < Ro::kParts; ++h) {
+                const int base = (t0 + j) * kN + (kN / Ro::kParts) * h + kKeys * half;
+                // P of the two warps lies side by side over S of the part, which both have read when they meet
+                const uint32_t ts = tmem + 128 * u + (kN / Ro::kParts) * h + kKeys * half + lane_base, tp = ts - (Ro::kHalves == 2 ? kKeys / 2 * half : 0);
+                if (!chunk_wait(&sm.s_full[u][h], i & 1, &sm.abort_flag)) failed = true;
+                // (two warps that share rows leave together: the one that gave up still meets the other at their barrier below)
+                if (failed && (Ro::kHalves == 1 || !warp_has_rows)) break;
+                tc::fence_after_sync();
+                if (warp_has_rows) {
+                    const bool bad_tile = sm.bad_tile[j & (kSlotsMeta - 1)] != 0;
+                    const bool masked = base + kKeys - 1 > min_pos || base + kKeys > kv_total || bad_tile;
+                    const int lim = bad_tile || !is_row ? -1 : min(my_pos, kv_total - 1) - base;  // last visible of this warp's keys
+                    auto mask = [&](uint32_t (&s)[32], int first) {                    // keys the row may not see at -inf
+                        if (masked) {
+#pragma unroll
+                            for (int e = 0; e < 32; ++e)
+                                if (first + e > lim) s[e] = 0xFF800000u;
+                        }
+                    };
+                    auto top = [&](const uint32_t (&s)[32]) {
+                        float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+                        for (int e = 0; e < 32; ++e) mx[e & 3] = fmaxf(mx[e & 3], __uint_as_float(s[e]));
+                        return fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+                    };
+                    // With split keys a row of S is read twice, 32 columns at a time: for its maximum, and for the exponentials.  What is read
+                    // last for the maximum stays in registers and is exponentiated first: P goes over columns already read.
+                    uint32_t s0[32], s1[Ro::kHalves == 1 ? 32 : 1];
+                    float mx;
+                    if constexpr (Ro::kHalves == 1) {
+                        tc::tmem_ld32(ts + 64, s0);
+                        tc::tmem_ld32(ts + 96, s1);
                         tc::tmem_ld_wait();
-#pragma unroll
-                        for (int e = 0; e < 32; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * alpha);
-                        tc::tmem_st32(to + 32 * c, r);
+                        mask(s0, 64);
+                        mask(s1, 96);
+                        mx = fmaxf(top(s0), top(s1));
+                        tc::tmem_ld32(ts, s0);
+                        tc::tmem_ld32(ts + 32, s1);
+                        tc::tmem_ld_wait();
+                        mask(s0, 0);
+                        mask(s1, 32);
+                        mx = fmaxf(mx, fmaxf(top(s0), top(s1)));
+                    } else {
+                        static_assert(Ro::kHalves == 1 || kKeys == 32, "columns of a warp");
+                        tc::tmem_ld32(ts, s0);
+                        tc::tmem_ld_wait();
+                        mask(s0, 0);
+                        mx = top(s0);
+                        sm.row_top[u][h][half][row] = mx;
+                        if (named_barrier_or(3 + 4 * u + (warp & 3), 64, failed)) { failed = true; break; }  // the two warps of these 32 rows
+                        mx = fmaxf(mx, sm.row_top[u][h][half ^ 1][row]);
                     }
+                    // The reference point of the row's exponentials follows the running maximum lazily: it moves only when the
+                    // maximum has grown by more than 2^kLazy, so P stays below 2^kLazy (exact enough in fp16, whose precision is
+                    // relative) and the O accumulator is rescaled a few times per walk instead of at every new maximum.
+                    constexpr float kLazy = 8.0f;
+                    const bool grown = mx > m_run + kLazy || (m_run == -INFINITY && mx > -INFINITY);
+                    const float m_new = grown ? mx : m_run;
+                    const float m_use = m_new == -INFINITY ? 0.0f : m_new;
+                    const float alpha = grown ? fast_exp2(m_run - m_use) : 1.0f;
+                    m_run = m_new;
+                    F2 sum[2] = {F2(0.0f, 0.0f), F2(0.0f, 0.0f)};
+                    const F2 off(-m_use, -m_use);
+                    auto weights = [&](const uint32_t (&s)[32], int c) {  // exponentials of columns 32 c .. -> 16 columns of P
+                        uint32_t pk[16];
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) {
+                            const float2 a = add2(F2(__uint_as_float(s[2 * e]), __uint_as_float(s[2 * e + 1])), off).get();
+                            const float p0 = fast_exp2(a.x), p1 = fast_exp2(a.y);
+                            sum[e & 1] = add2(sum[e & 1], F2(p0, p1));
+                            pk[e] = pack_half2(p0, p1);
+                        }
+                        tc::tmem_st16(tp + 16 * c, pk);
+                    };
+                    weights(s0, 0);
+                    if constexpr (Ro::kHalves == 1) {
+                        weights(s1, 1);
+#pragma unroll 1
+                        for (int c = 2; c < 4; ++c) {  // (unrolled, the two loads cost spills)
+                            tc::tmem_ld32(ts + 32 * c, s0);
+                            tc::tmem_ld_wait();
+                            mask(s0, 32 * c);
+                            weights(s0, c);
+                        }
+                    }
+                    const float2 sum2 = add2(sum[0], sum[1]).get();
+                    l_run = l_run * alpha + (sum2.x + sum2.y);
+                    if (i + h > 0 && __any_sync(0xffffffffu, grown)) {
+                        // P V of step i - 1 completed before S of step i was issued; that of this step's first part may still run
+                        if (h > 0 && !chunk_wait(&sm.o_done[u][0], i & 1, &sm.abort_flag)) failed = true;
+                        if (Ro::kParts == 2 && h == 0 && !chunk_wait(&sm.o_done[u][1], (i - 1) & 1, &sm.abort_flag)) failed = true;
+                        tc::fence_after_sync();
+#pragma unroll 1
+                        for (int c = 0; c < kCols / 32; ++c) {
+                            uint32_t r[32];
+                            tc::tmem_ld32(to + 32 * c, r);
+                            tc::tmem_ld_wait();
+#pragma unroll
+                            for (int e = 0; e < 32; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * alpha);
+                            tc::tmem_st32(to + 32 * c, r);
+                        }
+                    }
+                    tc::tmem_st_wait();
                 }
-                tc::tmem_st_wait();
+                tc::fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sm.p_full[u][h]);
             }
-            tc::fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.p_full[u]);
         }
         // ---- partial of this (row tile, key range): m (log2 units), l, o in tile dim order
-        if (steps > 0 && !failed && !chunk_wait(&sm.o_done[u], (steps - 1) & 1, &sm.abort_flag)) failed = true;
+#pragma unroll
+        for (int h = 0; h < Ro::kParts; ++h)
+            if (steps > 0 && !failed && !chunk_wait(&sm.o_done[u][h], (steps - 1) & 1, &sm.abort_flag)) failed = true;
         tc::fence_after_sync();
         if constexpr (Ro::kHalves == 2) {  // a row's sum has two halves; a warp that gave up comes here too
-            sm.row_top[u][half][row] = l_run;
+            sm.row_top[u][0][half][row] = l_run;
             named_barrier_sync(3 + 4 * u + (warp & 3), 64);
-            l_run += sm.row_top[u][half ^ 1][row];
+            l_run += sm.row_top[u][0][half ^ 1][row];
         }
         const bool have = steps > 0 && !failed && __any_sync(0xffffffffu, m_run != -INFINITY), seen = have && m_run != -INFINITY;
         if (P.out != nullptr) {
