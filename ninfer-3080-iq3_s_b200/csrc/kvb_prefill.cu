@@ -15,8 +15,8 @@
 // One stream's MMAs run while the other's softmax does; each stream has a warp that issues them (one warp for both, which waited for one
 // stream's hand-overs while the other's were due: 8-row verify step of a balanced cache of 100,003 tokens 62.0 us a layer, now 54.4).  With
 // two row tiles a key tile is two parts of 64 keys, each with its own S and P: a stream's MMAs of one part run beside its softmax of the
-// other (with one part and two issuing warps 1,024 tokens over 262,144 took 3.94 ms against 3.54).  Sixteen warps de-quantise K and V straight from the planes into
-// two-stage rings (thread = one key, 64 dims): nibbles -> fp16 with the exact unpack, then one fused multiply-add with the
+// other (with one part and two issuing warps 1,024 tokens over 262,144 took 3.94 ms against 3.54).  Eight or sixteen warps de-quantise K and V
+// straight from the planes into two-stage rings: nibbles -> fp16 with the exact unpack, then one fused multiply-add with the
 // tile's per-dim (K) or the key's (V) fp16 scale and zero point.  Dims inside every group of eight are kept in the order the
 // unpack yields (0,4,1,5,2,6,3,7); Q is written in the same order, so the contraction is unaffected, and what finishes a row
 // (the merge kernel, finish_rows) puts the output dims back.  Keys of the open tile come un-quantised from the stage.
@@ -73,6 +73,7 @@ struct __align__(1024) PrefillSmem {
     uint8_t k[2][kTileBytes];
     uint8_t v[2][kTileBytes];
     __half ks[2][D], kz[2][D], vo[2][D];  // per-dim factors by tile parity, in tile dim order
+    uint32_t ko[2][kN];                   // other_K of the keys, twice
     uint64_t k_full[2], k_free[2], v_full[2], v_free[2], s_full[kStreams][2], p_full[kStreams][2], o_done[kStreams][2], drain[kStreams];  // [2]: part of a tile
     uint32_t tmem_base;
     int bad_tile[kSlotsMeta];
@@ -98,134 +99,198 @@ __device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
     return r;
 }
 
-// One de-quantising role (kDqWarps warps, thread dt): K or V of the CTA's n tiles t0 .. t0 + n - 1, tile j into ring stage j & 1.
-// `other` (caches written with variance balancing): K is multiplied by the key's other_K, V by the per-dim other_V,
-// reference kvarn128_codec.cuh:331-347; fp16 like the rest of this kernel.
-template <bool kValue, bool kOther, int kDqWarps>
-__device__ __forceinline__ bool dequant_role(PrefillSmem& sm, const LayerView& L, int head, int dt, int t0, int n, int kv_total) {
-    // 64 dims of one key per thread with eight warps, all 128 with four; threads 0..127 also fetch the factors of dim dt
-    constexpr int kWords = 64 / kDqWarps;  // 16-byte chunks of the tile row a thread writes
-    const int lane = dt & 31, key = dt & 127, first = kDqWarps == 8 ? 64 * (dt >> 7) : 0;
-    const int32_t* tbl = L.table();
-    const uint8_t* const plane = kValue ? L.v_code : L.k_code;
-    const int sealed_tiles = kv_total / kN;
-    constexpr bool kTables = !kValue || kOther;
-    struct Fetch {
-        uint4 code[kWords / 4];
-        __half d0, d1, t0, t1;  // K: scale, zero point of the dim; other_K of the key.  V: other_V of the dim; scale, zero point of the key
-        bool bad;
-    };
-    // where this thread reads in page 0 of this head, and the page strides
-    const uint8_t* const code_at = plane + page_head_offset(64, L.kv_heads, 0, head) + (key & 63) * 64 + first / 2;
-    constexpr int kLead = kValue ? 4 : 5;  // halves per scale row
-    const __half* const scales = (kValue ? L.v_scale : L.k_scale) + page_head_offset(kLead, L.kv_heads, 0, head);
-    const __half* const tok_at = scales + (key & 63) * kLead + (kValue ? 2 : 4);       // V: scale, zero point of the key; K: other_K
-    const __half* const dim_at = scales + ((dt & 127) >> 1) * kLead + (dt & 1);        // V: other_V of the dim; K: its scale, zero point 2 further
-    const int code_stride = 64 * kPage * L.kv_heads, scale_stride = kLead * kPage * L.kv_heads;
-    int32_t ids[2] = {LayerView::kNoEntry, LayerView::kNoEntry};  // table entries of the tile the next fetch asks for, requested a tile earlier
-    auto lookup = [&](int j) {
+// What both de-quantising roles (kDqWarps warps each, thread dt) walk: the CTA's n tiles t0 .. t0 + n - 1, tile j into ring stage j & 1.
+// Table entries are requested a tile before the fetch that needs them.
+struct TilePages {
+    const LayerView& L;
+    const int32_t* tbl;
+    int t0, n, sealed_tiles;
+    int32_t ids[2];
+    __device__ __forceinline__ TilePages(const LayerView& view, int first, int count, int kv_total)
+        : L(view), tbl(view.table()), t0(first), n(count), sealed_tiles(kv_total / kN), ids{LayerView::kNoEntry, LayerView::kNoEntry} {}
+    __device__ __forceinline__ bool sealed(int j) const { return t0 + j < sealed_tiles; }
+    __device__ __forceinline__ void lookup(int j) {
         ids[0] = ids[1] = LayerView::kNoEntry;
-        if (j < n && t0 + j < sealed_tiles) {
+        if (j < n && sealed(j)) {
             ids[0] = L.page_entry(tbl, 2 * (t0 + j));
             ids[1] = L.page_entry(tbl, 2 * (t0 + j) + 1);
         }
+    }
+};
+
+// K: thread = the 16-byte chunk of eight dims dt % 16 of keys dt / 16, + kStep, ..: its dims' factors stay in registers for a tile, a warp
+// reads the code rows of two keys at once and writes whole swizzled rows, and a store's address is a constant away from the last one's.
+// Bound by its instructions (busy nine tenths of a step of split walks, three quarters with two row tiles).  Measured on B200 against
+// thread = key, which read both factors of every chunk from shared memory: 8 rows at 131,072 tokens 68.4 -> 62.6 us a layer, balanced at
+// 100,003 54.4 -> 53.4, 1,024 tokens over 262,144 alone 3,465 -> 3,325 us.
+// `other` (caches written with variance balancing): K is multiplied by the key's other_K, V by the per-dim other_V, reference
+// kvarn128_codec.cuh:331-347; fp16 like the rest of this kernel.
+template <bool kOther, int kDqWarps>
+__device__ __forceinline__ bool dequant_k(PrefillSmem& sm, const LayerView& L, int head, int dt, int t0, int n, int kv_total) {
+    constexpr int kStep = 2 * kDqWarps, kPer = kN / kStep, kPerPage = kPer / 2;
+    const int lane = dt & 31, chunk = dt & 15, first = dt >> 4;
+    TilePages T(L, t0, n, kv_total);
+    struct Fetch {
+        uint32_t code[kPer];
+        __half d0, d1, t0;  // scale, zero point of dim dt; other_K of key dt
+        bool bad;
     };
+    const uint8_t* const code_at = L.k_code + page_head_offset(64, L.kv_heads, 0, head) + first * 64 + chunk * 4;
+    const __half* const scales = L.k_scale + page_head_offset(5, L.kv_heads, 0, head);
+    const __half* const tok_at = scales + (dt & 63) * 5 + 4;
+    const __half* const dim_at = scales + ((dt & 127) >> 1) * 5 + (dt & 1);
+    const int code_stride = 64 * kPage * L.kv_heads, scale_stride = 5 * kPage * L.kv_heads;
     auto fetch = [&](int j, Fetch& f) {
-        const int32_t pg0 = L.checked_page(ids[0]), pg1 = L.checked_page(ids[1]);
+        const int32_t pg0 = L.checked_page(T.ids[0]), pg1 = L.checked_page(T.ids[1]);
         const bool here = pg0 >= 0 && pg1 >= 0;
-        f.bad = !here && j < n && t0 + j < sealed_tiles;  // reported in the error word; the tile is masked
+        f.bad = !here && j < n && T.sealed(j);  // reported in the error word; the tile is masked
+        f.d0 = f.d1 = f.t0 = __ushort_as_half(0);
+        const uint8_t* src = code_at + static_cast<int64_t>(pg0) * code_stride;
+        const uint8_t* src1 = code_at + static_cast<int64_t>(pg1) * code_stride;
 #pragma unroll
-        for (int c = 0; c < kWords / 4; ++c) f.code[c] = make_uint4(0u, 0u, 0u, 0u);
-        f.d0 = f.d1 = f.t0 = f.t1 = __ushort_as_half(0);
-        if (here) {
-            const int32_t page = key < kPage ? pg0 : pg1;
-            const uint4* src = reinterpret_cast<const uint4*>(code_at + static_cast<int64_t>(page) * code_stride);
-#pragma unroll
-            for (int c = 0; c < kWords / 4; ++c) f.code[c] = src[c];
-            const __half* tok = tok_at + static_cast<int64_t>(page) * scale_stride;
+        for (int i = 0; i < kPer; ++i) f.code[i] = here ? *reinterpret_cast<const uint32_t*>((i < kPerPage ? src : src1) + (i % kPerPage) * kStep * 64) : 0u;
+        if (here && dt < D) {
             const __half* dim = dim_at + static_cast<int64_t>(pg0) * scale_stride;
-            if constexpr (kValue) {
-                const __half2 sz = *reinterpret_cast<const __half2*>(tok);
-                f.t0 = __low2half(sz);
-                f.t1 = __high2half(sz);
-                if (kOther && dt < D) f.d0 = dim[0];
-            } else {
-                if (dt < D) {
-                    f.d0 = dim[0];
-                    f.d1 = dim[2];
-                }
-                if constexpr (kOther) f.t0 = tok[0];
-            }
+            f.d0 = dim[0];
+            f.d1 = dim[2];
+            if constexpr (kOther) f.t0 = *(tok_at + static_cast<int64_t>(dt < kPage ? pg0 : pg1) * scale_stride);
         }
     };
     Fetch cur, nxt;
     if (n > 0) {
-        lookup(0);
+        T.lookup(0);
         fetch(0, nxt);
-        lookup(1);
+        T.lookup(1);
     }
+    // chunk `chunk` of row `first` of a tile; the next row of this thread lies kStep / 8 groups of 1024 bytes further
+    const uint32_t at = tile_off(first, 8 * chunk);
     bool failed = false;
     for (int j = 0; j < n; ++j) {
         const int st = j & 1;
-        const bool sealed = t0 + j < sealed_tiles;
         cur = nxt;
         fetch(j + 1, nxt);
-        lookup(j + 2);
-        if constexpr (kTables) {
-            if (dt < D) {
-                if constexpr (kValue) {
-                    sm.vo[st][dim_slot(dt)] = cur.d0;
-                } else {
-                    sm.ks[st][dim_slot(dt)] = cur.d0;
-                    sm.kz[st][dim_slot(dt)] = cur.d1;
-                }
-            }
-            if (!kValue && dt == 0) sm.bad_tile[j & (kSlotsMeta - 1)] = cur.bad;
-            if (named_barrier_or(kValue ? 2 : 1, 32 * kDqWarps, failed)) return true;
+        T.lookup(j + 2);
+        if (dt < D) {
+            sm.ks[st][dim_slot(dt)] = cur.d0;
+            sm.kz[st][dim_slot(dt)] = cur.d1;
+            if constexpr (kOther) sm.ko[st][dt] = __half_as_ushort(cur.t0) * 0x10001u;
         }
+        if (dt == 0) sm.bad_tile[j & (kSlotsMeta - 1)] = cur.bad;
+        if (named_barrier_or(1, 32 * kDqWarps, failed)) return true;
         // the stage is free once the MMAs of tile j - 2 have completed
-        if (j > 1 && !chunk_wait(kValue ? &sm.v_free[st] : &sm.k_free[st], ((j >> 1) + 1) & 1, &sm.abort_flag)) {
+        if (j > 1 && !chunk_wait(&sm.k_free[st], ((j >> 1) + 1) & 1, &sm.abort_flag)) {
             failed = true;
-            if constexpr (!kTables) return true;
             continue;
         }
-        uint8_t* tile = kValue ? sm.v[st] : sm.k[st];
-        if (sealed) {
-            const uint32_t s2 = __half_as_ushort(cur.t0) * 0x10001u, z2 = __half_as_ushort(cur.t1) * 0x10001u;
+        uint8_t* const dst = sm.k[st] + at;
+        if (T.sealed(j)) {
+            const uint4 sc = *reinterpret_cast<const uint4*>(&sm.ks[st][8 * chunk]), zp = *reinterpret_cast<const uint4*>(&sm.kz[st][8 * chunk]);
 #pragma unroll
-            for (int c = 0; c < kWords; ++c) {
-                const uint4 cc = cur.code[c >> 2];
+            for (int i = 0; i < kPer; ++i) {
                 uint32_t u[4];
-                unpack8((c & 3) == 0 ? cc.x : (c & 3) == 1 ? cc.y : (c & 3) == 2 ? cc.z : cc.w, u);
-                const int at = first + 8 * c;
-                uint4 out;
-                if constexpr (kValue) {
-                    out = make_uint4(hfma2_u32(u[0], s2, z2), hfma2_u32(u[1], s2, z2), hfma2_u32(u[2], s2, z2), hfma2_u32(u[3], s2, z2));
-                    if constexpr (kOther) {
-                        const uint4 ot = *reinterpret_cast<const uint4*>(&sm.vo[st][at]);
-                        out = make_uint4(hmul2_u32(out.x, ot.x), hmul2_u32(out.y, ot.y), hmul2_u32(out.z, ot.z), hmul2_u32(out.w, ot.w));
-                    }
-                } else {
-                    const uint4 sc = *reinterpret_cast<const uint4*>(&sm.ks[st][at]), zp = *reinterpret_cast<const uint4*>(&sm.kz[st][at]);
-                    out = make_uint4(hfma2_u32(u[0], sc.x, zp.x), hfma2_u32(u[1], sc.y, zp.y), hfma2_u32(u[2], sc.z, zp.z), hfma2_u32(u[3], sc.w, zp.w));
-                    if constexpr (kOther) out = make_uint4(hmul2_u32(out.x, s2), hmul2_u32(out.y, s2), hmul2_u32(out.z, s2), hmul2_u32(out.w, s2));
+                unpack8(cur.code[i], u);
+                uint4 out = make_uint4(hfma2_u32(u[0], sc.x, zp.x), hfma2_u32(u[1], sc.y, zp.y), hfma2_u32(u[2], sc.z, zp.z), hfma2_u32(u[3], sc.w, zp.w));
+                if constexpr (kOther) {
+                    const uint32_t o2 = sm.ko[st][first + kStep * i];
+                    out = make_uint4(hmul2_u32(out.x, o2), hmul2_u32(out.y, o2), hmul2_u32(out.z, o2), hmul2_u32(out.w, o2));
                 }
-                *reinterpret_cast<uint4*>(tile + tile_off(key, at)) = out;
+                *reinterpret_cast<uint4*>(dst + i * (kStep / 8) * 1024) = out;
             }
         } else {  // un-quantised fp16 rows of the stage (dims re-ordered inside every group of eight)
             const int t = t0 + j;
-            const uint4* src = reinterpret_cast<const uint4*>(L.stage_row(kValue ? 1 : 0, t & 1, head, key) + first);
-            const bool live = t * kN + key < kv_total;
-#pragma unroll
-            for (int c = 0; c < kWords; ++c) {
-                const uint4 r = live ? src[c] : make_uint4(0u, 0u, 0u, 0u);
-                *reinterpret_cast<uint4*>(tile + tile_off(key, first + 8 * c)) =
+            const __half* src = L.stage_row(0, t & 1, head, first) + 8 * chunk;
+#pragma unroll 4
+            for (int i = 0; i < kPer; ++i) {
+                const uint4 r = t * kN + first + kStep * i < kv_total ? *reinterpret_cast<const uint4*>(src + i * kStep * D) : make_uint4(0u, 0u, 0u, 0u);
+                *reinterpret_cast<uint4*>(dst + i * (kStep / 8) * 1024) =
                     make_uint4(prmt(r.x, r.z, 0x5410), prmt(r.x, r.z, 0x7632), prmt(r.y, r.w, 0x5410), prmt(r.y, r.w, 0x7632));
             }
         }
         fence_proxy_async();
         __syncwarp();
-        if (lane == 0) mbar_arrive(kValue ? &sm.v_full[st] : &sm.k_full[st]);
+        if (lane == 0) mbar_arrive(&sm.k_full[st]);
+    }
+    return failed;
+}
+
+// V: thread = a key (its scale and zero point in registers), 64 dims with eight warps, all 128 with four; threads 0 .. 127 also fetch the
+// factor of dim dt.
+template <bool kOther, int kDqWarps>
+__device__ __forceinline__ bool dequant_v(PrefillSmem& sm, const LayerView& L, int head, int dt, int t0, int n, int kv_total) {
+    constexpr int kWords = 64 / kDqWarps;  // 16-byte chunks of the tile row a thread writes
+    const int lane = dt & 31, key = dt & 127, first = kDqWarps == 8 ? 64 * (dt >> 7) : 0;
+    TilePages T(L, t0, n, kv_total);
+    struct Fetch {
+        uint4 code[kWords / 4];
+        __half d0;    // other_V of the dim
+        uint32_t sz;  // scale, zero point of the key
+    };
+    const uint8_t* const code_at = L.v_code + page_head_offset(64, L.kv_heads, 0, head) + (key & 63) * 64 + first / 2;
+    const __half* const scales = L.v_scale + page_head_offset(4, L.kv_heads, 0, head);
+    const __half* const tok_at = scales + (key & 63) * 4 + 2;
+    const __half* const dim_at = scales + ((dt & 127) >> 1) * 4 + (dt & 1);
+    const int code_stride = 64 * kPage * L.kv_heads, scale_stride = 4 * kPage * L.kv_heads;
+    auto fetch = [&](Fetch& f) {
+        const int32_t pg0 = L.checked_page(T.ids[0]), pg1 = L.checked_page(T.ids[1]), page = key < kPage ? pg0 : pg1;
+        const bool here = pg0 >= 0 && pg1 >= 0;
+        const uint4* src = reinterpret_cast<const uint4*>(code_at + static_cast<int64_t>(page) * code_stride);
+#pragma unroll
+        for (int c = 0; c < kWords / 4; ++c) f.code[c] = here ? src[c] : make_uint4(0u, 0u, 0u, 0u);
+        f.sz = here ? *reinterpret_cast<const uint32_t*>(tok_at + static_cast<int64_t>(page) * scale_stride) : 0u;
+        f.d0 = kOther && here && dt < D ? dim_at[static_cast<int64_t>(pg0) * scale_stride] : __ushort_as_half(0);
+    };
+    Fetch cur, nxt;
+    if (n > 0) {
+        T.lookup(0);
+        fetch(nxt);
+        T.lookup(1);
+    }
+    // row `key` of a tile, its 16-byte chunks exchanged as the 128-byte swizzle has them: chunk c lies at (at ^ 16 (c % 8)) in its block
+    const uint32_t at = (key >> 3) * 1024 + (key & 7) * 128 + ((key & 7) << 4);
+    bool failed = false;
+    for (int j = 0; j < n; ++j) {
+        const int st = j & 1;
+        cur = nxt;
+        fetch(nxt);
+        T.lookup(j + 2);
+        if constexpr (kOther) {
+            if (dt < D) sm.vo[st][dim_slot(dt)] = cur.d0;
+            if (named_barrier_or(2, 32 * kDqWarps, failed)) return true;
+        }
+        if (j > 1 && !chunk_wait(&sm.v_free[st], ((j >> 1) + 1) & 1, &sm.abort_flag)) {
+            failed = true;
+            if constexpr (!kOther) return true;
+            continue;
+        }
+        uint8_t* const tile = sm.v[st] + (first >> 6) * 16384;
+        auto put = [&](int c, uint4 x) { *reinterpret_cast<uint4*>(tile + (c >> 3) * 16384 + (at ^ ((c & 7) << 4))) = x; };
+        if (T.sealed(j)) {
+            const uint32_t s2 = prmt(cur.sz, cur.sz, 0x1010), z2 = prmt(cur.sz, cur.sz, 0x3232);
+#pragma unroll
+            for (int c = 0; c < kWords; ++c) {
+                const uint4 cc = cur.code[c >> 2];
+                uint32_t u[4];
+                unpack8((c & 3) == 0 ? cc.x : (c & 3) == 1 ? cc.y : (c & 3) == 2 ? cc.z : cc.w, u);
+                uint4 out = make_uint4(hfma2_u32(u[0], s2, z2), hfma2_u32(u[1], s2, z2), hfma2_u32(u[2], s2, z2), hfma2_u32(u[3], s2, z2));
+                if constexpr (kOther) {
+                    const uint4 ot = *reinterpret_cast<const uint4*>(&sm.vo[st][first + 8 * c]);
+                    out = make_uint4(hmul2_u32(out.x, ot.x), hmul2_u32(out.y, ot.y), hmul2_u32(out.z, ot.z), hmul2_u32(out.w, ot.w));
+                }
+                put(c, out);
+            }
+        } else {
+            const int t = t0 + j;
+            const uint4* src = reinterpret_cast<const uint4*>(L.stage_row(1, t & 1, head, key) + first);
+            const bool live = t * kN + key < kv_total;
+#pragma unroll
+            for (int c = 0; c < kWords; ++c) {
+                const uint4 r = live ? src[c] : make_uint4(0u, 0u, 0u, 0u);
+                put(c, make_uint4(prmt(r.x, r.z, 0x5410), prmt(r.x, r.z, 0x7632), prmt(r.y, r.w, 0x5410), prmt(r.y, r.w, 0x7632)));
+            }
+        }
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.v_full[st]);
     }
     return failed;
 }
@@ -420,8 +485,8 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
         tc::regs_dec<Ro::kDqRegs>();
         if (P.after_append) grid_dependency_wait();
         const int dt = tid - 32 * kDqWarp;
-        if (dt < 32 * kDqWarps) failed = dequant_role<false, kOther, kDqWarps>(sm, L, head, dt, t0, n, kv_total);
-        else failed = dequant_role<true, kOther, kDqWarps>(sm, L, head, dt - 32 * kDqWarps, t0, n, kv_total);
+        if (dt < 32 * kDqWarps) failed = dequant_k<kOther, kDqWarps>(sm, L, head, dt, t0, n, kv_total);
+        else failed = dequant_v<kOther, kDqWarps>(sm, L, head, dt - 32 * kDqWarps, t0, n, kv_total);
     } else if (warp >= kMmaWarp) {
         // =========================== MMA issue (a warp a stream; the two beside them complete the warpgroup) ===========================
         tc::regs_dec<Ro::kMmaRegs>();
