@@ -207,6 +207,7 @@ __device__ __forceinline__ F2 add2(F2 a, F2 b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
     return r;
 }
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) { return fma2(b, F2(-1.0f, -1.0f), a); }  // exactly a - b, rounded once
 __device__ __forceinline__ F2 mul2(F2 a, F2 b) {
     F2 r;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
