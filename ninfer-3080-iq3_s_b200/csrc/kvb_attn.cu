@@ -1,16 +1,16 @@
 // kvb_attn.cu -- paged split-K attention over the quantised cache for 1..8 query tokens (decode, MTP
-// verify), de-quantisation fused into the QK and PV loops.  head_dim 128 (one 128-dim slice per key) and 256 (two: the
-// template parameter S).
+// verify), de-quantisation fused into the QK and PV loops.  Here for head_dim 128; head_dim 256: kvb_attn_pair.cuh.
 //
 // Grid (splits, kv heads, row blocks).  A CTA owns one KV head, one contiguous range of sealed pages and a block
 // of up to 16 GQA-merged query rows (row = token * G + q head within the KV head); the last split of a head also
 // reads the open tile, whose rows are still un-quantised fp16 in the stage.  Inside a CTA each of the 8, 12 or 16 warps
-// streams its own sub-range of pages through a private ring of two 4 KB slots (8 KB at 256 dims) in shared memory filled
+// streams its own sub-range of pages through a private ring of two 4 KB slots in shared memory filled
 // by bulk async copies (one mbarrier per slot) and never synchronises with another warp until the final merge.  A page
 // arrives as two chunks: its K codes together with a small header (the page's V scale rows; its K scale rows when
-// it is the first page of a tile the warp sees), then its V codes as 1 KB sub-blocks, each shifted 16 bytes
+// it is the first page of a tile the warp sees), then its V codes, with one row block a warp as 1 KB sub-blocks, each shifted 16 bytes
 // further, which makes the transposing ldmatrix reads of the V codes free of bank conflicts.  A slot is refilled
-// as soon as its chunk has been consumed.
+// as soon as its chunk has been consumed.  A CTA leaves one partial per row, which a kernel behind it merges; at short contexts the
+// splits of a head are a cluster and merge their own (attn_short_kernel).
 //
 // Math per page (quantised-domain identities, no per-element de-quantisation), all on the int8 tensor path:
 //   logit[r][j] = sum_d (q'[r][d] * scale_K[d]) * code_K[j][d]  +  sum_d q'[r][d] * zp_K[d]
@@ -26,19 +26,13 @@
 //     enter the running fp32 accumulators with the weight exp2(page max - running max).
 // The page-local reference keeps 16 significant bits below each page's own maximum, whatever the global one is.  What is fp32 runs on
 // packed pairs (two keys of a row, two rows of a dim).  Measured on B200 in graph replay against single values, us a layer: decode at
-// 378,944 tokens 47.1 -> 45.1, verify of 2 / 3 / 4 / 5 rows at 131,072 36.9 / 54.5 / 53.4 / 69.6 -> 36.2 / 52.6 / 51.9 / 67.2, 5 rows of 256 dims
-// at 20,000 40.1 -> 39.6.
-// At head_dim 256 each slice has its own query integers (one scale_K, zp_K table per slice) and weights (scale_V per slice),
-// with a third byte each; the slices meet in the fp32 logits.  Bound by latency, most of it of instructions: eight warps, two a
-// scheduler, run thousands of instructions a page once or twice (a 16 KB page costs about as much as two 8 KB ones).  Measured on
-// B200 in graph replay, 24 / 4 heads, balanced bf16 cache: decode at 30,011 tokens 22.9 us a layer against 178 for one warp per key
-// on fp32 FMAs, a 5-row verify step at 20,000 tokens 40.0 against 486 (no per-element de-quantisation, rows of a KV head share
-// every code read); the look for factors that are not finite is 0.4 and 1.0 us of it.
+// 378,944 tokens 47.1 -> 45.1, verify of 2 / 3 / 4 / 5 rows at 131,072 36.9 / 54.5 / 53.4 / 69.6 -> 36.2 / 52.6 / 51.9 / 67.2.
 #include <algorithm>
 #include <climits>
 #include <cstddef>
 #include <cstdlib>
 #include <functional>
+#include <type_traits>
 
 #include "kvb_common.cuh"
 #include "kvb_ptx.cuh"
@@ -47,7 +41,7 @@ namespace kvb {
 namespace {
 
 constexpr int D = 128;
-constexpr int kWarpsWide = 8;       // ... for 9..16 merged rows (two N blocks per warp), and at head_dim 256: twice the accumulators, 255 registers
+constexpr int kWarpsWide = 8;       // ... for 9..16 merged rows (two N blocks per warp: twice the accumulators, 255 registers)
 constexpr int kRows = 16;           // query rows per CTA: one or two 8-row N blocks
 constexpr int kSlots = 2;           // ring slots per warp: the chunk in work and the next one in flight
 constexpr int kHdrs = 2;            // header buffers per warp (a header lives from the issue of its page's K chunk to the end of the page)
@@ -56,34 +50,28 @@ constexpr float kMagic = 12582912.0f;   // 1.5 * 2^23: x + kMagic has round(x) i
 constexpr int kShortSplits = 8;     // most splits of a head that are a cluster, see attn_short_kernel
 constexpr int kTabPad = 4;          // the per-dim tables are padded by 4 floats per 32 dims: the 32-dim chunks a warp reads at once fall in different banks
 
-// What depends on the number of 128-dim slices of a head (head_dim 128 or 256).
-template <int S> struct Shape {
-    static constexpr int kDim = 128 * S;
-    static constexpr int kChunk = kPage * 64 * S;  // the K or the V codes of one page
-    static constexpr int kHdrV = 512 * S, kHdrK = 640 * S, kHdr = kHdrV + kHdrK;  // V scale rows of the page, then the K scale rows
-    static constexpr int kBlocks = 4 * S;          // 32-dim blocks
-    static constexpr int kTab = kDim + kBlocks * kTabPad;
-    // Bytes of a fixed-point query element or key weight: 16 bits at 128 dims; at 256 dims 22 and 23 bits, as much as the
-    // fp32 sums they enter keep.
-    static constexpr int kDigits = S == 1 ? 2 : 3;
-    static constexpr float kQMax = S == 1 ? 32639.0f : 4194000.0f;  // largest query integer
-    static constexpr float kPMagic = S == 1 ? kMagic : 8388608.0f;  // weights are >= 0: 2^23 leaves 23 bits
-    static constexpr float kPMax = S == 1 ? 65000.0f : 8380000.0f;  // largest weight (a margin below the full range absorbs the rounding of the factor)
+// What a page of a head holds at 128 dims (256: kvb_attn_pair.cuh).
+struct Shape {
+    static constexpr int kChunk = kPage * 64;  // the K or the V codes of one page
+    static constexpr int kHdrV = 512, kHdrK = 640, kHdr = kHdrV + kHdrK;  // V scale rows of the page, then the K scale rows
+    static constexpr int kBlocks = 4;          // 32-dim blocks
+    static constexpr int kTab = D + kBlocks * kTabPad;
+    static constexpr float kQMax = 32639.0f;   // largest query integer: 16 bits
+    static constexpr float kPMax = 65000.0f;   // largest weight, 16 bits (a margin below the full range absorbs the rounding of the factor)
     // Key of m-row g (+ 8: kKeyH further) of 16-key group grp: key_lo(g) + key_grp(grp); see attn_cta.
-    static constexpr int kKeyH = 2 / S;
-    static __device__ __forceinline__ int key_lo(int g) { return S == 1 ? 16 * (g >> 1) + (g & 1) : 8 * g; }
-    static __device__ __forceinline__ constexpr int key_grp(int grp) { return (8 / S) * (grp >> 1) + (4 / S) * (grp & 1); }
+    static constexpr int kKeyH = 2;
+    static __device__ __forceinline__ int key_lo(int g) { return 16 * (g >> 1) + (g & 1); }
+    static __device__ __forceinline__ constexpr int key_grp(int grp) { return 8 * (grp >> 1) + 4 * (grp & 1); }
 };
 
-// The V codes of a page in a slot.  With two row blocks a warp as they lie in the page, one copy; else as 1 KB sub-blocks (16 keys at 128
-// dims, 8 at 256), each shifted 16 bytes further: the eight rows of every transposing ldmatrix then fall in eight different bank groups.
-// The copies cost instructions, the conflicts shared-memory cycles, of which a page of 256 dims and warps with one row block (more of
-// them, or less work a page) have fewer to spare.  Measured on B200, us a layer, shifted against plain: 2 rows at 131,072 tokens 35.9 35.1,
-// balanced 2 / 4 / 5 rows at 100,003 33.3 / 55.0 / 55.2 32.7 / 53.5 / 53.6; one row block, 378,944 tokens 45.1 46.3, a batch of 32 278 282; 256 dims,
-// 131,072 tokens 46.3 50.0.
-template <int S, int NB> struct VSlot {
-    static constexpr int kShift = S == 1 && NB == 2 ? 0 : 16, kSubs = kShift ? 4 * S : 1, kSubBytes = Shape<S>::kChunk / kSubs;
-    static constexpr int kBytes = (Shape<S>::kChunk + (kSubs - 1) * kShift + 127) / 128 * 128;
+// The V codes of a page in a slot.  With two row blocks a warp as they lie in the page, one copy; else as 1 KB sub-blocks of 16 keys, each
+// shifted 16 bytes further: the eight rows of every transposing ldmatrix then fall in eight different bank groups.
+// The copies cost instructions, the conflicts shared-memory cycles, of which warps with one row block (more of them, or less work a
+// page) have fewer to spare.  Measured on B200, us a layer, shifted against plain: 2 rows at 131,072 tokens 35.9 35.1, balanced 2 / 4 / 5 rows at
+// 100,003 33.3 / 55.0 / 55.2 32.7 / 53.5 / 53.6; one row block, 378,944 tokens 45.1 46.3, a batch of 32 278 282.
+template <int NB> struct VSlot {
+    static constexpr int kShift = NB == 2 ? 0 : 16, kSubs = kShift ? 4 : 1, kSubBytes = Shape::kChunk / kSubs;
+    static constexpr int kBytes = (Shape::kChunk + (kSubs - 1) * kShift + 127) / 128 * 128;
 };
 
 struct AttnParams {
@@ -102,41 +90,40 @@ struct AttnParams {
     float* ws_o;         // [H][Z][nsplit][16][D]
 };
 
-template <int S, int NB> struct __align__(128) WarpRing {
-    uint8_t slots[kSlots][VSlot<S, NB>::kBytes];
-    uint8_t hdr[kHdrs][Shape<S>::kHdr];
-    float scale_k[Shape<S>::kTab], zp_k[Shape<S>::kTab];  // per-dim scale / zero point of K for the tile in work: dim d at d + kTabPad * (d / 32)
+template <int NB> struct __align__(128) WarpRing {
+    uint8_t slots[kSlots][VSlot<NB>::kBytes];
+    uint8_t hdr[kHdrs][Shape::kHdr];
+    float scale_k[Shape::kTab], zp_k[Shape::kTab];  // per-dim scale / zero point of K for the tile in work: dim d at d + kTabPad * (d / 32)
 };
 
-template <int S, int NB, int W> struct __align__(128) AttnSmem {
-    WarpRing<S, NB> ring[W];        // in the end the merge buffer of the warps
+template <int NB, int W> struct __align__(128) AttnSmem {
+    WarpRing<NB> ring[W];        // in the end the merge buffer of the warps
     // One per slot: completes when the copies of the chunk in the slot have landed.  Outside the rings: memory that holds an mbarrier
     // must not be used for anything else while it does.
     uint64_t bars[W][kSlots];
-    float4 qfrag[2 / S][8 * S][32];  // q' in per-lane fragment order: [row half][8 slice + j][lane] = dims 128 slice + 32t+4j..+3 of row g(+8)
+    float4 qfrag[2][8][32];  // q' in per-lane fragment order: [row half][j][lane] = dims 32t+4j..+3 of row g(+8)
     int row_pos[kRows];
-    int poison[2][kRows];    // 256 dims: the row sees a key whose V (in this slice) is not finite
 };
 
 // The partial of a CTA whose cluster merges it (attn_short_kernel), behind the rest.
-template <int S> struct ClusterPart {
-    float o[kRows][Shape<S>::kDim];
+struct ClusterPart {
+    float o[kRows][D];
     float m[kRows], l[kRows];
 };
 
 // Per-thread state of the running softmax.  Lane (g, t) owns query rows 8 nb + 2t, 2t+1 of n-block nb and dims
-// 32 db + 4g + i (db < 4 S, i < 4):  o[nb][db][xy][c] is dim 32 db + 4g + xy + 2 (c >> 1), row 8 nb + 2t + (c & 1) -- the
-// accumulator layout of the two MMAs per 32-dim block (xy = 0: even dims, 1: odd dims), kept in pairs of rows [c >> 1].  l and z (per slice) are partial
+// 32 db + 4g + i (db, i < 4):  o[nb][db][xy][c] is dim 32 db + 4g + xy + 2 (c >> 1), row 8 nb + 2t + (c & 1) -- the
+// accumulator layout of the two MMAs per 32-dim block (xy = 0: even dims, 1: odd dims), kept in pairs of rows [c >> 1].  l and z are partial
 // over the lane's keys; everything is relative to the running maximum m (log2 units).
-template <int S, int NB> struct Acc {
-    F2 o[NB][4 * S][2][2];
-    float m[NB][2], l[NB][2], z[S][NB][2];
+template <int NB> struct Acc {
+    F2 o[NB][4][2][2];
+    float m[NB][2], l[NB][2], z[NB][2];
 };
 
 // B fragments of (q')^T per n-block and k-block (b0, b1), high and low fp16 parts: the open tile's rows are fp16.
-template <int S, int NB> struct QFrag {
-    uint32_t hi[NB][8 * S][2];
-    uint32_t lo[NB][8 * S][2];
+template <int NB> struct QFrag {
+    uint32_t hi[NB][8][2];
+    uint32_t lo[NB][8][2];
 };
 
 __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {
@@ -178,14 +165,14 @@ __device__ __forceinline__ void imma_uu0(int (&d)[4], uint32_t a0, uint32_t a1, 
 }
 
 // Q-side fragments for the open tile from q' (shared memory, fragment order).  Lane (g, t) prepares row 8 nb + g, dims
-// 128 slice + 32t .. 32t+31 in natural pairs (2e, 2e+1), split into an fp16 high and low part so the product keeps fp32
+// 32t .. 32t+31 in natural pairs (2e, 2e+1), split into an fp16 high and low part so the product keeps fp32
 // accuracy.
-template <int S, int NB, typename Smem>
-__device__ __forceinline__ void build_qfrag(const Smem& sm, int lane, QFrag<S, NB>& f) {
+template <int NB, typename Smem>
+__device__ __forceinline__ void build_qfrag(const Smem& sm, int lane, QFrag<NB>& f) {
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) {
 #pragma unroll
-        for (int j = 0; j < 8 * S; ++j) {
+        for (int j = 0; j < 8; ++j) {
             const float4 qv = sm.qfrag[nb][j][lane];
             const float x[4] = {qv.x, qv.y, qv.z, qv.w};
 #pragma unroll
@@ -199,111 +186,91 @@ __device__ __forceinline__ void build_qfrag(const Smem& sm, int lane, QFrag<S, N
     }
 }
 
-// Integer form of (q' * scale_K)^T for the quantised pages: each row (of a slice) is scaled to integers of kDigits bytes
-// (row scale f = max|.| / kQMax), Qi = 256 hi + lo with hi = Qi >> 8 signed and lo = Qi & 255 unsigned (three bytes at
-// 256 dims), so that the key side can feed its packed code bytes to the int8 tensor path without unpacking nibbles: with
-// L = byte & 0x0F (even dim) and H = byte & 0xF0 (16 x odd dim),
+// Integer form of (q' * scale_K)^T for the quantised pages: each row is scaled to 16-bit integers (row scale
+// f = max|.| / kQMax), Qi = 256 hi + lo with hi = Qi >> 8 signed and lo = Qi & 255 unsigned, so that the key side can feed
+// its packed code bytes to the int8 tensor path without unpacking nibbles: with L = byte & 0x0F (even dim) and
+// H = byte & 0xF0 (16 x odd dim),
 //   sum_d Qi[d] code[d] = sum_b Qi[2b] L_b + (1/16) sum_b Qi[2b+1] H_b.
-// b[slice][nb][kb][part][digit] holds the B fragments (b0, b1) of 32-byte k-block kb: part 0 = even dims, 1 = odd dims;
-// digit 0 = highest (s8), then u8.  The bytes are read straight out of the float kMagic + Qi.
-template <int S, int NB> struct QInt {
-    uint32_t b[S][NB][2][2][Shape<S>::kDigits][2];
-    float f[S][NB][2];   // row scale / 16 of the lane's rows 2t, 2t+1
-    float qz[S][NB][2];  // sum_d q'[row][d] * zp_K[d]
+// b[nb][kb][part][digit] holds the B fragments (b0, b1) of 32-byte k-block kb: part 0 = even dims, 1 = odd dims;
+// digit 0 = high (s8), then u8.  The bytes are read straight out of the float kMagic + Qi.
+template <int NB> struct QInt {
+    uint32_t b[NB][2][2][2][2];
+    float f[NB][2];   // row scale / 16 of the lane's rows 2t, 2t+1
+    float qz[NB][2];  // sum_d q'[row][d] * zp_K[d]
 };
 
-template <int S, int NB, typename Smem, typename Ring>
-__device__ __forceinline__ void build_qint(const Smem& sm, const Ring& R, int lane, QInt<S, NB>& f) {
-    constexpr float kQMax = Shape<S>::kQMax;
+template <int NB, typename Smem, typename Ring>
+__device__ __forceinline__ void build_qint(const Smem& sm, const Ring& R, int lane, QInt<NB>& f) {
+    constexpr float kQMax = Shape::kQMax;
     const int t = lane & 3;
 #pragma unroll
-    for (int s = 0; s < S; ++s) {
+    for (int nb = 0; nb < NB; ++nb) {
+        F2 qs[16], qz2(0.0f, 0.0f);
+        float amax = 0.0f;
 #pragma unroll
-        for (int nb = 0; nb < NB; ++nb) {
-            F2 qs[16], qz2(0.0f, 0.0f);
-            float amax = 0.0f;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float4 qv = sm.qfrag[nb][8 * s + j][lane];
-                const float4 ks = *reinterpret_cast<const float4*>(&R.scale_k[(32 + kTabPad) * (4 * s + t) + 4 * j]);
-                const float4 kz = *reinterpret_cast<const float4*>(&R.zp_k[(32 + kTabPad) * (4 * s + t) + 4 * j]);
-                const F2 q0(qv.x, qv.y), q1(qv.z, qv.w);
-                qs[2 * j] = mul2(q0, F2(ks.x, ks.y));
-                qs[2 * j + 1] = mul2(q1, F2(ks.z, ks.w));
-                qz2 = fma2(q0, F2(kz.x, kz.y), qz2);
-                qz2 = fma2(q1, F2(kz.z, kz.w), qz2);
-                const float2 a = qs[2 * j].get(), b = qs[2 * j + 1].get();
-                amax = fmaxf(fmaxf(amax, fmaxf(fabsf(a.x), fabsf(a.y))), fmaxf(fabsf(b.x), fabsf(b.y)));
-            }
-            float qz = qz2.get().x + qz2.get().y;
-            qz += __shfl_xor_sync(0xffffffffu, qz, 1);
-            qz += __shfl_xor_sync(0xffffffffu, qz, 2);  // every lane of group g now holds qz of row 8 nb + g
-            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-            const float fr = amax > 0.0f ? amax * (1.0f / kQMax) : 1.0f, inv = amax > 0.0f ? kQMax / amax : 0.0f;
-            f.qz[s][nb][0] = __shfl_sync(0xffffffffu, qz, 8 * t);      // row 2t   lives in lanes 4 * (2t) ..
-            f.qz[s][nb][1] = __shfl_sync(0xffffffffu, qz, 8 * t + 4);  // row 2t+1 lives in lanes 4 * (2t+1) ..
-            f.f[s][nb][0] = __shfl_sync(0xffffffffu, fr, 8 * t) * 0.0625f;
-            f.f[s][nb][1] = __shfl_sync(0xffffffffu, fr, 8 * t + 4) * 0.0625f;
-            uint32_t x[32];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {  // low 16 bits (22 at 256 dims): Qi (two's complement)
-                const float2 y = fma2(qs[i], F2(inv, inv), F2(kMagic, kMagic)).get();
-                x[2 * i] = __float_as_uint(y.x);
-                x[2 * i + 1] = __float_as_uint(y.y);
-            }
-#pragma unroll
-            for (int kb = 0; kb < 2; ++kb)
-#pragma unroll
-                for (int part = 0; part < 2; ++part)
-#pragma unroll
-                    for (int r = 0; r < 2; ++r) {  // b0: local dims 16 kb + 2j + part, b1: +8
-                        const int i0 = 16 * kb + 8 * r + part;
-                        const uint32_t t01 = prmt(x[i0], x[i0 + 2], 0x5140), t23 = prmt(x[i0 + 4], x[i0 + 6], 0x5140);  // [lo lo hi hi]
-                        constexpr int kLast = Shape<S>::kDigits - 1;
-                        f.b[s][nb][kb][part][kLast][r] = prmt(t01, t23, 0x5410);
-                        f.b[s][nb][kb][part][kLast - 1][r] = prmt(t01, t23, 0x7632);
-                        if constexpr (S == 2) {  // third byte: 0x40 + (Qi >> 16), made a signed byte (flip bit 6, copy it to bit 7)
-                            const uint32_t h01 = prmt(x[i0], x[i0 + 2], 0x0062), h23 = prmt(x[i0 + 4], x[i0 + 6], 0x0062);
-                            const uint32_t h = prmt(h01, h23, 0x5410) ^ 0x40404040u;
-                            f.b[s][nb][kb][part][0][r] = h | ((h & 0x40404040u) << 1);
-                        }
-                    }
+        for (int j = 0; j < 8; ++j) {
+            const float4 qv = sm.qfrag[nb][j][lane];
+            const float4 ks = *reinterpret_cast<const float4*>(&R.scale_k[(32 + kTabPad) * t + 4 * j]);
+            const float4 kz = *reinterpret_cast<const float4*>(&R.zp_k[(32 + kTabPad) * t + 4 * j]);
+            const F2 q0(qv.x, qv.y), q1(qv.z, qv.w);
+            qs[2 * j] = mul2(q0, F2(ks.x, ks.y));
+            qs[2 * j + 1] = mul2(q1, F2(ks.z, ks.w));
+            qz2 = fma2(q0, F2(kz.x, kz.y), qz2);
+            qz2 = fma2(q1, F2(kz.z, kz.w), qz2);
+            const float2 a = qs[2 * j].get(), b = qs[2 * j + 1].get();
+            amax = fmaxf(fmaxf(amax, fmaxf(fabsf(a.x), fabsf(a.y))), fmaxf(fabsf(b.x), fabsf(b.y)));
         }
+        float qz = qz2.get().x + qz2.get().y;
+        qz += __shfl_xor_sync(0xffffffffu, qz, 1);
+        qz += __shfl_xor_sync(0xffffffffu, qz, 2);  // every lane of group g now holds qz of row 8 nb + g
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+        const float fr = amax > 0.0f ? amax * (1.0f / kQMax) : 1.0f, inv = amax > 0.0f ? kQMax / amax : 0.0f;
+        f.qz[nb][0] = __shfl_sync(0xffffffffu, qz, 8 * t);      // row 2t   lives in lanes 4 * (2t) ..
+        f.qz[nb][1] = __shfl_sync(0xffffffffu, qz, 8 * t + 4);  // row 2t+1 lives in lanes 4 * (2t+1) ..
+        f.f[nb][0] = __shfl_sync(0xffffffffu, fr, 8 * t) * 0.0625f;
+        f.f[nb][1] = __shfl_sync(0xffffffffu, fr, 8 * t + 4) * 0.0625f;
+        uint32_t x[32];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {  // low 16 bits: Qi (two's complement)
+            const float2 y = fma2(qs[i], F2(inv, inv), F2(kMagic, kMagic)).get();
+            x[2 * i] = __float_as_uint(y.x);
+            x[2 * i + 1] = __float_as_uint(y.y);
+        }
+#pragma unroll
+        for (int kb = 0; kb < 2; ++kb)
+#pragma unroll
+            for (int part = 0; part < 2; ++part)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {  // b0: local dims 16 kb + 2j + part, b1: +8
+                    const int i0 = 16 * kb + 8 * r + part;
+                    const uint32_t t01 = prmt(x[i0], x[i0 + 2], 0x5140), t23 = prmt(x[i0 + 4], x[i0 + 6], 0x5140);  // [lo lo hi hi]
+                    f.b[nb][kb][part][1][r] = prmt(t01, t23, 0x5410);
+                    f.b[nb][kb][part][0][r] = prmt(t01, t23, 0x7632);
+                }
     }
 }
 
-// Scale rows of K -> per-dim tables in natural dim order, fp32; lane l converts rows 2l and 2l+1.
-// 128 dims: a page row is 5 halves [scale(2r) scale(2r+1) zp(2r) zp(2r+1) other(r)]: dims 4l .. 4l+3.
-// 256 dims: 10 halves [scale(4r) .. scale(4r+3) zp(4r) .. zp(4r+3) other(r), other(r) of the second slice]: dims 8l .. 8l+7.
-template <int S, typename Ring>
+// Scale rows of K -> per-dim tables in natural dim order, fp32; lane l converts rows 2l and 2l+1.  A page row is 5 halves
+// [scale(2r) scale(2r+1) zp(2r) zp(2r+1) other(r)]: dims 4l .. 4l+3.
+template <typename Ring>
 __device__ __forceinline__ void transpose_k_scale(const uint8_t* kscale_rows, Ring& R, int lane) {
-    const uint32_t* w = reinterpret_cast<const uint32_t*>(kscale_rows + 20 * S * lane);
-    if constexpr (S == 1) {
-        const uint32_t w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3], w4 = w[4];
-        // halves: w0 = s(4l) s(4l+1) | w1 = z(4l) z(4l+1) | w2 = o(2l) s(4l+2) | w3 = s(4l+3) z(4l+2) | w4 = z(4l+3) o(2l+1)
-        const float2 s01 = unpack_half2(w0), s23 = unpack_half2(prmt(w2, w3, 0x5432));
-        const float2 z01 = unpack_half2(w1), z23 = unpack_half2(prmt(w3, w4, 0x5432));
-        *reinterpret_cast<float4*>(&R.scale_k[4 * lane + kTabPad * (lane >> 3)]) = make_float4(s01.x, s01.y, s23.x, s23.y);
-        *reinterpret_cast<float4*>(&R.zp_k[4 * lane + kTabPad * (lane >> 3)]) = make_float4(z01.x, z01.y, z23.x, z23.y);
-    } else {
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const float2 s01 = unpack_half2(w[5 * r]), s23 = unpack_half2(w[5 * r + 1]), z01 = unpack_half2(w[5 * r + 2]), z23 = unpack_half2(w[5 * r + 3]);
-            const int at = 8 * lane + 4 * r + kTabPad * (lane >> 2);
-            *reinterpret_cast<float4*>(&R.scale_k[at]) = make_float4(s01.x, s01.y, s23.x, s23.y);
-            *reinterpret_cast<float4*>(&R.zp_k[at]) = make_float4(z01.x, z01.y, z23.x, z23.y);
-        }
-    }
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(kscale_rows + 20 * lane);
+    const uint32_t w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3], w4 = w[4];
+    // halves: w0 = s(4l) s(4l+1) | w1 = z(4l) z(4l+1) | w2 = o(2l) s(4l+2) | w3 = s(4l+3) z(4l+2) | w4 = z(4l+3) o(2l+1)
+    const float2 s01 = unpack_half2(w0), s23 = unpack_half2(prmt(w2, w3, 0x5432));
+    const float2 z01 = unpack_half2(w1), z23 = unpack_half2(prmt(w3, w4, 0x5432));
+    *reinterpret_cast<float4*>(&R.scale_k[4 * lane + kTabPad * (lane >> 3)]) = make_float4(s01.x, s01.y, s23.x, s23.y);
+    *reinterpret_cast<float4*>(&R.zp_k[4 * lane + kTabPad * (lane >> 3)]) = make_float4(z01.x, z01.y, z23.x, z23.y);
 }
 
 // Running maximum moves to mnew: rescale the accumulators of one row pair.  alpha = exp2(m_old - m_new).
-template <int S, int NB>
-__device__ __forceinline__ void rescale(Acc<S, NB>& acc, const float (&alpha)[NB][2]) {
+template <int NB>
+__device__ __forceinline__ void rescale(Acc<NB>& acc, const float (&alpha)[NB][2]) {
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) {
 #pragma unroll
-        for (int db = 0; db < 4 * S; ++db)
+        for (int db = 0; db < 4; ++db)
 #pragma unroll
             for (int xy = 0; xy < 2; ++xy)
 #pragma unroll
@@ -311,69 +278,16 @@ __device__ __forceinline__ void rescale(Acc<S, NB>& acc, const float (&alpha)[NB
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             acc.l[nb][j] *= alpha[nb][j];
-#pragma unroll
-            for (int s = 0; s < S; ++s) acc.z[s][nb][j] *= alpha[nb][j];
+            acc.z[nb][j] *= alpha[nb][j];
         }
     }
-}
-
-// Values that are not finite (head_dim 256).  A weight of zero does not keep an infinite V away from the rows that may not see its
-// key: V enters the products clamped to finite values, and the rows that do see such a key are marked and end as NaN.
-__device__ __forceinline__ bool nonfinite_half2(uint32_t w) { return (((w & 0x7C007C00u) + 0x04000400u) & 0x80008000u) != 0u; }
-__device__ __forceinline__ uint32_t finite_half2(uint32_t w) {  // the same bits, or +-65504 in the place of an infinity or a NaN
-    asm("max.f16x2 %0, %0, %1;" : "+r"(w) : "r"(0xFBFFFBFFu));
-    asm("min.f16x2 %0, %0, %1;" : "+r"(w) : "r"(0x7BFF7BFFu));
-    return w;
-}
-// Marks the rows that see one of the keys first + i, bit i of `keys`, i < 64.
-__device__ __forceinline__ void poison_rows(int* poison, const int* row_pos, int lane, uint64_t keys, int first, int key_begin, int key_end) {
-    if (lane >= kRows) return;
-    const int lo = max(key_begin - first, 0), hi = min(min(key_end - 1, row_pos[lane]) - first, 63);
-    if (lo <= hi && ((keys >> lo) << (63 - hi + lo)) != 0) poison[lane] = 1;
-}
-// The V scale rows of a page (a key's row: other_V of four dims | its scales | its zero points), some of them not finite: such keys
-// and dims leave the page.  A call: what happens never stays out of the loop's instructions and registers.
-__device__ __noinline__ void sanitize_page(uint4* rows, int (*poison)[kRows], const int* row_pos, int lane, int first, int key_begin, int key_end) {
-    key_end = min(key_end, first + kPage);
-#pragma unroll 1
-    for (int h = 0; h < 2; ++h) {
-        uint4 r = rows[lane + 32 * h];
-        const bool dims = nonfinite_half2(r.x) || nonfinite_half2(r.y);
-        if (dims) r.x = r.y = 0u;
-        for (int s = 0; s < 2; ++s) {
-            const uint32_t keep = s ? 0x0000FFFFu : 0xFFFF0000u;
-            const bool key = nonfinite_half2(r.z & ~keep) || nonfinite_half2(r.w & ~keep);
-            if (key) { r.z &= keep; r.w &= keep; }
-            const uint32_t keys = __ballot_sync(0xffffffffu, key);
-            poison_rows(poison[s], row_pos, lane, static_cast<uint64_t>(keys) << (32 * h), first, key_begin, key_end);
-        }
-        if (__any_sync(0xffffffffu, dims)) poison_rows(poison[h], row_pos, lane, ~0ull, first, key_begin, key_end);  // rows 0 .. 31: dims of slice 0
-        rows[lane + 32 * h] = r;
-    }
-    fence_proxy_async();
-    __syncwarp();
-}
-// The same for 16 V rows of the open tile (256 dims; lanes 0 .. 15 look at slice 0, 16 .. 31 at slice 1).
-__device__ __noinline__ void poison_stage_group(const __half* vrow, int (*poison)[kRows], const int* row_pos, int lane, int first, int kv_total, int key_begin, int key_end) {
-    uint32_t keys[2] = {0u, 0u};
-#pragma unroll 1
-    for (int key = 0; key < 16 && first + key < kv_total; ++key) {
-        const uint4 r = *reinterpret_cast<const uint4*>(vrow + key * 256 + 8 * lane);
-        const uint32_t hit = __ballot_sync(0xffffffffu, nonfinite_half2(r.x) || nonfinite_half2(r.y) || nonfinite_half2(r.z) || nonfinite_half2(r.w));
-        if (hit & 0x0000FFFFu) keys[0] |= 1u << key;
-        if (hit & 0xFFFF0000u) keys[1] |= 1u << key;
-    }
-    for (int s = 0; s < 2; ++s) poison_rows(poison[s], row_pos, lane, keys[s], first, key_begin, key_end);
 }
 
 // 16 keys of the open tile, read un-quantised (fp16, rotated) straight from the stage.
 // krow/vrow point at the first of the 16 stage rows of this head (row stride D halves).
-// At 256 dims the weights enter as an fp16 high and low part, like the query.
-template <int S, int NB, typename Smem>
-__device__ __forceinline__ void process_stage_group(Smem& sm, const __half* krow, const __half* vrow, const QFrag<S, NB>& qf,
-                                                    Acc<S, NB>& acc, int lane, int first_pos, int kv_total,
+template <int NB>
+__device__ __forceinline__ void process_stage_group(const __half* krow, const __half* vrow, const QFrag<NB>& qf, Acc<NB>& acc, int lane, int first_pos, int kv_total,
                                                     const int (&row_lim)[NB][2], int key_begin, int key_end) {
-    constexpr int D = Shape<S>::kDim;
     const int g = lane >> 2, t = lane & 3;
     float s[NB][4];
     {
@@ -382,9 +296,8 @@ __device__ __forceinline__ void process_stage_group(Smem& sm, const __half* krow
 #pragma unroll
         for (int nb = 0; nb < NB; ++nb) s[nb][0] = s[nb][1] = s[nb][2] = s[nb][3] = 0.0f;
 #pragma unroll
-        for (int i = 0; i < 4 * S; ++i) {
-            const int at = 128 * (i >> 2) + 8 * (i & 3);
-            const uint4 a = *reinterpret_cast<const uint4*>(ka + at), b = *reinterpret_cast<const uint4*>(kb + at);
+        for (int i = 0; i < 4; ++i) {
+            const uint4 a = *reinterpret_cast<const uint4*>(ka + 8 * i), b = *reinterpret_cast<const uint4*>(kb + 8 * i);
 #pragma unroll
             for (int nb = 0; nb < NB; ++nb) {
                 mma16816(s[nb], a.x, b.x, a.y, b.y, qf.hi[nb][2 * i][0], qf.hi[nb][2 * i][1]);
@@ -420,8 +333,8 @@ __device__ __forceinline__ void process_stage_group(Smem& sm, const __half* krow
             acc.m[nb][j] = mnew;
         }
     }
-    if (__any_sync(0xffffffffu, moved)) rescale<S, NB>(acc, alpha);
-    uint32_t b0[NB], b1[NB], c0[NB], c1[NB];
+    if (__any_sync(0xffffffffu, moved)) rescale<NB>(acc, alpha);
+    uint32_t b0[NB], b1[NB];
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) {
 #pragma unroll
@@ -431,28 +344,17 @@ __device__ __forceinline__ void process_stage_group(Smem& sm, const __half* krow
         }
         b0[nb] = movmatrix_trans(pack_half2(s[nb][0], s[nb][1]));  // -> (row g; keys 2t, 2t+1)
         b1[nb] = movmatrix_trans(pack_half2(s[nb][2], s[nb][3]));  // -> (row g; keys 2t+8, 2t+9)
-        if constexpr (S == 2) {
-            const float2 h0 = unpack_half2(pack_half2(s[nb][0], s[nb][1])), h1 = unpack_half2(pack_half2(s[nb][2], s[nb][3]));
-            c0[nb] = movmatrix_trans(pack_half2(s[nb][0] - h0.x, s[nb][1] - h0.y));
-            c1[nb] = movmatrix_trans(pack_half2(s[nb][2] - h1.x, s[nb][3] - h1.y));
-        }
     }
     // A = V^T: the lane supplies dims 32 db + 4g .. +3 of keys 2t, 2t+1, 2t+8, 2t+9.  Keys at or beyond kv_total hold
-    // stale rows: their p is exactly 0; zero V there so 0 * inf cannot appear.  (At 256 dims V is clamped: see finite_half2.)
-    uint32_t odd = 0;
+    // stale rows: their p is exactly 0; zero V there so 0 * inf cannot appear.
 #pragma unroll
-    for (int db = 0; db < 4 * S; ++db) {
+    for (int db = 0; db < 4; ++db) {
         uint2 v[4];
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
             const int key = 2 * t + (kk & 1) + (kk >> 1) * 8;
             const bool live = first_pos + key < kv_total;
             v[kk] = live ? *reinterpret_cast<const uint2*>(vrow + key * D + 32 * db + 4 * g) : make_uint2(0u, 0u);
-            if constexpr (S == 2) {
-                const uint2 f = make_uint2(finite_half2(v[kk].x), finite_half2(v[kk].y));
-                odd |= (f.x ^ v[kk].x) | (f.y ^ v[kk].y);
-                v[kk] = f;
-            }
         }
         const uint32_t x0 = prmt(v[0].x, v[1].x, 0x5410), x1 = prmt(v[0].y, v[1].y, 0x5410);  // dims 4g, 4g+2 of keys 2t, 2t+1
         const uint32_t x2 = prmt(v[2].x, v[3].x, 0x5410), x3 = prmt(v[2].y, v[3].y, 0x5410);  // ... of keys 2t+8, 2t+9
@@ -468,19 +370,12 @@ __device__ __forceinline__ void process_stage_group(Smem& sm, const __half* krow
             }
             mma16816(o[0], x0, x1, x2, x3, b0[nb], b1[nb]);
             mma16816(o[1], y0, y1, y2, y3, b0[nb], b1[nb]);
-            if constexpr (S == 2) {
-                mma16816(o[0], x0, x1, x2, x3, c0[nb], c1[nb]);
-                mma16816(o[1], y0, y1, y2, y3, c0[nb], c1[nb]);
-            }
 #pragma unroll
             for (int xy = 0; xy < 2; ++xy) {
                 acc.o[nb][db][xy][0] = F2(o[xy][0], o[xy][1]);
                 acc.o[nb][db][xy][1] = F2(o[xy][2], o[xy][3]);
             }
         }
-    }
-    if constexpr (S == 2) {
-        if (__any_sync(0xffffffffu, odd != 0u)) poison_stage_group(vrow, sm.poison, sm.row_pos, lane, first_pos, kv_total, key_begin, key_end);
     }
 }
 
@@ -492,33 +387,33 @@ __device__ __forceinline__ void process_stage_group(Smem& sm, const __half* krow
 // its logits and every dim of a tile a factor other_V on its output (reference kvarn128_codec.cuh:331-347); both are 1
 // otherwise and the arithmetic for them is compiled out.
 // kCluster: the partial stays in shared memory, for the cluster (attn_short_kernel).
-template <int S, int NB, int W, bool kOther = false, bool kCluster = false>
+template <int NB, int W, bool kOther = false, bool kCluster = false>
 __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int head, int zb, int64_t pidx) {
-    using Sh = Shape<S>;
-    constexpr int D = Sh::kDim, kChunkBytes = Sh::kChunk, kHdrV = Sh::kHdrV, kHdrK = Sh::kHdrK, kDigits = Sh::kDigits;
+    using Sh = Shape;
+    constexpr int kChunkBytes = Sh::kChunk, kHdrV = Sh::kHdrV, kHdrK = Sh::kHdrK;
     constexpr int kWarps = W, kThreads = W * 32;
     constexpr int kGroups = kPage / 16;            // 16-key groups of a page
-    constexpr int kORow = D + 4, kWarpFloats = (2 + S) * kRows + kRows * kORow;  // merge buffer of a warp: m, l, z (per slice) per row, then o
-    using Smem = AttnSmem<S, NB, W>;
+    constexpr int kORow = D + 4, kWarpFloats = 3 * kRows + kRows * kORow;  // merge buffer of a warp: m, l, z per row, then o
+    using Smem = AttnSmem<NB, W>;
     static_assert(kWarps * kWarpFloats * 4 <= offsetof(Smem, bars), "the merge buffer ends before the barriers");
     extern __shared__ __align__(128) unsigned char smem_raw[];
     Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
     const LayerView& L = P.L;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int G = L.q_heads / L.kv_heads;
-    WarpRing<S, NB>& R = sm.ring[warp];
-    using Vs = VSlot<S, NB>;
+    WarpRing<NB>& R = sm.ring[warp];
+    using Vs = VSlot<NB>;
     uint64_t (&bars)[kSlots] = sm.bars[warp];
     // ---- order of the first memory requests: the few bytes everything waits for (positions, q rows, page table
     //      entries) go out first, then the first chunk of every warp, then -- after the rotation of q -- the rest of
     //      the ring.
     constexpr int kQIter = (8 * NB + W - 1) / W;  // warp w prepares rows w, w + W, ... of the block
-    uint16_t qraw[kQIter][4 * S];
+    uint16_t qraw[kQIter][4];
     int qpos[kQIter];
 #pragma unroll
     for (int i = 0; i < kQIter; ++i) {
 #pragma unroll
-        for (int j = 0; j < 4 * S; ++j) qraw[i][j] = 0;
+        for (int j = 0; j < 4; ++j) qraw[i][j] = 0;
         qpos[i] = INT_MAX;  // no such row: never masked, never stored
         const int r = warp + W * i;
         if (r < 8 * NB) {
@@ -526,7 +421,7 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
             if (tq < P.T) {
                 const uint16_t* qrow = P.q + (static_cast<int64_t>(tq) * L.q_heads + head * G + gq) * D;
 #pragma unroll
-                for (int j = 0; j < 4 * S; ++j) qraw[i][j] = qrow[lane + 32 * j];
+                for (int j = 0; j < 4; ++j) qraw[i][j] = qrow[lane + 32 * j];
                 qpos[i] = P.pos[tq];
             }
         }
@@ -535,7 +430,6 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
     const int key_end = min(P.key_end, kv_total), key_begin = max(P.key_begin, 0);
     const int sealed_pages = 2 * (kv_total / kTile);
 
-    if (S == 2 && threadIdx.x < 2 * kRows) (&sm.poison[0][0])[threadIdx.x] = 0;
     if (lane == 0) {
 #pragma unroll
         for (int s = 0; s < kSlots; ++s) mbar_init(&bars[s], 1);
@@ -611,15 +505,15 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
     for (int i = 0; i < kQIter; ++i) {
         const int r = warp + W * i;
         if (r < 8 * NB) {
-            float v[4 * S];
+            float v[4];
 #pragma unroll
-            for (int j = 0; j < 4 * S; ++j) v[j] = L.dtype == KVB_DTYPE_BF16 ? in_to_f32<true>(qraw[i][j]) : in_to_f32<false>(qraw[i][j]);
+            for (int j = 0; j < 4; ++j) v[j] = L.dtype == KVB_DTYPE_BF16 ? in_to_f32<true>(qraw[i][j]) : in_to_f32<false>(qraw[i][j]);
             hadamard_warp<D>(v, lane);  // rows beyond T are zeros and stay zeros
             if (lane == 0) sm.row_pos[r] = qpos[i];
             float* dst = reinterpret_cast<float*>(sm.qfrag);
 #pragma unroll
-            for (int j = 0; j < 4 * S; ++j)  // dim lane + 32 j -> lane' = (r%8)*4 + (d%128)/32, slot j' = 8 slice + (d%32)/4, component d%4
-                dst[(((r >> 3) * 8 * S + 8 * (j >> 2) + (lane >> 2)) * 32 + (r & 7) * 4 + (j & 3)) * 4 + (lane & 3)] = v[j] * P.scale_log2;
+            for (int j = 0; j < 4; ++j)  // dim lane + 32 j -> lane' = (r%8)*4 + d/32, slot j' = (d%32)/4, component d%4
+                dst[(((r >> 3) * 8 + (lane >> 2)) * 32 + (r & 7) * 4 + j) * 4 + (lane & 3)] = v[j] * P.scale_log2;
         }
     }
     while (n_issued < kSlots && n_issued < nchunks) issue_next(n_issued);
@@ -636,7 +530,7 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
     }
     for (int r = 0; r < 8 * NB; ++r) min_lim = min(min_lim, sm.row_pos[r]);  // (a negative position: a row that sees no key)
 
-    Acc<S, NB> acc;
+    Acc<NB> acc;
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) {
 #pragma unroll
@@ -647,8 +541,7 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
                 for (int h = 0; h < 2; ++h) acc.o[nb][db][xy][h] = F2(0.0f, 0.0f);
         acc.m[nb][0] = acc.m[nb][1] = -INFINITY;
         acc.l[nb][0] = acc.l[nb][1] = 0.0f;
-#pragma unroll
-        for (int s = 0; s < S; ++s) acc.z[s][nb][0] = acc.z[s][nb][1] = 0.0f;
+        acc.z[nb][0] = acc.z[nb][1] = 0.0f;
     }
 
     // ---- open tile (last split of the head): its eight 16-key groups are dealt to the consumer warps, un-quantised,
@@ -658,9 +551,9 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
         for (int grp = warp; grp < 8; grp += W) {
             const int first = base + 16 * grp;
             if (first < key_end && first + 16 > key_begin && first < kv_total) {
-                QFrag<S, NB> qf;
-                build_qfrag<S, NB>(sm, lane, qf);
-                process_stage_group<S, NB>(sm, L.stage_row(0, tile & 1, head, 16 * grp), L.stage_row(1, tile & 1, head, 16 * grp), qf,
+                QFrag<NB> qf;
+                build_qfrag<NB>(sm, lane, qf);
+                process_stage_group<NB>(L.stage_row(0, tile & 1, head, 16 * grp), L.stage_row(1, tile & 1, head, 16 * grp), qf,
                                         acc, lane, first, kv_total, row_lim, key_begin, key_end);
             }
         }
@@ -674,7 +567,7 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
     // a converged warp.  Two forms of the same: a vote on the first probe, which usually succeeds in all lanes, for K; a verdict per lane
     // (a lane that has to keep probing finds the barrier complete as soon as any lane has) and __syncwarp for V.  Measured on B200, us
     // a layer, these / votes for both / __syncwarp for both / neither: decode at 131,072 tokens 21.8 22.0 21.7 21.9, at 378,944 47.1 47.0 47.9 47.0,
-    // 2 rows at 131,072 36.9 36.8 38.5 38.6, 5 rows 69.5 70.1 68.9 69.1, 5 rows of 256 dims at 131,000 174.7 177.2 179.4 178.3.
+    // 2 rows at 131,072 36.9 36.8 38.5 38.6, 5 rows 69.5 70.1 68.9 69.1.
     auto wait_k = [&](int s) {
         if (timed_out) return;
         timed_out = !__all_sync(0xffffffffu, mbar_try_wait(&bars[s], (phases >> s) & 1u)) && !mbar_wait_bounded(&bars[s], (phases >> s) & 1u);
@@ -694,14 +587,13 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
         slot = slot + 1 == kSlots ? 0 : slot + 1;
     };
     // Key order inside a page: m-row i of 16-key group grp (lane g holds rows g and g + 8) is key
-    //   16 ((i & 7) >> 1) + 8 (grp >> 1) + 4 (grp & 1) + 2 (i >> 3) + (i & 1)     at 128 dims,
-    //   8 (i & 7) + 4 (grp >> 1) + 2 (grp & 1) + (i >> 3)                         at 256 dims,
+    //   16 ((i & 7) >> 1) + 8 (grp >> 1) + 4 (grp & 1) + 2 (i >> 3) + (i & 1)
     // so that, after the accumulator -> operand transposition, the weights of a group line up with the keys ldmatrix
     // gathers from the shifted sub-blocks of the V chunk.
     const int key_lo = Sh::key_lo(g);
     constexpr int kKeyH = Sh::kKeyH;
 
-    QInt<S, NB> qi;
+    QInt<NB> qi;
     float ov[Sh::kBlocks][2][2];  // kOther: other_V of dims 32 db + 4g + xy + 2h of the current tile
     int cur_tile = -1;
     for (int pi = 0; pi < npages; ++pi) {
@@ -716,33 +608,18 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
         // ---- K chunk + header
         wait_k(slot);
         const uint8_t* hdr = R.hdr[pi % kHdrs];
-        uint32_t sc = 0;  // 256 dims: the lane's largest scales of V, one slice a half
-        if constexpr (S == 2) {
-            uint4* rows = reinterpret_cast<uint4*>(R.hdr[pi % kHdrs]);
-            constexpr uint32_t kAbs = 0x7FFF7FFFu;
-            auto look = [&]() {  // whether a factor of V is not finite
-                const uint4 a = rows[lane], b = rows[lane + 32];
-                sc = __vmaxu2(a.z & kAbs, b.z & kAbs);
-                const uint32_t all = __vmaxu2(__vmaxu2(__vmaxu2(a.x & kAbs, b.x & kAbs), __vmaxu2(a.y & kAbs, b.y & kAbs)), __vmaxu2(__vmaxu2(a.w & kAbs, b.w & kAbs), sc));
-                return __any_sync(0xffffffffu, nonfinite_half2(all));
-            };
-            if (look()) {
-                sanitize_page(rows, sm.poison, sm.row_pos, lane, lp * kPage, key_begin, key_end);
-                sc = __vmaxu2(rows[lane].z & kAbs, rows[lane + 32].z & kAbs);
-            }
-        }
         if ((lp >> 1) != cur_tile) {  // per-dim scale / zero point of K belong to the tile
             cur_tile = lp >> 1;
             __syncwarp();
-            transpose_k_scale<S>(hdr + kHdrV, R, lane);
+            transpose_k_scale(hdr + kHdrV, R, lane);
             __syncwarp();
-            build_qint<S, NB>(sm, R, lane, qi);
-            if constexpr (kOther) {  // other_V of the lane's dims: V scale row d / (2 S) starts with the other_V of its 2 S dims
+            build_qint<NB>(sm, R, lane, qi);
+            if constexpr (kOther) {  // other_V of the lane's dims: V scale row d / 2 starts with the other_V of its two dims
 #pragma unroll
                 for (int db = 0; db < Sh::kBlocks; ++db)
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        const float2 o2 = unpack_half2(*reinterpret_cast<const uint32_t*>(hdr + (S == 1 ? (16 * db + 2 * g + h) * 8 : (8 * db + g) * 16 + 4 * h)));
+                        const float2 o2 = unpack_half2(*reinterpret_cast<const uint32_t*>(hdr + (16 * db + 2 * g + h) * 8));
                         ov[db][0][h] = o2.x;
                         ov[db][1][h] = o2.y;
                     }
@@ -750,75 +627,45 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
         }
         const int first = lp * kPage;
         const bool need_mask = first + kPage - 1 > min_lim || first < key_begin || first + kPage > key_end;
-        // ---- QK: integer sums of the page.  One slice keeps them as integers (the row maximum is an integer maximum); with
-        //      two slices, each with its own row scale, they become fp32 logits right away.
+        // ---- QK: integer sums of the page
         int tot[NB][kGroups][4];
-        float sl[NB][kGroups][4];  // logits, then logits relative to the page maximum (log2 units)
+        float sl[NB][kGroups][4];  // logits relative to the page maximum (log2 units)
         {
-            const uint8_t* ch = R.slots[slot] + key_lo * 64 * S + 16 * t;
+            const uint8_t* ch = R.slots[slot] + key_lo * 64 + 16 * t;
 #pragma unroll
             for (int grp = 0; grp < kGroups; ++grp) {
-                const int koff = Sh::key_grp(grp) * 64 * S;
+                const int koff = Sh::key_grp(grp) * 64;
+                const uint4 ka = *reinterpret_cast<const uint4*>(ch + koff);
+                const uint4 kb8 = *reinterpret_cast<const uint4*>(ch + koff + kKeyH * 64);
+                const uint32_t wa[4] = {ka.x, ka.y, ka.z, ka.w}, wb[4] = {kb8.x, kb8.y, kb8.z, kb8.w};
+                int ce[NB][2][4], co[NB][2][4];  // even dims, odd dims (x 16)
 #pragma unroll
-                for (int s = 0; s < S; ++s) {
-                    const uint4 ka = *reinterpret_cast<const uint4*>(ch + koff + 64 * s);
-                    const uint4 kb8 = *reinterpret_cast<const uint4*>(ch + koff + kKeyH * 64 * S + 64 * s);
-                    const uint32_t wa[4] = {ka.x, ka.y, ka.z, ka.w}, wb[4] = {kb8.x, kb8.y, kb8.z, kb8.w};
-                    int ce[NB][kDigits][4], co[NB][kDigits][4];  // even dims, odd dims (x 16)
+                for (int kb = 0; kb < 2; ++kb) {
+                    const uint32_t l0 = wa[2 * kb] & 0x0F0F0F0Fu, l1 = wb[2 * kb] & 0x0F0F0F0Fu, l2 = wa[2 * kb + 1] & 0x0F0F0F0Fu,
+                                   l3 = wb[2 * kb + 1] & 0x0F0F0F0Fu;
+                    const uint32_t h0 = wa[2 * kb] & 0xF0F0F0F0u, h1 = wb[2 * kb] & 0xF0F0F0F0u, h2 = wa[2 * kb + 1] & 0xF0F0F0F0u,
+                                   h3 = wb[2 * kb + 1] & 0xF0F0F0F0u;
 #pragma unroll
-                    for (int kb = 0; kb < 2; ++kb) {
-                        const uint32_t l0 = wa[2 * kb] & 0x0F0F0F0Fu, l1 = wb[2 * kb] & 0x0F0F0F0Fu, l2 = wa[2 * kb + 1] & 0x0F0F0F0Fu,
-                                       l3 = wb[2 * kb + 1] & 0x0F0F0F0Fu;
-                        const uint32_t h0 = wa[2 * kb] & 0xF0F0F0F0u, h1 = wb[2 * kb] & 0xF0F0F0F0u, h2 = wa[2 * kb + 1] & 0xF0F0F0F0u,
-                                       h3 = wb[2 * kb + 1] & 0xF0F0F0F0u;
-#pragma unroll
-                        for (int nb = 0; nb < NB; ++nb) {
-#pragma unroll
-                            for (int d = 0; d < kDigits; ++d) {
-                                const uint32_t(&be)[2] = qi.b[s][nb][kb][0][d], (&bo)[2] = qi.b[s][nb][kb][1][d];
-                                if (d == 0) {
-                                    if (kb == 0) {
-                                        imma_us0(ce[nb][d], l0, l1, l2, l3, be[0], be[1]);
-                                        imma_us0(co[nb][d], h0, h1, h2, h3, bo[0], bo[1]);
-                                    } else {
-                                        imma_us(ce[nb][d], l0, l1, l2, l3, be[0], be[1]);
-                                        imma_us(co[nb][d], h0, h1, h2, h3, bo[0], bo[1]);
-                                    }
-                                } else {
-                                    if (kb == 0) {
-                                        imma_uu0(ce[nb][d], l0, l1, l2, l3, be[0], be[1]);
-                                        imma_uu0(co[nb][d], h0, h1, h2, h3, bo[0], bo[1]);
-                                    } else {
-                                        imma_uu(ce[nb][d], l0, l1, l2, l3, be[0], be[1]);
-                                        imma_uu(co[nb][d], h0, h1, h2, h3, bo[0], bo[1]);
-                                    }
-                                }
-                            }
+                    for (int nb = 0; nb < NB; ++nb) {
+                        const uint32_t (&be)[2][2] = qi.b[nb][kb][0], (&bo)[2][2] = qi.b[nb][kb][1];
+                        if (kb == 0) {
+                            imma_us0(ce[nb][0], l0, l1, l2, l3, be[0][0], be[0][1]);
+                            imma_us0(co[nb][0], h0, h1, h2, h3, bo[0][0], bo[0][1]);
+                            imma_uu0(ce[nb][1], l0, l1, l2, l3, be[1][0], be[1][1]);
+                            imma_uu0(co[nb][1], h0, h1, h2, h3, bo[1][0], bo[1][1]);
+                        } else {
+                            imma_us(ce[nb][0], l0, l1, l2, l3, be[0][0], be[0][1]);
+                            imma_us(co[nb][0], h0, h1, h2, h3, bo[0][0], bo[0][1]);
+                            imma_uu(ce[nb][1], l0, l1, l2, l3, be[1][0], be[1][1]);
+                            imma_uu(co[nb][1], h0, h1, h2, h3, bo[1][0], bo[1][1]);
                         }
                     }
-                    float ok[2] = {1.0f, 1.0f};
-                    if constexpr (S == 2 && kOther) {
-#pragma unroll
-                        for (int h = 0; h < 2; ++h)
-                            ok[h] = __half2float(*reinterpret_cast<const __half*>(hdr + kHdrV + (key_lo + Sh::key_grp(grp) + kKeyH * h) * 20 + 16 + 2 * s));
-                    }
-#pragma unroll
-                    for (int nb = 0; nb < NB; ++nb)
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            if constexpr (S == 1) {
-                                // 16 * sum = 256 (16 even_hi + odd_hi) + (16 even_lo + odd_lo); |.| < 2^31
-                                tot[nb][grp][e] = ((ce[nb][0][e] * 16 + co[nb][0][e]) << 8) + (ce[nb][1][e] * 16 + co[nb][1][e]);
-                            } else {
-                                // the two low bytes' sums stay below 2^31 together; the high byte's joins in fp32
-                                const int low = ((ce[nb][1][e] * 16 + co[nb][1][e]) << 8) + (ce[nb][2][e] * 16 + co[nb][2][e]);
-                                const float sum = fmaf(static_cast<float>(ce[nb][0][e] * 16 + co[nb][0][e]), 65536.0f, static_cast<float>(low));
-                                const float x = fmaf(sum, qi.f[s][nb][e & 1], qi.qz[s][nb][e & 1]);
-                                if constexpr (kOther) sl[nb][grp][e] = s == 0 ? x * ok[e >> 1] : fmaf(x, ok[e >> 1], sl[nb][grp][e]);
-                                else sl[nb][grp][e] = s == 0 ? x : sl[nb][grp][e] + x;
-                            }
-                        }
                 }
+#pragma unroll
+                for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)  // 16 * sum = 256 (16 even_hi + odd_hi) + (16 even_lo + odd_lo); |.| < 2^31
+                        tot[nb][grp][e] = ((ce[nb][0][e] * 16 + co[nb][0][e]) << 8) + (ce[nb][1][e] * 16 + co[nb][1][e]);
             }
         }
         release_chunk(true);
@@ -831,32 +678,18 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
                     const bool out = p < key_begin || p >= key_end;
 #pragma unroll
                     for (int nb = 0; nb < NB; ++nb)
-                        if (out || p > row_lim[nb][e & 1]) {
-                            if constexpr (S == 1) tot[nb][grp][e] = INT_MIN;
-                            else sl[nb][grp][e] = -INFINITY;
-                        }
+                        if (out || p > row_lim[nb][e & 1]) tot[nb][grp][e] = INT_MIN;
                 }
         }
         // ---- softmax of the page relative to its own row maxima; weights of the page against the running state
-        float wq[S][NB][2];     // weight of the integer sums of this page in the running accumulators
-        float zfull[S][NB][2];  // kOther: sum over the page's keys of p * zp_V, weighted like the integer sums
-        uint32_t bw[S][NB][kDigits][kGroups];  // weights as B fragments, one byte each: highest digit first
+        float wq[NB][2];     // weight of the integer sums of this page in the running accumulators
+        float zfull[NB][2];  // kOther: sum over the page's keys of p * zp_V, weighted like the integer sums
+        uint32_t bw[NB][2][kGroups];  // weights as B fragments, one byte each: high, low
         {
             // per-key scale of V: the largest of the page bounds p * scale_V; one factor for all rows
-            float F[S], invF[S];
-            if constexpr (S == 1) {
-                const uint32_t a = *reinterpret_cast<const uint16_t*>(hdr + lane * 8 + 4) & 0x7FFFu, b = *reinterpret_cast<const uint16_t*>(hdr + (lane + 32) * 8 + 4) & 0x7FFFu;
-                const float svmax = __half2float(__ushort_as_half(static_cast<uint16_t>(__reduce_max_sync(0xffffffffu, max(a, b)))));
-                F[0] = svmax > 0.0f ? Sh::kPMax / svmax : 0.0f;
-                invF[0] = svmax * (1.0f / Sh::kPMax);
-            } else {
-#pragma unroll
-                for (int s = 0; s < S; ++s) {
-                    const float svmax = __half2float(__ushort_as_half(static_cast<uint16_t>(__reduce_max_sync(0xffffffffu, s ? sc >> 16 : sc & 0xFFFFu))));
-                    F[s] = svmax > 0.0f ? Sh::kPMax / svmax : 0.0f;
-                    invF[s] = svmax * (1.0f / Sh::kPMax);
-                }
-            }
+            const uint32_t sa = *reinterpret_cast<const uint16_t*>(hdr + lane * 8 + 4) & 0x7FFFu, sb = *reinterpret_cast<const uint16_t*>(hdr + (lane + 32) * 8 + 4) & 0x7FFFu;
+            const float svmax = __half2float(__ushort_as_half(static_cast<uint16_t>(__reduce_max_sync(0xffffffffu, max(sa, sb)))));
+            const float F = svmax > 0.0f ? Sh::kPMax / svmax : 0.0f, invF = svmax * (1.0f / Sh::kPMax);
             float alpha[NB][2], wpass[NB][2], cst[NB][2];
             bool moved = false;
             auto page_weights = [&](int nb, int j, float mpass) {  // the page's row maximum against the running one
@@ -866,28 +699,25 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
                 alpha[nb][j] = fast_exp2(acc.m[nb][j] - muse);
                 wpass[nb][j] = fast_exp2(mpass - muse);
                 acc.m[nb][j] = mnew;
-#pragma unroll
-                for (int s = 0; s < S; ++s) wq[s][nb][j] = wpass[nb][j] * invF[s];
+                wq[nb][j] = wpass[nb][j] * invF;
             };
-            if constexpr (kOther || S == 2) {
-                if constexpr (S == 1) {
-                    // logits = other_K(key) * (f * integer sum + qz): the page maximum is taken on the floats
-                    float ok[kGroups][2];
+            if constexpr (kOther) {
+                // logits = other_K(key) * (f * integer sum + qz): the page maximum is taken on the floats
+                float ok[kGroups][2];
+#pragma unroll
+                for (int grp = 0; grp < kGroups; ++grp)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        ok[grp][h] = __half2float(*reinterpret_cast<const __half*>(hdr + kHdrV + (key_lo + Sh::key_grp(grp) + kKeyH * h) * 10 + 8));
+#pragma unroll
+                for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
                     for (int grp = 0; grp < kGroups; ++grp)
 #pragma unroll
-                        for (int h = 0; h < 2; ++h)
-                            ok[grp][h] = __half2float(*reinterpret_cast<const __half*>(hdr + kHdrV + (key_lo + Sh::key_grp(grp) + kKeyH * h) * 10 + 8));
-#pragma unroll
-                    for (int nb = 0; nb < NB; ++nb)
-#pragma unroll
-                        for (int grp = 0; grp < kGroups; ++grp)
-#pragma unroll
-                            for (int e = 0; e < 4; ++e)
-                                sl[nb][grp][e] = tot[nb][grp][e] == INT_MIN
-                                                     ? -INFINITY
-                                                     : fmaf(static_cast<float>(tot[nb][grp][e]), qi.f[0][nb][e & 1], qi.qz[0][nb][e & 1]) * ok[grp][e >> 1];
-                }
+                        for (int e = 0; e < 4; ++e)
+                            sl[nb][grp][e] = tot[nb][grp][e] == INT_MIN
+                                                 ? -INFINITY
+                                                 : fmaf(static_cast<float>(tot[nb][grp][e]), qi.f[nb][e & 1], qi.qz[nb][e & 1]) * ok[grp][e >> 1];
 #pragma unroll
                 for (int nb = 0; nb < NB; ++nb) {
 #pragma unroll
@@ -902,7 +732,7 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
                         cst[nb][j] = mpass == -INFINITY ? 0.0f : mpass;
                     }
                 }
-                if (__any_sync(0xffffffffu, moved)) rescale<S, NB>(acc, alpha);
+                if (__any_sync(0xffffffffu, moved)) rescale<NB>(acc, alpha);
 #pragma unroll
                 for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
@@ -920,19 +750,19 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
                         mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
                         mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
                         mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-                        const float mpass = mx == INT_MIN ? -INFINITY : fmaf(static_cast<float>(mx), qi.f[0][nb][j], qi.qz[0][nb][j]);
+                        const float mpass = mx == INT_MIN ? -INFINITY : fmaf(static_cast<float>(mx), qi.f[nb][j], qi.qz[nb][j]);
                         page_weights(nb, j, mpass);
-                        cst[nb][j] = qi.qz[0][nb][j] - (mpass == -INFINITY ? 0.0f : mpass);
+                        cst[nb][j] = qi.qz[nb][j] - (mpass == -INFINITY ? 0.0f : mpass);
                     }
                 }
-                if (__any_sync(0xffffffffu, moved)) rescale<S, NB>(acc, alpha);
+                if (__any_sync(0xffffffffu, moved)) rescale<NB>(acc, alpha);
 #pragma unroll
                 for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
                     for (int grp = 0; grp < kGroups; ++grp)
 #pragma unroll
                         for (int j = 0; j < 2; ++j) {  // the keys of m-rows g and g + 8 of one row
-                            const float2 y = fma2(F2(static_cast<float>(tot[nb][grp][j]), static_cast<float>(tot[nb][grp][2 + j])), F2(qi.f[0][nb][j], qi.f[0][nb][j]), F2(cst[nb][j], cst[nb][j])).get();
+                            const float2 y = fma2(F2(static_cast<float>(tot[nb][grp][j]), static_cast<float>(tot[nb][grp][2 + j])), F2(qi.f[nb][j], qi.f[nb][j]), F2(cst[nb][j], cst[nb][j])).get();
                             sl[nb][grp][j] = y.x;
                             sl[nb][grp][2 + j] = y.y;
                         }
@@ -949,29 +779,16 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
                         }
                 }
             }
-            F2 lp_[NB][2], zp_[S][NB][2];  // per row, the keys of m-rows g and g + 8
+            F2 lp_[NB][2], zp_[NB][2];  // per row, the keys of m-rows g and g + 8
 #pragma unroll
             for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    lp_[nb][j] = F2(0.0f, 0.0f);
-#pragma unroll
-                    for (int s = 0; s < S; ++s) zp_[s][nb][j] = F2(0.0f, 0.0f);
-                }
-            const uint8_t* vs = hdr + key_lo * 8 * S + 4 * S;  // V scale rows per key: 2 S other_V, S scales, S zero points
+                for (int j = 0; j < 2; ++j) lp_[nb][j] = zp_[nb][j] = F2(0.0f, 0.0f);
+            const uint8_t* vs = hdr + key_lo * 8 + 4;  // V scale rows per key: 2 other_V, scale, zero point
 #pragma unroll
             for (int grp = 0; grp < kGroups; ++grp) {
-                const int koff = Sh::key_grp(grp) * 8 * S;
-                float sc0[S], zz0[S], sc1[S], zz1[S];  // scale and zero point of the keys of m-rows g and g + 8
-                if constexpr (S == 1) {
-                    const float2 sz0 = unpack_half2(*reinterpret_cast<const uint32_t*>(vs + koff)), sz1 = unpack_half2(*reinterpret_cast<const uint32_t*>(vs + koff + kKeyH * 8));
-                    sc0[0] = sz0.x; zz0[0] = sz0.y; sc1[0] = sz1.x; zz1[0] = sz1.y;
-                } else {
-                    const uint2 a = *reinterpret_cast<const uint2*>(vs + koff), b = *reinterpret_cast<const uint2*>(vs + koff + kKeyH * 16);
-                    const float2 sa = unpack_half2(a.x), za = unpack_half2(a.y), sb = unpack_half2(b.x), zb2 = unpack_half2(b.y);
-                    sc0[0] = sa.x; sc0[S - 1] = sa.y; zz0[0] = za.x; zz0[S - 1] = za.y;
-                    sc1[0] = sb.x; sc1[S - 1] = sb.y; zz1[0] = zb2.x; zz1[S - 1] = zb2.y;
-                }
+                const int koff = Sh::key_grp(grp) * 8;
+                const float2 sz0 = unpack_half2(*reinterpret_cast<const uint32_t*>(vs + koff)), sz1 = unpack_half2(*reinterpret_cast<const uint32_t*>(vs + koff + kKeyH * 8));  // of the keys of m-rows g and g + 8
 #pragma unroll
                 for (int nb = 0; nb < NB; ++nb) {
                     F2 p[2];
@@ -980,51 +797,40 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
                         p[j] = F2(fast_exp2(sl[nb][grp][j]), fast_exp2(sl[nb][grp][2 + j]));
                         lp_[nb][j] = add2(lp_[nb][j], p[j]);
                     }
+                    // accumulator layout (m-row g; rows 2t, 2t+1) -> operand layout (row g; m-rows 2t, 2t+1 | 2t+8, 2t+9)
+                    const F2 sf = mul2(F2(sz0.x, sz1.x), F2(F, F));
+                    uint32_t w[4];
 #pragma unroll
-                    for (int s = 0; s < S; ++s) {
-                        // accumulator layout (m-row g; rows 2t, 2t+1) -> operand layout (row g; m-rows 2t, 2t+1 | 2t+8, 2t+9)
-                        const F2 sf = mul2(F2(sc0[s], sc1[s]), F2(F[s], F[s]));
-                        uint32_t w[4];
-#pragma unroll
-                        for (int j = 0; j < 2; ++j) {
-                            zp_[s][nb][j] = fma2(p[j], F2(zz0[s], zz1[s]), zp_[s][nb][j]);
-                            const float2 y = fma2(p[j], sf, F2(Sh::kPMagic, Sh::kPMagic)).get();
-                            w[j] = __float_as_uint(y.x);
-                            w[2 + j] = __float_as_uint(y.y);
-                        }
-                        const uint32_t y0 = movmatrix_trans(prmt(w[0], w[1], 0x5410)), y1 = movmatrix_trans(prmt(w[2], w[3], 0x5410));
-                        bw[s][nb][kDigits - 1][grp] = prmt(y0, y1, 0x6420);
-                        bw[s][nb][kDigits - 2][grp] = prmt(y0, y1, 0x7531);
-                        if constexpr (S == 2) {  // the third bytes of both m-rows travel in one 16-bit element
-                            const uint32_t y2 = movmatrix_trans(prmt(prmt(w[0], w[2], 0x0062), prmt(w[1], w[3], 0x0062), 0x5410));
-                            bw[s][nb][0][grp] = prmt(y2, y2, 0x3120);
-                        }
+                    for (int j = 0; j < 2; ++j) {
+                        zp_[nb][j] = fma2(p[j], F2(sz0.y, sz1.y), zp_[nb][j]);
+                        const float2 y = fma2(p[j], sf, F2(kMagic, kMagic)).get();
+                        w[j] = __float_as_uint(y.x);
+                        w[2 + j] = __float_as_uint(y.y);
                     }
+                    const uint32_t y0 = movmatrix_trans(prmt(w[0], w[1], 0x5410)), y1 = movmatrix_trans(prmt(w[2], w[3], 0x5410));
+                    bw[nb][1][grp] = prmt(y0, y1, 0x6420);
+                    bw[nb][0][grp] = prmt(y0, y1, 0x7531);
                 }
             }
 #pragma unroll
             for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
-                    const float2 lp2 = lp_[nb][j].get();
+                    const float2 lp2 = lp_[nb][j].get(), zp2 = zp_[nb][j].get();
                     acc.l[nb][j] = fmaf(lp2.x + lp2.y, wpass[nb][j], acc.l[nb][j]);
-#pragma unroll
-                    for (int s = 0; s < S; ++s) {
-                        const float2 zp2 = zp_[s][nb][j].get();
-                        if constexpr (kOther) {  // the zero-point term takes other_V of the tile per dim: it enters the accumulators with the page
-                            float zs = zp2.x + zp2.y;
-                            zs += __shfl_xor_sync(0xffffffffu, zs, 4);
-                            zs += __shfl_xor_sync(0xffffffffu, zs, 8);
-                            zs += __shfl_xor_sync(0xffffffffu, zs, 16);
-                            zfull[s][nb][j] = zs * wpass[nb][j];
-                        } else {
-                            acc.z[s][nb][j] = fmaf(zp2.x + zp2.y, wpass[nb][j], acc.z[s][nb][j]);
-                        }
+                    if constexpr (kOther) {  // the zero-point term takes other_V of the tile per dim: it enters the accumulators with the page
+                        float zs = zp2.x + zp2.y;
+                        zs += __shfl_xor_sync(0xffffffffu, zs, 4);
+                        zs += __shfl_xor_sync(0xffffffffu, zs, 8);
+                        zs += __shfl_xor_sync(0xffffffffu, zs, 16);
+                        zfull[nb][j] = zs * wpass[nb][j];
+                    } else {
+                        acc.z[nb][j] = fmaf(zp2.x + zp2.y, wpass[nb][j], acc.z[nb][j]);
                     }
                 }
         }
         // ---- PV on the int8 path.  Matrix i' of half c of the page (8 rows) gathers keys 2i', 2i'+1 (+ 8c) of each of the four
-        //      sub-blocks at 128 dims, key i' + 4c of each of the eight at 256: eight distinct 16-byte bank groups.
+        //      sub-blocks: eight distinct 16-byte bank groups when they are shifted.
         //      ldmatrix.trans hands lane (g, t) the code bytes of dims 32 db + 4g .. +3 of matrix rows 2t, 2t+1; one byte permute
         //      gathers the rows of two matrices of a dim pair, one AND isolates the even dim (x) or 16 x the odd dim (y): the k
         //      slots of MMA c, matching groups 2c and 2c + 1.
@@ -1032,14 +838,11 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
         {
             // lane L addresses row L & 7 of matrix L >> 3, shifted with its sub-block
             const int vrow = lane & 7, vmat = lane >> 3;
-            const uint8_t* ch = S == 1 ? R.slots[slot] + (16 * (vrow >> 1) + 2 * vmat + (vrow & 1)) * 64 + Vs::kShift * (vrow >> 1)
-                                       : R.slots[slot] + (8 * vrow + vmat) * 128 + Vs::kShift * vrow;
+            const uint8_t* ch = R.slots[slot] + (16 * (vrow >> 1) + 2 * vmat + (vrow & 1)) * 64 + Vs::kShift * (vrow >> 1);
             // swept one 32-dim block at a time: a quarter of the integer accumulators live (measured 1.6 % faster than two halves)
 #pragma unroll
             for (int db = 0; db < Sh::kBlocks; ++db) {
-                constexpr int kHi = 0;
-                const int s = db >> 2;
-                int ix[NB][2][kDigits][4];  // [nb][xy][digit][c]
+                int ix[NB][2][2][4];  // [nb][xy][digit][c]
 #pragma unroll
                 for (int c = 0; c < 2; ++c) {  // 32-key halves of the page
                     uint32_t r[4];
@@ -1051,13 +854,13 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
 #pragma unroll
                     for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
-                        for (int d = 0; d < kDigits; ++d) {
+                        for (int d = 0; d < 2; ++d) {
                             if (c == 0) {
-                                imma_uu0(ix[nb][0][d], ax0, ax1, ax2, ax3, bw[s][nb][d][0], bw[s][nb][d][1]);
-                                imma_uu0(ix[nb][1][d], ay0, ay1, ay2, ay3, bw[s][nb][d][0], bw[s][nb][d][1]);
+                                imma_uu0(ix[nb][0][d], ax0, ax1, ax2, ax3, bw[nb][d][0], bw[nb][d][1]);
+                                imma_uu0(ix[nb][1][d], ay0, ay1, ay2, ay3, bw[nb][d][0], bw[nb][d][1]);
                             } else {
-                                imma_uu(ix[nb][0][d], ax0, ax1, ax2, ax3, bw[s][nb][d][2], bw[s][nb][d][3]);
-                                imma_uu(ix[nb][1][d], ay0, ay1, ay2, ay3, bw[s][nb][d][2], bw[s][nb][d][3]);
+                                imma_uu(ix[nb][0][d], ax0, ax1, ax2, ax3, bw[nb][d][2], bw[nb][d][3]);
+                                imma_uu(ix[nb][1][d], ay0, ay1, ay2, ay3, bw[nb][d][2], bw[nb][d][3]);
                             }
                         }
                 }
@@ -1067,19 +870,18 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
 #pragma unroll
                     for (int xy = 0; xy < 2; ++xy) {
                         const float nibble = xy ? 0.0625f : 1.0f;
-                        const F2 w(wq[s][nb][0] * nibble, wq[s][nb][1] * nibble);
+                        const F2 w(wq[nb][0] * nibble, wq[nb][1] * nibble);
 #pragma unroll
                         for (int h = 0; h < 2; ++h) {  // a dim, rows 2t and 2t + 1
                             float v[2];
 #pragma unroll
                             for (int j = 0; j < 2; ++j) {
                                 const int c = 2 * h + j;
-                                v[j] = static_cast<float>((ix[nb][xy][kDigits - 2][c] << 8) + ix[nb][xy][kDigits - 1][c]);
-                                if constexpr (S == 2) v[j] = fmaf(static_cast<float>(ix[nb][xy][kHi][c]), 65536.0f, v[j]);
+                                v[j] = static_cast<float>((ix[nb][xy][0][c] << 8) + ix[nb][xy][1][c]);
                             }
                             F2& o = acc.o[nb][db][xy][h];
                             if constexpr (kOther)  // (sum p code scale_V + sum p zp_V) * other_V(dim)
-                                o = fma2(fma2(F2(v[0], v[1]), w, F2(zfull[s][nb][0], zfull[s][nb][1])), F2(ov[db][xy][h], ov[db][xy][h]), o);
+                                o = fma2(fma2(F2(v[0], v[1]), w, F2(zfull[nb][0], zfull[nb][1])), F2(ov[db][xy][h], ov[db][xy][h]), o);
                             else
                                 o = fma2(F2(v[0], v[1]), w, o);
                         }
@@ -1106,22 +908,20 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
 #pragma unroll
             for (int o = 4; o <= 16; o <<= 1) {
                 acc.l[nb][j] += __shfl_xor_sync(0xffffffffu, acc.l[nb][j], o);
-#pragma unroll
-                for (int s = 0; s < S; ++s) acc.z[s][nb][j] += __shfl_xor_sync(0xffffffffu, acc.z[s][nb][j], o);
+                acc.z[nb][j] += __shfl_xor_sync(0xffffffffu, acc.z[nb][j], o);
             }
             if (g == 0) {
                 const int row = 8 * nb + 2 * t + j;
                 mbuf[row] = acc.m[nb][j];
                 mbuf[kRows + row] = acc.l[nb][j];
-#pragma unroll
-                for (int s = 0; s < S; ++s) mbuf[(2 + s) * kRows + row] = acc.z[s][nb][j];
+                mbuf[2 * kRows + row] = acc.z[nb][j];
             }
         }
 #pragma unroll
         for (int db = 0; db < Sh::kBlocks; ++db)
 #pragma unroll
             for (int j = 0; j < 2; ++j) {  // row 8 nb + 2t + j, dims 32 db + 4g .. +3
-                float* dst = mbuf + (2 + S) * kRows + (8 * nb + 2 * t + j) * kORow + 32 * db + 4 * g;
+                float* dst = mbuf + 3 * kRows + (8 * nb + 2 * t + j) * kORow + 32 * db + 4 * g;
                 const float2 a = acc.o[nb][db][0][0].get(), b = acc.o[nb][db][1][0].get(), c = acc.o[nb][db][0][1].get(), d = acc.o[nb][db][1][1].get();
                 *reinterpret_cast<float4*>(dst) = j ? make_float4(a.y, b.y, c.y, d.y) : make_float4(a.x, b.x, c.x, d.x);
             }
@@ -1140,15 +940,14 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
             for (int w = 0; w < kWarps; ++w) {
                 const float* wb = all + w * kWarpFloats;
                 const float wt = fast_exp2(wb[row] - m);  // exp2(-inf) = 0 for a warp that saw no key
-                const float4 v = *reinterpret_cast<const float4*>(wb + (2 + S) * kRows + row * kORow + d);
-                const float z = wb[(2 + d / 128) * kRows + row];
+                const float4 v = *reinterpret_cast<const float4*>(wb + 3 * kRows + row * kORow + d);
+                const float z = wb[2 * kRows + row];
                 l += wt * wb[kRows + row];
                 o.x += wt * (v.x + z); o.y += wt * (v.y + z); o.z += wt * (v.z + z); o.w += wt * (v.w + z);
             }
         }
-        if (S == 2 && sm.poison[d / 128][row] != 0) o.x = o.y = o.z = o.w = __uint_as_float(0x7FC00000u);
         if constexpr (kCluster) {
-            ClusterPart<S>& part = *reinterpret_cast<ClusterPart<S>*>(smem_raw + sizeof(Smem));
+            ClusterPart& part = *reinterpret_cast<ClusterPart*>(smem_raw + sizeof(Smem));
             *reinterpret_cast<float4*>(&part.o[row][d]) = o;
             if (d == 0) { part.m[row] = m; part.l[row] = l; }
         } else {
@@ -1158,12 +957,18 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
     }
 }
 
-template <int S, int NB, int W, bool kOther = false>
+}  // namespace
+}  // namespace kvb
+#include "kvb_attn_pair.cuh"
+namespace kvb {
+namespace {
+
+template <int NB, int W, bool kOther = false>
 __global__ void __launch_bounds__(W * 32, 1) attn_kernel(const AttnParams P) {
     // q, the positions and the cache come from the kernels before this one; an append has waited for those before it
     if (!P.after_append) grid_dependency_wait();
     const int head = blockIdx.y, zb = blockIdx.z, split = blockIdx.x;
-    attn_cta<S, NB, W, kOther>(P, split, head, zb, ((static_cast<int64_t>(head) * gridDim.z + zb) * P.nsplit + split) * kRows);
+    attn_cta<NB, W, kOther>(P, split, head, zb, ((static_cast<int64_t>(head) * gridDim.z + zb) * P.nsplit + split) * kRows);
     if (P.after_append) grid_dependency_wait();  // nobody leaves before the append is over: what waits for this grid finds both done
 }
 
@@ -1171,16 +976,18 @@ __global__ void __launch_bounds__(W * 32, 1) attn_kernel(const AttnParams P) {
 // partials in the workspace, no merge kernel.  CTA c of the cluster finishes rows c, c + n, .., a warp each: every split's partial of the
 // row, in the order and with the roundings of the merge kernel, normalised, rotated back, stored.
 template <int S, int NB, bool kOther>
-__global__ void __launch_bounds__(kWarpsWide * 32, 1) attn_short_kernel(const AttnParams P, uint16_t* __restrict__ out) {
-    constexpr int W = kWarpsWide, D = Shape<S>::kDim;
+__global__ void __launch_bounds__((S == 1 ? kWarpsWide : kPairWarps) * 32, 1) attn_short_kernel(const AttnParams P, uint16_t* __restrict__ out) {
+    constexpr int W = S == 1 ? kWarpsWide : kPairWarps, D = 128 * S;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    using Smem = AttnSmem<S, NB, W>;
+    using Smem = std::conditional_t<S == 1, AttnSmem<NB, W>, PairSmem>;
+    using Part = std::conditional_t<S == 1, ClusterPart, PairPart>;
     Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
-    ClusterPart<S>& part = *reinterpret_cast<ClusterPart<S>*>(smem_raw + sizeof(Smem));
+    Part& part = *reinterpret_cast<Part*>(smem_raw + (S == 1 ? sizeof(Smem) : offsetof(PairSmem, swap)));
     static_assert(sizeof(Smem) % 16 == 0, "alignment");
     if (!P.after_append) grid_dependency_wait();
     const int head = blockIdx.y, zb = blockIdx.z, split = blockIdx.x, n = P.nsplit;
-    attn_cta<S, NB, W, kOther, true>(P, split, head, zb, 0);
+    if constexpr (S == 1) attn_cta<NB, W, kOther, true>(P, split, head, zb, 0);
+    else attn_pair_cta<true>(P, split, head, zb, 0);
     cluster_sync();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, G = P.L.q_heads / P.L.kv_heads;
     for (int r = split + n * warp; r < 8 * NB; r += n * W) {
@@ -1299,7 +1106,7 @@ __global__ void __launch_bounds__(W * 32, kPerSm) attn_batch_kernel(const BatchP
     P.ws_m = B.ws_m;
     P.ws_l = B.ws_l;
     P.ws_o = B.ws_o;
-    attn_cta<1, NB, W>(P, part - B.plan.prefix[b], head, 0, pidx);
+    attn_cta<NB, W>(P, part - B.plan.prefix[b], head, 0, pidx);
 }
 
 // Merge the partials of all splits of one query row, normalise, rotate back (H is its own inverse) and
@@ -1348,7 +1155,7 @@ __global__ void __launch_bounds__(kReduceWarps * 32) reduce_kernel(const float* 
                                                                   float* __restrict__ part_m, float* __restrict__ part_l,
                                                                   float* __restrict__ part_o, const PushTarget push,
                                                                   const BatchPlan plan) {
-    constexpr int D = Shape<S>::kDim;
+    constexpr int D = 128 * S;
     __shared__ float4 so[kReduceWarps][S][32];
     __shared__ float sl[kReduceWarps];
     const int row = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1609,12 +1416,12 @@ int launch_chunk_attention_256(const kvb_layer* layer, const void* q, const int3
 namespace {
 
 // One attention launch with W warps per CTA (the opt-in to large dynamic shared memory is made once per device and W).
-template <int S, int NB, int W, bool kOther = false>
+template <int NB, int W, bool kOther = false>
 cudaError_t launch_attn(dim3 grid, cudaStream_t stream, const AttnParams& P) {
-    constexpr int smem = static_cast<int>(sizeof(AttnSmem<S, NB, W>));
+    constexpr int smem = static_cast<int>(sizeof(AttnSmem<NB, W>));
     static OncePerDevice opted;
-    if (const cudaError_t e = allow_smem(opted, attn_kernel<S, NB, W, kOther>, smem)) return e;
-    return launch_early(attn_kernel<S, NB, W, kOther>, grid, dim3(W * 32), smem, stream, P);
+    if (const cudaError_t e = allow_smem(opted, attn_kernel<NB, W, kOther>, smem)) return e;
+    return launch_early(attn_kernel<NB, W, kOther>, grid, dim3(W * 32), smem, stream, P);
 }
 
 // The merge asks for as little shared memory as an SM can be set to.  Left to itself the driver sets an SM up for as many of its
@@ -1639,19 +1446,29 @@ cudaError_t launch_reduce(int rows, cudaStream_t stream, const float* ws_m, cons
                         block_rows, dtype, out, part_m, part_l, part_o, push, plan);
 }
 
+cudaError_t launch_attn_pair(dim3 grid, cudaStream_t stream, const AttnParams& P) {
+    constexpr int smem = static_cast<int>(sizeof(PairSmem));
+    static OncePerDevice opted;
+    if (const cudaError_t e = allow_smem(opted, attn_pair_kernel, smem)) return e;
+    return launch_early(attn_pair_kernel, grid, dim3(kPairWarps * 32), smem, stream, P);
+}
+
 // Up to this many keys, and with up to this many clusters, the splits of a head and row block are a cluster (attn_short_kernel).  Beyond
 // the keys, eight CTAs have more than a round of pages; beyond the clusters, they are not all on the GPU at once.  Measured on B200 in
 // graph replay, append and attention, 24 / 4 heads, merge kernel against clusters, us a layer: 300 tokens 9.0 8.5, 1,500 9.6 9.1, 2,500 9.6
-// 9.2, 4,000 9.0 9.4, 6,000 9.9 12.3; 256 dims 1,500 16.0 14.9, 3,000 16.0 16.0, 4,000 15.7 16.2; verify at 1,500 tokens, 4 rows (12
-// clusters) 9.5 9.2, 5 rows (16) 9.6 16.4.  Launched one by one (3 us of the host each), 16 layers at 1,500 tokens take 206 and 164 us.
-constexpr int kShortKeys = 3072, kShortClusters = 12;
+// 9.2, 4,000 9.0 9.4, 6,000 9.9 12.3; 256 dims 300 13.3 12.5, 800 13.4 12.5, 1,500 14.7 14.2, 2,000 14.7 15.6, 3,000 14.2 15.4; verify at
+// 1,500 tokens, 4 rows (12 clusters) 9.5 9.2, 5 rows (16) 9.6 16.4.  Launched one by one (3 us of the host each), 16 layers at 1,500
+// tokens take 206 and 164 us.
+constexpr int kShortClusters = 12;
+constexpr int short_keys(int head_dim) { return head_dim == 128 ? 3072 : 1536; }
 // The same as clusters: the splits of a head and row block.
 template <int S, int NB, bool kOther>
 cudaError_t launch_short(dim3 grid, cudaStream_t stream, const AttnParams& P, uint16_t* out) {
-    constexpr int smem = static_cast<int>(sizeof(AttnSmem<S, NB, kWarpsWide>) + sizeof(ClusterPart<S>));
+    constexpr int warps = S == 1 ? kWarpsWide : kPairWarps;
+    constexpr int smem = static_cast<int>(S == 1 ? sizeof(AttnSmem<NB, kWarpsWide>) + sizeof(ClusterPart) : sizeof(PairSmem));
     static OncePerDevice opted;
     if (const cudaError_t e = allow_smem(opted, attn_short_kernel<S, NB, kOther>, smem)) return e;
-    return launch_early_cluster(attn_short_kernel<S, NB, kOther>, grid, dim3(kWarpsWide * 32), smem, static_cast<int>(grid.x), stream, P, out);
+    return launch_early_cluster(attn_short_kernel<S, NB, kOther>, grid, dim3(warps * 32), smem, static_cast<int>(grid.x), stream, P, out);
 }
 
 // Warps per CTA for a decode call: 8, 12 or 16 (whole warp quartets: an SM hands registers and issue slots out per
@@ -1711,7 +1528,7 @@ int launch_attention(const kvb_layer* layer, const void* q, const int32_t* pos_d
     const RowPlan plan = plan_rows(kv_len_max, layer->kv_heads, layer->q_heads, layer->head_dim, T, layer->sinkhorn_iters != 0);
     // The output may be stored while others still read q, the positions and, behind an append, its rows?
     const size_t out_bytes = static_cast<size_t>(T) * layer->q_heads * layer->head_dim * sizeof(uint16_t);
-    const bool clustered = kv_len_max <= kShortKeys && layer->kv_heads * plan.zblocks <= kShortClusters && out != nullptr && part_m == nullptr && push == nullptr &&
+    const bool clustered = kv_len_max <= short_keys(layer->head_dim) && layer->kv_heads * plan.zblocks <= kShortClusters && out != nullptr && part_m == nullptr && push == nullptr &&
                            stores_beside(span_of(out, out_bytes), span_of(q, out_bytes), span_of(pos_dev, T * sizeof(int32_t)), span_of(total_pos_dev, sizeof(int32_t)));
     const int Z = plan.zblocks, nsplit = clustered ? std::min(plan.nsplit, kShortSplits) : plan.nsplit;
     const int parts = nsplit;
@@ -1742,22 +1559,21 @@ int launch_attention(const kvb_layer* layer, const void* q, const int32_t* pos_d
         KVB_CUDA_OK(launch(grid, stream, P, to));
         return KVB_OK;
     }
-    if (layer->head_dim != 128) {  // two slices per head: twice the accumulators and the wider integers leave room for 8 warps.  The
-        // factors of balanced caches are applied whatever the descriptor says: at this head dim a reader need not know the count
-        KVB_CUDA_OK((launch_attn<2, 1, kWarpsWide, true>(grid, stream, P)));
+    if (layer->head_dim != 128) {  // the factors of balanced caches are applied whatever the descriptor says: at this head dim a reader need not know the count
+        KVB_CUDA_OK(launch_attn_pair(grid, stream, P));
     } else if (layer->sinkhorn_iters != 0) {  // balanced caches: other_K per key, other_V per dim (more registers: 8 warps)
         if (upper) {
-            KVB_CUDA_OK((launch_attn<1, 2, kWarpsWide, true>(grid, stream, P)));
+            KVB_CUDA_OK((launch_attn<2, kWarpsWide, true>(grid, stream, P)));
         } else {
-            KVB_CUDA_OK((launch_attn<1, 1, 8, true>(grid, stream, P)));
+            KVB_CUDA_OK((launch_attn<1, 8, true>(grid, stream, P)));
         }
     } else if (upper) {
-        KVB_CUDA_OK((launch_attn<1, 2, kWarpsWide>(grid, stream, P)));
+        KVB_CUDA_OK((launch_attn<2, kWarpsWide>(grid, stream, P)));
     } else {
         switch (plan.warps) {
-            case 8: KVB_CUDA_OK((launch_attn<1, 1, 8>(grid, stream, P))); break;
-            case 12: KVB_CUDA_OK((launch_attn<1, 1, 12>(grid, stream, P))); break;
-            default: KVB_CUDA_OK((launch_attn<1, 1, 16>(grid, stream, P))); break;
+            case 8: KVB_CUDA_OK((launch_attn<1, 8>(grid, stream, P))); break;
+            case 12: KVB_CUDA_OK((launch_attn<1, 12>(grid, stream, P))); break;
+            default: KVB_CUDA_OK((launch_attn<1, 16>(grid, stream, P))); break;
         }
     }
     const int total_rows = T * layer->q_heads;
@@ -2057,7 +1873,7 @@ extern "C" int kvb_attn_decode_batch(const kvb_layer* layers_dev, int batch, int
     B.ws_m = workspace_base(workspace);
     B.ws_l = B.ws_m + rows;
     B.ws_o = B.ws_l + rows;
-    constexpr int smem = static_cast<int>(sizeof(AttnSmem<1, 1, kWarpsWide>));
+    constexpr int smem = static_cast<int>(sizeof(AttnSmem<1, kWarpsWide>));
     static_assert(kBatchPerSm * (smem + 1024) <= 228 * 1024, "CTAs beside each other");
     static OncePerDevice opted1, opted2;
     KVB_CUDA_OK(allow_smem(opted1, attn_batch_kernel<1, kWarpsWide, kBatchPerSm>, smem));
