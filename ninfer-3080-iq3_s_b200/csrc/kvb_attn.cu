@@ -74,6 +74,13 @@ template <int NB> struct VSlot {
     static constexpr int kBytes = (Shape::kChunk + (kSubs - 1) * kShift + 127) / 128 * 128;
 };
 
+// Division by a number of splits as a multiplication; exact below 2^26.
+struct SplitBy {
+    uint32_t all, others;  // 2^32 / nsplit, / (nsplit - 1), rounded up (0: by one)
+    __host__ __device__ static uint32_t inverse(int d) { return d > 1 ? 0xFFFFFFFFu / static_cast<uint32_t>(d) + 1u : 0u; }
+    __device__ static int divide(int n, uint32_t inv) { return inv != 0u ? static_cast<int>(__umulhi(static_cast<uint32_t>(n), inv)) : n; }
+};
+
 struct AttnParams {
     LayerView L;
     const uint16_t* q;   // [T][q_heads][D]
@@ -81,6 +88,7 @@ struct AttnParams {
     const int32_t* total_pos;  // position of the newest token in the cache (kv_total = *total_pos + 1)
     int T;
     float scale_log2;    // softmax scale * log2(e)
+    SplitBy by;
     int nsplit;          // CTAs over the sealed tiles of a head; the last one also reads the open tile
     int block_rows;      // GQA-merged query rows per row block (grid z): 8 (one 8-row block per warp) or 16 (two)
     int key_begin, key_end;
@@ -379,6 +387,35 @@ __device__ __forceinline__ void process_stage_group(const __half* krow, const __
     }
 }
 
+// Pages of split `split` of `n` pages, which its CTA walks W at a time.  The last split has the open tile as well, whose 16-key groups (a
+// warp or pair each) count as 3/4 of a page; it takes no page that would be a round more for those with a group.  Neither may cost the
+// other splits a round.  Measured on B200 in graph replay, append and attention, us a layer, equal shares (by 64-bit divisions, the first
+// position read behind the newest, the next kernel's start by every warp) against this: decode at 300 / 1,500 / 8,000 / 32,768 / 65,536 /
+// 378,944 tokens 8.6 / 9.1 / 10.2 / 12.6 / 17.8 / 49.4 8.1 7.8 8.7 12.6 17.6 49.1, 256 dims 1,500 / 4,000 / 30,011 14.2 / 13.2 / 23.1 11.5 11.6 21.0, verify of 4
+// rows at 1,500 / 8,000 / 131,072 9.2 / 11.6 / 52.0 7.8 10.7 52.2, of 5 rows of 256 dims at 20,000 35.9 35.3.  A CTA with the open tile was
+// some 2,000 cycles behind the others.
+template <int W> __device__ __forceinline__ void split_pages(int n, int open_keys, int split, int nsplit, SplitBy by, int& begin, int& end) {
+    const int groups = (open_keys + 15) / 16, weighted = n + groups * 3 / 4;
+    int share = SplitBy::divide(n, by.all), more = n - share * nsplit;  // `more` splits have a page more
+    const int rounds = (share + (more != 0) + W - 1) / W, keep = rounds * W - groups;
+    if (weighted <= rounds * W * nsplit) {
+        share = SplitBy::divide(weighted, by.all);
+        more = weighted - share * nsplit;
+    }
+    if (nsplit > 1 && n - share * (nsplit - 1) - more > keep && n - keep <= rounds * W * (nsplit - 1)) {
+        share = SplitBy::divide(n - keep, by.others);
+        more = n - keep - share * (nsplit - 1);
+    }
+    begin = min(share * split + min(split, more), n);
+    end = split == nsplit - 1 ? n : min(begin + share + (split < more), n);
+}
+// Pages of warp (or pair) w of the W of a CTA with n.  Over few rounds, and beside the open tile, whose groups the first ones have, the last
+// ones take a page more (the first ones rotate the query before they begin); over many, every so many-th.
+template <int W> __device__ __forceinline__ int warp_pages(int n, int w, bool last_first) {
+    const int share = n / W;
+    return last_first ? share * w + max(w - (W - (n - share * W)), 0) : n * w / W;
+}
+
 // The work of one CTA: split `split` of KV head `head`, row block `zb`; its partial goes to rows pidx .. pidx + 15 of
 // the workspace.  NB = 8-row blocks of query rows per warp.  A pass = one page: its 64 logits per row are held at
 // once.  Within a page the keys are taken in a fixed permutation (see key_lo below) that lets the QK accumulators
@@ -426,7 +463,7 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
             }
         }
     }
-    const int kv_total = *P.total_pos + 1;
+    const int pos0 = P.pos[0], kv_total = *P.total_pos + 1;
     const int key_end = min(P.key_end, kv_total), key_begin = max(P.key_begin, 0);
     const int sealed_pages = 2 * (kv_total / kTile);
 
@@ -440,13 +477,13 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
     int w0, w1;
     {
         const int pb = min(key_begin / kPage, sealed_pages), pe = min((key_end + kPage - 1) / kPage, sealed_pages);
-        const int n = max(pe - pb, 0);
-        const int c0 = pb + static_cast<int>(static_cast<int64_t>(n) * split / P.nsplit);
-        const int c1 = pb + static_cast<int>(static_cast<int64_t>(n) * (split + 1) / P.nsplit);
-        w0 = c0 + (c1 - c0) * warp / kWarps;
-        w1 = c0 + (c1 - c0) * (warp + 1) / kWarps;
+        int c0, c1;
+        split_pages<kWarps>(max(pe - pb, 0), kv_total % kTile, split, P.nsplit, P.by, c0, c1);
+        const bool last_first = c1 - c0 < 3 * kWarps || split == P.nsplit - 1;
+        w0 = pb + c0 + warp_pages<kWarps>(c1 - c0, warp, last_first);
+        w1 = pb + c0 + warp_pages<kWarps>(c1 - c0, warp + 1, last_first);
         // the stage, and tiles from that of the first appended row on
-        if (P.after_append && (split == P.nsplit - 1 || c1 * kPage > P.pos[0] / kTile * kTile)) grid_dependency_wait();
+        if (P.after_append && (split == P.nsplit - 1 || (pb + c1) * kPage > pos0 / kTile * kTile)) grid_dependency_wait();
     }
     const int npages = w1 - w0, nchunks = 2 * npages;
     // ---- the refill side of the ring.  Chunk n of this warp is page w0 + n / 2: even n = K codes + header, odd n = V
@@ -517,18 +554,17 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
         }
     }
     while (n_issued < kSlots && n_issued < nchunks) issue_next(n_issued);
-    launch_dependents();  // the reduce kernel may take its place on the SMs; it waits for this grid's completion
+    if (warp == kWarps - 1) launch_dependents();  // the reduce kernel may take its place on the SMs; it waits for this grid's completion
     __syncthreads();
 
     const int g = lane >> 2, t = lane & 3;
     int row_lim[NB][2];
-    int min_lim = INT_MAX;
+    const int min_lim = __reduce_min_sync(0xffffffffu, sm.row_pos[lane % (8 * NB)]);  // (a negative position: a row that sees no key)
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) {
         row_lim[nb][0] = sm.row_pos[8 * nb + 2 * t];
         row_lim[nb][1] = sm.row_pos[8 * nb + 2 * t + 1];
     }
-    for (int r = 0; r < 8 * NB; ++r) min_lim = min(min_lim, sm.row_pos[r]);  // (a negative position: a row that sees no key)
 
     Acc<NB> acc;
 #pragma unroll
@@ -1099,6 +1135,7 @@ __global__ void __launch_bounds__(W * 32, kPerSm) attn_batch_kernel(const BatchP
     P.T = 1;
     P.scale_log2 = B.scale_log2;
     P.nsplit = B.plan.prefix[b + 1] - B.plan.prefix[b];
+    P.by = {SplitBy::inverse(P.nsplit), SplitBy::inverse(P.nsplit - 1)};
     P.block_rows = kRows;
     P.key_begin = 0;
     P.key_end = INT_MAX;
@@ -1454,11 +1491,10 @@ cudaError_t launch_attn_pair(dim3 grid, cudaStream_t stream, const AttnParams& P
 }
 
 // Up to this many keys, and with up to this many clusters, the splits of a head and row block are a cluster (attn_short_kernel).  Beyond
-// the keys, eight CTAs have more than a round of pages; beyond the clusters, they are not all on the GPU at once.  Measured on B200 in
-// graph replay, append and attention, 24 / 4 heads, merge kernel against clusters, us a layer: 300 tokens 9.0 8.5, 1,500 9.6 9.1, 2,500 9.6
-// 9.2, 4,000 9.0 9.4, 6,000 9.9 12.3; 256 dims 300 13.3 12.5, 800 13.4 12.5, 1,500 14.7 14.2, 2,000 14.7 15.6, 3,000 14.2 15.4; verify at
-// 1,500 tokens, 4 rows (12 clusters) 9.5 9.2, 5 rows (16) 9.6 16.4.  Launched one by one (3 us of the host each), 16 layers at 1,500
-// tokens take 206 and 164 us.
+// the keys, eight CTAs have more than a round of pages; beyond the clusters, they are not all on the GPU at once.  Measured on B200, 24 / 4
+// heads, merge kernel against clusters: launched one by one (3 us of the host each), 16 layers at 1,500 tokens 206 and 164 us; in graph
+// replay, append and attention, us a layer: 300 tokens 8.1 8.0, 1,500 7.8 8.0, 3,000 8.1 8.4, 256 dims 300 12.0 11.7, 1,500 11.1 11.4, verify
+// of 4 rows (12 clusters) at 1,500 8.2 7.8; before, 4,000 9.0 9.4, 6,000 9.9 12.3, 256 dims 2,000 14.7 15.6, 5 rows (16 clusters) 9.6 16.4.
 constexpr int kShortClusters = 12;
 constexpr int short_keys(int head_dim) { return head_dim == 128 ? 3072 : 1536; }
 // The same as clusters: the splits of a head and row block.
@@ -1475,10 +1511,12 @@ cudaError_t launch_short(dim3 grid, cudaStream_t stream, const AttnParams& P, ui
 // quartet; 10 or 14 warps measured no faster per warp than 12 or 16).  A warp works on whole pages, so a CTA with n
 // pages needs ceil(n / W) rounds; a round and the fixed part (set-up, merge of the warps) take longer the more warps
 // share the SM.  Times in microseconds, fitted to sweeps over 32K .. 379K tokens on B200: with 8 warps the SM is
-// not yet saturated (a round of 8 pages takes 2.5 us, one of 16 pages 3.9 us).
+// not yet saturated (a round of 8 pages takes 2.5 us, one of 16 pages 3.9 us).  Append and attention in graph replay with 8 / 12 / 16
+// warps: 16,384 tokens 9.9 10.3 11.0, 32,768 12.6 13.8 13.3, 57,000 16.1 15.7, 65,536 17.6 16.5 17.5, 75,000 17.7 17.2, 131,072 25.1 23.7 25.7,
+// 378,944 57.8 50.2 49.3.
 int decode_warps(int kv_len_max, int nsplit, float* cost_us = nullptr) {
     static const int forced = [] { const char* e = std::getenv("KVB_DECODE_WARPS"); return e ? std::atoi(e) : 0; }();
-    static const struct { int warps; float fixed_us, round_us; } kChoice[3] = {{16, 8.8f, 3.93f}, {12, 7.3f, 2.98f}, {8, 6.1f, 2.52f}};
+    static const struct { int warps; float fixed_us, round_us; } kChoice[3] = {{16, 8.8f, 3.93f}, {12, 7.0f, 2.98f}, {8, 6.1f, 2.52f}};
     const int pages = 2 * (kv_len_max / kTile), per_cta = (pages + nsplit - 1) / nsplit;
     int best = 16;
     float best_cost = 1e30f;
@@ -1540,6 +1578,7 @@ int launch_attention(const kvb_layer* layer, const void* q, const int32_t* pos_d
     P.T = T;
     P.scale_log2 = scale * 1.4426950408889634f;
     P.nsplit = nsplit;
+    P.by = {SplitBy::inverse(nsplit), SplitBy::inverse(nsplit - 1)};
     P.block_rows = plan.block_rows;
     P.key_begin = key_begin;
     P.key_end = key_end;

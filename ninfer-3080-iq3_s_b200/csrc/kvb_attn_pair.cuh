@@ -188,7 +188,7 @@ __device__ __forceinline__ void attn_pair_cta(const AttnParams& P, int split, in
             qpos = P.pos[tq];
         }
     }
-    const int kv_total = *P.total_pos + 1;
+    const int pos0 = P.pos[0], kv_total = *P.total_pos + 1;
     const int key_end = min(P.key_end, kv_total), key_begin = max(P.key_begin, 0);
     const int sealed_pages = 2 * (kv_total / kTile);
     if (threadIdx.x < 2 * kRows) (&sm.poison[0][0])[threadIdx.x] = 0;
@@ -201,13 +201,13 @@ __device__ __forceinline__ void attn_pair_cta(const AttnParams& P, int split, in
     int w0, w1;
     {
         const int pb = min(key_begin / kPage, sealed_pages), pe = min((key_end + kPage - 1) / kPage, sealed_pages);
-        const int n = max(pe - pb, 0);
-        const int c0 = pb + static_cast<int>(static_cast<int64_t>(n) * split / P.nsplit);
-        const int c1 = pb + static_cast<int>(static_cast<int64_t>(n) * (split + 1) / P.nsplit);
-        w0 = c0 + (c1 - c0) * pair / kPairs;
-        w1 = c0 + (c1 - c0) * (pair + 1) / kPairs;
+        int c0, c1;
+        split_pages<kPairs>(max(pe - pb, 0), kv_total % kTile, split, P.nsplit, P.by, c0, c1);
+        const bool last_first = c1 - c0 < 3 * kPairs || split == P.nsplit - 1;
+        w0 = pb + c0 + warp_pages<kPairs>(c1 - c0, pair, last_first);
+        w1 = pb + c0 + warp_pages<kPairs>(c1 - c0, pair + 1, last_first);
         // the stage, and tiles from that of the first appended row on
-        if (P.after_append && (split == P.nsplit - 1 || c1 * kPage > P.pos[0] / kTile * kTile)) grid_dependency_wait();
+        if (P.after_append && (split == P.nsplit - 1 || (pb + c1) * kPage > pos0 / kTile * kTile)) grid_dependency_wait();
     }
     const int npages = w1 - w0, nchunks = 2 * npages;
     // ---- the refill side of the ring (see attn_cta): both warps follow it; lane 0 of the first issues K, of the second V
@@ -268,13 +268,12 @@ __device__ __forceinline__ void attn_pair_cta(const AttnParams& P, int split, in
         for (int j = 0; j < 8; ++j)  // dim lane + 32 j -> lane' = row * 4 + (d%128)/32, slot j' = 8 slice + (d%32)/4, component d%4
             dst[((8 * (j >> 2) + (lane >> 2)) * 32 + warp * 4 + (j & 3)) * 4 + (lane & 3)] = v[j] * P.scale_log2;
     }
-    launch_dependents();  // the merge kernel may take its place on the SMs; it waits for this grid's completion
+    if (warp == kPairWarps - 1) launch_dependents();  // the merge kernel may take its place on the SMs; it waits for this grid's completion
     __syncthreads();
 
     const int g = lane >> 2, t = lane & 3;
     const int row_lim[2] = {sm.row_pos[2 * t], sm.row_pos[2 * t + 1]};
-    int min_lim = INT_MAX;
-    for (int r = 0; r < 8; ++r) min_lim = min(min_lim, sm.row_pos[r]);  // (a negative position: a row that sees no key)
+    const int min_lim = __reduce_min_sync(0xffffffffu, sm.row_pos[lane & 7]);  // (a negative position: a row that sees no key)
     F2 o[4][2][2];  // [32-dim block of the slice][even, odd dims][c >> 1], see Acc
 #pragma unroll
     for (int db = 0; db < 4; ++db)
