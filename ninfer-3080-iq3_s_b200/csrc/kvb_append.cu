@@ -382,13 +382,13 @@ __device__ __forceinline__ void rotate_rows(const uint16_t* __restrict__ src, in
 template <int D, bool kBf16>
 __global__ void __launch_bounds__(kThreads, 1) append_kernel(LayerView L, const uint16_t* __restrict__ k,
                                                              const uint16_t* __restrict__ v,
-                                                             const int32_t* __restrict__ positions, int tokens, bool starts_next) {
+                                                             const int32_t* __restrict__ positions, int tokens) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     AppendSmem& sm = *reinterpret_cast<AppendSmem*>(smem_raw);
     using G = Geo<D>;
     constexpr int S = G::S;
     grid_dependency_wait();  // launched while its predecessor still runs: nothing is read or written before it is over
-    if (starts_next) launch_dependents();
+    launch_dependents();
     const int pos0 = positions[0], last = positions[tokens - 1];
     if (pos0 < 0 || last - pos0 != tokens - 1) {  // positions must be contiguous and non-negative
         if (threadIdx.x == 0) L.flag(KVB_ERR_POSITIONS);
@@ -525,7 +525,7 @@ int launch_append(const LayerView& V, const void* k, const void* v, const int32_
     KVB_CUDA_OK(allow_smem(opted, append_kernel<D, kBf16>, smem));
     const dim3 grid(tokens / kTile + 2, V.kv_heads, 2 * Geo<D>::S);
     KVB_CUDA_OK(launch_early(append_kernel<D, kBf16>, grid, dim3(kThreads), smem, stream, V, static_cast<const uint16_t*>(k), static_cast<const uint16_t*>(v),
-                             positions, tokens, append_starts_next(D, tokens)));
+                             positions, tokens));
     return KVB_OK;
 }
 
