@@ -1,7 +1,7 @@
 // kvb_append.cu -- quantise-append into the paged pool, and the tile decode used for verification.
 //
 // One launch covers any token count: the grid is (tile slot of the append, kv head, K|V x 128-dim slice).  A CTA rotates the
-// new rows with one warp per row (Walsh-Hadamard in registers + shuffles), keeps its slice of the 128-token tile in shared
+// new rows with 32 dims of a row a lane (Walsh-Hadamard in registers, shuffles last), keeps its slice of the 128-token tile in shared
 // memory, and -- when the append completes the tile -- quantises it: per-row min/max -> fp16 scale / zero-point -> 4-bit
 // codes, written to the two pages of the tile.  At head_dim 256 the slices are separate CTAs (each rotates the whole row:
 // cheap beside the balancing of its slice).  There is no intermediate record and no bit-serial packing.
@@ -95,14 +95,14 @@ __device__ __forceinline__ float rcp_newton(float x) {
 // outside the row sums, so the deviations after it come from the sums before it.  Threads 0..127 own column i and row i and hold
 // their factors; the reference's running sum of clamped logarithms is kept as the running product it stands for, clamped to the same
 // range, which leaves a reciprocal square root, a few products and a reciprocal between the sums and the next factors.  Threads
-// 128..255 judge the states meanwhile: the extremes of a state's deviations while the rows of the next are updated, the verdict while
+// 128..255 rate the states meanwhile: the extremes of a state's deviations while the rows of the next are updated, the verdict while
 // its columns are.  Two passes (in pairs of elements) and four barriers a round; bound by the chain pass, barrier, factors, barrier: 1.0
 // us a round.  Measured on B200, 1,024 tokens, 4 heads of 256 dims, 16 rounds: 36.3 -> 31.8 us a call (logf and expf per round, the
 // owners judging, single elements before).
 template <bool kValue>
 __device__ void sinkhorn(AppendSmem& sm, const float (&by_token)[kPer], const float (&by_dim)[kPer], int iters) {
     const int i = threadIdx.x, j = i & (kSlice - 1);
-    const bool owner = i < kSlice, judge = i >= kSlice && i < 2 * kSlice;
+    const bool owner = i < kSlice, rater = i >= kSlice && i < 2 * kSlice;
     auto sums = [&](const float (&x)[kPer], const float* factors, int part, int index) {
         F2 s(0.0f, 0.0f), q(0.0f, 0.0f);
 #pragma unroll
@@ -174,7 +174,7 @@ __device__ void sinkhorn(AppendSmem& sm, const float (&by_token)[kPer], const fl
             rcp_col = rcp_newton(cur_col);
             set_col(rcp_col);
         }
-        if (judge && it > 0) keep_best();
+        if (rater && it > 0) keep_best();
         __syncthreads();
         row_pass();
         __syncthreads();
@@ -185,7 +185,7 @@ __device__ void sinkhorn(AppendSmem& sm, const float (&by_token)[kPer], const fl
             set_row(rcp_row);
             dev_row = dev * rcp_row;
         }
-        if (judge) {
+        if (rater) {
             look();
             seen = sm.state_fac[j];
         }
@@ -197,14 +197,14 @@ __device__ void sinkhorn(AppendSmem& sm, const float (&by_token)[kPer], const fl
         dev_col = deviation() * rcp_col;
         hand_over();
     }
-    if (judge && iters > 0) keep_best();
+    if (rater && iters > 0) keep_best();
     __syncthreads();
-    if (judge) {
+    if (rater) {
         look();
         seen = sm.state_fac[j];
     }
     __syncthreads();
-    if (judge) {
+    if (rater) {
         keep_best();
         sm.best_col[j] = best_col;
         sm.best_row[j] = best_row;

@@ -1628,8 +1628,8 @@ int launch_attention(const kvb_layer* layer, const void* q, const int32_t* pos_d
 
 // From this many GQA-merged query rows per KV head on, steps run on the tcgen05 kernel.  Measured on B200 in graph replay, 24 / 4
 // heads, 131,072 tokens, us a layer for widths 3 .. 8 (18 .. 48 rows) on the warp-level kernel and on this one: unbalanced
-// 54.3 53.1 69.3 85.6 99.6 96.9 against 64.0 65.2 65.6 66.4 68.3 68.5, balanced 71.8 71.3 71.6 99.7 99.4 97.2 against 70.0 70.3
-// 70.7 71.4 73.2 73.5.  (At 30 rows the tensor cores would be faster, but K and V are rounded to fp16 there.)
+// 53.4 52.4 67.0 83.1 96.6 95.3 against 58.7 59.4 59.8 60.5 62.4 63.3, balanced 68.7 68.8 69.6 97.0 97.0 95.5 against 59.4 62.5
+// 63.7 61.2 63.3 63.8.  (At 30 rows, balanced from 18 on, the tensor cores would be faster, but K and V are rounded to fp16 there.)
 static constexpr int kDenseRows = 32;
 extern "C" int kvb_split_capacity(int kv_len_max, int kv_heads, int q_heads, int rows, int batch) {
     (void)batch;

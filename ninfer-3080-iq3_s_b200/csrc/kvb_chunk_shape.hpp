@@ -17,10 +17,10 @@ struct ShapeCost {
     int min_steps;     // key steps a range has at least (one range always goes)
     int parts;         // partials a row gets per range
 };
-// head_dim 128, in fifths of the time a row tile takes for a key tile with two row tiles a CTA (1.2 us, measured at 1,024 tokens over
+// head_dim 128, in fifths of the time a row tile takes for a key tile with two row tiles a CTA (1.15 us, measured at 1,024 tokens over
 // 262,144; with split keys 1.7 us): a step of two row tiles costs 10, one with split keys 7, set-up and epilogue about 17 and 12 us.
-// Measured, the kernel alone: 1,024 tokens over 262,144 3.30 ms with two row tiles, 4.70 ms with split keys; 777 tokens alone 36.4 and
-// 25.0 us (their append included 38.3 and 35.2).  The costs are those of ranges that are merged: that one range writes no partials and
+// Measured, the kernel alone: 1,024 tokens over 262,144 3.06 ms with two row tiles, 4.49 ms with split keys; 777 tokens alone 35.6 and
+// 23.9 us (their append included 36.8 and 29.2).  The costs are those of ranges that are merged: that one range writes no partials and
 // needs no merge kernel is not in them.
 constexpr ShapeCost kTwoTiles{70, 10, 2, 1}, kSplitKeys{50, 7, 2, 2};
 // head_dim 256: a CTA costs its pages plus about six pages' worth of set-up and epilogue.
