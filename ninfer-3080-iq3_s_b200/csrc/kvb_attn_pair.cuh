@@ -202,7 +202,7 @@ __device__ __forceinline__ void attn_pair_cta(const AttnParams& P, int split, in
     {
         const int pb = min(key_begin / kPage, sealed_pages), pe = min((key_end + kPage - 1) / kPage, sealed_pages);
         int c0, c1;
-        split_pages<kPairs>(max(pe - pb, 0), kv_total % kTile, split, P.nsplit, P.by, c0, c1);
+        split_pages<kPairs, 2>(max(pe - pb, 0), kv_total % kTile, split, P.nsplit, P.by, c0, c1);
         const bool last_first = c1 - c0 < 3 * kPairs || split == P.nsplit - 1;
         w0 = pb + c0 + warp_pages<kPairs>(c1 - c0, pair, last_first);
         w1 = pb + c0 + warp_pages<kPairs>(c1 - c0, pair + 1, last_first);
