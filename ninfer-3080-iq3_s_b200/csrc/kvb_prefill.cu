@@ -27,6 +27,7 @@
 #include "kvb_chunk_merge.cuh"
 #include "kvb_common.cuh"
 #include "kvb_tcgen05.cuh"
+#include "kvb_walk.hpp"
 
 #include <cstddef>
 
@@ -554,16 +555,16 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
         const int min_pos = __reduce_min_sync(0xffffffffu, is_row ? my_pos : INT_MAX);
         const int steps = steps_of(u);
         float m_run = -INFINITY, l_run = 0.0f;
-        for (int i = 0; i < steps && !failed; ++i) {
+        Walk<Ro::kHalves == 2> walk;
+        for (int i = 0; i < steps; ++i) {
             const int j = kSplit ? 2 * i + u : i;
 #pragma unroll 1
             for (int h = 0; h < Ro::kParts; ++h) {
                 const int base = (t0 + j) * kN + (kN / Ro::kParts) * h + kKeys * half;
                 // P of the two warps lies side by side over S of the part, which both have read when they meet
                 const uint32_t ts = tmem + 128 * u + (kN / Ro::kParts) * h + kKeys * half + lane_base, tp = ts - (Ro::kHalves == 2 ? kKeys / 2 * half : 0);
-                if (!chunk_wait(&sm.s_full[u][h], i & 1, &sm.abort_flag)) failed = true;
-                // (two warps that share rows leave together: the one that gave up still meets the other at their barrier below)
-                if (failed && (Ro::kHalves == 1 || !warp_has_rows)) break;
+                walk.waited(chunk_wait(&sm.s_full[u][h], i & 1, &sm.abort_flag));
+                if (walk.leaves_alone(warp_has_rows)) { i = steps; break; }
                 tc::fence_after_sync();
                 if (warp_has_rows) {
                     const bool bad_tile = sm.bad_tile[j & (kSlotsMeta - 1)] != 0;
@@ -606,7 +607,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
                         mask(s0, 0);
                         mx = top(s0);
                         sm.row_top[u][h][half][row] = mx;
-                        if (named_barrier_or(3 + 4 * u + (warp & 3), 64, failed)) { failed = true; break; }  // the two warps of these 32 rows
+                        if (walk.leaves_together(named_barrier_or(3 + 4 * u + (warp & 3), 64, walk.failed))) { i = steps; break; }  // the two warps of these 32 rows
                         mx = fmaxf(mx, sm.row_top[u][h][half ^ 1][row]);
                     }
                     // The reference point of the row's exponentials follows the running maximum lazily: it moves only when the
@@ -646,8 +647,8 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
                     l_run = l_run * alpha + (sum2.x + sum2.y);
                     if (i + h > 0 && __any_sync(0xffffffffu, grown)) {
                         // P V of step i - 1 completed before S of step i was issued; that of this step's first part may still run
-                        if (h > 0 && !chunk_wait(&sm.o_done[u][0], i & 1, &sm.abort_flag)) failed = true;
-                        if (Ro::kParts == 2 && h == 0 && !chunk_wait(&sm.o_done[u][1], (i - 1) & 1, &sm.abort_flag)) failed = true;
+                        if (h > 0) walk.waited(chunk_wait(&sm.o_done[u][0], i & 1, &sm.abort_flag));
+                        if (Ro::kParts == 2 && h == 0) walk.waited(chunk_wait(&sm.o_done[u][1], (i - 1) & 1, &sm.abort_flag));
                         tc::fence_after_sync();
 #pragma unroll 1
                         for (int c = 0; c < kCols / 32; ++c) {
@@ -666,6 +667,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
                 if (lane == 0) mbar_arrive(&sm.p_full[u][h]);
             }
         }
+        failed = walk.failed;
         // ---- partial of this (row tile, key range): m (log2 units), l, o in tile dim order
 #pragma unroll
         for (int h = 0; h < Ro::kParts; ++h)
