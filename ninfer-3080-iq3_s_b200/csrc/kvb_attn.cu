@@ -36,6 +36,7 @@
 
 #include "kvb_common.cuh"
 #include "kvb_ptx.cuh"
+#include "kvb_shares.hpp"
 
 namespace kvb {
 namespace {
@@ -72,13 +73,6 @@ struct Shape {
 template <int NB> struct VSlot {
     static constexpr int kShift = NB == 2 ? 0 : 16, kSubs = kShift ? 4 : 1, kSubBytes = Shape::kChunk / kSubs;
     static constexpr int kBytes = (Shape::kChunk + (kSubs - 1) * kShift + 127) / 128 * 128;
-};
-
-// Division by a number of splits as a multiplication; exact below 2^26.
-struct SplitBy {
-    uint32_t all, others;  // 2^32 / nsplit, / (nsplit - 1), rounded up (0: by one)
-    __host__ __device__ static uint32_t inverse(int d) { return d > 1 ? 0xFFFFFFFFu / static_cast<uint32_t>(d) + 1u : 0u; }
-    __device__ static int divide(int n, uint32_t inv) { return inv != 0u ? static_cast<int>(__umulhi(static_cast<uint32_t>(n), inv)) : n; }
 };
 
 struct AttnParams {
@@ -387,42 +381,6 @@ __device__ __forceinline__ void process_stage_group(const __half* krow, const __
     }
 }
 
-// Pages of split `split` of `n` pages, which its CTA walks W at a time.  The last split has the open tile as well, whose 16-key groups (a
-// warp or pair each) count as 3/4 of a page; it takes no page that would be a round more for those with a group.  Neither may cost the
-// other splits a round.  From eight rounds on (128 dims) the pages alone are shared, evenly: 4-row verify at 126,000 / 127,526 tokens 49.0 /
-// 51.1 -> 48.3 / 48.9, at 129,000 51.4 -> 52.0, decode at 378,944 45.7 -> 46.1; 256 dims 45,000 62.0 63.5, not there.  Measured on B200 in graph replay, append and attention, us a layer, equal shares (by 64-bit divisions, the first
-// position read behind the newest, the next kernel's start by every warp) against this: decode at 300 / 1,500 / 8,000 / 32,768 / 65,536 /
-// 378,944 tokens 8.6 / 9.1 / 10.2 / 12.6 / 17.8 / 49.4 8.1 7.8 8.7 12.6 17.6 49.1, 256 dims 1,500 / 4,000 / 30,011 14.2 / 13.2 / 23.1 11.5 11.6 21.0, verify of 4
-// rows at 1,500 / 8,000 / 131,072 9.2 / 11.6 / 52.0 7.8 10.7 52.2, of 5 rows of 256 dims at 20,000 35.9 35.3.  A CTA with the open tile was
-// some 2,000 cycles behind the others.
-constexpr int kManyRounds = 8;
-template <int W, int kSlices> __device__ __forceinline__ void split_pages(int n, int open_keys, int split, int nsplit, SplitBy by, int& begin, int& end) {
-    const int groups = (open_keys + 15) / 16, weighted = n + groups * 3 / 4;
-    int share = SplitBy::divide(n, by.all), more = n - share * nsplit;  // `more` splits have a page more
-    const int rounds = (share + (more != 0) + W - 1) / W, keep = rounds * W - groups;
-    if (kSlices == 1 && rounds >= kManyRounds) {
-        begin = share * split + SplitBy::divide(more * split, by.all);
-        end = share * (split + 1) + SplitBy::divide(more * (split + 1), by.all);
-        return;
-    }
-    if (weighted <= rounds * W * nsplit) {
-        share = SplitBy::divide(weighted, by.all);
-        more = weighted - share * nsplit;
-    }
-    if (nsplit > 1 && n - share * (nsplit - 1) - more > keep && n - keep <= rounds * W * (nsplit - 1)) {
-        share = SplitBy::divide(n - keep, by.others);
-        more = n - keep - share * (nsplit - 1);
-    }
-    begin = min(share * split + min(split, more), n);
-    end = split == nsplit - 1 ? n : min(begin + share + (split < more), n);
-}
-// Pages of warp (or pair) w of the W of a CTA with n.  Over few rounds, and beside the open tile, whose groups the first ones have, the last
-// ones take a page more (the first ones rotate the query before they begin); over many, every so many-th.
-template <int W> __device__ __forceinline__ int warp_pages(int n, int w, bool last_first) {
-    const int share = n / W;
-    return last_first ? share * w + max(w - (W - (n - share * W)), 0) : n * w / W;
-}
-
 // The work of one CTA: split `split` of KV head `head`, row block `zb`; its partial goes to rows pidx .. pidx + 15 of
 // the workspace.  NB = 8-row blocks of query rows per warp.  A pass = one page: its 64 logits per row are held at
 // once.  Within a page the keys are taken in a fixed permutation (see key_lo below) that lets the QK accumulators
@@ -470,7 +428,7 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
             }
         }
     }
-    const int pos0 = P.pos[0], kv_total = *P.total_pos + 1;
+    const int pos0 = P.pos[0], kv_total = max(*P.total_pos + 1, 0);  // (a negative position: no key)
     const int key_end = min(P.key_end, kv_total), key_begin = max(P.key_begin, 0);
     const int sealed_pages = 2 * (kv_total / kTile);
 

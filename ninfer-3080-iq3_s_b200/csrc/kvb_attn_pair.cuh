@@ -188,7 +188,7 @@ __device__ __forceinline__ void attn_pair_cta(const AttnParams& P, int split, in
             qpos = P.pos[tq];
         }
     }
-    const int pos0 = P.pos[0], kv_total = *P.total_pos + 1;
+    const int pos0 = P.pos[0], kv_total = max(*P.total_pos + 1, 0);  // (a negative position: no key)
     const int key_end = min(P.key_end, kv_total), key_begin = max(P.key_begin, 0);
     const int sealed_pages = 2 * (kv_total / kTile);
     if (threadIdx.x < 2 * kRows) (&sm.poison[0][0])[threadIdx.x] = 0;

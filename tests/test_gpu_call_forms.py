@@ -318,3 +318,32 @@ def test_bad_page_in_the_prefix_of_a_chunk(D, H, QH, ctx, tokens, bad):
     want = _chunk_reference(tw, qn, at, T, without=(page // 2 * 128, (page // 2 + 1) * 128) if tile else (64 * page, 64 * (page + 1)))
     ok, msg = attn_close(out.float().cpu().numpy(), want, *((PREFILL_MAX_ABS, PREFILL_REL_L2) if tile else (ATTN_MAX_ABS, ATTN_REL_L2)))
     assert ok, msg
+
+
+@pytest.mark.parametrize("D", [128, 256])
+@pytest.mark.parametrize("bound", [400, 20000])
+@pytest.mark.parametrize("newest", [-48, -50, -129, -100000])
+def test_a_newest_position_below_zero(D, bound, newest):
+    """No key is there: zeros by every entry point, on any number of splits, and what an append says of the positions."""
+    import torch
+
+    H, QH, scale = 4, 24, 1.0 / np.sqrt(D)
+    tw = _filled(D, H, QH, 300, room=20000)
+    L, bad = tw.gpu, pkg().capi.ERR_POSITIONS
+
+    def rows(n, heads):
+        return torch.ones((n, heads, D), dtype=torch.float16, device=tw.dev)
+
+    def zeros(out, errors):
+        torch.cuda.synchronize()
+        assert torch.all(out == 0.0) and L.errors() == errors
+        L.error_word.zero_()
+
+    at = torch.arange(newest - 39, newest + 1, dtype=torch.int32, device=tw.dev)
+    zeros(L.attn_decode(rows(1, QH)[0], at[39:], scale, bound), 0)
+    zeros(L.append_decode(rows(1, QH)[0], rows(1, H), rows(1, H), at[39:], scale, bound), bad)
+    for n in (2, 5, 8):
+        zeros(L.attn_verify(rows(n, QH), rows(n, H), rows(n, H), at[40 - n:], scale, bound), bad)
+    zeros(L.attn_prefill(rows(40, QH), rows(40, H), rows(40, H), at, scale, bound), bad)
+    if D == 128:
+        zeros(pkg().DecodeBatch([L, L], [bound, bound]).attn_decode(rows(2, QH), at[39:].repeat(2), scale), 0)
