@@ -564,18 +564,19 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
     bool timed_out = false;
     int slot = 0;          // slot of the oldest chunk not yet released
     uint32_t phases = 0;   // bit s: parity the next wait on slot s expects
-    // Wait for the chunk in slot s (bounded).  Behind it the warp is together again: ldmatrix, movmatrix and the MMAs are instructions of
-    // a converged warp.  Two forms of the same: a vote on the first probe, which usually succeeds in all lanes, for K; a verdict per lane
-    // (a lane that has to keep probing finds the barrier complete as soon as any lane has) and __syncwarp for V.  Measured on B200, us
-    // a layer, these / votes for both / __syncwarp for both / neither: decode at 131,072 tokens 21.8 22.0 21.7 21.9, at 378,944 47.1 47.0 47.9 47.0,
-    // 2 rows at 131,072 36.9 36.8 38.5 38.6, 5 rows 69.5 70.1 68.9 69.1.
+    // Wait for the chunk in slot s (bounded).  Behind it the warp is together again, with one verdict: ldmatrix, movmatrix and the MMAs are
+    // instructions of a converged warp.  A chunk that was given up is still on its way: the warp leaves the walk with the chunk's slot
+    // as it is, for the last wait below.  A vote on the first probe, which usually succeeds in all lanes, for K; for V a verdict per lane (a
+    // lane that has to keep probing finds the barrier complete as soon as any lane has), then a vote.  Measured on B200 in graph replay, us a
+    // layer, __syncwarp behind V and a vote at the next page / this / the vote behind the products of V: decode at 131,072 tokens 21.5
+    // 21.2 21.2, at 378,944 46.4 45.3 45.9, verify of 2 / 4 / 5 rows at 131,072 39.9 / 51.9 / 66.9  39.1 / 50.9 / 65.6  39.1 / 51.2 / 66.0,
+    // append and decode at 1,500 / 4,000 7.9 / 8.2  7.9 / 8.2  8.2 / 8.5.
     auto wait_k = [&](int s) {
-        if (timed_out) return;
-        timed_out = !__all_sync(0xffffffffu, mbar_try_wait(&bars[s], (phases >> s) & 1u)) && !mbar_wait_bounded(&bars[s], (phases >> s) & 1u);
+        timed_out = !kStepWaitsK || (!__all_sync(0xffffffffu, mbar_try_wait(&bars[s], (phases >> s) & 1u)) && !mbar_wait_bounded(&bars[s], (phases >> s) & 1u));
     };
     auto wait_v = [&](int s) {
-        if (!timed_out && !mbar_try_wait(&bars[s], (phases >> s) & 1u) && !mbar_wait_lane_bounded(&bars[s], (phases >> s) & 1u)) timed_out = true;
-        __syncwarp();
+        if (!kStepWaitsV || (!mbar_try_wait(&bars[s], (phases >> s) & 1u) && !mbar_wait_lane_bounded(&bars[s], (phases >> s) & 1u))) timed_out = true;
+        timed_out = __any_sync(0xffffffffu, timed_out);
     };
     auto release_chunk = [&](bool was_live) {  // the chunk in `slot` has been read by every lane: refill the slot, advance
         if (was_live) phases ^= 1u << slot;
@@ -599,8 +600,6 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
     int cur_tile = -1;
     for (int pi = 0; pi < npages; ++pi) {
         const int lp = w0 + pi;
-        timed_out = __any_sync(0xffffffffu, timed_out);  // one verdict for the warp before anything branches on it
-        if (timed_out) break;
         if (!((live >> slot) & 1u)) {  // a page that could not be addressed: nothing was copied, nothing is read
             release_chunk(false);
             release_chunk(false);
@@ -608,6 +607,7 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
         }
         // ---- K chunk + header
         wait_k(slot);
+        if (timed_out) break;
         const uint8_t* hdr = R.hdr[pi % kHdrs];
         if ((lp >> 1) != cur_tile) {  // per-dim scale / zero point of K belong to the tile
             cur_tile = lp >> 1;
@@ -836,6 +836,7 @@ __device__ __forceinline__ void attn_cta(const AttnParams& P, int split, int hea
         //      gathers the rows of two matrices of a dim pair, one AND isolates the even dim (x) or 16 x the odd dim (y): the k
         //      slots of MMA c, matching groups 2c and 2c + 1.
         wait_v(slot);
+        if (timed_out) break;
         {
             // lane L addresses row L & 7 of matrix L >> 3, shifted with its sub-block
             const int vrow = lane & 7, vmat = lane >> 3;

@@ -387,8 +387,8 @@ __device__ __forceinline__ void attn_pair_cta(const AttnParams& P, int split, in
     bool timed_out = false;
     int slot = 0;          // slot of the oldest chunk not yet released
     uint32_t phases = 0;   // bit i: parity the next wait on slot i expects
-    auto wait_chunk = [&](int i) {  // bounded; behind it the warp is together again (see attn_cta)
-        if (!__all_sync(0xffffffffu, mbar_try_wait(&bars[i], (phases >> i) & 1u)) && !mbar_wait_bounded(&bars[i], (phases >> i) & 1u)) timed_out = true;
+    auto wait_chunk = [&](int i, bool waits) {  // bounded; behind it the warp is together again (see attn_cta)
+        if (!waits || (!__all_sync(0xffffffffu, mbar_try_wait(&bars[i], (phases >> i) & 1u)) && !mbar_wait_bounded(&bars[i], (phases >> i) & 1u))) timed_out = true;
     };
     auto release_chunk = [&](bool was_live) {  // the chunk in `slot` has been read by both warps: refill the slot, advance
         if (was_live) phases ^= 1u << slot;
@@ -411,7 +411,7 @@ __device__ __forceinline__ void attn_pair_cta(const AttnParams& P, int split, in
             continue;
         }
         // ---- K chunk + header
-        wait_chunk(slot);
+        wait_chunk(slot, kStepWaitsK);
         uint8_t* const hdr = R.hdr[pi % kHdrs];
         uint32_t sc;  // the lane's largest scale of V
         {
@@ -569,7 +569,7 @@ __device__ __forceinline__ void attn_pair_cta(const AttnParams& P, int split, in
             wq = F2(wpass[0] * invF, wpass[1] * invF);
         }
         // ---- PV on the int8 path, see attn_cta: key i' + 4c of each of the eight shifted sub-blocks
-        wait_chunk(slot);
+        wait_chunk(slot, kStepWaitsV);
         {
             const int vrow = lane & 7, vmat = lane >> 3;
             const uint8_t* ch = R.slots[slot] + (8 * vrow + vmat) * 128 + Pair::kShift * vrow + 64 * s;
@@ -616,7 +616,8 @@ __device__ __forceinline__ void attn_pair_cta(const AttnParams& P, int split, in
                     }
             }
         }
-        named_barrier_sync(pair_barrier, 64);  // V and the header have been read by both
+        // V and the header have been read by both, or one has given it up: it is still on its way, and its slot stays as it is
+        if (named_barrier_or(pair_barrier, 64, timed_out)) { timed_out = true; break; }
         release_chunk(true);
     }
     if (timed_out) {

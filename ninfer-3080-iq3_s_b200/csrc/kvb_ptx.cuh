@@ -48,6 +48,16 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     return __all_sync(0xffffffffu, ok);
 }
 
+// The waits of a decode or verify step for a chunk of K or of V: the same.  (A test builds that kernel with waits that give up at once,
+// for chunks that then land all the same.)
+#ifndef KVB_STEP_PROBES_K
+#define KVB_STEP_PROBES_K kSpinLimit
+#endif
+#ifndef KVB_STEP_PROBES_V
+#define KVB_STEP_PROBES_V kSpinLimit
+#endif
+constexpr bool kStepWaitsK = (KVB_STEP_PROBES_K) > 0, kStepWaitsV = (KVB_STEP_PROBES_V) > 0;
+
 // The same wait for lanes that may have diverged (some found the barrier complete at their first probe): no vote.
 // Every lane probes the same barrier phase, so a lane can run out of probes only if no lane ever saw it complete.
 __device__ __forceinline__ bool mbar_wait_lane_bounded(uint64_t* bar, uint32_t parity) {
