@@ -1464,14 +1464,39 @@ cudaError_t launch_attn_pair(dim3 grid, cudaStream_t stream, const AttnParams& P
 constexpr int kShortClusters = 12;
 constexpr int short_keys(int head_dim) { return head_dim == 128 ? 3072 : 1536; }
 // The same as clusters: the splits of a head and row block.
-template <int S, int NB, bool kOther>
-cudaError_t launch_short(dim3 grid, cudaStream_t stream, const AttnParams& P, uint16_t* out) {
-    constexpr int warps = S == 1 ? kWarpsWide : kPairWarps;
-    constexpr int smem = static_cast<int>(S == 1 ? sizeof(AttnSmem<NB, kWarpsWide>) + sizeof(ClusterPart) : sizeof(PairSmem));
-    static OncePerDevice opted;
-    if (const cudaError_t e = allow_smem(opted, attn_short_kernel<S, NB, kOther>, smem)) return e;
-    return launch_early_cluster(attn_short_kernel<S, NB, kOther>, grid, dim3(warps * 32), smem, static_cast<int>(grid.x), stream, P, out);
-}
+template <int S, int NB, bool kOther> struct Short {
+    static constexpr int kThreads = 32 * (S == 1 ? kWarpsWide : kPairWarps);
+    static constexpr int kSmem = static_cast<int>(S == 1 ? sizeof(AttnSmem<NB, kWarpsWide>) + sizeof(ClusterPart) : sizeof(PairSmem));
+    // Whether the device holds the largest such cluster at all: an SM holds one of its CTAs, and a part of a GPU may have fewer SMs beside each
+    // other.  Asked once per device, behind the opt-in to the shared memory, which the launch needs.
+    static bool held() {
+#ifdef KVB_NO_CLUSTERS  // (a test builds it for a device that holds none)
+        return false;
+#endif
+        static std::atomic<int> cache[64];  // 0: not asked yet, 1: no, 2: yes
+        const int dev = current_device();
+        int known = dev < 0 || dev >= 64 ? 0 : cache[dev].load(std::memory_order_acquire);
+        if (known == 0) {
+            int clusters = 0;
+            known = 1;
+            if (cudaFuncSetAttribute(attn_short_kernel<S, NB, kOther>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) == cudaSuccess &&
+                clusters_held(attn_short_kernel<S, NB, kOther>, kShortSplits, dim3(kThreads), kSmem, &clusters) == cudaSuccess && clusters > 0)
+                known = 2;
+            cudaGetLastError();  // the merge kernel's route needs none
+            if (dev >= 0 && dev < 64) cache[dev].store(known, std::memory_order_release);
+        }
+        return known == 2;
+    }
+    // Behind held().
+    static cudaError_t launch(dim3 grid, cudaStream_t stream, const AttnParams& P, uint16_t* out) {
+        return launch_early_cluster(attn_short_kernel<S, NB, kOther>, grid, dim3(kThreads), kSmem, static_cast<int>(grid.x), stream, P, out);
+    }
+};
+struct ShortCall {
+    bool (*held)();
+    cudaError_t (*launch)(dim3, cudaStream_t, const AttnParams&, uint16_t*);
+};
+template <int S, int NB, bool kOther> ShortCall short_call() { return {Short<S, NB, kOther>::held, Short<S, NB, kOther>::launch}; }
 
 // Warps per CTA for a decode call: 8, 12 or 16 (whole warp quartets: an SM hands registers and issue slots out per
 // quartet; 10 or 14 warps measured no faster per warp than 12 or 16).  A warp works on whole pages, so a CTA with n
@@ -1532,8 +1557,13 @@ int launch_attention(const kvb_layer* layer, const void* q, const int32_t* pos_d
     const RowPlan plan = plan_rows(kv_len_max, layer->kv_heads, layer->q_heads, layer->head_dim, T, layer->sinkhorn_iters != 0);
     // The output may be stored while others still read q, the positions and, behind an append, its rows?
     const size_t out_bytes = static_cast<size_t>(T) * layer->q_heads * layer->head_dim * sizeof(uint16_t);
+    const bool upper = plan.nb == 2, other = layer->sinkhorn_iters != 0;
+    const ShortCall as_clusters = layer->head_dim != 128 ? short_call<2, 1, true>()
+                                  : upper                ? (other ? short_call<1, 2, true>() : short_call<1, 2, false>())
+                                                         : (other ? short_call<1, 1, true>() : short_call<1, 1, false>());
     const bool clustered = kv_len_max <= short_keys(layer->head_dim) && layer->kv_heads * plan.zblocks <= kShortClusters && out != nullptr && part_m == nullptr && push == nullptr &&
-                           stores_beside(span_of(out, out_bytes), span_of(q, out_bytes), span_of(pos_dev, T * sizeof(int32_t)), span_of(total_pos_dev, sizeof(int32_t)));
+                           stores_beside(span_of(out, out_bytes), span_of(q, out_bytes), span_of(pos_dev, T * sizeof(int32_t)), span_of(total_pos_dev, sizeof(int32_t))) &&
+                           as_clusters.held();
     const int Z = plan.zblocks, nsplit = clustered ? std::min(plan.nsplit, kShortSplits) : plan.nsplit;
     const int parts = nsplit;
     AttnParams P;
@@ -1553,20 +1583,14 @@ int launch_attention(const kvb_layer* layer, const void* q, const int32_t* pos_d
     P.ws_l = P.ws_m + rows;
     P.ws_o = P.ws_l + rows;
     P.after_append = starts_beside(behind, clustered ? span_of(out, out_bytes) : span_of(P.ws_m, rows * (2 + layer->head_dim) * sizeof(float)));
-    const bool upper = plan.nb == 2;
     const dim3 grid(parts, layer->kv_heads, Z);
     if (clustered) {
-        uint16_t* const to = static_cast<uint16_t*>(out);
-        const bool other = layer->sinkhorn_iters != 0;
-        const auto launch = layer->head_dim != 128 ? launch_short<2, 1, true>
-                            : upper                ? (other ? launch_short<1, 2, true> : launch_short<1, 2, false>)
-                                                   : (other ? launch_short<1, 1, true> : launch_short<1, 1, false>);
-        KVB_CUDA_OK(launch(grid, stream, P, to));
+        KVB_CUDA_OK(as_clusters.launch(grid, stream, P, static_cast<uint16_t*>(out)));
         return KVB_OK;
     }
     if (layer->head_dim != 128) {  // the factors of balanced caches are applied whatever the descriptor says: at this head dim a reader need not know the count
         KVB_CUDA_OK(launch_attn_pair(grid, stream, P));
-    } else if (layer->sinkhorn_iters != 0) {  // balanced caches: other_K per key, other_V per dim (more registers: 8 warps)
+    } else if (other) {  // balanced caches: other_K per key, other_V per dim (more registers: 8 warps)
         if (upper) {
             KVB_CUDA_OK((launch_attn<2, kWarpsWide, true>(grid, stream, P)));
         } else {

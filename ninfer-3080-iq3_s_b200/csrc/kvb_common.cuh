@@ -126,6 +126,21 @@ inline cudaError_t launch_early_cluster(void (*kernel)(KArgs...), dim3 grid, dim
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// How many clusters of `cluster` such CTAs the device can run at once.
+template <typename K> cudaError_t clusters_held(K* kernel, int cluster, dim3 block, size_t smem, int* clusters) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(cluster);
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = static_cast<unsigned>(cluster);
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaOccupancyMaxActiveClusters(clusters, kernel, &cfg);
+}
+
 inline int current_device() {  // -1: unknown
     int dev = -1;
     return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
