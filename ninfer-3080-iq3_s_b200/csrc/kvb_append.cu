@@ -299,20 +299,15 @@ __device__ void quantize_slice(AppendSmem& sm, float (&x)[kPer]) {
     __syncthreads();
 }
 
-__device__ __noinline__ uint4 load8(const uint16_t* p) {  // from any 2-byte boundary
-    return make_uint4(p[0] | static_cast<uint32_t>(p[1]) << 16, p[2] | static_cast<uint32_t>(p[3]) << 16, p[4] | static_cast<uint32_t>(p[5]) << 16,
-                      p[6] | static_cast<uint32_t>(p[7]) << 16);
-}
-
 // The new rows begin .. end - 1 of tile `base`, rotated (stages, order and roundings of hadamard_warp).  A lane holds 32 neighbouring
 // dims of a row: D / 32 lanes a row, 1024 / D rows a warp at a time; the strides up to 16 stay inside a lane, in pairs of dims, those of
 // 32 and more cross lanes, and rows are read and stored 16 bytes at a time.  A warp has up to 8 rows of the tile and reads them all before
 // rotating any: it waits for global memory once.  `keep(row, d, x)` takes dims d .. d + 7 of the slice.  Measured on B200 against a
 // warp a row with dims l + 32 r in lane l (five strides by shuffles, two bytes an access) and a division a code, 1,024 tokens, us a call:
 // 128 dims 9.9 -> 7.4, 256 dims 13.2 -> 9.8, with 16 rounds of balancing 31.8 -> 27.1; a prompt of 777 tokens 32.6 -> 29.2.
-// `wide`: the rows start at 16-byte boundaries.
+// The rows start at 16-byte boundaries.
 template <int D, bool kBf16, typename Keep>
-__device__ __forceinline__ void rotate_rows(const uint16_t* __restrict__ src, int64_t row_stride, bool wide, int begin, int end, int slice, Keep keep) {
+__device__ __forceinline__ void rotate_rows(const uint16_t* __restrict__ src, int64_t row_stride, int begin, int end, int slice, Keep keep) {
     constexpr int kLanes = D / 32, kAtOnce = 32 / kLanes, kWarpsPerCta = kThreads / 32, kPasses = kTile / (kWarpsPerCta * kAtOnce);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, block = lane % kLanes;
     uint4 raw[kPasses][4];
@@ -321,7 +316,7 @@ __device__ __forceinline__ void rotate_rows(const uint16_t* __restrict__ src, in
         const int tt = begin + warp + kWarpsPerCta * (u * kAtOnce + lane / kLanes);
         const uint16_t* row = src + (tt - begin) * row_stride + 32 * block;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) raw[u][c] = tt >= end ? make_uint4(0u, 0u, 0u, 0u) : wide ? reinterpret_cast<const uint4*>(row)[c] : load8(row + 8 * c);
+        for (int c = 0; c < 4; ++c) raw[u][c] = tt >= end ? make_uint4(0u, 0u, 0u, 0u) : reinterpret_cast<const uint4*>(row)[c];
     }
 #pragma unroll
     for (int u = 0; u < kPasses; ++u) {
@@ -372,6 +367,42 @@ __device__ __forceinline__ void rotate_rows(const uint16_t* __restrict__ src, in
     }
 }
 
+// The same, a warp a row with dims l + 32 r in lane l: from any 2-byte boundary, up to 16 kBatch rows.  `keep(row, d, h)` takes dim d of the
+// slice.
+template <int D, bool kBf16, int kBatch, typename Keep>
+__device__ __forceinline__ void rotate_rows_singly(const uint16_t* __restrict__ src, int64_t row_stride, int begin, int end, int slice, Keep keep) {
+    constexpr int kWarpsPerCta = kThreads / 32;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint16_t raw[kBatch][D / 32];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+        const int tt = begin + warp + u * kWarpsPerCta;
+        if (tt < end) {
+            const uint16_t* row = src + (tt - begin) * row_stride;
+#pragma unroll
+            for (int r = 0; r < D / 32; ++r) raw[u][r] = row[lane + 32 * r];
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+        const int tt = begin + warp + u * kWarpsPerCta;
+        if (tt >= end) break;
+        float val[D / 32];
+#pragma unroll
+        for (int r = 0; r < D / 32; ++r) val[r] = in_to_f32<kBf16>(raw[u][r]);
+        hadamard_warp<D>(val, lane);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) keep(tt, lane + 32 * r, __float2half_rn(D == 128 || slice == 0 ? val[r] : val[D / 32 - 4 + r]));
+    }
+}
+
+// Whether the rows of a tile are rotated a warp each though they could go 32 dims a lane: up to 16 rows have a warp each either way, and a lane
+// with 32 dims of one is the longer chain.  Measured on B200 in graph replay, us an append that completes no tile, 32 dims a lane / a warp a
+// row, three rows a warp asked for at once: 128 dims 1 / 8 / 16 / 48 rows 1.9 2.3 2.9 3.0 / 1.8 1.8 1.9 2.6, at 64 rows 3.2 / 3.3 (eight at once); 256
+// dims 1 / 8 / 16 / 32 rows 2.1 2.5 3.2 3.3 / 1.8 1.9 2.3 2.8, at 48 rows 3.4 / 3.7 (eight).  Rows off the 16-byte boundary (a warp a row: no
+// other way reads them together): 1,024 tokens 7.7 and 10.3, by elements in the lanes that need them 10.7 and 16.6.
+template <int D> __device__ __forceinline__ bool rotates_singly(int rows, bool wide) { return rows <= (D == 256 && wide ? 32 : 48); }
+
 // Rotate + stage + seal.
 //
 // Which tiles keep their rows in the stage: only the last two tiles of an append (one per slot) can be
@@ -414,20 +445,25 @@ __global__ void __launch_bounds__(kThreads, 1) append_kernel(LayerView L, const 
     const int64_t row_stride = static_cast<int64_t>(L.kv_heads) * D;
     const uint16_t* src = (which ? v : k) + static_cast<int64_t>(head) * D;
     const bool wide = (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
-    auto stage_at = [&](int tile, int tt, int d) { return reinterpret_cast<uint4*>(L.stage_row(which, tile & 1, head, tt) + slice * kSlice + d); };
-    rotate_rows<D, kBf16>(src + (t.base + t.begin - pos0) * row_stride, row_stride, wide, t.begin, t.end, slice, [&](int tt, int d, uint4 x) {
-        *reinterpret_cast<uint4*>(&sm.rows[tt * kRowStride + d]) = x;
-        if (write_stage) *stage_at(t.tile, tt, d) = x;
-    });
+    // the new rows of a tile into shared memory and its stage rows, 16 bytes or one element at a time
+    auto rotate = [&](const AppendTile& a, bool here, bool to_stage) {
+        const uint16_t* const rows = src + (a.base + a.begin - pos0) * row_stride;
+        __half* const stage = L.stage_row(which, a.tile & 1, head, 0) + slice * kSlice;
+        auto keep = [&](int tt, int d, auto x) {
+            using X = decltype(x);
+            if (here) *reinterpret_cast<X*>(&sm.rows[tt * kRowStride + d]) = x;
+            if (to_stage) *reinterpret_cast<X*>(&stage[tt * D + d]) = x;
+        };
+        if (rotates_singly<D>(a.end - a.begin, wide)) rotate_rows_singly<D, kBf16, 3>(rows, row_stride, a.begin, a.end, slice, keep);
+        else if (wide) rotate_rows<D, kBf16>(rows, row_stride, a.begin, a.end, slice, keep);
+        else rotate_rows_singly<D, kBf16, 8>(rows, row_stride, a.begin, a.end, slice, keep);
+    };
+    rotate(t, true, write_stage);
     if (!seal) return;
     __syncthreads();
     if (inside && t.tile == t.t0 && t.tlast >= t.t0 + 2) {
         const int later = ((t.tlast ^ t.t0) & 1) == 0 ? t.tlast : t.tlast - 1;  // of the last two tiles, the one with this slot
-        if (later >= t.t0 + 2) {
-            const AppendTile u = append_tile(pos0, last, later - t.t0);
-            rotate_rows<D, kBf16>(src + (u.base - pos0) * row_stride, row_stride, wide, 0, u.end, slice,
-                                  [&](int tt, int d, uint4 x) { *stage_at(later, tt, d) = x; });
-        }
+        if (later >= t.t0 + 2) rotate(append_tile(pos0, last, later - t.t0), false, true);
     }
 
     const int32_t* tbl = L.table();

@@ -66,3 +66,29 @@ def test_codes_at_the_middle(kind):
     assert all((np.asarray(a).reshape(-1) == np.asarray(b).reshape(-1)).all() for a, b in zip(got, want))
     if kind == "middles":
         assert got[1].max() > 0x0F
+
+
+@pytest.mark.parametrize("D", [128, 256])
+@pytest.mark.parametrize("shift", [0, 3])
+@pytest.mark.parametrize("before,T", [(0, 16), (3, 17), (0, 32), (5, 33), (0, 48), (0, 49), (60, 64), (100, 30), (90, 300), (120, 140)])
+def test_few_rows_and_many(D, shift, before, T):
+    """Rows of a tile that a warp each rotates, and more: tiles left open, completed, and a long append that begins inside one.  The oracle's
+    stage and planes."""
+    import torch
+
+    H, QH = 4, 24
+    tw = Twin(D=D, H=H, QH=QH, capacity_tokens=before + T, seed=2)
+    k, v = (orc.synth_kv(T, before + T, H, D, i) for i in (1, 2))
+    if before:
+        tw.append(k[:before], v[:before])
+    rows = []
+    for x in (k, v):
+        x = torch.from_numpy(x[before:]).cuda()
+        buf = torch.zeros(x.numel() + 8, dtype=x.dtype, device="cuda")
+        rows.append(buf[shift:shift + x.numel()].view(x.shape))
+        rows[-1].copy_(x)
+    tw.gpu.append(*rows, torch.arange(before, before + T, dtype=torch.int32, device="cuda"))
+    tw.cpu.append(k[before:].view(np.uint16), v[before:].view(np.uint16), before, 0)
+    tw.len = before + T
+    assert tw.live_stage_equal()
+    assert all(tw.planes_equal().values()) and tw.gpu.errors() == 0
