@@ -31,9 +31,9 @@
 #include <climits>
 #include <cstddef>
 #include <cstdlib>
-#include <functional>
 #include <type_traits>
 
+#include "kvb_batch_plan.hpp"
 #include "kvb_common.cuh"
 #include "kvb_ptx.cuh"
 #include "kvb_shares.hpp"
@@ -1784,82 +1784,18 @@ static_assert(sizeof(LayerView) == sizeof(kvb_layer) && offsetof(LayerView, erro
                   offsetof(LayerView, iters) == offsetof(kvb_layer, sinkhorn_iters),
               "the device reads kvb_layer structs as LayerView");
 
-// Parts (splits over the sealed tiles; the last one also reads the open tile) of every sequence from the host's
-// bounds of their lengths: chunks of at least 4 tiles, at most 64 splits per sequence.  A CTA of 8 warps takes `fixed` us (set-up,
-// first fetch, merge) and `round` us per 8 pages; `beside` of them share an SM, so that one's set-up and end lie beside the
-// others' work.  Chunk sizes that make about 1/2 .. 4 waves of CTAs are costed by the work per place plus 0.45 of what the last CTA
-// ends later than that, the CTAs of a head taken in order by its share of the places (a CTA left alone on its SM runs faster, hence not
-// all of it: fitted to sweeps of the chunk size over six batches).  Measured on B200, calls in a row, one CTA of 16 warps an SM with 2 ..
-// 12 CTAs per SM in total against this, us: 32 sequences of up to 131,072 tokens (24 / 4 heads) 317 -> 286, 8 of them 117 -> 84, 48 of
-// 30,000 130 -> 124, 40 of 4,096 34.4 -> 31.5, 24 of 100,000 (32 / 8) 353 -> 342, 20 of 60,000 (16 / 2) 73.5 -> 52.8.
-struct BatchCost {
-    int beside;
-    float fixed, round;
-};
-constexpr int kBatchLeast = 4;     // tiles of a chunk: a page for each of the 8 warps
-constexpr int kBatchPlaces = 512;  // the most places of a head that are modelled
-constexpr BatchCost kBatchNarrow{kBatchPerSm, 3.0f, 4.3f}, kBatchBroad{1, 6.1f, 4.4f};  // up to 8 merged rows, more
-int batch_parts(int kv_len_max, int chunk) { return std::min(std::max((kv_len_max / kTile + chunk - 1) / chunk, 1), kReduceWarps * kMaxPartsPerWarp); }
-int plan_batch_chunk(const int32_t* kv_len_max, int batch, int kv_heads, int sms, const BatchCost& cost) {
-    constexpr int kMost = kReduceWarps * kMaxPartsPerWarp;
-    int64_t total_tiles = 0;
-    int most_tiles = 0;
-    for (int b = 0; b < batch; ++b) {
-        total_tiles += kv_len_max[b] / kTile;
-        most_tiles = std::max(most_tiles, kv_len_max[b] / kTile);
-    }
-    const int places = std::min(std::max(1, cost.beside * sms / kv_heads), kBatchPlaces);  // of a head
-    int best_chunk = kBatchLeast, last_chunk = 0;
-    float best = 1e30f, ends[kBatchPlaces];
-    static const float kWaves[] = {0.5f, 0.98f, 1.48f, 1.95f, 2.45f, 2.9f, 3.9f};
-    for (float waves : kWaves) {
-        const int want = static_cast<int>(static_cast<float>(total_tiles) / (waves * static_cast<float>(places))) + 1;
-        const int chunk = (std::max({kBatchLeast, want, (most_tiles + kMost - 1) / kMost}) + 3) / 4 * 4;
-        if (chunk == last_chunk) continue;
-        last_chunk = chunk;
-        std::fill(ends, ends + places, 0.0f);  // a heap, the earliest end first
-        float work = 0.0f, end = 0.0f;
-        for (int b = 0; b < batch; ++b) {
-            const int parts = batch_parts(kv_len_max[b], chunk);
-            const float t = cost.fixed + cost.round * static_cast<float>(((kv_len_max[b] / kTile + parts - 1) / parts + 3) / 4);
-            work += t * static_cast<float>(parts);
-            for (int i = 0; i < parts; ++i) {
-                std::pop_heap(ends, ends + places, std::greater<float>());
-                ends[places - 1] += t;
-                end = std::max(end, ends[places - 1]);
-                std::push_heap(ends, ends + places, std::greater<float>());
-            }
-        }
-        const float per_place = work / static_cast<float>(places), us = per_place + 0.45f * (end - per_place);
-        if (us < best) {
-            best = us;
-            best_chunk = chunk;
-        }
-    }
-    return best_chunk;
-}
-// The chunk size of the thread's last plan is kept with the numbers it follows from: a serving loop asks for the same ones at
-// every step, and costing them takes up to 0.1 ms.
+// (The broad kernel's costs are those of a verify step's row blocks of 16; nothing was fitted for it.)
+constexpr BatchCost kBatchNarrow{kBatchPerSm, 30, 43}, kBatchBroad{1, 61, 44};  // up to 8 merged rows, more
 int plan_batch(const int32_t* kv_len_max, int batch, int kv_heads, int group, BatchPlan& plan) {
-    struct Last {
-        int32_t bounds[kBatchMax];
-        int batch = 0, kv_heads = 0, sms = 0, chunk = kBatchLeast;
-        bool broad = false;
-    };
-    static thread_local Last last;
+    static thread_local LastBatch last;
+    static_assert(kBatchMax == kBatchMost && kBatchParts == kReduceWarps * kMaxPartsPerWarp, "what a call and the merge kernel hold");
+    int32_t tiles[kBatchMax];
+    for (int b = 0; b < batch; ++b) tiles[b] = kv_len_max[b] / kTile;
     const bool broad = group > 8;
-    const int sms = sm_count();
-    if (last.batch != batch || last.kv_heads != kv_heads || last.sms != sms || last.broad != broad || !std::equal(kv_len_max, kv_len_max + batch, last.bounds)) {
-        last.chunk = plan_batch_chunk(kv_len_max, batch, kv_heads, sms, broad ? kBatchBroad : kBatchNarrow);
-        std::copy(kv_len_max, kv_len_max + batch, last.bounds);
-        last.batch = batch;
-        last.kv_heads = kv_heads;
-        last.sms = sms;
-        last.broad = broad;
-    }
+    const int chunk = last.chunk_of(tiles, batch, kv_heads, sm_count(), broad, broad ? kBatchBroad : kBatchNarrow);
     plan.n = batch;
     plan.prefix[0] = 0;
-    for (int b = 0; b < batch; ++b) plan.prefix[b + 1] = plan.prefix[b] + batch_parts(kv_len_max[b], last.chunk);
+    for (int b = 0; b < batch; ++b) plan.prefix[b + 1] = plan.prefix[b] + batch_parts(tiles[b], chunk);
     return plan.prefix[batch];
 }
 

@@ -82,6 +82,11 @@ def test_every_page_is_dealt_once(tmp_path):
     assert "shares: ok" in _run_host_check(tmp_path, "shares_check")
 
 
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs a C++ compiler")
+def test_the_schedule_of_a_batch(tmp_path):
+    assert "batch plan: ok" in _run_host_check(tmp_path, "batch_plan_check")
+
+
 def test_chunk_workspaces_are_what_a_call_can_use():
     """24 / 4 heads, 148 SMs: an 8-row verify step takes 74 partials a row at 128 dims and the narrow kernel's at 256; a short prompt
     takes one key range, a chunk at 256 dims three."""
