@@ -1052,6 +1052,7 @@ __global__ void __launch_bounds__((S == 1 ? kWarpsWide : kPairWarps) * 32, 1) at
 // short sequences give CTAs of similar size.
 constexpr int kBatchMax = 64;
 constexpr int kBatchPerSm = 2;  // CTAs of 8 warps beside each other on an SM (up to 8 merged rows)
+constexpr int kWarpsAlone = 16;  // of a CTA that has its SM to itself (choose_batch)
 struct BatchPlan {
     int n;                      // sequences; 0 = not a batched call
     int prefix[kBatchMax + 1];  // parts before sequence b
@@ -1786,16 +1787,16 @@ static_assert(sizeof(LayerView) == sizeof(kvb_layer) && offsetof(LayerView, erro
 
 // (The broad kernel's costs are those of a verify step's row blocks of 16; nothing was fitted for it.)
 constexpr BatchCost kBatchNarrow{kBatchPerSm, 30, 43}, kBatchBroad{1, 61, 44};  // up to 8 merged rows, more
-int plan_batch(const int32_t* kv_len_max, int batch, int kv_heads, int group, BatchPlan& plan) {
+int plan_batch(const int32_t* kv_len_max, int batch, int kv_heads, int group, BatchPlan& plan, bool* alone = nullptr) {
     static thread_local LastBatch last;
     static_assert(kBatchMax == kBatchMost && kBatchParts == kReduceWarps * kMaxPartsPerWarp, "what a call and the merge kernel hold");
     int32_t tiles[kBatchMax];
     for (int b = 0; b < batch; ++b) tiles[b] = kv_len_max[b] / kTile;
-    const bool broad = group > 8;
-    const int chunk = last.chunk_of(tiles, batch, kv_heads, sm_count(), broad, broad ? kBatchBroad : kBatchNarrow);
+    const BatchChoice choice = last.of(tiles, batch, kv_heads, group, sm_count(), group > 8 ? kBatchBroad : kBatchNarrow);
+    if (alone != nullptr) *alone = choice.alone;
     plan.n = batch;
     plan.prefix[0] = 0;
-    for (int b = 0; b < batch; ++b) plan.prefix[b + 1] = plan.prefix[b] + batch_parts(tiles[b], chunk);
+    for (int b = 0; b < batch; ++b) plan.prefix[b + 1] = plan.prefix[b] + batch_parts(tiles[b], choice.chunk);
     return plan.prefix[batch];
 }
 
@@ -1826,7 +1827,8 @@ extern "C" int kvb_attn_decode_batch(const kvb_layer* layers_dev, int batch, int
     for (int b = 0; b < batch; ++b)
         if (kv_len_max[b] < 1) return fail(KVB_EINVAL, "kvb_attn_decode_batch: kv_len_max[%d] = %d", b, kv_len_max[b]);
     BatchParams B;
-    const int total = plan_batch(kv_len_max, batch, kv_heads, q_heads / kv_heads, B.plan);
+    bool alone = false;
+    const int total = plan_batch(kv_len_max, batch, kv_heads, q_heads / kv_heads, B.plan, &alone);
     const size_t rows = static_cast<size_t>(kv_heads) * total * kRows;
     B.layers = reinterpret_cast<const LayerView*>(layers_dev);
     B.q = static_cast<const uint16_t*>(q);
@@ -1838,14 +1840,15 @@ extern "C" int kvb_attn_decode_batch(const kvb_layer* layers_dev, int batch, int
     B.ws_m = workspace_base(workspace);
     B.ws_l = B.ws_m + rows;
     B.ws_o = B.ws_l + rows;
-    constexpr int smem = static_cast<int>(sizeof(AttnSmem<1, kWarpsWide>));
-    static_assert(kBatchPerSm * (smem + 1024) <= 228 * 1024, "CTAs beside each other");
-    static OncePerDevice opted1, opted2;
+    constexpr int smem = static_cast<int>(sizeof(AttnSmem<1, kWarpsWide>)), smem_alone = static_cast<int>(sizeof(AttnSmem<1, kWarpsAlone>));
+    static_assert(kBatchPerSm * (smem + 1024) <= 228 * 1024 && sizeof(AttnSmem<2, kWarpsWide>) <= smem, "CTAs beside each other");
+    static OncePerDevice opted1, opted2, opted3;
     KVB_CUDA_OK(allow_smem(opted1, attn_batch_kernel<1, kWarpsWide, kBatchPerSm>, smem));
     KVB_CUDA_OK(allow_smem(opted2, attn_batch_kernel<2, kWarpsWide, 1>, smem));
+    KVB_CUDA_OK(allow_smem(opted3, attn_batch_kernel<1, kWarpsAlone, 1>, smem_alone));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (q_heads / kv_heads > 8) KVB_CUDA_OK(launch_early(attn_batch_kernel<2, kWarpsWide, 1>, dim3(total, kv_heads, 1), dim3(kWarpsWide * 32), smem, st, B));
-    else KVB_CUDA_OK(launch_early(attn_batch_kernel<1, kWarpsWide, kBatchPerSm>, dim3(total, kv_heads, 1), dim3(kWarpsWide * 32), smem, st, B));
+    const auto kernel = q_heads / kv_heads > 8 ? attn_batch_kernel<2, kWarpsWide, 1> : alone ? attn_batch_kernel<1, kWarpsAlone, 1> : attn_batch_kernel<1, kWarpsWide, kBatchPerSm>;
+    KVB_CUDA_OK(launch_early(kernel, dim3(total, kv_heads, 1), dim3(32 * (alone ? kWarpsAlone : kWarpsWide)), alone ? smem_alone : smem, st, B));
     KVB_CUDA_OK((launch_reduce<1, false>(batch * q_heads, st, B.ws_m, B.ws_l, B.ws_o, 0, batch, q_heads, kv_heads, 1, kRows, dtype, static_cast<uint16_t*>(out),
                                          nullptr, nullptr, nullptr, PushTarget{}, B.plan)));
     return KVB_OK;

@@ -101,23 +101,48 @@ inline int plan_batch_chunk(const int32_t* tiles, int batch, int kv_heads, int s
     return best_chunk;
 }
 
-// The chunk size of a thread's last plan, with what it follows from: a serving loop asks for the same one at every step until a sequence
-// enters its next tile.  Costing it takes a host core 2 .. 13 us for 8 .. 64 sequences (10 .. 47 with a heap of places).
+// How a batch runs: tiles of a chunk, and whether its CTAs (up to 8 merged rows) are `alone` on their SMs, with 16 warps.  They are where chunks
+// of 4 or 8 tiles, no more than a page a warp, give every CTA an SM of its own: nothing beside it would hide a longer round.  Not where
+// the CTAs of the merge, one a row, find SMs that had none of the attention's: 8 warps merge sooner.  Measured on B200 in graph replay, us a call,
+// two CTAs of 8 warps an SM / one of 16: 6 sequences of up to 500 / 1,500 / 4,788 tokens (24 / 4 heads) 11.0 11.8 12.3 / 9.2 9.5 9.9, 2 of 10,000
+// and 20,000 12.0 13.1 / 9.8 12.1; 2 of 1,500 and 4,788 9.2 8.5 / 9.5 9.0; in chunks of 16 tiles, alone too, 3 of 30,000 15.4 / 16.0.
+struct BatchChoice {
+    int chunk;
+    bool alone;
+};
+inline BatchChoice choose_batch(const int32_t* tiles, int batch, int kv_heads, int group, int sms, const BatchCost& cost) {
+    for (int chunk = kBatchLeast; chunk <= 2 * kBatchLeast && group <= 8; chunk *= 2) {
+        int parts = 0;
+        bool whole = true;  // no sequence has more chunks than splits
+        for (int b = 0; b < batch; ++b) {
+            parts += batch_parts(tiles[b], chunk);
+            whole = whole && tiles[b] <= chunk * kBatchParts;
+        }
+        if (whole && parts * kv_heads <= sms) {
+            if ((parts + batch * group) * kv_heads <= sms) break;
+            return {chunk, true};
+        }
+    }
+    return {plan_batch_chunk(tiles, batch, kv_heads, sms, cost), false};
+}
+
+// A thread's last choice, with what it follows from: a serving loop asks for the same one at every step until a sequence
+// enters its next tile.  Modelling it takes a host core 2 .. 13 us for 8 .. 64 sequences (10 .. 47 with a heap of places).
 struct LastBatch {
     int32_t tiles[kBatchMost];
-    int batch = 0, kv_heads = 0, sms = 0, chunk = kBatchLeast;
-    bool broad = false;
+    int batch = 0, kv_heads = 0, group = 0, sms = 0;
+    BatchChoice choice{kBatchLeast, false};
 
-    int chunk_of(const int32_t* now, int n, int heads, int processors, bool is_broad, const BatchCost& cost) {
-        if (batch != n || kv_heads != heads || sms != processors || broad != is_broad || !std::equal(now, now + n, tiles)) {
-            chunk = plan_batch_chunk(now, n, heads, processors, cost);
+    BatchChoice of(const int32_t* now, int n, int heads, int rows, int processors, const BatchCost& cost) {
+        if (batch != n || kv_heads != heads || group != rows || sms != processors || !std::equal(now, now + n, tiles)) {
+            choice = choose_batch(now, n, heads, rows, processors, cost);
             std::copy(now, now + n, tiles);
             batch = n;
             kv_heads = heads;
+            group = rows;
             sms = processors;
-            broad = is_broad;
         }
-        return chunk;
+        return choice;
     }
 };
 

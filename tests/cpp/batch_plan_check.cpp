@@ -54,14 +54,34 @@ int main() {
     int32_t tiles[3] = {100, 700, 1000};
     for (int i = 0; i < 200; ++i) {
         const int n = between(1, 3), heads = 1 << between(0, 3), sms = between(0, 1) ? 148 : 74;
-        const bool broad = between(0, 1);
-        const BatchCost cost = broad ? BatchCost{1, 61, 44} : BatchCost{2, 30, 43};
+        const int group = between(1, 16);
+        const BatchCost cost = group > 8 ? BatchCost{1, 61, 44} : BatchCost{2, 30, 43};
         if (between(0, 2) == 0) tiles[between(0, 2)] = between(1, 3000);
         for (int again = 0; again < 2; ++again)
-            if (last.chunk_of(tiles, n, heads, sms, broad, cost) != plan_batch_chunk(tiles, n, heads, sms, cost)) {
-                std::printf("a plan of other numbers\n");
-                ++bad;
+            {
+                const BatchChoice kept = last.of(tiles, n, heads, group, sms, cost), made = choose_batch(tiles, n, heads, group, sms, cost);
+                if (kept.chunk != made.chunk || kept.alone != made.alone) {
+                    std::printf("a plan of other numbers\n");
+                    ++bad;
+                }
             }
+    }
+    // CTAs that are alone on their SMs: no more of them than SMs, no more than 16 pages each
+    for (int i = 0; i < 2000 && bad < 5; ++i) {
+        const int n = between(1, kBatchMost), heads = 1 << between(0, 3), most = 1 << between(0, 12);
+        int32_t t[kBatchMost];
+        for (int b = 0; b < n; ++b) t[b] = between(0, most);
+        const BatchChoice c = choose_batch(t, n, heads, between(1, 8), 148, {2, 30, 43});
+        int all = 0, pages = 0;
+        for (int b = 0; b < n; ++b) {
+            const int parts = batch_parts(t[b], c.chunk);
+            all += parts * heads;
+            pages = std::max(pages, (2 * t[b] + parts - 1) / parts);
+        }
+        if ((c.alone && (all > 148 || pages > 16)) || choose_batch(t, n, heads, 9, 148, {1, 61, 44}).alone) {
+            std::printf("alone: %d CTAs, %d pages\n", all, pages);
+            ++bad;
+        }
     }
     std::printf(bad ? "batch plan: %d wrong\n" : "batch plan: ok\n", bad);
     return bad != 0;
