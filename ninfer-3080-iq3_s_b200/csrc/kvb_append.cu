@@ -401,7 +401,11 @@ __device__ __forceinline__ void rotate_rows_singly(const uint16_t* __restrict__ 
 // row, three rows a warp asked for at once: 128 dims 1 / 8 / 16 / 48 rows 1.9 2.3 2.9 3.0 / 1.8 1.8 1.9 2.6, at 64 rows 3.2 / 3.3 (eight at once); 256
 // dims 1 / 8 / 16 / 32 rows 2.1 2.5 3.2 3.3 / 1.8 1.9 2.3 2.8, at 48 rows 3.4 / 3.7 (eight).  Rows off the 16-byte boundary (a warp a row: no
 // other way reads them together): 1,024 tokens 7.7 and 10.3, by elements in the lanes that need them 10.7 and 16.6.
-template <int D> __device__ __forceinline__ bool rotates_singly(int rows, bool wide) { return rows <= (D == 256 && wide ? 32 : 48); }
+// Not in balanced caches of 128 dims, whose verify steps of two rows a warp take longer behind the shorter append (2 / 5 rows at 497 tokens 11.8 /
+// 11.8 us a layer, a warp a row 12.1 / 12.3, the same and held up for as long 11.8 / 12.0: it is when the append ends that counts).
+template <int D> __device__ __forceinline__ bool rotates_singly(int rows, bool wide, bool balanced) {
+    return rows <= (D == 256 && wide ? 32 : 48) && !(D == 128 && wide && balanced);
+}
 
 // Rotate + stage + seal.
 //
@@ -454,7 +458,7 @@ __global__ void __launch_bounds__(kThreads, 1) append_kernel(LayerView L, const 
             if (here) *reinterpret_cast<X*>(&sm.rows[tt * kRowStride + d]) = x;
             if (to_stage) *reinterpret_cast<X*>(&stage[tt * D + d]) = x;
         };
-        if (rotates_singly<D>(a.end - a.begin, wide)) rotate_rows_singly<D, kBf16, 3>(rows, row_stride, a.begin, a.end, slice, keep);
+        if (rotates_singly<D>(a.end - a.begin, wide, L.iters > 0)) rotate_rows_singly<D, kBf16, 3>(rows, row_stride, a.begin, a.end, slice, keep);
         else if (wide) rotate_rows<D, kBf16>(rows, row_stride, a.begin, a.end, slice, keep);
         else rotate_rows_singly<D, kBf16, 8>(rows, row_stride, a.begin, a.end, slice, keep);
     };
