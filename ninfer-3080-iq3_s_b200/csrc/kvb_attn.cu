@@ -1457,11 +1457,14 @@ cudaError_t launch_attn_pair(dim3 grid, cudaStream_t stream, const AttnParams& P
     return launch_early(attn_pair_kernel, grid, dim3(kPairWarps * 32), smem, stream, P);
 }
 
-// Up to this many keys, and with up to this many clusters, the splits of a head and row block are a cluster (attn_short_kernel).  Beyond
-// the keys, eight CTAs have more than a round of pages; beyond the clusters, they are not all on the GPU at once.  Measured on B200, 24 / 4
-// heads, merge kernel against clusters: launched one by one (3 us of the host each), 16 layers at 1,500 tokens 206 and 164 us; in graph
-// replay, append and attention, us a layer: 300 tokens 8.1 8.0, 1,500 7.8 8.0, 3,000 8.1 8.4, 256 dims 300 12.0 11.7, 1,500 11.1 11.4, verify
-// of 4 rows (12 clusters) at 1,500 8.2 7.8; before, 4,000 9.0 9.4, 6,000 9.9 12.3, 256 dims 2,000 14.7 15.6, 5 rows (16 clusters) 9.6 16.4.
+// Up to this many keys, and with up to this many clusters, the splits of a head and row block are a cluster (attn_short_kernel).  What that
+// saves is a launch, 3 us of the host: 16 layers launched one by one at 1,500 tokens take 206 us with the merge kernel and 164 as clusters.
+// On the device the merge kernel's route is the faster one where a head has one split, whose CTA would finish all rows alone, and at 256 dims:
+// a step that is captured, whose launches cost the host nothing, takes it there.  Graph replay, 24 / 4 heads, append and attention, us a layer,
+// merge kernel / clusters: 60 tokens 1 / 4 rows 6.6 8.2 / 6.6 9.1, 200 tokens 8.5 8.2 / 8.6 8.2, 600 tokens 8.1 8.0 / 7.9 7.7, 1,500 tokens
+// 8.0 8.3 / 8.0 8.0, 2,500 tokens 8.2 8.5 / 8.5 8.3, 256 dims 60 tokens 9.2 10.1 / 9.5 10.5, 600 tokens 10.8 11.4 / 11.6 11.8, 1,500 tokens 11.0
+// 11.8 / 11.6 12.1.  Beyond the keys, eight CTAs have more than a round of pages (4,000 tokens 9.0 / 9.4, 6,000 9.9 / 12.3, 256 dims 2,000 14.7 /
+// 15.6); beyond the clusters, they are not all on the GPU at once (5 rows of 256 dims, 16 clusters, 9.6 / 16.4).
 constexpr int kShortClusters = 12;
 constexpr int short_keys(int head_dim) { return head_dim == 128 ? 3072 : 1536; }
 // The same as clusters: the splits of a head and row block.
@@ -1562,10 +1565,12 @@ int launch_attention(const kvb_layer* layer, const void* q, const int32_t* pos_d
     const ShortCall as_clusters = layer->head_dim != 128 ? short_call<2, 1, true>()
                                   : upper                ? (other ? short_call<1, 2, true>() : short_call<1, 2, false>())
                                                          : (other ? short_call<1, 1, true>() : short_call<1, 1, false>());
-    const bool clustered = kv_len_max <= short_keys(layer->head_dim) && layer->kv_heads * plan.zblocks <= kShortClusters && out != nullptr && part_m == nullptr && push == nullptr &&
-                           stores_beside(span_of(out, out_bytes), span_of(q, out_bytes), span_of(pos_dev, T * sizeof(int32_t)), span_of(total_pos_dev, sizeof(int32_t))) &&
-                           as_clusters.held();
-    const int Z = plan.zblocks, nsplit = clustered ? std::min(plan.nsplit, kShortSplits) : plan.nsplit;
+    const int Z = plan.zblocks;
+    // (as many splits by either route: the same bits)
+    const bool few = kv_len_max <= short_keys(layer->head_dim) && layer->kv_heads * Z <= kShortClusters && out != nullptr && part_m == nullptr && push == nullptr;
+    const int nsplit = few ? std::min(plan.nsplit, kShortSplits) : plan.nsplit;
+    const bool clustered = few && stores_beside(span_of(out, out_bytes), span_of(q, out_bytes), span_of(pos_dev, T * sizeof(int32_t)), span_of(total_pos_dev, sizeof(int32_t))) &&
+                           as_clusters.held() && !((layer->head_dim != 128 || nsplit == 1) && is_captured(stream));
     const int parts = nsplit;
     AttnParams P;
     P.L = make_view(*layer);

@@ -141,6 +141,13 @@ template <typename K> cudaError_t clusters_held(K* kernel, int cluster, dim3 blo
     return cudaOccupancyMaxActiveClusters(clusters, kernel, &cfg);
 }
 
+inline bool is_captured(cudaStream_t stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) == cudaSuccess) return status != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return false;
+}
+
 inline int current_device() {  // -1: unknown
     int dev = -1;
     return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;

@@ -1,4 +1,4 @@
-"""A device, or a part of one, that holds no cluster of a short step's CTAs: the step takes the merge kernel's route."""
+"""A device, or a part of one, that holds no cluster of a short step's CTAs: the step takes the merge kernel's route, to the same bits."""
 import ctypes as C
 import os
 import shutil
@@ -24,7 +24,7 @@ def without(tmp_path_factory):
     return C.CDLL(lib)
 
 
-@pytest.mark.parametrize("D,H,QH,T,rows,iters", [(128, 4, 24, 1500, 1, 0), (128, 4, 24, 3000, 2, 16), (128, 2, 16, 130, 3, 0), (256, 4, 24, 1400, 1, 2)])
+@pytest.mark.parametrize("D,H,QH,T,rows,iters", [(128, 4, 24, 1500, 1, 0), (128, 4, 24, 3000, 2, 16), (128, 2, 16, 130, 3, 0), (128, 4, 24, 100, 4, 0), (256, 4, 24, 1400, 1, 2), (256, 4, 24, 1536, 3, 0)])
 def test_short_steps_without_clusters(without, D, H, QH, T, rows, iters):
     import torch
 
@@ -35,6 +35,7 @@ def test_short_steps_without_clusters(without, D, H, QH, T, rows, iters):
     q = torch.from_numpy(qn).to(tw.dev)
     ws = tw.gpu.workspace(T, rows)
     want = cpu_twin_of(tw.gpu).attention(qn, list(range(T - rows, T)), 1.0 / np.sqrt(D), QH, threads=4, kv_total=T)
+    outs = []
     for lib, merged in ((pkg().capi.load(), False), (without, True)):
         ws.fill_(float("nan"))
         out = torch.empty_like(q)
@@ -44,4 +45,6 @@ def test_short_steps_without_clusters(without, D, H, QH, T, rows, iters):
         assert torch.isnan(ws).all() != merged  # partials for the merge kernel
         ok, msg = attn_close(out.float().cpu().numpy(), want, ATTN_MAX_ABS, ATTN_REL_L2)
         assert ok, msg
+        outs.append(out)
+    assert torch.equal(*outs)
     assert tw.gpu.errors() == 0
