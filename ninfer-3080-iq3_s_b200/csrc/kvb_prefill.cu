@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
         const int steps = steps_of(u);
         float m_run = -INFINITY, l_run = 0.0f;
         Walk<Ro::kHalves == 2> walk;
-        for (int i = 0; i < steps; ++i) {
+        for (int i = 0; i < steps && (Ro::kHalves == 2 || !walk.failed); ++i) {
             const int j = kSplit ? 2 * i + u : i;
 #pragma unroll 1
             for (int h = 0; h < Ro::kParts; ++h) {
@@ -564,7 +564,10 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
                 // P of the two warps lies side by side over S of the part, which both have read when they meet
                 const uint32_t ts = tmem + 128 * u + (kN / Ro::kParts) * h + kKeys * half + lane_base, tp = ts - (Ro::kHalves == 2 ? kKeys / 2 * half : 0);
                 walk.waited(chunk_wait(&sm.s_full[u][h], i & 1, &sm.abort_flag));
-                if (walk.leaves_alone(warp_has_rows)) { i = steps; break; }
+                if (walk.leaves_alone(warp_has_rows)) {
+                    if constexpr (Ro::kHalves == 2) i = steps;
+                    break;
+                }
                 tc::fence_after_sync();
                 if (warp_has_rows) {
                     const bool bad_tile = sm.bad_tile[j & (kSlotsMeta - 1)] != 0;
