@@ -121,9 +121,9 @@ struct TilePages {
 
 // K: thread = the 16-byte chunk of eight dims dt % 16 of keys dt / 16, + kStep, ..: its dims' factors stay in registers for a tile, a warp
 // reads the code rows of two keys at once and writes whole swizzled rows, and a store's address is a constant away from the last one's.
-// Bound by its instructions (busy nine tenths of a step of split walks, three quarters with two row tiles).  Measured on B200 against
+// Bound by its instructions (busy nine tenths of a step of split walks, three quarters with two row tiles).  Measured on B200 in graph replay against
 // thread = key, which read both factors of every chunk from shared memory: 8 rows at 131,072 tokens 68.4 -> 62.6 us a layer, balanced at
-// 100,003 54.4 -> 53.4, 1,024 tokens over 262,144 alone 3,465 -> 3,325 us.
+// 100,003 54.4 -> 53.4; one call of 1,024 tokens over 262,144 3,465 -> 3,325 us.
 // `other` (caches written with variance balancing): K is multiplied by the key's other_K, V by the per-dim other_V, reference
 // kvarn128_codec.cuh:331-347; fp16 like the rest of this kernel.
 template <bool kOther, int kDqWarps>
@@ -555,19 +555,14 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
         const int min_pos = __reduce_min_sync(0xffffffffu, is_row ? my_pos : INT_MAX);
         const int steps = steps_of(u);
         float m_run = -INFINITY, l_run = 0.0f;
-        Walk<Ro::kHalves == 2> walk;
-        for (int i = 0; i < steps && (Ro::kHalves == 2 || !walk.failed); ++i) {
+        for (int i = 0; i < steps && !failed; ++i) {
             const int j = kSplit ? 2 * i + u : i;
 #pragma unroll 1
             for (int h = 0; h < Ro::kParts; ++h) {
                 const int base = (t0 + j) * kN + (kN / Ro::kParts) * h + kKeys * half;
                 // P of the two warps lies side by side over S of the part, which both have read when they meet
                 const uint32_t ts = tmem + 128 * u + (kN / Ro::kParts) * h + kKeys * half + lane_base, tp = ts - (Ro::kHalves == 2 ? kKeys / 2 * half : 0);
-                walk.waited(chunk_wait(&sm.s_full[u][h], i & 1, &sm.abort_flag));
-                if (walk.leaves_alone(warp_has_rows)) {
-                    if constexpr (Ro::kHalves == 2) i = steps;
-                    break;
-                }
+                if (leaves_alone<Ro::kHalves == 2>(failed, chunk_wait(&sm.s_full[u][h], i & 1, &sm.abort_flag), warp_has_rows)) break;
                 tc::fence_after_sync();
                 if (warp_has_rows) {
                     const bool bad_tile = sm.bad_tile[j & (kSlotsMeta - 1)] != 0;
@@ -610,7 +605,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
                         mask(s0, 0);
                         mx = top(s0);
                         sm.row_top[u][h][half][row] = mx;
-                        if (walk.leaves_together(named_barrier_or(3 + 4 * u + (warp & 3), 64, walk.failed))) { i = steps; break; }  // the two warps of these 32 rows
+                        if (leaves_together(failed, named_barrier_or(3 + 4 * u + (warp & 3), 64, failed))) break;  // the two warps of these 32 rows
                         mx = fmaxf(mx, sm.row_top[u][h][half ^ 1][row]);
                     }
                     // The reference point of the row's exponentials follows the running maximum lazily: it moves only when the
@@ -650,8 +645,8 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
                     l_run = l_run * alpha + (sum2.x + sum2.y);
                     if (i + h > 0 && __any_sync(0xffffffffu, grown)) {
                         // P V of step i - 1 completed before S of step i was issued; that of this step's first part may still run
-                        if (h > 0) walk.waited(chunk_wait(&sm.o_done[u][0], i & 1, &sm.abort_flag));
-                        if (Ro::kParts == 2 && h == 0) walk.waited(chunk_wait(&sm.o_done[u][1], (i - 1) & 1, &sm.abort_flag));
+                        if (h > 0) chunk_wait(&sm.o_done[u][0], i & 1, &sm.abort_flag);
+                        if (Ro::kParts == 2 && h == 0) chunk_wait(&sm.o_done[u][1], (i - 1) & 1, &sm.abort_flag);
                         tc::fence_after_sync();
 #pragma unroll 1
                         for (int c = 0; c < kCols / 32; ++c) {
@@ -670,11 +665,11 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_kernel(const PrefillParams 
                 if (lane == 0) mbar_arrive(&sm.p_full[u][h]);
             }
         }
-        failed = walk.failed;
         // ---- partial of this (row tile, key range): m (log2 units), l, o in tile dim order
+        // (a wait ahead of a rescaling that was given up by a warp of this stream raised the flag before its last P was handed over)
 #pragma unroll
         for (int h = 0; h < Ro::kParts; ++h)
-            if (steps > 0 && !failed && !chunk_wait(&sm.o_done[u][h], (steps - 1) & 1, &sm.abort_flag)) failed = true;
+            if (steps > 0 && !failed && !chunk_wait<Ro::kHalves == 2>(&sm.o_done[u][h], (steps - 1) & 1, &sm.abort_flag)) failed = true;
         tc::fence_after_sync();
         if constexpr (Ro::kHalves == 2) {  // a row's sum has two halves; a warp that gave up comes here too
             sm.row_top[u][0][half][row] = l_run;

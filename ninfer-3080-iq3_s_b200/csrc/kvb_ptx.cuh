@@ -71,12 +71,14 @@ __device__ __forceinline__ bool mbar_wait_lane_bounded(uint64_t* bar, uint32_t p
 #ifndef KVB_CHUNK_PROBES
 #define KVB_CHUNK_PROBES kSpinLimit
 #endif
-__device__ __forceinline__ bool chunk_wait(uint64_t* bar, uint32_t parity, int* abort_flag) {
+// kSound: also reports a flag that was raised, by any wait of the CTA, before what it waits for came about.
+template <bool kSound = false> __device__ __forceinline__ bool chunk_wait(uint64_t* bar, uint32_t parity, int* abort_flag) {
     bool ok = false;
     for (uint32_t i = 0; i < KVB_CHUNK_PROBES && !ok; ++i) {
         ok = mbar_try_wait(bar, parity);
         if (!ok && *reinterpret_cast<volatile int*>(abort_flag) != 0) break;
     }
+    if constexpr (kSound) ok = ok && *reinterpret_cast<volatile int*>(abort_flag) == 0;
     ok = __all_sync(0xffffffffu, ok);
     if (!ok) *reinterpret_cast<volatile int*>(abort_flag) = 1;
     return ok;

@@ -1,4 +1,5 @@
 // Two warps that share rows walk the parts of their key tiles and give up at every wait they have, alike or not: each meeting has both.
+#include <atomic>
 #include <condition_variable>
 #include <cstdio>
 #include <mutex>
@@ -49,35 +50,41 @@ struct Warp {
 };
 
 // The softmax warps' walk: a part is waited for, two warps that share its rows meet, and before the sums are scaled the products before them
-// are waited for.  Returns the parts that were worked on.
-template <bool kMeets, typename Meet> int walk(int steps, bool rows, Warp w, bool& failed, Meet meet) {
+// are waited for.  A wait that is given up raises the abort flag.  Returns the parts that were worked on.
+template <typename Meet> int walk(int steps, Warp w, bool& failed, std::atomic<bool>& abort, Meet meet) {
     int waits = 0, parts = 0;
-    auto wait = [&] { return waits++ < w.first || (waits - 1 > w.first && !w.again); };
-    kvb::Walk<kMeets> walk;
-    for (int i = 0; i < steps; ++i)
+    auto wait = [&] {
+        const bool whole = waits++ < w.first || (waits - 1 > w.first && !w.again);
+        if (!whole) abort = true;
+        return whole;
+    };
+    failed = false;
+    for (int i = 0; i < steps && !failed; ++i)
         for (int h = 0; h < 2; ++h) {
-            walk.waited(wait());
-            if (walk.leaves_alone(rows)) { i = steps; break; }
-            if (kMeets && walk.leaves_together(meet(walk.failed))) { i = steps; break; }
+            if (kvb::leaves_alone<true>(failed, wait(), true)) break;
+            if (kvb::leaves_together(failed, meet(failed))) break;
             ++parts;
-            if (i + h > 0) walk.waited(wait());
+            if (i + h > 0) wait();
         }
-    failed = walk.failed;
     return parts;
 }
 
+// Whether no warp is left alone, and both know in the end if either has given up.
 bool two_warps(int steps, Warp a, Warp b) {
     Barrier barrier;
+    std::atomic<bool> abort{false};
+    bool known[2];
     auto run = [&](int who, Warp w) {
         bool failed;
-        walk<true>(steps, true, w, failed, [&](bool mine) { return barrier.come(who, kVerdict, mine); });
+        walk(steps, w, failed, abort, [&](bool mine) { return barrier.come(who, kVerdict, mine); });
         barrier.come(who, kEnd, failed);
+        known[who] = failed || abort;
         barrier.leave(who);
     };
     std::thread other(run, 1, b);
     run(0, a);
     other.join();
-    return barrier.sound;
+    return barrier.sound && known[0] == abort && known[1] == abort;
 }
 
 }  // namespace
@@ -90,14 +97,19 @@ int main() {
             for (int y = 0; y <= waits; ++y)
                 for (int again = 0; again < 4; ++again)
                     if (!two_warps(steps, {x, (again & 1) != 0}, {y, (again & 2) != 0})) {
-                        if (bad++ < 5) std::printf("%d steps, given up at waits %d and %d (%d): a warp is left alone\n", steps, x, y, again);
+                        if (bad++ < 5) std::printf("%d steps, given up at waits %d and %d (%d): a warp is left alone, or does not know\n", steps, x, y, again);
                     }
     }
-    // a warp that shares no rows leaves behind the first wait for a part that finds it given up
-    for (int at = 0; at <= 7; ++at) {
-        bool failed;
-        const int parts = walk<false>(2, true, {at, true}, failed, [](bool) { return false; });
-        if (parts != (at == 0 ? 0 : at / 2 + 1) || failed != (at < 7)) { std::printf("alone, given up at %d: %d parts\n", at, parts); ++bad; }
+    // a warp that shares no rows leaves behind the first wait for a part that is given up (it has no others)
+    for (int at = 0; at <= 4; ++at) {
+        int waits = 0, parts = 0;
+        bool failed = false;
+        for (int i = 0; i < 2 && !failed; ++i)
+            for (int h = 0; h < 2; ++h) {
+                if (at & 1 ? kvb::leaves_alone<false>(failed, waits++ != at, true) : kvb::leaves_alone<true>(failed, waits++ != at, false)) break;
+                ++parts;
+            }
+        if (parts != at || failed != (at < 4)) { std::printf("alone, given up at %d: %d parts\n", at, parts); ++bad; }
     }
     std::printf(bad ? "walk: %d wrong\n" : "walk: ok\n", bad);
     return bad != 0;
