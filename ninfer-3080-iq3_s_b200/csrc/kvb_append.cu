@@ -97,7 +97,7 @@ __device__ __forceinline__ float rcp_newton(float x) {
 // range, which leaves a reciprocal square root, a few products and a reciprocal between the sums and the next factors.  Threads
 // 128..255 rate the states meanwhile: the extremes of a state's deviations while the rows of the next are updated, the verdict while
 // its columns are.  Two passes (in pairs of elements) and four barriers a round; bound by the chain pass, barrier, factors, barrier: 1.0
-// us a round.  Measured on B200, 1,024 tokens, 4 heads of 256 dims, 16 rounds: 36.3 -> 31.8 us a call (logf and expf per round, the
+// us a round.  Measured on B200, 1,024 tokens, 4 heads of 256 dims, 16 rounds, calls in a row: 36.3 -> 31.8 us (logf and expf per round, the
 // owners judging, single elements before).
 template <bool kValue>
 __device__ void sinkhorn(AppendSmem& sm, const float (&by_token)[kPer], const float (&by_dim)[kPer], int iters) {
@@ -303,8 +303,8 @@ __device__ void quantize_slice(AppendSmem& sm, float (&x)[kPer]) {
 // dims of a row: D / 32 lanes a row, 1024 / D rows a warp at a time; the strides up to 16 stay inside a lane, in pairs of dims, those of
 // 32 and more cross lanes, and rows are read and stored 16 bytes at a time.  A warp has up to 8 rows of the tile and reads them all before
 // rotating any: it waits for global memory once.  `keep(row, d, x)` takes dims d .. d + 7 of the slice.  Measured on B200 against a
-// warp a row with dims l + 32 r in lane l (five strides by shuffles, two bytes an access) and a division a code, 1,024 tokens, us a call:
-// 128 dims 9.9 -> 7.4, 256 dims 13.2 -> 9.8, with 16 rounds of balancing 31.8 -> 27.1; a prompt of 777 tokens 32.6 -> 29.2.
+// warp a row with dims l + 32 r in lane l (five strides by shuffles, two bytes an access) and a division a code, us a call, graph replay of 1,024
+// tokens: 128 dims 9.9 -> 7.0, 256 dims 12.5 -> 9.3; calls in a row: with 16 rounds of balancing 31.8 -> 27.1, a prompt of 777 tokens 32.6 -> 29.2.
 // The rows start at 16-byte boundaries.
 template <int D, bool kBf16, typename Keep>
 __device__ __forceinline__ void rotate_rows(const uint16_t* __restrict__ src, int64_t row_stride, int begin, int end, int slice, Keep keep) {

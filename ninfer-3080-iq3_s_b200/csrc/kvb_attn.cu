@@ -68,8 +68,8 @@ struct Shape {
 // The V codes of a page in a slot.  With two row blocks a warp as they lie in the page, one copy; else as 1 KB sub-blocks of 16 keys, each
 // shifted 16 bytes further: the eight rows of every transposing ldmatrix then fall in eight different bank groups.
 // The copies cost instructions, the conflicts shared-memory cycles, of which warps with one row block (more of them, or less work a
-// page) have fewer to spare.  Measured on B200, us a layer, shifted against plain: 2 rows at 131,072 tokens 35.9 35.1, balanced 2 / 4 / 5 rows at
-// 100,003 33.3 / 55.0 / 55.2 32.7 / 53.5 / 53.6; one row block, 378,944 tokens 45.1 46.3, a batch of 32 278 282.
+// page) have fewer to spare.  Measured on B200 in graph replay, us a layer, shifted against plain: 2 rows at 131,072 tokens 35.9 35.1, balanced 2 / 4 / 5 rows at
+// 100,003 33.3 / 55.0 / 55.2 32.7 / 53.5 / 53.6; one row block, 378,944 tokens 45.1 46.3, a batch of 32 (calls in a row) 278 282.
 template <int NB> struct VSlot {
     static constexpr int kShift = NB == 2 ? 0 : 16, kSubs = kShift ? 4 : 1, kSubBytes = Shape::kChunk / kSubs;
     static constexpr int kBytes = (Shape::kChunk + (kSubs - 1) * kShift + 127) / 128 * 128;
@@ -1432,8 +1432,8 @@ cudaError_t launch_attn(dim3 grid, cudaStream_t stream, const AttnParams& P) {
 // CTAs as the registers allow (four: 64 KB), and the SM's change between that and the attention kernel's 132 KB or more lies
 // between the two in a chain of layers.  Measured on B200 in graph replay, a decode call at 16,384 / 32,768 / 131,072 tokens:
 // 9.4 / 12.0 / 23.1 us left to the driver, 8.6 / 11.2 / 22.2 with 0, 9.7 / 12.3 / 23.3 with both kernels asking for all of it.
-// The least there is holds one CTA an SM: with more rows than SMs (a batch: 768) the driver's choice is the better one
-// (32 sequences, 315 us against 320).
+// The least there is holds one CTA an SM: with more rows than SMs (batches) the driver's choice is the better one (graph replay, 40 sequences
+// of 4,096 tokens 29.5 us a call against 35.5, 8 and 32 of 131,072 79.2 and 272 against 81.5 and 278).
 template <int S, bool kPush>
 cudaError_t launch_reduce(int rows, cudaStream_t stream, const float* ws_m, const float* ws_l, const float* ws_o, int parts, int T, int q_heads, int kv_heads,
                           int zblocks, int block_rows, int dtype, uint16_t* out, float* part_m, float* part_l, float* part_o, const PushTarget& push,
@@ -1459,8 +1459,8 @@ cudaError_t launch_attn_pair(dim3 grid, cudaStream_t stream, const AttnParams& P
 
 // Up to this many keys, and with up to this many clusters, the splits of a head and row block are a cluster (attn_short_kernel).  What that
 // saves is a launch, 3 us of the host: 16 layers launched one by one at 1,500 tokens take 206 us with the merge kernel and 164 as clusters.
-// On the device the merge kernel's route is the faster one where a head has one split, whose CTA would finish all rows alone, and at 256 dims:
-// a step that is captured, whose launches cost the host nothing, takes it there.  Graph replay, 24 / 4 heads, append and attention, us a layer,
+// On the device the merge kernel's route is the faster one where a head has one split whose CTA would finish two rows a warp alone, and at 256
+// dims (attention alone within 3 % either way): a step that is captured, whose launches cost the host nothing, takes it there.  Graph replay, 24 / 4 heads, append and attention, us a layer,
 // merge kernel / clusters: 60 tokens 1 / 4 rows 6.6 8.2 / 6.6 9.1, 200 tokens 8.5 8.2 / 8.6 8.2, 600 tokens 8.1 8.0 / 7.9 7.7, 1,500 tokens
 // 8.0 8.3 / 8.0 8.0, 2,500 tokens 8.2 8.5 / 8.5 8.3, 256 dims 60 tokens 9.2 10.1 / 9.5 10.5, 600 tokens 10.8 11.4 / 11.6 11.8, 1,500 tokens 11.0
 // 11.8 / 11.6 12.1.  Beyond the keys, eight CTAs have more than a round of pages (4,000 tokens 9.0 / 9.4, 6,000 9.9 / 12.3, 256 dims 2,000 14.7 /
@@ -1570,7 +1570,7 @@ int launch_attention(const kvb_layer* layer, const void* q, const int32_t* pos_d
     const bool few = kv_len_max <= short_keys(layer->head_dim) && layer->kv_heads * Z <= kShortClusters && out != nullptr && part_m == nullptr && push == nullptr;
     const int nsplit = few ? std::min(plan.nsplit, kShortSplits) : plan.nsplit;
     const bool clustered = few && stores_beside(span_of(out, out_bytes), span_of(q, out_bytes), span_of(pos_dev, T * sizeof(int32_t)), span_of(total_pos_dev, sizeof(int32_t))) &&
-                           as_clusters.held() && !((layer->head_dim != 128 || nsplit == 1) && is_captured(stream));
+                           as_clusters.held() && !((layer->head_dim != 128 || (nsplit == 1 && upper)) && is_captured(stream));
     const int parts = nsplit;
     AttnParams P;
     P.L = make_view(*layer);

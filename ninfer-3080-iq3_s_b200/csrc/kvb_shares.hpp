@@ -23,12 +23,17 @@ struct SplitBy {
 
 // Pages of split `split` of `n` pages, which its CTA walks W at a time.  The last split has the open tile as well, whose 16-key groups (a
 // warp or pair each) count as 3/4 of a page; it takes no page that would be a round more for those with a group.  Neither may cost the
-// other splits a round.  From eight rounds on (128 dims) the pages alone are shared, evenly: 4-row verify at 126,000 / 127,526 tokens 49.0 /
-// 51.1 -> 48.3 / 48.9, at 129,000 51.4 -> 52.0, decode at 378,944 45.7 -> 46.1; 256 dims 45,000 62.0 63.5, not there.  Measured on B200 in graph replay, append and attention, us a layer, equal shares (by 64-bit divisions, the first
-// position read behind the newest, the next kernel's start by every warp) against this: decode at 300 / 1,500 / 8,000 / 32,768 / 65,536 /
-// 378,944 tokens 8.6 / 9.1 / 10.2 / 12.6 / 17.8 / 49.4 8.1 7.8 8.7 12.6 17.6 49.1, 256 dims 1,500 / 4,000 / 30,011 14.2 / 13.2 / 23.1 11.5 11.6 21.0, verify of 4
-// rows at 1,500 / 8,000 / 131,072 9.2 / 11.6 / 52.0 7.8 10.7 52.2, of 5 rows of 256 dims at 20,000 35.9 35.3.  A CTA with the open tile was
-// some 2,000 cycles behind the others.
+// other splits a round.  A CTA with the open tile was some 2,000 cycles behind the others.
+// Measured on B200 in graph replay, append and attention, us a layer, equal shares (by 64-bit divisions, the first position read behind the
+// newest, the next kernel's start by every warp) / this:
+//   decode at 300, 1,500, 8,000, 32,768, 65,536, 378,944 tokens   8.6  9.1 10.2 12.6 17.8 49.4 / 8.1  7.8  8.7 12.6 17.6 49.1
+//   decode of 256 dims at 1,500, 4,000, 30,011                    14.2 13.2 23.1 / 11.5 11.6 21.0
+//   4 rows at 1,500, 8,000, 131,072                               9.2 11.6 52.0 / 7.8 10.7 52.2
+//   5 rows of 256 dims at 20,000                                  35.9 / 35.3
+// From eight rounds on (128 dims) the pages alone are shared, evenly; with the open tile counted / without:
+//   4 rows at 126,000, 127,526, 129,000                           49.0 51.1 51.4 / 48.3 48.9 52.0
+//   decode at 378,944                                             45.7 / 46.1
+//   256 dims at 45,000 (not there)                                62.0 / 63.5
 constexpr int kManyRounds = 8;
 template <int W, int kSlices> KVB_SHARES void split_pages(int n, int open_keys, int split, int nsplit, SplitBy by, int& begin, int& end) {
     const int groups = larger(open_keys + 15, 0) / 16, weighted = n + groups * 3 / 4;

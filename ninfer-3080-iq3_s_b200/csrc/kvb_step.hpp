@@ -16,11 +16,11 @@ inline Span span_of(const void* p, size_t bytes) {
 inline bool overlap(Span a, Span b) { return a.begin < b.end && b.begin < a.end; }
 
 // Whether the attention of a step starts its work beside the append (whose trigger lets every kernel behind it be launched), and only what
-// of it reads the rows written there waits for the append's end.  Measured on B200, a step of one layer: 32,768 tokens 13.8 -> 13.4 us,
-// 8-row verify of 100,003 67.6 -> 63.6, a prompt of 777 35.9 -> 33.0.  Not for several rows of a verify step at 256 dims, whose row blocks
-// (four, for 5 rows at 24 / 4 heads) share their pages through L2: 41.2 -> 42.5 with one warp a page.  (With two warps a page it gains
-// there too, 5 rows at 20,000 tokens 34.7 -> 33.9; the line has not been moved.)  Launched early but waiting, 2 / 4 / 5 / 8 rows at 20,000
-// tokens take 25.2 / 29.8 / 35.3 / 46.6 -> 24.6 / 29.5 / 34.7 / 46.2.
+// of it reads the rows written there waits for the append's end.  Measured on B200, a layer of a step launched one by one: 32,768 tokens 13.8 ->
+// 13.4 us, 8-row verify of 100,003 67.6 -> 63.6, a prompt of 777 35.9 -> 33.0.  Several rows of a verify step at 256 dims are launched early
+// and wait (2 / 4 / 5 / 8 rows at 20,000 tokens, graph replay, 25.2 / 29.8 / 35.3 / 46.6 -> 24.6 / 29.5 / 34.7 / 46.2).  The kernel with one warp a
+// page lost by starting beside the append (5 rows 41.2 -> 42.5); the one with two, which is there now, would gain (34.7 -> 33.9): the line is
+// older than it.
 inline bool append_starts_next(int head_dim, int tokens) { return head_dim == 128 || tokens == 1 || tokens > 8; }
 
 // An append right before the attention: whether the attention starts its work beside it, and what it reads.
